@@ -13,7 +13,9 @@ REPO = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 def _train(args, cwd):
     cmd = [sys.executable, "-m", "llm_kittens_b200.cli.train_gpt2cu", *args]
     r = subprocess.run(cmd, cwd=cwd, env=dict(os.environ, PYTHONPATH=REPO), capture_output=True, text=True, timeout=600)
-    assert r.returncode == 0, (r.stdout[-2000:], r.stderr[-2000:])
+    if r.returncode != 0:   # the error's text stands in front of the backtrace, which alone can be longer than the tail
+        err = r.stderr if len(r.stderr) <= 6000 else r.stderr[:4000] + "\n[...]\n" + r.stderr[-2000:]
+        pytest.fail(f"exit code {r.returncode}\n--- stdout\n{r.stdout[-2000:]}\n--- stderr\n{err}", pytrace=False)
     return r.stdout
 
 
