@@ -147,7 +147,6 @@ attn_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_c
     const int failed = threadIdx.x == 0 && status != nullptr ? *reinterpret_cast<volatile int*>(status) : 0;
     if (ptx::smem_u32(smem) & 1023u) {
         if (threadIdx.x == 0 && status != nullptr) atomicCAS(status, 0, LLMK_ST_BOUNDS);
-        grid_dep_wait();
         return;
     }
     uint8_t* sK = smem + C::OFF_K;
@@ -201,7 +200,6 @@ attn_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_c
         ptx::fence_barrier_init();
         ptx::fence_proxy_async_smem();
         skip = failed;
-        grid_dep_wait();
         if (!failed) {   // the first tiles are on their way while TMEM is allocated
             ptx::mbar_arrive_expect_tx(kv_full, 2 * C::TILE);
             load_tile<HS, BM>(sK, &tmQKV, kv_full, k_col, kv0, b);
@@ -217,8 +215,6 @@ attn_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_c
     __syncthreads();
     ptx::tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
-    grid_dep_launch();   // this block has its TMEM columns
-    grid_dep_wait();
     if (skip) {
         if (warp == 1) ptx::tmem_dealloc(tmem_base, C::TMEM);
         return;
@@ -454,7 +450,6 @@ attn_bwd_dkv2_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_con
     const int failed = threadIdx.x == 0 && status != nullptr ? *reinterpret_cast<volatile int*>(status) : 0;
     if (ptx::smem_u32(smem) & 1023u) {
         if (threadIdx.x == 0 && status != nullptr) atomicCAS(status, 0, LLMK_ST_BOUNDS);
-        grid_dep_wait();
         return;
     }
     uint8_t* sK = smem + OFF_K;
@@ -509,7 +504,6 @@ attn_bwd_dkv2_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_con
         ptx::fence_barrier_init();
         ptx::fence_proxy_async_smem();
         skip = failed;
-        grid_dep_wait();
         if (!failed) {
             ptx::mbar_arrive_expect_tx(kv_full, 2 * TILE);
             load_tile<HS, BM>(sK, &tmQKV, kv_full, k_col, kv0, b);
@@ -525,8 +519,6 @@ attn_bwd_dkv2_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_con
     __syncthreads();
     ptx::tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
-    grid_dep_launch();   // this block has its TMEM columns
-    grid_dep_wait();
     if (skip) {
         if (warp == 1) ptx::tmem_dealloc(tmem_base, 512);
         return;
@@ -725,7 +717,6 @@ attn_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_co
     const int failed = threadIdx.x == 0 && status != nullptr ? *reinterpret_cast<volatile int*>(status) : 0;
     if (ptx::smem_u32(smem) & 1023u) {
         if (threadIdx.x == 0 && status != nullptr) atomicCAS(status, 0, LLMK_ST_BOUNDS);
-        grid_dep_wait();
         return;
     }
     uint8_t* sQ = smem + C::OFF_Q;
@@ -774,7 +765,6 @@ attn_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_co
         ptx::fence_barrier_init();
         ptx::fence_proxy_async_smem();
         skip = failed;
-        grid_dep_wait();
         if (!failed) {
             ptx::mbar_arrive_expect_tx(q_full, 2 * C::TILE);
             load_tile<HS, BM>(sQ, &tmQKV, q_full, q_col, q0, b);
@@ -790,8 +780,6 @@ attn_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_co
     __syncthreads();
     ptx::tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
-    grid_dep_launch();   // this block has its TMEM columns
-    grid_dep_wait();
     if (skip) {
         if (warp == 1) ptx::tmem_dealloc(tmem_base, C::TMEM);
         return;
@@ -999,14 +987,17 @@ static int launch(const void* qkv, const void* dout, bf16* dqkv, const float* ls
         CUtensorMap tq_in64, tdo_in64;
         if ((rc = gemm::make_tmap_3d(&tq_in64, qkv, width, T, B, 64, 64))) return rc;
         if ((rc = gemm::make_tmap_3d(&tdo_in64, dout, cw, T, B, 64, 64))) return rc;
-        LLMK_CUDA_TRY(launch_chained(dkv2::attn_bwd_dkv2_kernel, dim3(dkv_order.tiles * dkv_order.heads), dim3(dkv2::THREADS2), dkv2::SMEM_BYTES, stream, tq, tq_in64, tdo_in64, tdqkv, lse, dvec,
-                                                                                                    T, NH, NKVH, scale, status, rope, dkv_order));
+        dkv2::attn_bwd_dkv2_kernel<<<dkv_order.tiles * dkv_order.heads, dkv2::THREADS2, dkv2::SMEM_BYTES, stream>>>(tq, tq_in64,
+            tdo_in64, tdqkv, lse, dvec, T, NH, NKVH, scale, status, rope, dkv_order);
+        LLMK_LAUNCH_CHECK();
     } else {
-        LLMK_CUDA_TRY(launch_chained(attn_bwd_dkv_tc_kernel<HS>, dim3(dkv_order.tiles * dkv_order.heads), dim3(THREADS), DkvCfg<HS>::SMEM_BYTES, stream, 
-            tkv, tq_in, tdo_in, tdkv, lse, dvec, T, NH, NKVH, scale, status, rope, Tkv, causal, dkv_order));
+        attn_bwd_dkv_tc_kernel<HS><<<dkv_order.tiles * dkv_order.heads, THREADS, DkvCfg<HS>::SMEM_BYTES, stream>>>(tkv, tq_in, tdo_in,
+            tdkv, lse, dvec, T, NH, NKVH, scale, status, rope, Tkv, causal, dkv_order);
+        LLMK_LAUNCH_CHECK();
     }
-    LLMK_CUDA_TRY(launch_chained(attn_bwd_dq_tc_kernel<HS>, dim3(dq_order.tiles * dq_order.heads), dim3(THREADS), DqCfg<HS>::SMEM_BYTES, stream, tq, tdo, tkv_in, tdqkv, lse, dvec, T, NH,
-                                                                                             NKVH, scale, status, rope, Tkv, causal, dq_order));
+    attn_bwd_dq_tc_kernel<HS><<<dq_order.tiles * dq_order.heads, THREADS, DqCfg<HS>::SMEM_BYTES, stream>>>(tq, tdo, tkv_in, tdqkv, lse,
+        dvec, T, NH, NKVH, scale, status, rope, Tkv, causal, dq_order);
+    LLMK_LAUNCH_CHECK();
     return LLMK_OK;
 }
 

@@ -152,7 +152,6 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_const
     const int failed = threadIdx.x == 0 && status != nullptr ? *reinterpret_cast<volatile int*>(status) : 0;
     if (ptx::smem_u32(smem) & 1023u) {  // swizzled tiles need a 1024-byte aligned window: refuse instead of corrupting
         if (threadIdx.x == 0 && status != nullptr) atomicCAS(status, 0, LLMK_ST_BOUNDS);
-        grid_dep_wait();
         return;
     }
     uint8_t* sQ = smem;
@@ -202,7 +201,6 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_const
         ptx::fence_barrier_init();
         ptx::fence_proxy_async_smem();
         skip = failed;
-        grid_dep_wait();
         if (!failed) {   // the first tiles are on their way while TMEM is allocated
             ptx::mbar_arrive_expect_tx(q_full, C::TILE_BYTES);
 #pragma unroll
@@ -218,8 +216,6 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_const
     __syncthreads();
     ptx::tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
-    grid_dep_launch();   // this block has its TMEM columns
-    grid_dep_wait();
     if (skip) {
         if (warp == 1) ptx::tmem_dealloc(tmem_base, C::TMEM_COLS);
         return;
@@ -401,8 +397,9 @@ static int launch(const CUtensorMap& tm, const CUtensorMap& tm_kv, bf16* out, fl
     }
     const float scale_log2 = 1.4426950408889634f / sqrtf((float)HS);
     const TileOrder order = make_tile_order(ceil_div(T, BQ), NH * B, 4l * Tkv * HS * NKVH / NH);
-    LLMK_CUDA_TRY(launch_chained(attn_fwd_tc_kernel<HS, ROUND>, dim3(order.tiles * order.heads), dim3(THREADS), Cfg<HS>::SMEM_BYTES, stream, tm, tm_kv, out, lse, T, Tkv, causal,
-                                                                                                       NH, NKVH, scale_log2, status, order));
+    attn_fwd_tc_kernel<HS, ROUND><<<order.tiles * order.heads, THREADS, Cfg<HS>::SMEM_BYTES, stream>>>(tm, tm_kv, out, lse, T, Tkv,
+        causal, NH, NKVH, scale_log2, status, order);
+    LLMK_LAUNCH_CHECK();
     return LLMK_OK;
 }
 
@@ -439,7 +436,6 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_con
     const int failed = threadIdx.x == 0 && status != nullptr ? *reinterpret_cast<volatile int*>(status) : 0;
     if (ptx::smem_u32(smem) & 1023u) {
         if (threadIdx.x == 0 && status != nullptr) atomicCAS(status, 0, LLMK_ST_BOUNDS);
-        grid_dep_wait();
         return;
     }
     uint8_t* sQ = smem;                                  // [2]
@@ -493,7 +489,6 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_con
         ptx::fence_barrier_init();
         ptx::fence_proxy_async_smem();
         skip = failed;
-        grid_dep_wait();
         if (!failed) {   // the first tiles are on their way while TMEM is allocated
             ptx::mbar_arrive_expect_tx(q_full, (n1 ? 2 : 1) * TILE_BYTES);
             ptx::tma_load_3d(sQ, &tmQKV, q_full, q_col, qb2 * 2 * BQ, b);
@@ -510,8 +505,6 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_con
     __syncthreads();
     ptx::tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
-    grid_dep_launch();   // this block has its TMEM columns
-    grid_dep_wait();
     if (skip) {
         if (warp == 1) ptx::tmem_dealloc(tmem_base, 512);
         return;
@@ -705,7 +698,9 @@ static int launch(const CUtensorMap& tm, const CUtensorMap& tm_out, float* lse, 
     }
     const float scale_log2 = 1.4426950408889634f / sqrtf((float)HS);
     const TileOrder order = make_tile_order(ceil_div(T, 2 * BQ), NH * B, 4l * T * HS * NKVH / NH);
-    LLMK_CUDA_TRY(launch_chained(attn_fwd_pair_kernel<ROUND>, dim3(order.tiles * order.heads), dim3(THREADS), SMEM_BYTES, stream, tm, tm_out, lse, T, NH, NKVH, scale_log2, status, order));
+    attn_fwd_pair_kernel<ROUND><<<order.tiles * order.heads, THREADS, SMEM_BYTES, stream>>>(tm, tm_out, lse, T, NH, NKVH, scale_log2,
+        status, order);
+    LLMK_LAUNCH_CHECK();
     return LLMK_OK;
 }
 }  // namespace pair

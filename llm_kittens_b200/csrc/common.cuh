@@ -98,34 +98,6 @@ static inline int sm_count_current_device() {
     return sms[dev];
 }
 
-// ---- programmatic dependent launch -------------------------------------------------------------
-// The kernels of a model step are a chain of launches of 3 to 300 us; between two of them the chip drains, launches and
-// runs the next kernel's prologue (barriers, TMEM, descriptors), 2 to 4 us. A kernel launched with this attribute may start
-// while its predecessor in the stream still runs, once all blocks of that one have called grid_dep_launch() or ended, and
-// blocks in grid_dep_wait() until the predecessor has completed and its writes are visible. So: every kernel launched this
-// way calls grid_dep_wait() in every thread before its first access to global memory (reads, writes, early returns
-// alike: a grid that ended without waiting would let its successor start beside its predecessor). A kernel that polls
-// flags of other kernels or ranks does not call grid_dep_launch(): its successor must not take the resources that those
-// need. A kernel with TMEM calls grid_dep_launch() only once its block has its columns: a successor that took them first
-// would wait for a block that waits for them. Without the attribute both calls do nothing.
-__device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-
-template <typename... KArgs, typename... Args>
-static inline cudaError_t launch_chained(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
-}
-
 // ---- 128-bit packed access -------------------------------------------------------------------
 struct alignas(16) bf16x8 {
     __nv_bfloat162 v[4];

@@ -13,8 +13,6 @@ namespace ew {
 constexpr int TPB = 256;
 
 __global__ void gelu_fwd_kernel(bf16* __restrict__ out, const bf16* __restrict__ inp, size_t n) {
-    grid_dep_launch();
-    grid_dep_wait();
     size_t i = ((size_t)blockIdx.x * TPB + threadIdx.x) * 8;
     if (i >= n) return;
     float f[8];
@@ -39,8 +37,6 @@ __device__ __forceinline__ float sigmoidf_(float x) { return 1.0f / (1.0f + __ex
 
 // out = silu(gate) * up
 __global__ void swiglu_fwd_kernel(bf16* __restrict__ out, const bf16* __restrict__ gate, const bf16* __restrict__ up, size_t n) {
-    grid_dep_launch();
-    grid_dep_wait();
     size_t i = ((size_t)blockIdx.x * TPB + threadIdx.x) * 8;
     if (i >= n) return;
     float g[8], u[8];
@@ -53,8 +49,6 @@ __global__ void swiglu_fwd_kernel(bf16* __restrict__ out, const bf16* __restrict
 // dgate = dout * up * silu'(gate) ; dup = dout * silu(gate)
 __global__ void swiglu_bwd_kernel(bf16* __restrict__ dgate, bf16* __restrict__ dup, const bf16* __restrict__ dout,
                                   const bf16* __restrict__ gate, const bf16* __restrict__ up, size_t n) {
-    grid_dep_launch();
-    grid_dep_wait();
     size_t i = ((size_t)blockIdx.x * TPB + threadIdx.x) * 8;
     if (i >= n) return;
     float g[8], u[8], d[8], dg[8], du[8];
@@ -414,7 +408,8 @@ using namespace llmk::ew;
 
 LLMK_API int llmk_gelu_fwd(void* out, const void* inp, long n, void* stream) {
     if (n % 8) return LLMK_ERR_SHAPE;
-    LLMK_CUDA_TRY(launch_chained(gelu_fwd_kernel, dim3(VEC_GRID(n)), dim3(TPB), 0, (cudaStream_t)stream, (bf16*)out, (const bf16*)inp, (size_t)n));
+    gelu_fwd_kernel<<<VEC_GRID(n), TPB, 0, (cudaStream_t)stream>>>((bf16*)out, (const bf16*)inp, (size_t)n);
+    LLMK_LAUNCH_CHECK();
     return LLMK_OK;
 }
 LLMK_API int llmk_gelu_bwd_inplace(void* dinout, const void* inp, long n, void* stream) {
@@ -425,13 +420,15 @@ LLMK_API int llmk_gelu_bwd_inplace(void* dinout, const void* inp, long n, void* 
 }
 LLMK_API int llmk_swiglu_fwd(void* out, const void* gate, const void* up, long n, void* stream) {
     if (n % 8) return LLMK_ERR_SHAPE;
-    LLMK_CUDA_TRY(launch_chained(swiglu_fwd_kernel, dim3(VEC_GRID(n)), dim3(TPB), 0, (cudaStream_t)stream, (bf16*)out, (const bf16*)gate, (const bf16*)up, (size_t)n));
+    swiglu_fwd_kernel<<<VEC_GRID(n), TPB, 0, (cudaStream_t)stream>>>((bf16*)out, (const bf16*)gate, (const bf16*)up, (size_t)n);
+    LLMK_LAUNCH_CHECK();
     return LLMK_OK;
 }
 LLMK_API int llmk_swiglu_bwd(void* dgate, void* dup, const void* dout, const void* gate, const void* up, long n, void* stream) {
     if (n % 8) return LLMK_ERR_SHAPE;
-    LLMK_CUDA_TRY(launch_chained(swiglu_bwd_kernel, dim3(VEC_GRID(n)), dim3(TPB), 0, (cudaStream_t)stream, (bf16*)dgate, (bf16*)dup, (const bf16*)dout,
-                                                                     (const bf16*)gate, (const bf16*)up, (size_t)n));
+    swiglu_bwd_kernel<<<VEC_GRID(n), TPB, 0, (cudaStream_t)stream>>>((bf16*)dgate, (bf16*)dup, (const bf16*)dout, (const bf16*)gate,
+        (const bf16*)up, (size_t)n);
+    LLMK_LAUNCH_CHECK();
     return LLMK_OK;
 }
 LLMK_API int llmk_swiglu_fused_fwd(void* out, const void* upgate, int rows, int H, void* stream) {

@@ -119,8 +119,6 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     ptx::tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
     const bool skip = *skip_word != 0;
-    grid_dep_launch();   // this block has its TMEM columns
-    grid_dep_wait();     // (the status word was read early: a failure seen late only costs the work of one more kernel)
 
     // Producer and issuer are one thread each: a warp that waits and then branches to one lane per k-block spends more
     // cycles on that than the tensor core on a 128 x 64 x 64 product (0.28 us per k-block that way, 0.14 this way).
@@ -393,15 +391,13 @@ static int launch(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensor
     cfg.blockDim = dim3(THREADS);
     cfg.dynamicSmemBytes = smem_bytes(G::STAGE_BYTES, G::ACC_BYTES, p.stages, tmem_cols(BN, (EPI & EPI_DBIAS) != 0));
     cfg.stream = stream;
-    cudaLaunchAttribute attr[2];
+    cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = p.S;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
-    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 2;
+    cfg.numAttrs = 1;
     LLMK_CUDA_TRY(cudaLaunchKernelEx(&cfg, gemm_small_kernel<MODE, EPI, BN>, tmA, tmB, tmB2, p));
     return LLMK_OK;
 }

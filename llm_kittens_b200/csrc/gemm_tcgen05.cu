@@ -117,7 +117,6 @@ struct Params {
     int M, N, K;
     int tiles_m, tiles_n, splits, kb_total, kb_per_split;   // tiles_m counts 256-row tiles when `pair`
     int pair;
-    int chained;               // launched as a dependent of its predecessor, and lets its successor start early
     // Grouped (batched) problems: `group_m` rows of C per group (0 = one problem). Group g of a tile is m0 / group_m.
     // NT: B is [G*N, K] and bias [G*N]; NN: B is [G*K, N]; TN: A is [G*K, M_g], B is [G*K, N], C is [G*M_g, N].
     int group_m;
@@ -311,8 +310,6 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
     ptx::tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
     const bool skip = (PAIR ? ptx::ld_shared_cluster_u32(&skip_word, 0) : (uint32_t)skip_word) != 0;
-    if (p.chained) grid_dep_launch();   // both blocks of the pair have their TMEM columns
-    grid_dep_wait();
 
     if (skip) {
         // nothing to do: fall through to the teardown
@@ -894,8 +891,6 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
 __global__ void splitk_reduce_kernel(bf16* __restrict__ out, const float* __restrict__ partial, size_t n, int splits,
                                      int accumulate, bf16* __restrict__ dbias, const float* __restrict__ db_partial, int M,
                                      int db_rows) {
-    grid_dep_launch();
-    grid_dep_wait();
     size_t i = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * 8;
     if (i >= n) return;
     if (dbias != nullptr && i < (size_t)M) {
@@ -1003,15 +998,13 @@ static int launch(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensor
         cfg.blockDim = dim3(Cfg<EPI, true>::NTHREADS);
         cfg.dynamicSmemBytes = SMEM_BYTES;
         cfg.stream = stream;
-        cudaLaunchAttribute attr[2];
+        cudaLaunchAttribute attr[1];
         attr[0].id = cudaLaunchAttributeClusterDimension;
         attr[0].val.clusterDim.x = 2;
         attr[0].val.clusterDim.y = 1;
         attr[0].val.clusterDim.z = 1;
         cfg.attrs = attr;
-        attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[1].val.programmaticStreamSerializationAllowed = 1;
-        cfg.numAttrs = p.chained ? 2 : 1;
+        cfg.numAttrs = 1;
         LLMK_CUDA_TRY(cudaLaunchKernelEx(&cfg, gemm_kernel<MODE, EPI, true>, tmA, tmB, tmC, tmX, xm, p));
         return LLMK_OK;
     }
@@ -1248,7 +1241,6 @@ static int gemm_impl(int mode, int epi, const void* A, const void* B, void* C, v
     p.M = M; p.N = N; p.K = K;
     const int pair_clusters = query_pair_clusters();
     p.pair = pair_clusters > 0 ? 1 : 0;
-    p.chained = max_ctas <= 0 && ready.b_ready == nullptr && ready.a_ready == nullptr && ready.b_ready2 == nullptr && !(epi & EPI_SCATTER);
     p.group_m = 0;
     if (groups > 1) {
         // a tile must not straddle two groups, and a k-block must not run into the next group's rows
@@ -1394,9 +1386,9 @@ static int gemm_impl(int mode, int epi, const void* A, const void* B, void* C, v
     if (rc) return rc;
     if (epi & EPI_PARTIAL) {
         const size_t n = (size_t)M * N;
-        LLMK_CUDA_TRY(launch_chained(splitk_reduce_kernel, dim3(ceil_div((long)(n / 8), 256)), dim3(256), 0, stream, static_cast<bf16*>(C), p.partial, n, p.splits,
-                                                                            split_accumulate ? 1 : 0, with_dbias ? p.dbias : nullptr,
-                                                                            p.db_partial, M, p.splits * p.tiles_n));
+        splitk_reduce_kernel<<<ceil_div((long)(n / 8), 256), 256, 0, stream>>>(static_cast<bf16*>(C), p.partial, n, p.splits,
+            split_accumulate ? 1 : 0, with_dbias ? p.dbias : nullptr, p.db_partial, M, p.splits * p.tiles_n);
+        LLMK_LAUNCH_CHECK();
     }
     return LLMK_OK;
 }

@@ -21,8 +21,6 @@ namespace norm {
 constexpr int FIN_LANES = 32;
 __global__ void __launch_bounds__(32 * FIN_LANES)
 norm_bwd_finish_kernel(bf16* __restrict__ dweight, bf16* __restrict__ dbias, const float* __restrict__ scratch, int nblocks, int C) {
-    grid_dep_launch();
-    grid_dep_wait();
     // block = (32 columns, FIN_LANES partial-row lanes); lane y sums partials y, y + FIN_LANES, ...; then the lanes are
     // added in fixed order, so the result does not depend on scheduling
     __shared__ float shw[FIN_LANES][33], shb[FIN_LANES][33];
@@ -74,8 +72,6 @@ __global__ void __launch_bounds__(REG_WARPS * 32)
 norm_fwd_reg_kernel(bf16* __restrict__ normed, float* __restrict__ mean_out, float* __restrict__ rstd_out,
                     bf16* residual_out, const bf16* inp1, const bf16* __restrict__ inp2, const bf16* __restrict__ weight,
                     const bf16* __restrict__ bias, int N, int C_, float eps) {
-    grid_dep_launch();
-    grid_dep_wait();
     const int C = RAGGED ? C_ : NVEC * 256;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const float inv_c = 1.0f / (float)C;
@@ -162,8 +158,6 @@ __global__ void __launch_bounds__(256, NV <= 2 ? 4 : (NV <= 4 ? 2 : 1))
 norm_fwd_wide_kernel(bf16* __restrict__ normed, float* __restrict__ mean_out, float* __restrict__ rstd_out,
                      bf16* residual_out, const bf16* inp1, const bf16* __restrict__ inp2, const bf16* __restrict__ weight,
                      const bf16* __restrict__ bias, int N, int C, float eps) {
-    grid_dep_launch();
-    grid_dep_wait();
     __shared__ float red[2][2][8];   // [parity][sum | squares][warp]
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const float inv_c = 1.0f / (float)C;
@@ -283,8 +277,6 @@ __global__ void __launch_bounds__(BulkCfg<NVEC>::WARPS * 32, 1)
 norm_bwd_bulk_kernel(bf16* __restrict__ dinp, float* __restrict__ scratch, const bf16* __restrict__ dout,
                      const bf16* __restrict__ inp, const bf16* __restrict__ weight, const float* __restrict__ mean,
                      const float* __restrict__ rstd, int N, int accumulate_dinp, int* status) {
-    grid_dep_launch();
-    grid_dep_wait();
     using B = BulkCfg<NVEC>;
     constexpr int C = B::C, ROW = B::ROW, STAGES = B::STAGES, WARPS = B::WARPS;
     constexpr int PLANES = RMS ? 1 : 2;
@@ -413,8 +405,6 @@ __global__ void __launch_bounds__(256, NV <= 2 ? 2 : 1)
 norm_bwd_wide_kernel(bf16* __restrict__ dinp, float* __restrict__ scratch, const bf16* __restrict__ dout,
                      const bf16* __restrict__ inp, const bf16* __restrict__ weight, const float* __restrict__ mean,
                      const float* __restrict__ rstd, int N, int C_, int accumulate_dinp) {
-    grid_dep_launch();
-    grid_dep_wait();
     const int C = RAGGED ? C_ : NV * 2048;
     __shared__ float red[2][2][8];   // [parity][s1 | s2][warp]
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -539,8 +529,8 @@ static int launch_fwd(bf16* normed, float* mean, float* rstd, bf16* residual, co
         cap *= num_sms();                                                                                                   \
         int grid = ceil_div(N, ROWS_PER_BLOCK);                                                                             \
         if (grid > cap) grid = cap;                                                                                         \
-        LLMK_CUDA_TRY(launch_chained(KERNEL, dim3(grid), dim3(REG_WARPS * 32), 0, stream, normed, mean, rstd, residual, inp1, \
-                                     inp2, weight, bias, N, C, eps));                                                       \
+        KERNEL<<<grid, REG_WARPS * 32, 0, stream>>>(normed, mean, rstd, residual, inp1, inp2, weight, bias, N, C, eps);     \
+        LLMK_LAUNCH_CHECK();                                                                                                \
         return LLMK_OK;                                                                                                     \
     }
 #define LLMK_NORM_FWD_CASE(NV)                                                                                              \
@@ -614,9 +604,11 @@ static int launch_bwd_bulk(bf16* dinp, bf16* dweight, bf16* dbias, float* scratc
     int grid = num_sms();
     const int need = ceil_div(N, B::WARPS);
     if (grid > need) grid = need;
-    LLMK_CUDA_TRY(launch_chained(norm_bwd_bulk_kernel<RMS, NVEC>, dim3(grid), dim3(B::WARPS * 32), B::SMEM, stream, dinp, scratch, dout, inp, weight, mean, rstd, N,
-                                                                             accumulate_dinp, current_status_word()));
-    LLMK_CUDA_TRY(launch_chained(norm_bwd_finish_kernel, dim3(ceil_div(C, 32)), dim3(32, FIN_LANES), 0, stream, dweight, dbias, scratch, grid, C));
+    norm_bwd_bulk_kernel<RMS, NVEC><<<grid, B::WARPS * 32, B::SMEM, stream>>>(dinp, scratch, dout, inp, weight, mean, rstd, N,
+        accumulate_dinp, current_status_word());
+    LLMK_LAUNCH_CHECK();
+    norm_bwd_finish_kernel<<<ceil_div(C, 32), dim3(32, FIN_LANES), 0, stream>>>(dweight, dbias, scratch, grid, C);
+    LLMK_LAUNCH_CHECK();
     return LLMK_OK;
 }
 template <bool RMS, int NV, bool RAGGED = false>
@@ -625,9 +617,10 @@ static int launch_bwd_wide(bf16* dinp, bf16* dweight, bf16* dbias, float* scratc
                            cudaStream_t stream) {
     int grid = num_sms() * (NV <= 2 ? 2 : 1);
     if (grid > N) grid = N;
-    LLMK_CUDA_TRY(launch_chained(norm_bwd_wide_kernel<RMS, NV, RAGGED>, dim3(grid), dim3(256), 0, stream, dinp, scratch, dout, inp, weight, mean, rstd, N, C,
-                                                                  accumulate_dinp));
-    LLMK_CUDA_TRY(launch_chained(norm_bwd_finish_kernel, dim3(ceil_div(C, 32)), dim3(32, FIN_LANES), 0, stream, dweight, dbias, scratch, grid, C));
+    norm_bwd_wide_kernel<RMS, NV, RAGGED><<<grid, 256, 0, stream>>>(dinp, scratch, dout, inp, weight, mean, rstd, N, C, accumulate_dinp);
+    LLMK_LAUNCH_CHECK();
+    norm_bwd_finish_kernel<<<ceil_div(C, 32), dim3(32, FIN_LANES), 0, stream>>>(dweight, dbias, scratch, grid, C);
+    LLMK_LAUNCH_CHECK();
     return LLMK_OK;
 }
 }  // namespace norm

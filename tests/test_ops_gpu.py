@@ -152,7 +152,7 @@ def test_zeroing_ends_at_the_tensor(n):
 
 
 @pytest.mark.parametrize("rows,C,NH", [(64, 768, 12), (320, 2048, 32), (4096, 768, 12)])
-def test_kernels_launched_ahead_of_their_predecessor_keep_the_stream_order(rows, C, NH):
+def test_chains_of_kernels_keep_the_stream_order(rows, C, NH):
     """Chains in which every launch reads what the one before wrote and overwrites what the one before read, with work of
     another stream forked and joined in between: the same bits with a synchronisation after every call, without any, and
     replayed from a CUDA graph."""

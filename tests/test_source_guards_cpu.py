@@ -68,6 +68,15 @@ def test_device_code_has_no_trap_and_every_polling_loop_has_a_time_limit():
             assert re.search(r"globaltimer_ns|now_ns\(\)|clock64|break|return", window), f"{path}: endless loop near {window[:80]!r}"
 
 
+def test_every_kernel_starts_after_its_predecessor_has_ended():
+    """Kernels read what earlier kernels of the stream wrote through ``const __restrict__`` pointers, i.e. with loads that
+    assume the data to be constant for the kernel's lifetime: no launch asks for a start beside its predecessor."""
+    for path in _files(CSRC, (".cu", ".cuh", ".h")):
+        code = _strip_comments(_read(path))
+        assert not re.search(r"griddepcontrol|[Pp]rogrammaticStreamSerialization|LaunchAttributeProgrammatic|GridDependencySynchronize|"
+                             r"TriggerProgrammaticLaunch", code), path
+
+
 def test_every_profiler_command_line_leaves_the_clocks_alone():
     hits = 0
     for path in list(_files(PKG, (".py",))) + list(_files(os.path.join(REPO, "profiles"), (".md",))) + [os.path.join(REPO, "README.md")]:
