@@ -426,7 +426,8 @@ class Transformer:
                 def attention_side_work():
                     prep[0] = attn_ops.attention_bwd_prep(d_btc, a["atty"][k], a["dvec"], B, T, cfg.num_heads, cfg.head_size)
 
-                self._fork(attention_side_work)
+                if attn_ops.fused_rope_available(T):   # (the warp-level kernels compute D themselves: nothing to fork for)
+                    self._fork(attention_side_work)
             self._dweight(dres, a["atty"][k], g["attprojw"][l], None if self.is_llama else g["attprojb"][l])
             self._join()   # D is needed now, and the next kernel overwrites the buffer that the MLP's column sum read
             dqkv = a["d_wide"].view(-1)[: BT * QW].view(BT, QW)

@@ -1,0 +1,54 @@
+"""The launch schedule of the models without a GPU: the native library is replaced by a recorder, so that the order of the
+calls, and what each is handed, can be looked at."""
+import pytest
+import torch
+
+from llm_kittens_b200.models.config import ModelConfig
+from llm_kittens_b200.models.transformer import Transformer
+from llm_kittens_b200.ops import _native, gemm
+
+
+class _Lib:
+    """Every entry point exists and returns 0."""
+
+    def __getattr__(self, name):
+        return lambda *a: 0
+
+
+@pytest.fixture
+def calls(monkeypatch):
+    """List of (entry point, arguments) of the native calls made so far."""
+    out = []
+    monkeypatch.setattr(_native, "lib", lambda: _Lib())
+    monkeypatch.setattr(_native, "call", lambda name, *a: out.append((name, a)))
+    monkeypatch.setattr(_native, "require_cuda_tensor", lambda *a, **k: None)
+    monkeypatch.setattr(_native, "status_word", lambda: None)
+    monkeypatch.setattr(_native, "scratch_buffer", lambda pool, nbytes, min_bytes, name: torch.empty(16, dtype=torch.uint8))
+    monkeypatch.setattr(gemm, "tile_rows", lambda: 256)
+    return out
+
+
+def _model(head_size, recompute=0):
+    cfg = ModelConfig(family="gpt2", max_seq_len=512, vocab_size=250, padded_vocab_size=256, num_layers=2, num_heads=2,
+                      num_kv_heads=2, channels=2 * head_size, hidden_dim=8 * head_size)
+    return Transformer(cfg, device="cpu", recompute=recompute)
+
+
+@pytest.mark.parametrize("head_size,T,forks", [(64, 64, 0), (64, 192, 0), (64, 128, 0), (128, 64, 0), (128, 192, 0), (128, 128, 2),
+                                               (128, 320, 2)])
+def test_the_side_stream_is_used_only_for_work(calls, monkeypatch, head_size, T, forks):
+    """The backward pass forks to the side stream only where something is launched there: the pre-pass of the attention
+    backward, once per layer, when the tcgen05 kernels run and the pre-pass is not in the epilogue of a GEMM (heads of 64)."""
+    model = _model(head_size)
+    work = []
+
+    def fork(fn):
+        before = len(calls)
+        fn()
+        work.append([name for name, _ in calls[before:]])
+
+    monkeypatch.setattr(model, "_fork", fork)
+    tokens = torch.zeros(1, T, dtype=torch.int32)
+    model.forward(tokens, tokens)
+    model.backward()
+    assert work == [["llmk_attention_bwd_prep"]] * forks
