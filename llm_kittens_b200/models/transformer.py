@@ -42,6 +42,29 @@ _LAYERED_ACTS = {"block_in", "ln1", "ln1_rstd", "ln1_mean", "ln2", "ln2_rstd", "
                  "gate", "act", "fch"}
 
 
+class _Stacked(dict):
+    """Named tensors, many of them stacked over the layers, with a place for their per-layer views (``layers``), which is
+    emptied when an entry is replaced, added or removed."""
+
+    layers: dict | None = None
+
+    @classmethod
+    def of(cls, d: dict) -> "_Stacked":
+        return d if isinstance(d, cls) else cls(d)
+
+
+def _dropping_views(method):
+    def changed(self, *args, **kwargs):
+        self.layers = None
+        return method(self, *args, **kwargs)
+
+    return changed
+
+
+for _name in ("__setitem__", "__delitem__", "__ior__", "update", "setdefault", "pop", "popitem", "clear"):
+    setattr(_Stacked, _name, _dropping_views(getattr(dict, _name)))
+
+
 class Transformer:
     def __init__(self, config: ModelConfig, device: str | torch.device = "cuda", recompute: int = 1,
                  rope_interleaved: bool = True):
@@ -77,14 +100,14 @@ class Transformer:
     # ------------------------------------------------------------------ per-layer views
     # Indexing a stacked tensor makes a tensor object, 2 us on the host; the dozen that a block's forward needs were a
     # third of a launch-bound forward (124M sampler at T = 64: 1.10 ms, 0.69 without them). They are made at the first
-    # forward after the stacked tensors were set, by whoever set them.
+    # forward after the stacked tensors, or one of them, were set, by whoever set them.
     @property
     def p(self) -> dict:
         return self._p
 
     @p.setter
     def p(self, views: dict) -> None:
-        self._p, self._p_layers = views, None
+        self._p = _Stacked.of(views)
 
     @property
     def acts(self) -> dict | None:
@@ -92,17 +115,17 @@ class Transformer:
 
     @acts.setter
     def acts(self, a: dict | None) -> None:
-        self._acts, self._acts_layers = a, None
+        self._acts = None if a is None else _Stacked.of(a)
 
     def _layers(self) -> tuple[dict, dict]:
         """(activations, parameters) with every stacked tensor as a tuple of its layers."""
-        if self._acts_layers is None:
-            self._acts_layers = {n: (v.unbind(0) if n in _LAYERED_ACTS and isinstance(v, torch.Tensor) else v)
-                                 for n, v in self._acts.items()}
-        if self._p_layers is None:
+        a, p = self._acts, self._p
+        if a.layers is None:
+            a.layers = {n: (v.unbind(0) if n in _LAYERED_ACTS and isinstance(v, torch.Tensor) else v) for n, v in a.items()}
+        if p.layers is None:
             layered = {s.spec.name for s in self.layout.slots if s.spec.layered}
-            self._p_layers = {n: (v.unbind(0) if n in layered and isinstance(v, torch.Tensor) else v) for n, v in self._p.items()}
-        return self._acts_layers, self._p_layers
+            p.layers = {n: (v.unbind(0) if n in layered and isinstance(v, torch.Tensor) else v) for n, v in p.items()}
+        return a.layers, p.layers
 
     # ------------------------------------------------------------------ parameters
     def init_weights(self, seed: int = 42) -> None:

@@ -52,3 +52,28 @@ def test_the_side_stream_is_used_only_for_work(calls, monkeypatch, head_size, T,
     model.forward(tokens, tokens)
     model.backward()
     assert work == [["llmk_attention_bwd_prep"]] * forks
+
+
+def test_a_replaced_tensor_is_used_by_every_layer_of_the_next_forward(calls):
+    """Per-layer views are made once; replacing one stacked tensor, in whatever way, makes them again."""
+    model = _model(64)
+    tokens = torch.zeros(1, 64, dtype=torch.int32)
+    model.forward(tokens)
+
+    def pointers(entry, position):
+        calls.clear()
+        model.forward(tokens)
+        return [a[position].data_ptr() for name, a in calls if name == entry]
+
+    for put in (lambda t: model.p.__setitem__("qkvw", t), lambda t: model.p.update(qkvw=t), lambda t: setattr(model, "p", {**model.p, "qkvw": t})):
+        mine = torch.randn_like(model.p["qkvw"])
+        put(mine)
+        seen = pointers("llmk_gemm", 3)
+        assert all(mine[layer].data_ptr() in seen for layer in range(2))
+        assert model.p["qkvw"] is mine
+    mine = torch.empty_like(model.acts["lse"])
+    model.acts["lse"] = mine
+    assert pointers("llmk_attention_fwd", 1) == [mine[0].data_ptr(), mine[1].data_ptr()]
+    acts = model.acts
+    model.acts = acts                       # handing the same table back keeps it (and what identifies it)
+    assert model.acts is acts
