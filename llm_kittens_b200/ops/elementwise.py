@@ -139,9 +139,10 @@ def encoder_bwd(dwte, dwpe, dout, tokens):
 
 
 def zero_(t: torch.Tensor) -> torch.Tensor:
-    """Zeroes a contiguous CUDA tensor in place at the write rate of the memory (gradient buffers of several GB)."""
+    """Zeroes a contiguous CUDA tensor in place at the write rate of the memory (gradient buffers of several GB). A tensor
+    of another device than the current one, whose stream a kernel would be launched on, goes to PyTorch."""
     N.require_cuda_tensor(t, None, "t")
-    if t.data_ptr() % 16:
+    if t.data_ptr() % 16 or t.device.index != torch._C._cuda_getDevice():
         return t.zero_()
     N.call("llmk_zero", t, t.numel() * t.element_size())
     return t

@@ -5,7 +5,7 @@ import torch
 
 from llm_kittens_b200.models.config import ModelConfig
 from llm_kittens_b200.models.transformer import Transformer
-from llm_kittens_b200.ops import _native, gemm
+from llm_kittens_b200.ops import _native, elementwise, gemm
 
 
 class _Lib:
@@ -77,3 +77,30 @@ def test_a_replaced_tensor_is_used_by_every_layer_of_the_next_forward(calls):
     acts = model.acts
     model.acts = acts                       # handing the same table back keeps it (and what identifies it)
     assert model.acts is acts
+
+
+@pytest.mark.parametrize("index,address,native", [(0, 4096, True), (1, 4096, False), (0, 4098, False)])
+def test_zeroing_a_tensor_of_another_device_is_left_to_pytorch(calls, monkeypatch, index, address, native):
+    """Kernels are launched on the current device's stream: a tensor of another device would be written there without order
+    to the work of its own device."""
+    class Tensor:
+        device = torch.device("cuda", index)
+        zeroed = False
+
+        def data_ptr(self):
+            return address
+
+        def numel(self):
+            return 8
+
+        def element_size(self):
+            return 2
+
+        def zero_(self):
+            self.zeroed = True
+            return self
+
+    monkeypatch.setattr(torch._C, "_cuda_getDevice", lambda: 0)
+    t = Tensor()
+    assert elementwise.zero_(t) is t
+    assert (t.zeroed, [name for name, _ in calls]) == ((False, ["llmk_zero"]) if native else (True, []))
