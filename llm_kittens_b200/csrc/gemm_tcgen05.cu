@@ -1068,8 +1068,17 @@ using namespace llmk::gemm;
 // How many CTA pairs the pair (cta_group::2) kernel keeps resident; 0 when that path is off (LLMK_GEMM_PAIR=0).
 LLMK_API int llmk_gemm_pair_clusters() { return query_pair_clusters(); }
 
-// Bytes of fp32 workspace that llmk_gemm needs for (mode, M, N, K) with the split count it will pick.
-LLMK_API long llmk_gemm_workspace_bytes(int mode, int M, int N, int K, int num_sms);
+// Bytes of fp32 workspace that llmk_gemm needs for (mode, M, N, K) with the split count it will pick on the current device
+// under the same `max_ctas` (0 = no limit).
+LLMK_API long llmk_gemm_workspace_bytes(int mode, int M, int N, int K, int max_ctas);
+
+// CTAs (pair kernel: CTA pairs) that work on a product under a limit of `max_ctas` CTAs (0 = none).
+static int gemm_workers(int max_ctas, int pair_clusters, int sms) {
+    const int workers = pair_clusters > 0 ? pair_clusters : sms;
+    if (max_ctas <= 0) return workers;
+    const int cap = pair_clusters > 0 ? (max_ctas / 2 > 0 ? max_ctas / 2 : 1) : max_ctas;
+    return cap < workers ? cap : workers;
+}
 
 static int pick_splits(int mode, int M, int N, int K, int num_sms, int tile_rows = BM, double* estimate = nullptr) {
     if (mode != MODE_TN) return 1;
@@ -1098,11 +1107,11 @@ static int pick_splits(int mode, int M, int N, int K, int num_sms, int tile_rows
     return best;
 }
 
-long llmk_gemm_workspace_bytes(int mode, int M, int N, int K, int num_sms) {
-    // the larger of what the single-CTA and the pair kernel would pick (the choice is made at launch time)
-    int s = pick_splits(mode, M, N, K, num_sms > 0 ? num_sms : 148);
-    const int s2 = pick_splits(mode, M, N, K, (num_sms > 0 ? num_sms : 148) / 2, 2 * BM);
-    if (s2 > s) s = s2;
+long llmk_gemm_workspace_bytes(int mode, int M, int N, int K, int max_ctas) {
+    // the launch's own choice: the split count does not grow or fall steadily with the number of workers
+    const int pair_clusters = query_pair_clusters();
+    const int sms = sm_count_current_device();
+    const int s = pick_splits(mode, M, N, K, gemm_workers(max_ctas, pair_clusters, sms > 0 ? sms : 148), pair_clusters > 0 ? 2 * BM : BM);
     return s > 1 ? (long)s * M * N * 4 + (long)s * ceil_div(N, BN) * M * 4 /* bias-gradient partials */ : 0;
 }
 
@@ -1311,9 +1320,7 @@ static int gemm_impl(int mode, int epi, const void* A, const void* B, void* C, v
     bool split_accumulate = false;
     const int with_dbias = epi & EPI_DBIAS;
     if (mode == MODE_TN && ((epi & ~EPI_DBIAS) == 0 || (epi & ~EPI_DBIAS) == EPI_ADD)) {
-        const int workers = p.pair ? pair_clusters : g_num_sms;
-        const int cap = max_ctas > 0 ? (p.pair ? (max_ctas / 2 > 0 ? max_ctas / 2 : 1) : max_ctas) : workers;
-        int s = pick_splits(mode, M, N, K, cap < workers ? cap : workers, p.pair ? 2 * BM : BM);
+        const int s = pick_splits(mode, M, N, K, gemm_workers(max_ctas, pair_clusters, g_num_sms), p.pair ? 2 * BM : BM);
         if (s > 1) {
             if (workspace == nullptr || workspace_bytes < (long)s * M * N * 4 + (with_dbias ? (long)s * p.tiles_n * M * 4 : 0)) return LLMK_ERR_WORKSPACE;
             p.splits = s;

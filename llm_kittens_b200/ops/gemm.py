@@ -80,7 +80,7 @@ def _gemm(mode, epi, a, b, c, c2, bias, aux, M, Nn, K, groups=1, a_ready=None):
     ws = None
     ws_bytes = 0
     if mode == MODE_TN:
-        ws_bytes = int(N.lib().llmk_gemm_workspace_bytes(mode, M * groups, Nn, K, 0))
+        ws_bytes = int(N.lib().llmk_gemm_workspace_bytes(mode, M * groups, Nn, K, _MAX_CTAS))
         if ws_bytes:
             ws = workspace(ws_bytes)
             ws_bytes = ws.numel()
@@ -265,7 +265,7 @@ def gemm_tn(a, b, out=None, accumulate=False, groups=1, dbias=None):
     if fused:
         for t, nm in ((a, "A"), (b, "B"), (out2, "C"), (dbias, "dbias")):
             N.require_cuda_tensor(t, torch.bfloat16, nm)
-        ws_bytes = int(N.lib().llmk_gemm_workspace_bytes(MODE_TN, M * groups, Nn, K, 0))
+        ws_bytes = int(N.lib().llmk_gemm_workspace_bytes(MODE_TN, M * groups, Nn, K, _MAX_CTAS))
         ws = workspace(ws_bytes) if ws_bytes else None
         ws_n = ws.numel() if ws is not None else 0
         if groups == 1:

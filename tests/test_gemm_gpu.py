@@ -366,3 +366,27 @@ def test_fused_epilogues_of_few_tiles(M, T, H, K):
     want = (dout.double() * o.double()).view(M // T, T, NH, 64).sum(-1).transpose(1, 2)
     assert ((dvec.double() - want).abs() <= 1e-5 * 64).all()
     _native.check_status()
+
+
+@pytest.mark.parametrize("max_ctas", [0, 2, 24, 100, 132, 146, 148])
+@pytest.mark.parametrize("M,N,K", [(256, 4224, 38976), (768, 3072, 16384), (1024, 1024, 8200), (2304, 768, 4096)])
+def test_split_products_get_the_workspace_of_their_split_count(M, N, K, max_ctas):
+    """The split count depends on how many CTAs work on a product and does not change steadily with it; buffers here hold
+    exactly what is asked for, whatever the limit."""
+    from llm_kittens_b200.ops import gemm, _native
+
+    a, b = _rand(K, M, scale=0.1), _rand(K, N)
+    want = a.double().T @ b.double()
+    _native.set_guards(True)
+    gemm.set_max_ctas(max_ctas)
+    try:
+        db = torch.empty(M, device="cuda", dtype=torch.bfloat16)
+        out = gemm.gemm_tn(a, b, dbias=db)
+        assert _native.check_guards() >= 0
+    finally:
+        gemm.set_max_ctas(0)
+        _native.set_guards(False)
+    # fp32 sums of K products (of order 0.1), one rounding to bf16
+    assert ((out.double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-5 * K ** 0.5).all()
+    assert ((db.double() - a.double().sum(0)).abs() <= 2.0 ** -8 * a.double().sum(0).abs() + 1e-5 * K ** 0.5).all()
+    _native.check_status()
