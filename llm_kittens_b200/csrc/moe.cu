@@ -89,8 +89,9 @@ __device__ __forceinline__ bool wait_entries_block(const int* flags, int n, int 
 
 // ------------------------------------------------------------------ router
 // One warp per ROUTER_ROWS tokens: logits = x . Wr^T (fp32), softmax over E, top-K (ties -> lower expert index),
-// weights renormalised to sum 1. Several tokens share a router weight's trip from shared memory and its conversion.
-constexpr int ROUTER_ROWS = 4;
+// weights renormalised to sum 1. Two tokens share a router weight's trip from shared memory and its conversion, where there
+// are enough of them to fill the chip with warps: see launch_router.
+template <int ROUTER_ROWS>
 __global__ void __launch_bounds__(256)
 router_fwd_kernel(float* __restrict__ probs, int* __restrict__ top_idx, float* __restrict__ top_w, const bf16* __restrict__ x,
                   const bf16* __restrict__ wr, int N, int C, int E, int K) {
@@ -128,8 +129,8 @@ router_fwd_kernel(float* __restrict__ probs, int* __restrict__ top_idx, float* _
         for (int e = 0; e < MAXE; e++)
             if (e < E) acc[r][e] = warp_sum(acc[r][e]);
     // Lane e takes expert e. Sums and comparisons go through the experts in order, by shuffles, so the probabilities and
-    // the choices among equal ones are those of a serial loop (which one lane ran over arrays in local memory: 54 us at
-    // 16384 x 1024 with 8 experts, now 36 with four rows a warp).
+    // the choices among equal ones are those of a serial loop (which one lane ran over arrays in local memory: 52 us at
+    // 16384 x 1024 with 8 experts, 43 this way, 29 with two rows a warp).
 #pragma unroll
     for (int r = 0; r < ROUTER_ROWS; r++) {
         const int row = row0 + r;
@@ -177,7 +178,8 @@ router_fwd_kernel(float* __restrict__ probs, int* __restrict__ top_idx, float* _
 __global__ void __launch_bounds__(1024)
 assign_slots_kernel(int* __restrict__ slot, int* __restrict__ counts, const int* __restrict__ top_idx, int NK, int cap) {
     // 4096 entries per round, ranks from ballots, one barrier per round (two sets of warp totals) and the next round's
-    // entries already loaded: 29 us at 32768 entries with 1024 a round, a shuffle scan and three barriers, now 6.8
+    // entries already loaded: 27.7 us at 32768 entries with 1024 a round, a shuffle scan and three barriers, now 8.2
+    // (with the fill of the table, as called)
     constexpr int PER = 4, ROUND = 1024 * PER;
     __shared__ int warp_tot[2][32];
     const int e = blockIdx.x;
@@ -506,7 +508,7 @@ combine_dweight_kernel(float* __restrict__ dw, const bf16* __restrict__ dout, co
 // ------------------------------------------------------------------ load-balance statistics + router backward
 // density[e] = mean_t probs[t,e]  (one block, fixed order). The table is read once, in order: a thread's elements all
 // belong to one expert because the number of threads at work is a multiple of E. (A pass per expert with a stride of E took
-// 31 us at 16384 x 8, now 7.6.)
+// 31.7 us at 16384 x 8, now 7.3.)
 __global__ void __launch_bounds__(1024)
 density_kernel(float* __restrict__ density, float* __restrict__ aux_loss, const float* __restrict__ probs, int N, int E,
                float coef, int accumulate) {
@@ -586,18 +588,33 @@ static inline Peers make_peers(const long long* ptrs, int P) {
 using namespace llmk;
 using namespace llmk::moe;
 
+namespace llmk {
+namespace moe {
+// Rows per warp. The work per row is the same trip over the router however many rows share it, so with few tokens one row
+// per warp is the shortest chain, and with many the shared trip pays. us at C = 1024, 8 experts, top 2, one / two / four
+// rows: 64 tokens 7.7 / 10.4 / 14.1, 2048 9.7 / 10.9 / 14.8, 4096 14.0 / 12.4 / 14.9, 16384 43 / 29 / 33, 65536 154 / 110 / 118;
+// four are ahead by 10 % at 8192 tokens with 16 experts only. (768 channels and 4 experts: 2048 tokens 6.1 / 7.1 / 10.2, 4096
+// 7.8 / 8.1 / 10.6, 16384 21 / 17 / 22.)
+template <int ROWS>
+static int launch_router(float* probs, int* top_idx, float* top_w, const bf16* x, const bf16* wr, int N, int C, int E, int K,
+                         cudaStream_t stream) {
+    static PerDeviceOnce once_configured;
+    if (once_configured.first()) {
+        LLMK_CUDA_TRY(cudaFuncSetAttribute(router_fwd_kernel<ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    }
+    router_fwd_kernel<ROWS><<<ceil_div(N, 8 * ROWS), 256, E * C * 2, stream>>>(probs, top_idx, top_w, x, wr, N, C, E, K);
+    LLMK_LAUNCH_CHECK();
+    return LLMK_OK;
+}
+}  // namespace moe
+}  // namespace llmk
+
 LLMK_API int llmk_moe_router_fwd(void* probs, void* top_idx, void* top_w, const void* x, const void* wr, int N, int C, int E, int K,
                                  void* stream) {
     if (E > MAXE || K > MAXK || K > E || C % 8 || (long)E * C * 2 > 200 * 1024) return LLMK_ERR_SHAPE;
-    const int smem = E * C * 2;
-    static PerDeviceOnce once_configured;
-    if (once_configured.first()) {
-        LLMK_CUDA_TRY(cudaFuncSetAttribute(router_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    }
-    router_fwd_kernel<<<ceil_div(N, 8 * ROUTER_ROWS), 256, smem, (cudaStream_t)stream>>>((float*)probs, (int*)top_idx, (float*)top_w,
-                                                                          (const bf16*)x, (const bf16*)wr, N, C, E, K);
-    LLMK_LAUNCH_CHECK();
-    return LLMK_OK;
+#define LLMK_ROUTER(ROWS) launch_router<ROWS>((float*)probs, (int*)top_idx, (float*)top_w, (const bf16*)x, (const bf16*)wr, N, C, E, K, (cudaStream_t)stream)
+    return N <= 2048 ? LLMK_ROUTER(1) : LLMK_ROUTER(2);
+#undef LLMK_ROUTER
 }
 LLMK_API int llmk_moe_assign_slots(void* slot, void* counts, const void* top_idx, int N, int K, int E, int cap, void* stream) {
     cudaStream_t st = (cudaStream_t)stream;
