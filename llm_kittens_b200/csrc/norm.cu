@@ -49,10 +49,11 @@ norm_bwd_finish_kernel(bf16* __restrict__ dweight, bf16* __restrict__ dbias, con
 }
 
 // ------------------------------------------------------------------------------------------------
-// Forward. Both kernels keep the row in registers between the statistics passes and the normalise pass and load the next
-// row before they reduce the current one: they are bound by the memory latency per row, and without the prefetch a warp
-// has nothing in flight while it reduces. The grid is what fits on the chip at once, so every warp has several rows to
-// pipeline and there is no second, nearly empty wave.
+// Forward. Both kernels keep the row in registers between the statistics passes and the normalise pass, and are bound by the
+// memory latency per row. Without more, a warp has nothing in flight while it reduces; loading the next row before the
+// current one is reduced (AHEAD) keeps the memory busy but takes the registers of a second row, i.e. warps. With it the
+// grid is what fits on the chip at once, so every warp has several rows to pipeline and there is no second, nearly empty
+// wave; which one wins is in reads_ahead().
 //
 // Rows of up to 1280 columns: one warp per row; lane l owns the 16-byte vectors l, l + 32, ...
 // RAGGED: C is any multiple of 8 up to 256 * NVEC; the lanes whose last vector lies beyond the row keep zeros there.
@@ -67,7 +68,8 @@ __device__ __forceinline__ bf16x8 add8(const bf16x8& x, const bf16x8& y) {
     return pack8(a);
 }
 
-template <bool RMS, bool FUSED_RESIDUAL, int NVEC, bool RAGGED>
+// AHEAD: the next row is loaded before the current one is reduced.
+template <bool RMS, bool FUSED_RESIDUAL, int NVEC, bool RAGGED, bool AHEAD>
 __global__ void __launch_bounds__(REG_WARPS * 32)
 norm_fwd_reg_kernel(bf16* __restrict__ normed, float* __restrict__ mean_out, float* __restrict__ rstd_out,
                     bf16* residual_out, const bf16* inp1, const bf16* __restrict__ inp2, const bf16* __restrict__ weight,
@@ -82,11 +84,15 @@ norm_fwd_reg_kernel(bf16* __restrict__ normed, float* __restrict__ mean_out, flo
     };
     bf16x8 xn[NVEC], yn[FUSED_RESIDUAL ? NVEC : 1];
     int row = blockIdx.x * REG_WARPS + warp;
-    if (row < N) {
+    if (AHEAD && row < N) {
         load(inp1, row, xn);
         if (FUSED_RESIDUAL) load(inp2, row, yn);
     }
     for (; row < N; row += gridDim.x * REG_WARPS) {
+        if (!AHEAD) {
+            load(inp1, row, xn);
+            if (FUSED_RESIDUAL) load(inp2, row, yn);
+        }
         bf16x8 xv[NVEC];
 #pragma unroll
         for (int k = 0; k < NVEC; k++) {
@@ -97,7 +103,7 @@ norm_fwd_reg_kernel(bf16* __restrict__ normed, float* __restrict__ mean_out, flo
             }
         }
         const int next = row + gridDim.x * REG_WARPS;
-        if (next < N) {
+        if (AHEAD && next < N) {
             load(inp1, next, xn);
             if (FUSED_RESIDUAL) load(inp2, next, yn);
         }
@@ -152,7 +158,7 @@ norm_fwd_reg_kernel(bf16* __restrict__ normed, float* __restrict__ mean_out, flo
 
 // Wider rows: one block per row, every thread owns NV 16-byte vectors (C is any multiple of 8 up to NV * 2048). With a warp
 // per row these have few warps and one row each: 4096 x 1600 took 14.5 us, 4096 x 2048 11.8, 4096 x 4096 24.5, 320 x 2048
-// 4.1; here 9.6, 8.4, 13.7 and 2.3. At 4096 x 1280 the warp is still ahead, 8.5 against 9.0 us.
+// 4.1; here 9.6, 8.4, 13.7 and 2.3. At 4096 x 1280 the warp is still ahead, 8.5 against 9.0 us (and for 1536: WARP_ROWS_1536).
 template <bool RMS, bool FUSED_RESIDUAL, int NV>
 __global__ void __launch_bounds__(256, NV <= 2 ? 4 : (NV <= 4 ? 2 : 1))
 norm_fwd_wide_kernel(bf16* __restrict__ normed, float* __restrict__ mean_out, float* __restrict__ rstd_out,
@@ -515,17 +521,33 @@ static int num_sms() {
     return g_sms;
 }
 
+// Whole 256-column widths on the warp-per-row kernel, measured with rows from HBM and from the L2. Without a residual the
+// plain loop is ahead or even (us at 65536 rows, plain / ahead, RMSNorm: 768 columns 35.4 / 40.4, 1024 54.3 / 65.8, 1280 67.0 /
+// 80.1, but 256 15.1 / 15.1 and from the L2 11.7 / 10.8; LayerNorm 1024 at 16384 rows from the L2 17.7 / 18.5, 1280 24.4 / 25.3).
+// With a residual the loads per row double, and so does the gain where the registers allow it: LayerNorm 512 56.4 / 49.9
+// and 1280 147.7 / 122.6, but 1024 105.4 / 106.5 and at 8192 rows from the L2 14.0 / 15.6; RMSNorm 256 27.9 / 24.9, 1280 138 / 131,
+// but 768 70.5 / 76.0. (The other widths of up to 1280 columns always read ahead.)
+constexpr bool reads_ahead(bool rms, bool fused, int nvec) {
+    return fused ? nvec == 5 || nvec == (rms ? 1 : 2) : rms && nvec == 1;
+}
+// LayerNorm at 1536 columns: the block-per-row kernel has a quarter of its threads idle, the warp-per-row one fewer warps.
+// us, block / warp: 1024 rows 4.2 / 4.7, 4096 9.7 / 10.9, 8192 17.1 / 17.2 (from the L2 15.4 / 14.5), 16384 30.4 / 28.7, 65536 108 / 97.
+// (RMSNorm, and both with a residual: the block is ahead at every count.)
+constexpr int WARP_ROWS_1536 = 8192;
+
 template <bool RMS, bool FUSED>
 static int launch_fwd(bf16* normed, float* mean, float* rstd, bf16* residual, const bf16* inp1, const bf16* inp2,
                       const bf16* weight, const bf16* bias, int N, int C, float eps, cudaStream_t stream) {
     if (C % 8 != 0 || C > 16384) return LLMK_ERR_SHAPE;
-#define LLMK_NORM_FWD_LAUNCH(KERNEL, ROWS_PER_BLOCK)                                                                        \
+#define LLMK_NORM_FWD_LAUNCH(KERNEL, ROWS_PER_BLOCK, AHEAD)                                                                 \
     {                                                                                                                       \
-        static PerDeviceInt resident;                                                                                       \
-        int cap = 0;                                                                                                        \
-        LLMK_CUDA_TRY(resident.get(&cap, [](int* v) {                                                                       \
-            return cudaOccupancyMaxActiveBlocksPerMultiprocessor(v, KERNEL, REG_WARPS * 32, 0);                             \
-        }));                                                                                                                \
+        int cap = 16;                                                                                                       \
+        if (AHEAD) {                                                                                                        \
+            static PerDeviceInt resident;                                                                                   \
+            LLMK_CUDA_TRY(resident.get(&cap, [](int* v) {                                                                   \
+                return cudaOccupancyMaxActiveBlocksPerMultiprocessor(v, KERNEL, REG_WARPS * 32, 0);                         \
+            }));                                                                                                            \
+        }                                                                                                                   \
         cap *= num_sms();                                                                                                   \
         int grid = ceil_div(N, ROWS_PER_BLOCK);                                                                             \
         if (grid > cap) grid = cap;                                                                                         \
@@ -535,8 +557,11 @@ static int launch_fwd(bf16* normed, float* mean, float* rstd, bf16* residual, co
     }
 #define LLMK_NORM_FWD_CASE(NV)                                                                                              \
     case NV:                                                                                                                \
-        if (C == NV * 256) LLMK_NORM_FWD_LAUNCH((norm_fwd_reg_kernel<RMS, FUSED, NV, false>), REG_WARPS)                    \
-        LLMK_NORM_FWD_LAUNCH((norm_fwd_reg_kernel<RMS, FUSED, NV, true>), REG_WARPS)
+        if (C == NV * 256) {                                                                                                \
+            constexpr bool AHEAD = reads_ahead(RMS, FUSED, NV);                                                             \
+            LLMK_NORM_FWD_LAUNCH((norm_fwd_reg_kernel<RMS, FUSED, NV, false, AHEAD>), REG_WARPS, AHEAD)                     \
+        }                                                                                                                   \
+        LLMK_NORM_FWD_LAUNCH((norm_fwd_reg_kernel<RMS, FUSED, NV, true, true>), REG_WARPS, true)
     switch (ceil_div(C, 256)) {
         LLMK_NORM_FWD_CASE(1)
         LLMK_NORM_FWD_CASE(2)
@@ -545,12 +570,15 @@ static int launch_fwd(bf16* normed, float* mean, float* rstd, bf16* residual, co
         LLMK_NORM_FWD_CASE(5)
         default: break;
     }
+    if constexpr (!RMS && !FUSED) {
+        if (C == 1536 && N >= WARP_ROWS_1536) LLMK_NORM_FWD_LAUNCH((norm_fwd_reg_kernel<RMS, FUSED, 6, false, false>), REG_WARPS, false)
+    }
     switch (ceil_div(C, 2048)) {
-        case 1: LLMK_NORM_FWD_LAUNCH((norm_fwd_wide_kernel<RMS, FUSED, 1>), 1)
-        case 2: LLMK_NORM_FWD_LAUNCH((norm_fwd_wide_kernel<RMS, FUSED, 2>), 1)
+        case 1: LLMK_NORM_FWD_LAUNCH((norm_fwd_wide_kernel<RMS, FUSED, 1>), 1, true)
+        case 2: LLMK_NORM_FWD_LAUNCH((norm_fwd_wide_kernel<RMS, FUSED, 2>), 1, true)
         case 3:
-        case 4: LLMK_NORM_FWD_LAUNCH((norm_fwd_wide_kernel<RMS, FUSED, 4>), 1)
-        default: LLMK_NORM_FWD_LAUNCH((norm_fwd_wide_kernel<RMS, FUSED, 8>), 1)
+        case 4: LLMK_NORM_FWD_LAUNCH((norm_fwd_wide_kernel<RMS, FUSED, 4>), 1, true)
+        default: LLMK_NORM_FWD_LAUNCH((norm_fwd_wide_kernel<RMS, FUSED, 8>), 1, true)
     }
 #undef LLMK_NORM_FWD_CASE
 #undef LLMK_NORM_FWD_LAUNCH

@@ -141,6 +141,28 @@ def test_norm_forward_of_wide_rows(N, C):
     assert torch.equal(a2, r) and ((out.double() - want).abs() <= ulp * want.abs() + 1e-4).all()
 
 
+@pytest.mark.parametrize("N,C", [(20001, 256), (19000, 512), (20001, 768), (19000, 1024), (19000, 1280), (8191, 1536), (8192, 1536),
+                                 (20001, 1536)])
+def test_norm_forward_of_more_rows_than_the_grid_has_warps(N, C):
+    """Every variant of the warp-per-row and block-per-row kernels over several rows per warp, with and without a residual."""
+    from llm_kittens_b200.ops import norm
+
+    a, b, w, bias = rnd(N, C), rnd(N, C), rnd(C, scale=0.5) + 1, rnd(C, scale=0.1)
+    ulp = 2.0 ** -8     # one rounding to bf16
+    for x, ln, rms in ((a, norm.layernorm_fwd(a, w, bias), norm.rmsnorm_fwd(a, w, 1e-5)),
+                       ((a.float() + b.float()).to(BF), norm.residual_layernorm_fwd(a, b, w, bias), norm.residual_rmsnorm_fwd(a, b, w, 1e-5))):
+        if len(ln) == 4:
+            assert torch.equal(ln[0], x) and torch.equal(rms[0], x)
+            ln, rms = ln[1:], rms[1:]
+        want = torch.nn.functional.layer_norm(x.double(), (C,), w.double(), bias.double(), 1e-5)
+        assert ((ln[0].double() - want).abs() <= ulp * want.abs() + 1e-4).all()
+        assert (ln[1] - x.double().mean(-1)).abs().max() < 1e-5
+        rs = torch.rsqrt(x.double().pow(2).mean(-1) + 1e-5)
+        want = x.double() * rs[:, None] * w.double()
+        assert ((rms[0].double() - want).abs() <= ulp * want.abs() + 1e-4).all()
+        assert (rms[1] / rs - 1).abs().max() < 1e-5
+
+
 @pytest.mark.parametrize("n", [1, 7, 8, 9, 2047, 2048, 2049, 1000003])
 def test_zeroing_ends_at_the_tensor(n):
     from llm_kittens_b200.ops import elementwise as ew
