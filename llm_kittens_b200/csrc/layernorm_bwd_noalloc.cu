@@ -57,7 +57,7 @@ LLMK_API int llmk_layernorm_bwd_noalloc(void* dinp, void* dweight, void* dbias, 
     int sms = 0;
     const int rc = setup_current_device(&scratch, &sms);
     if (rc != LLMK_OK) return rc;
-    // the backward launches at most 4 blocks per SM, each leaving 2 * C partial sums
+    // the backward launches at most 2 blocks per SM, each leaving 2 * C partial sums; the limit counts 4, as callers know it
     const long long needed = 4LL * sms * 2LL * C;
     if (needed > (long long)LLMK_LN_BWD_NOALLOC_SCRATCH_FLOATS) return LLMK_ERR_LIMIT;
     return llmk::norm::layernorm_bwd_impl(static_cast<bf16*>(dinp), static_cast<bf16*>(dweight), static_cast<bf16*>(dbias),

@@ -265,10 +265,10 @@ norm_fwd_wide_kernel(bf16* __restrict__ normed, float* __restrict__ mean_out, fl
 // warps x STAGES x 3 x C x 2 bytes are in flight per SM whatever the register budget (with one row per warp in
 // registers alone it reached well under half of the copy bandwidth). The dweight / dbias sums stay in registers over all
 // rows of a warp. scratch layout: [gridDim.x][2][C] fp32 (second plane unused for RMSNorm). Every wait is bounded; a
-// failure goes to `status`.
+// failure goes to `status`. RAGGED: C is any multiple of 8 up to 256 * NVEC (a row is then still whole 16-byte pieces).
 template <int NVEC>
 struct BulkCfg {
-    static constexpr int C = NVEC * 256;
+    static constexpr int C = NVEC * 256;   // widest row
     static constexpr int ROW = C * 2;
     // narrow rows: 16 warps (two per scheduler hide the reduction latency) with a 2-deep ring; wide rows: 8 warps
     static constexpr int WARPS = NVEC <= 3 ? 16 : 8;
@@ -278,17 +278,20 @@ struct BulkCfg {
     static constexpr int SMEM = OFF_BAR + WARPS * STAGES * 8;
 };
 
-template <bool RMS, int NVEC>
+template <bool RMS, int NVEC, bool RAGGED>
 __global__ void __launch_bounds__(BulkCfg<NVEC>::WARPS * 32, 1)
 norm_bwd_bulk_kernel(bf16* __restrict__ dinp, float* __restrict__ scratch, const bf16* __restrict__ dout,
                      const bf16* __restrict__ inp, const bf16* __restrict__ weight, const float* __restrict__ mean,
-                     const float* __restrict__ rstd, int N, int accumulate_dinp, int* status) {
+                     const float* __restrict__ rstd, int N, int C_, int accumulate_dinp, int* status) {
     using B = BulkCfg<NVEC>;
-    constexpr int C = B::C, ROW = B::ROW, STAGES = B::STAGES, WARPS = B::WARPS;
+    constexpr int SLOT = B::ROW, STAGES = B::STAGES, WARPS = B::WARPS;
     constexpr int PLANES = RMS ? 1 : 2;
+    const int C = RAGGED ? C_ : B::C;
+    const uint32_t ROW = (uint32_t)C * 2;
     extern __shared__ __align__(128) uint8_t smem_raw[];
     __shared__ int abort_word;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    auto in_row = [&](int k) { return !RAGGED || (lane + 32 * k) * 8 < C; };
     uint8_t* ring = smem_raw + (size_t)warp * B::WARP_RING;
     uint64_t* full = reinterpret_cast<uint64_t*>(smem_raw + B::OFF_BAR) + warp * STAGES;
     volatile int* abort_flag = &abort_word;
@@ -305,11 +308,11 @@ norm_bwd_bulk_kernel(bf16* __restrict__ dinp, float* __restrict__ scratch, const
     auto issue = [&](int i) {   // lane 0 only
         const int st = i % STAGES;
         const size_t off = (size_t)(first + (size_t)i * stride) * C;
-        uint8_t* dst = ring + st * 3 * ROW;
+        uint8_t* dst = ring + st * 3 * SLOT;
         ptx::mbar_arrive_expect_tx(&full[st], tx);
         ptx::bulk_load_1d(dst, dout + off, ROW, &full[st]);
-        ptx::bulk_load_1d(dst + ROW, inp + off, ROW, &full[st]);
-        if (accumulate_dinp) ptx::bulk_load_1d(dst + 2 * ROW, dinp + off, ROW, &full[st]);
+        ptx::bulk_load_1d(dst + SLOT, inp + off, ROW, &full[st]);
+        if (accumulate_dinp) ptx::bulk_load_1d(dst + 2 * SLOT, dinp + off, ROW, &full[st]);
     };
     if (lane == 0)
         for (int i = 0; i < STAGES && i < nrows; i++) issue(i);
@@ -330,13 +333,13 @@ norm_bwd_bulk_kernel(bf16* __restrict__ dinp, float* __restrict__ scratch, const
         const int row = first + i * stride;
         ok = ptx::mbar_wait(&full[st], (i / STAGES) & 1, abort_flag, status, LLMK_ST_TIMEOUT_TMA_FULL, 8000 + st);
         if (!ok) break;
-        const uint8_t* src = ring + st * 3 * ROW;
+        const uint8_t* src = ring + st * 3 * SLOT;
         bf16x8 dv[NVEC], xv[NVEC], ov[NVEC];
 #pragma unroll
-        for (int k = 0; k < NVEC; k++) {
-            dv[k] = *reinterpret_cast<const bf16x8*>(src + (lane + 32 * k) * 16);
-            xv[k] = *reinterpret_cast<const bf16x8*>(src + ROW + (lane + 32 * k) * 16);
-            if (accumulate_dinp) ov[k] = *reinterpret_cast<const bf16x8*>(src + 2 * ROW + (lane + 32 * k) * 16);
+        for (int k = 0; k < NVEC; k++) {   // lanes beyond the row hold zeros: nothing was copied there
+            dv[k] = in_row(k) ? *reinterpret_cast<const bf16x8*>(src + (lane + 32 * k) * 16) : zero8();
+            xv[k] = in_row(k) ? *reinterpret_cast<const bf16x8*>(src + SLOT + (lane + 32 * k) * 16) : zero8();
+            if (accumulate_dinp && in_row(k)) ov[k] = *reinterpret_cast<const bf16x8*>(src + 2 * SLOT + (lane + 32 * k) * 16);
         }
         __syncwarp();   // the stage has been copied into registers by every lane: refill it
         if (lane == 0 && i + STAGES < nrows) issue(i + STAGES);
@@ -348,7 +351,7 @@ norm_bwd_bulk_kernel(bf16* __restrict__ dinp, float* __restrict__ scratch, const
             float fd[8], fx[8], fw[8];
             unpack8(dv[k], fd);
             unpack8(xv[k], fx);
-            unpack8(ld128(weight + (lane + 32 * k) * 8), fw);
+            unpack8(in_row(k) ? ld128(weight + (lane + 32 * k) * 8) : zero8(), fw);
 #pragma unroll
             for (int j = 0; j < 8; j++) {
                 const float n = (fx[j] - m) * rs;
@@ -363,6 +366,7 @@ norm_bwd_bulk_kernel(bf16* __restrict__ dinp, float* __restrict__ scratch, const
         s2 = warp_sum(s2) * inv_c;
 #pragma unroll
         for (int k = 0; k < NVEC; k++) {
+            if (!in_row(k)) continue;
             float fd[8], fx[8], fo[8], fw[8];
             unpack8(dv[k], fd);
             unpack8(xv[k], fx);
@@ -383,12 +387,14 @@ norm_bwd_bulk_kernel(bf16* __restrict__ dinp, float* __restrict__ scratch, const
     if (*abort_flag) return;
     float* sh = reinterpret_cast<float*>(smem_raw);   // [WARPS][PLANES][C]
 #pragma unroll
-    for (int k = 0; k < NVEC; k++)
+    for (int k = 0; k < NVEC; k++) {
+        if (!in_row(k)) continue;
 #pragma unroll
         for (int j = 0; j < 8; j++) {
             sh[(size_t)warp * PLANES * C + (lane + 32 * k) * 8 + j] = dw[k][j];
             if (!RMS) sh[(size_t)warp * PLANES * C + C + (lane + 32 * k) * 8 + j] = db[k][j];
         }
+    }
     __syncthreads();
     float* dst = scratch + (size_t)blockIdx.x * 2 * C;
     for (int i = threadIdx.x; i < PLANES * C; i += blockDim.x) {
@@ -613,26 +619,25 @@ LLMK_API int llmk_residual_rmsnorm_fwd(void* residual, void* normed, void* rstd,
                                   (const bf16*)weight, nullptr, N, C, eps, (cudaStream_t)stream);
 }
 
-// Upper bound over both backward implementations (at most 4 blocks per SM).
-LLMK_API long llmk_norm_bwd_scratch_bytes(int N, int C) { return (long)num_sms() * 4 * 2 * C * 4; }
+// An upper bound: no backward kernel launches more than 2 blocks per SM.
+LLMK_API long llmk_norm_bwd_scratch_bytes(int N, int C) { return (long)num_sms() * 2 * 2 * C * 4; }
 
 namespace llmk {
 namespace norm {
-template <bool RMS, int NVEC>
+template <bool RMS, int NVEC, bool RAGGED = false>
 static int launch_bwd_bulk(bf16* dinp, bf16* dweight, bf16* dbias, float* scratch, const bf16* dout, const bf16* inp,
-                           const bf16* weight, const float* mean, const float* rstd, int N, int accumulate_dinp,
+                           const bf16* weight, const float* mean, const float* rstd, int N, int C, int accumulate_dinp,
                            cudaStream_t stream) {
-    constexpr int C = NVEC * 256;
     using B = BulkCfg<NVEC>;
-    static_assert(B::OFF_BAR >= B::WARPS * 2 * C * 4, "the rings must be able to hold the final reduction buffer");
+    static_assert(B::OFF_BAR >= B::WARPS * 2 * B::C * 4, "the rings must be able to hold the final reduction buffer");
     static PerDeviceOnce once_bulk_configured;
     if (once_bulk_configured.first()) {
-        LLMK_CUDA_TRY(cudaFuncSetAttribute(norm_bwd_bulk_kernel<RMS, NVEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, B::SMEM));
+        LLMK_CUDA_TRY(cudaFuncSetAttribute(norm_bwd_bulk_kernel<RMS, NVEC, RAGGED>, cudaFuncAttributeMaxDynamicSharedMemorySize, B::SMEM));
     }
     int grid = num_sms();
     const int need = ceil_div(N, B::WARPS);
     if (grid > need) grid = need;
-    norm_bwd_bulk_kernel<RMS, NVEC><<<grid, B::WARPS * 32, B::SMEM, stream>>>(dinp, scratch, dout, inp, weight, mean, rstd, N,
+    norm_bwd_bulk_kernel<RMS, NVEC, RAGGED><<<grid, B::WARPS * 32, B::SMEM, stream>>>(dinp, scratch, dout, inp, weight, mean, rstd, N, C,
         accumulate_dinp, current_status_word());
     LLMK_LAUNCH_CHECK();
     norm_bwd_finish_kernel<<<ceil_div(C, 32), dim3(32, FIN_LANES), 0, stream>>>(dweight, dbias, scratch, grid, C);
@@ -656,33 +661,60 @@ static int launch_bwd_wide(bf16* dinp, bf16* dweight, bf16* dbias, float* scratc
 
 namespace llmk {
 namespace norm {
-// LayerNorm backward: launch of the row kernel plus the fixed-order partial reduction.
+// From how many rows on the rings of the warp-per-row kernel pay for their set-up where a row is not whole vectors per lane;
+// below, every row has a block of its own anyway. us, block per row / rings, LayerNorm: 128 columns 256 rows 5.3 / 5.3, 512
+// 6.4 / 5.4, 16384 58 / 13; 384 columns 512 rows 6.9 / 7.5, 1024 8.6 / 7.9, 16384 62 / 19; 640 columns 1024 rows 9.9 / 10.8, 2048
+// 13.6 / 11.3; 1272 columns 512 rows 10.2 / 11.1, 1024 12.4 / 11.8, 16384 74 / 50.
+constexpr int ragged_bulk_rows(int C) { return C <= 256 ? 512 : 1024; }
+
+// The row kernel plus the fixed-order reduction of its partials.
+template <bool RMS>
+static int launch_bwd(bf16* dinp, bf16* dweight, bf16* dbias, float* scratch, const bf16* dout, const bf16* inp, const bf16* weight,
+                      const float* mean, const float* rstd, int N, int C, int accumulate_dinp, cudaStream_t stream) {
+    if (C % 8 != 0 || C > 12288) return LLMK_ERR_SHAPE;
+#define LLMK_NORM_BWD(LAUNCH, ...) \
+    return LAUNCH<RMS, __VA_ARGS__>(dinp, dweight, dbias, scratch, dout, inp, weight, mean, rstd, N, C, accumulate_dinp, stream);
+    switch (C % 2048 == 0 ? C / 2048 : 0) {
+        case 1: LLMK_NORM_BWD(launch_bwd_wide, 1)
+        case 2: LLMK_NORM_BWD(launch_bwd_wide, 2)
+        case 3: LLMK_NORM_BWD(launch_bwd_wide, 3)
+        case 4: LLMK_NORM_BWD(launch_bwd_wide, 4)
+        case 6: LLMK_NORM_BWD(launch_bwd_wide, 6)
+        default: break;
+    }
+#define LLMK_NORM_BWD_BULK(NVEC)                                                    \
+    case NVEC:                                                                      \
+        if (C == NVEC * 256) LLMK_NORM_BWD(launch_bwd_bulk, NVEC)                   \
+        if (N >= ragged_bulk_rows(C)) LLMK_NORM_BWD(launch_bwd_bulk, NVEC, true) \
+        break;
+    switch (ceil_div(C, 256)) {
+        LLMK_NORM_BWD_BULK(1)
+        LLMK_NORM_BWD_BULK(2)
+        LLMK_NORM_BWD_BULK(3)
+        LLMK_NORM_BWD_BULK(4)
+        LLMK_NORM_BWD_BULK(5)
+        default: break;
+    }
+    switch (ceil_div(C, 2048)) {
+        case 1: LLMK_NORM_BWD(launch_bwd_wide, 1, true)
+        case 2: LLMK_NORM_BWD(launch_bwd_wide, 2, true)
+        case 3: LLMK_NORM_BWD(launch_bwd_wide, 3, true)
+        default: break;
+    }
+    if constexpr (RMS) {
+        if (C <= 8192) LLMK_NORM_BWD(launch_bwd_wide, 4, true)
+        LLMK_NORM_BWD(launch_bwd_wide, 6, true)
+    }
+#undef LLMK_NORM_BWD_BULK
+#undef LLMK_NORM_BWD
+    return LLMK_ERR_SHAPE;
+}
+
+// (a symbol of its own for layernorm_bwd_noalloc.cu)
 int layernorm_bwd_impl(bf16* dinp, bf16* dweight, bf16* dbias, float* scratch, const bf16* dout, const bf16* inp,
                        const bf16* weight, const float* mean, const float* rstd, int N, int C, int accumulate_dinp,
                        cudaStream_t stream) {
-    if (C % 8 != 0 || C > 12288) return LLMK_ERR_SHAPE;
-    switch (C % 2048 == 0 ? C / 2048 : 0) {
-        case 1: return launch_bwd_wide<false, 1>(dinp, dweight, dbias, scratch, dout, inp, weight, mean, rstd, N, C, accumulate_dinp, stream);
-        case 2: return launch_bwd_wide<false, 2>(dinp, dweight, dbias, scratch, dout, inp, weight, mean, rstd, N, C, accumulate_dinp, stream);
-        case 3: return launch_bwd_wide<false, 3>(dinp, dweight, dbias, scratch, dout, inp, weight, mean, rstd, N, C, accumulate_dinp, stream);
-        case 4: return launch_bwd_wide<false, 4>(dinp, dweight, dbias, scratch, dout, inp, weight, mean, rstd, N, C, accumulate_dinp, stream);
-        case 6: return launch_bwd_wide<false, 6>(dinp, dweight, dbias, scratch, dout, inp, weight, mean, rstd, N, C, accumulate_dinp, stream);
-        default: break;
-    }
-    switch (C % 256 == 0 ? C / 256 : 0) {
-        case 1: return launch_bwd_bulk<false, 1>(dinp, dweight, dbias, scratch, dout, inp, weight, mean, rstd, N, accumulate_dinp, stream);
-        case 2: return launch_bwd_bulk<false, 2>(dinp, dweight, dbias, scratch, dout, inp, weight, mean, rstd, N, accumulate_dinp, stream);
-        case 3: return launch_bwd_bulk<false, 3>(dinp, dweight, dbias, scratch, dout, inp, weight, mean, rstd, N, accumulate_dinp, stream);
-        case 4: return launch_bwd_bulk<false, 4>(dinp, dweight, dbias, scratch, dout, inp, weight, mean, rstd, N, accumulate_dinp, stream);
-        case 5: return launch_bwd_bulk<false, 5>(dinp, dweight, dbias, scratch, dout, inp, weight, mean, rstd, N, accumulate_dinp, stream);
-        default: break;
-    }
-    if (C > 6144) return LLMK_ERR_SHAPE;
-    switch (ceil_div(C, 2048)) {
-        case 1: return launch_bwd_wide<false, 1, true>(dinp, dweight, dbias, scratch, dout, inp, weight, mean, rstd, N, C, accumulate_dinp, stream);
-        case 2: return launch_bwd_wide<false, 2, true>(dinp, dweight, dbias, scratch, dout, inp, weight, mean, rstd, N, C, accumulate_dinp, stream);
-        default: return launch_bwd_wide<false, 3, true>(dinp, dweight, dbias, scratch, dout, inp, weight, mean, rstd, N, C, accumulate_dinp, stream);
-    }
+    return launch_bwd<false>(dinp, dweight, dbias, scratch, dout, inp, weight, mean, rstd, N, C, accumulate_dinp, stream);
 }
 }  // namespace norm
 }  // namespace llmk
@@ -697,47 +729,7 @@ LLMK_API int llmk_layernorm_bwd(void* dinp, void* dweight, void* dbias, void* sc
 }
 
 LLMK_API int llmk_rmsnorm_bwd(void* dinp, void* dweight, void* scratch, const void* dout, const void* inp, const void* weight,
-                              const void* rstd, int N, int C, int accumulate_dinp, void* stream_) {
-    cudaStream_t stream = (cudaStream_t)stream_;
-    if (C % 8 != 0 || C > 12288) return LLMK_ERR_SHAPE;
-#define LLMK_RMS_BWD_CASE(NV)                                                                                             \
-    case NV:                                                                                                              \
-        return launch_bwd_bulk<true, NV>((bf16*)dinp, (bf16*)dweight, nullptr, (float*)scratch, (const bf16*)dout,         \
-                                        (const bf16*)inp, (const bf16*)weight, nullptr, (const float*)rstd, N,            \
-                                        accumulate_dinp, stream);
-#define LLMK_RMS_WIDE_CASE(NV)                                                                                            \
-    case NV:                                                                                                              \
-        return launch_bwd_wide<true, NV>((bf16*)dinp, (bf16*)dweight, nullptr, (float*)scratch, (const bf16*)dout,        \
-                                         (const bf16*)inp, (const bf16*)weight, nullptr, (const float*)rstd, N, C,        \
-                                         accumulate_dinp, stream);
-    switch (C % 2048 == 0 ? C / 2048 : 0) {
-        LLMK_RMS_WIDE_CASE(1)
-        LLMK_RMS_WIDE_CASE(2)
-        LLMK_RMS_WIDE_CASE(3)
-        LLMK_RMS_WIDE_CASE(4)
-        LLMK_RMS_WIDE_CASE(6)
-        default: break;
-    }
-#undef LLMK_RMS_WIDE_CASE
-    switch (C % 256 == 0 ? C / 256 : 0) {
-        LLMK_RMS_BWD_CASE(1)
-        LLMK_RMS_BWD_CASE(2)
-        LLMK_RMS_BWD_CASE(3)
-        LLMK_RMS_BWD_CASE(4)
-        LLMK_RMS_BWD_CASE(5)
-        default: break;
-    }
-#undef LLMK_RMS_BWD_CASE
-#define LLMK_RMS_RAGGED(NV)                                                                                                  \
-    return launch_bwd_wide<true, NV, true>((bf16*)dinp, (bf16*)dweight, nullptr, (float*)scratch, (const bf16*)dout,         \
-                                           (const bf16*)inp, (const bf16*)weight, nullptr, (const float*)rstd, N, C,        \
-                                           accumulate_dinp, stream);
-    switch (ceil_div(C, 2048)) {
-        case 1: LLMK_RMS_RAGGED(1)
-        case 2: LLMK_RMS_RAGGED(2)
-        case 3: LLMK_RMS_RAGGED(3)
-        case 4: LLMK_RMS_RAGGED(4)
-        default: LLMK_RMS_RAGGED(6)
-    }
-#undef LLMK_RMS_RAGGED
+                              const void* rstd, int N, int C, int accumulate_dinp, void* stream) {
+    return launch_bwd<true>((bf16*)dinp, (bf16*)dweight, nullptr, (float*)scratch, (const bf16*)dout, (const bf16*)inp,
+                            (const bf16*)weight, nullptr, (const float*)rstd, N, C, accumulate_dinp, (cudaStream_t)stream);
 }

@@ -81,7 +81,8 @@ def test_rmsnorm(N, C):
 
 
 @pytest.mark.parametrize("rms", [False, True])
-@pytest.mark.parametrize("N,C", [(1, 8), (5, 248), (9, 264), (700, 1600), (3, 1912), (300, 2040), (7, 2056), (5, 3200), (4, 6136)])
+@pytest.mark.parametrize("N,C", [(1, 8), (5, 248), (9, 264), (700, 1600), (3, 1912), (300, 2040), (7, 2056), (5, 3200), (4, 6136),
+                                 (512, 8), (4100, 128), (513, 248), (1024, 264), (2500, 384), (1023, 504), (1025, 776), (1030, 1272)])
 def test_norms_of_widths_that_are_not_whole_vectors_per_lane(N, C, rms):
     """Row widths around the edges of the per-lane (256) and per-block (2048) vectors. Every tensor is followed by a row of
     NaNs that must be neither read into a result nor overwritten."""
