@@ -19,6 +19,12 @@ def maxerr(a, b):
     return (a.float() - b.float()).abs().max().item()
 
 
+def rounded(got, want, rest):
+    """``got`` is ``want`` rounded to bf16 (at most 2^-9 of the value; 2^-8 leaves room for a result that lies on the other side
+    of a rounding boundary) but for ``rest``, the error of the fp32 arithmetic in front of the rounding."""
+    return ((got.double() - want.double()).abs() <= 2.0 ** -8 * want.double().abs() + rest).all().item()
+
+
 @pytest.mark.parametrize("N,C", [(64, 768), (1000, 768), (3, 1024), (257, 2048), (128, 4096), (33, 1600)])
 def test_layernorm_fwd_bwd(N, C):
     from llm_kittens_b200.ops import norm
@@ -28,7 +34,7 @@ def test_layernorm_fwd_bwd(N, C):
     xf = x.float().requires_grad_(True)
     wf, bf_ = w.float().requires_grad_(True), b.float().requires_grad_(True)
     ref = torch.nn.functional.layer_norm(xf, (C,), wf, bf_, 1e-5)
-    assert maxerr(out, ref) < 0.04
+    assert rounded(out, ref, 1e-4)
     assert maxerr(mean, x.float().mean(-1)) < 1e-3
     assert maxerr(rstd, 1 / torch.sqrt(x.float().var(-1, unbiased=False) + 1e-5)) < 1e-2
     dout = rnd(N, C)
@@ -37,7 +43,7 @@ def test_layernorm_fwd_bwd(N, C):
     dinp = dinp0.clone()
     dw, db = torch.zeros(C, device="cuda", dtype=BF), torch.zeros(C, device="cuda", dtype=BF)
     norm.layernorm_bwd(dinp, dw, db, dout, x, w, mean, rstd, accumulate_dinp=True)
-    assert maxerr(dinp, xf.grad + dinp0.float()) < 0.06
+    assert rounded(dinp, xf.grad + dinp0.float(), 1e-3)
     assert maxerr(dw, wf.grad) < 0.02 * max(1.0, wf.grad.abs().max().item())
     assert maxerr(db, bf_.grad) < 0.02 * max(1.0, bf_.grad.abs().max().item())
     # deterministic
@@ -55,7 +61,7 @@ def test_residual_layernorm():
     r = (a.float() + b.float()).to(BF)
     assert torch.equal(res, r)
     ref = torch.nn.functional.layer_norm(r.float(), (C,), w.float(), bias.float(), 1e-5)
-    assert maxerr(out, ref) < 0.04
+    assert rounded(out, ref, 1e-4)     # (outputs above 16, one draw in ten, are rounded by up to 0.06)
 
 
 @pytest.mark.parametrize("N,C", [(64, 2048), (100, 4096), (5, 768)])
@@ -66,14 +72,14 @@ def test_rmsnorm(N, C):
     out, rstd = norm.rmsnorm_fwd(x, w, 1e-5)
     xf, wf = x.float().requires_grad_(True), w.float().requires_grad_(True)
     ref = xf * torch.rsqrt(xf.pow(2).mean(-1, keepdim=True) + 1e-5) * wf
-    assert maxerr(out, ref) < 0.04
+    assert rounded(out, ref, 1e-4)
     assert maxerr(rstd, torch.rsqrt(x.float().pow(2).mean(-1) + 1e-5)) < 0.01
     dout = rnd(N, C)
     ref.backward(dout.float())
     dinp = torch.zeros(N, C, device="cuda", dtype=BF)
     dw = torch.zeros(C, device="cuda", dtype=BF)
     norm.rmsnorm_bwd(dinp, dw, dout, x, w, rstd, accumulate_dinp=False)
-    assert maxerr(dinp, xf.grad) < 0.04
+    assert rounded(dinp, xf.grad, 1e-3)
     assert maxerr(dw, wf.grad) < 0.02 * max(1.0, wf.grad.abs().max().item())
     a, b = rnd(N, C), rnd(N, C)
     res, out2, _ = norm.residual_rmsnorm_fwd(a, b, w, 1e-5)
@@ -312,13 +318,13 @@ def test_dbias_and_encoder():
     tok = torch.randint(0, V, (B, T), device="cuda", dtype=torch.int32)
     tok[0, :10] = 7  # repeated token
     out = ew.encoder_fwd(tok, wte, wpe)
-    assert maxerr(out, wte.float()[tok.long()] + wpe.float()[None]) < 0.02
+    assert rounded(out, wte.float()[tok.long()] + wpe.float()[None], 0.0)
     d = rnd(B, T, C)
     dwte, dwpe = torch.zeros_like(wte), torch.zeros_like(wpe)
     ew.encoder_bwd(dwte, dwpe, d, tok)
     ref_wte = torch.zeros(V, C, device="cuda").index_add_(0, tok.reshape(-1).long(), d.float().view(-1, C))
-    assert maxerr(dwte, ref_wte) < 0.06
-    assert maxerr(dwpe, d.float().sum(0)) < 0.05
+    assert rounded(dwte, ref_wte, 1e-5)
+    assert rounded(dwpe, d.float().sum(0), 1e-5)
     dwte2, dwpe2 = torch.zeros_like(wte), torch.zeros_like(wpe)
     ew.encoder_bwd(dwte2, dwpe2, d, tok)
     assert torch.equal(dwte, dwte2)
