@@ -282,24 +282,34 @@ __global__ void wpe_bwd_kernel(bf16* __restrict__ dwpe, const bf16* __restrict__
 // dwte[tok,:] += sum over the positions holding `tok`. `sorted_tok`/`sorted_pos` list the B*T positions ordered by token
 // id (stable, so positions ascend inside a run of one token). Token frequencies are far from even (the most frequent
 // token of a text is several per cent of it), and a row read by a dependent chain costs a memory latency, so runs are
-// cut: block j takes the WTE_ROWS sorted positions from j * WTE_ROWS and sums each run inside them in fp32. A run that
-// lies inside the block is added to dwte; a piece of a run that crosses a block edge goes to partial[j][0] (it started
-// in an earlier block) or partial[j][1] (it starts here), and wte_bwd_join_kernel adds the pieces of such a run in block
-// order. Fixed summation order => deterministic. (One block per run, whole: 1614 us at 65536 x 768 with Zipf-distributed
-// ids, where the longest run has some 2400 rows; cut: 42 us, of which the bytes take 20.)
-constexpr int WTE_ROWS = 32;
+// cut: block j takes the `rows` sorted positions from j * rows and sums each run inside them in fp32. A run that lies
+// inside the block is added to dwte; a piece of a run that crosses a block edge goes to partial[j][0] (it started in an
+// earlier block) or partial[j][1] (it starts here), and wte_bwd_join_kernel adds the pieces of such a run in block order.
+// Fixed summation order => deterministic. (One block per run, whole: 1614 us at 65536 x 768 with Zipf-distributed ids,
+// where the longest run has some 2400 rows; cut: 42 us, of which the bytes take 20.)
+constexpr int WTE_MAX_ROWS = 32;
+// Rows per block: few where there are few positions, for blocks on more SMs and shorter chains of rows, but every cut of a run
+// is one more piece for the join, which adds them one after the other. us for the whole gradient, sort included, at 768
+// columns, 8 / 16 / 32 rows: 64 positions of distinct tokens 25.5 / 27.8 / 32.1, 1024 Zipf 57.4 / 58.4 / 62.7, 1024 of one token
+// 62 / 56 / 54, 4096 Zipf 92.9 / 90.2 / 92.3, 4096 of one token 138 / 103 / 89, 16384 Zipf 151 / 129 / 115.
+static inline int wte_rows(int BT) { return BT <= 1024 ? 8 : (BT <= 4096 ? 16 : WTE_MAX_ROWS); }
+// AHEAD: the rows of dwte that a batch ends on are loaded with the batch. One after the other they cost a memory latency each
+// (64 distinct tokens at 32 rows per block 37.8 us, 32.1 with them ahead; 16384 Zipf 121.7 / 115.3), but with some 2000 blocks
+// the others hide that and the registers are better spent on warps (65536 Zipf 194 / 200).
+constexpr int WTE_AHEAD_BLOCKS = 1024;
+template <bool AHEAD>
 __global__ void wte_bwd_kernel(bf16* __restrict__ dwte, float* __restrict__ partial, const bf16* __restrict__ dout,
-                               const int* __restrict__ sorted_tok, const int* __restrict__ sorted_pos, int BT, int C) {
-    __shared__ int tok[WTE_ROWS], pos[WTE_ROWS];
-    __shared__ int before, after;   // the tokens next to the block's range (-1: none)
-    const int base = blockIdx.x * WTE_ROWS, n = min(WTE_ROWS, BT - base);
+                               const int* __restrict__ sorted_tok, const int* __restrict__ sorted_pos, int BT, int C, int rows) {
+    __shared__ int tok[WTE_MAX_ROWS + 1], pos[WTE_MAX_ROWS];
+    __shared__ int before;   // the token in front of the block's range (-1: none); tok[n]: the one behind it
+    const int base = blockIdx.x * rows, n = min(rows, BT - base);
     if ((int)threadIdx.x < n) {
         tok[threadIdx.x] = sorted_tok[base + threadIdx.x];
         pos[threadIdx.x] = sorted_pos[base + threadIdx.x];
     }
     if (threadIdx.x == 0) {
         before = base > 0 ? sorted_tok[base - 1] : -1;
-        after = base + n < BT ? sorted_tok[base + n] : -1;
+        tok[n] = base + n < BT ? sorted_tok[base + n] : -1;
     }
     __syncthreads();
     const int cvecs = C / 8;
@@ -308,12 +318,16 @@ __global__ void wte_bwd_kernel(bf16* __restrict__ dwte, float* __restrict__ part
         float acc[8];
 #pragma unroll
         for (int j = 0; j < 8; j++) acc[j] = 0.f;
-        int first = 0;         // where the current run starts in this block
         for (int k0 = 0; k0 < n; k0 += BATCH) {
-            bf16x8 v[BATCH];
+            // the rows of dout and, where a run that lies inside the block ends, the row of dwte that it is added to (tokens
+            // are sorted: the run of a token that also stands in front of the block comes from there)
+            bf16x8 v[BATCH], w[BATCH];
 #pragma unroll
-            for (int k = 0; k < BATCH; k++)
-                if (k0 + k < n) v[k] = ld128_stream(dout + (size_t)pos[k0 + k] * C + cv * 8);
+            for (int k = 0; k < BATCH; k++) {
+                const int i = k0 + k;
+                if (i < n) v[k] = ld128_stream(dout + (size_t)pos[i] * C + cv * 8);
+                if (AHEAD && i < n && tok[i + 1] != tok[i] && tok[i] != before) w[k] = ld128(dwte + (size_t)tok[i] * C + cv * 8);
+            }
 #pragma unroll
             for (int k = 0; k < BATCH; k++) {
                 const int i = k0 + k;
@@ -323,42 +337,41 @@ __global__ void wte_bwd_kernel(bf16* __restrict__ dwte, float* __restrict__ part
 #pragma unroll
                 for (int j = 0; j < 8; j++) acc[j] += f[j];
                 const int t = tok[i];
-                const int next = i + 1 < n ? tok[i + 1] : after;
-                if (i + 1 < n && next == t) continue;
+                const bool last = i + 1 == n;
+                if (!last && tok[i + 1] == t) continue;
                 // the run's piece in this block ends here
-                const bool from_left = first == 0 && before == t, to_right = i + 1 == n && next == t;
+                const bool from_left = t == before, to_right = last && tok[n] == t;
                 if (from_left || to_right) {
                     float4* dst = reinterpret_cast<float4*>(partial + ((size_t)blockIdx.x * 2 + (from_left ? 0 : 1)) * C + cv * 8);
                     dst[0] = make_float4(acc[0], acc[1], acc[2], acc[3]);
                     dst[1] = make_float4(acc[4], acc[5], acc[6], acc[7]);
                 } else {
                     bf16* dst = dwte + (size_t)t * C + cv * 8;
-                    unpack8(ld128(dst), f);
+                    unpack8(AHEAD ? w[k] : ld128(dst), f);
 #pragma unroll
                     for (int j = 0; j < 8; j++) f[j] += acc[j];
                     st128(dst, pack8(f));
                 }
 #pragma unroll
                 for (int j = 0; j < 8; j++) acc[j] = 0.f;
-                first = i + 1;
             }
         }
     }
 }
 // Block j finishes the run that starts in wte_bwd_kernel's block j and goes on in block j + 1, if there is one.
 __global__ void wte_bwd_join_kernel(bf16* __restrict__ dwte, const float* __restrict__ partial, const int* __restrict__ sorted_tok,
-                                    int BT, int C) {
-    const int base = blockIdx.x * WTE_ROWS, end = base + WTE_ROWS;
+                                    int BT, int C, int rows) {
+    const int base = blockIdx.x * rows, end = base + rows;
     if (end >= BT) return;
     const int t = sorted_tok[end];
     if (sorted_tok[end - 1] != t) return;                                             // no run crosses this edge
     if (base > 0 && sorted_tok[base] == t && sorted_tok[base - 1] == t) return;       // it started further left
     // blocks to the right that start with t: they are consecutive, so counting them is enough
-    const int blocks = (BT + WTE_ROWS - 1) / WTE_ROWS;
+    const int blocks = (BT + rows - 1) / rows;
     int pieces = 0;
     for (int j0 = blockIdx.x + 1; j0 < blocks; j0 += blockDim.x) {
         const int j = j0 + (int)threadIdx.x;
-        const int hit = __syncthreads_count(j < blocks && sorted_tok[(size_t)j * WTE_ROWS] == t);
+        const int hit = __syncthreads_count(j < blocks && sorted_tok[(size_t)j * rows] == t);
         pieces += hit;
         if (hit < (int)blockDim.x) break;
     }
@@ -613,7 +626,7 @@ LLMK_API int llmk_bucket_sort(void* sorted_tok, void* sorted_pos, const void* to
 }
 
 // fp32 elements of scratch that llmk_encoder_bwd needs for B * T = BT positions.
-LLMK_API long llmk_encoder_bwd_scratch_floats(int BT, int C) { return (long)ceil_div(BT, WTE_ROWS) * 2 * C; }
+LLMK_API long llmk_encoder_bwd_scratch_floats(int BT, int C) { return (long)ceil_div(BT, wte_rows(BT)) * 2 * C; }
 // dwte += scatter of dout rows by token, dwpe += sum over batch (dwpe may be null for models without wpe).
 LLMK_API int llmk_encoder_bwd(void* dwte, void* dwpe, const void* dout, const void* sorted_tok, const void* sorted_pos,
                               void* scratch, int B, int T, int C, void* stream) {
@@ -625,12 +638,12 @@ LLMK_API int llmk_encoder_bwd(void* dwte, void* dwpe, const void* dout, const vo
     int threads = C / 8;
     if (threads > 256) threads = 256;
     threads = ((threads + 31) / 32) * 32;
-    const int blocks = ceil_div(B * T, WTE_ROWS);
-    wte_bwd_kernel<<<blocks, threads, 0, (cudaStream_t)stream>>>((bf16*)dwte, (float*)scratch, (const bf16*)dout,
-                                                                 (const int*)sorted_tok, (const int*)sorted_pos, B * T, C);
+    const int rows = wte_rows(B * T), blocks = ceil_div(B * T, rows);
+    (blocks <= WTE_AHEAD_BLOCKS ? wte_bwd_kernel<true> : wte_bwd_kernel<false>)<<<blocks, threads, 0, (cudaStream_t)stream>>>(
+        (bf16*)dwte, (float*)scratch, (const bf16*)dout, (const int*)sorted_tok, (const int*)sorted_pos, B * T, C, rows);
     LLMK_LAUNCH_CHECK();
     wte_bwd_join_kernel<<<blocks, threads, 0, (cudaStream_t)stream>>>((bf16*)dwte, (const float*)scratch, (const int*)sorted_tok,
-                                                                      B * T, C);
+                                                                      B * T, C, rows);
     LLMK_LAUNCH_CHECK();
     return LLMK_OK;
 }

@@ -331,7 +331,10 @@ def test_dbias_and_encoder():
 
 
 @pytest.mark.parametrize("B,T,C,V,kind", [(1, 64, 768, 50, "same"), (3, 64, 64, 9, "few"), (2, 1024, 768, 50304, "zipf"),
-                                          (1, 64, 2056, 1000, "distinct"), (33, 64, 768, 3, "few"), (9, 1024, 128, 1, "same")])
+                                          (1, 64, 2056, 1000, "distinct"), (33, 64, 768, 3, "few"), (9, 1024, 128, 1, "same"),
+                                          (1, 8, 64, 50, "distinct"), (1, 7, 64, 3, "few"), (16, 64, 384, 50304, "zipf"),
+                                          (1, 1025, 384, 700, "few"), (4, 1024, 384, 50304, "zipf"), (1, 4097, 256, 50304, "distinct"),
+                                          (33, 1024, 256, 50304, "zipf"), (33, 1024, 64, 5, "few")])
 def test_embedding_gradient_of_runs_that_cross_block_edges(B, T, C, V, kind):
     """Runs of one token that end at, cross, or cover whole blocks of sorted positions, against fp64 sums."""
     from llm_kittens_b200.ops import elementwise as ew
