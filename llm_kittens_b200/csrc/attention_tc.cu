@@ -2,8 +2,8 @@
 // TMEM), for MHA and GQA, reading the packed QKV activation [B*T, (NH+2*NKVH)*HS] through one TMA
 // tensor map and writing O as [B*T, NH*HS] plus the log-sum-exp. Same job as attention_forward /
 // attention_gqa_forward of the reference (llmc/attention.cuh:261-338, llmc/attention_gqa.cuh:415-481),
-// which has no sm_100 path; the warp-level implementation in attention.cu remains as the fallback for
-// sequence lengths that are not a multiple of 128.
+// which has no sm_100 path; the warp-level implementation in attention.cu remains for short sequences and
+// small calls whose length is not a multiple of 128 (ops/attention.py has the rule).
 //
 // One CTA per (128 query rows, head, batch); 6 warps:
 //   warp 0     TMA producer: Q once, then K/V tiles of 128 rows through a 2-stage ring

@@ -15,18 +15,44 @@ IMPL = os.environ.get("LLMK_ATTENTION", "tc")
 
 def _tc_length(T: int) -> bool:
     """Whether the tcgen05 kernels take sequences of this length. They work on 128-row tiles; a ragged last tile costs them
-    half a tile, which the warp-level kernels (64-row tiles) undercut only when it is most of the sequence: forward and
-    backward in us at B7 T448 12 heads of 64 18 + 38 against 20 + 59, at B1 T320 32/8 heads 10 + 44 against 9 + 50 and with
-    heads of 128 13 + 57 against 13 + 91, but at B64 T192 12 heads 50 + 98 against 32 + 104 and at B32 T64 20 + 24 against
-    5 + 17."""
+    half a tile, which the warp-level kernels (64-row tiles) undercut in the backward pass only when it is most of the
+    sequence: us at B7 T448 12 heads of 64 38 against 59, at B1 T320 32/8 heads 37 against 50 and with heads of 128 57 against
+    91, but at B64 T192 12 heads 98 against 104 with 50 against 32 in front of it, and at B32 T64 24 against 17."""
     return T % 128 == 0 or (T % 64 == 0 and T > 256)
 
 
+_SMS: dict[int, int] = {}
+
+
+def _sms() -> int:
+    dev = torch._C._cuda_getDevice()
+    if dev not in _SMS:
+        _SMS[dev] = int(N.lib().llmk_num_sms())
+    return _SMS[dev]
+
+
+def _tc_forward(B: int, T: int, NH: int, HS: int) -> bool:
+    """Whether the forward of these sequences is faster on the tcgen05 kernels. Lengths that are multiples of 128 always are.
+    With a ragged last tile and heads of 64 the time of a launch that the chip holds at once is that of its longest tile,
+    2.07 us per 128 keys on the warp-level kernel and 2.25 on the other, on top of 2.5 and 3.4; with more tiles than that
+    their throughput decides. us, warp level / tcgen05: B1 T320 12 heads 7.7 / 10.2, B2 T320 25 heads 9.8 / 10.2 and 32 heads
+    11.3 / 10.4, B7 T448 6 heads 12.3 / 13.9 and 12 heads 20.5 / 17.6, B2 T576 6 heads 12.1 / 13.6 and 12 heads 15.2 / 13.6, B1 T1088
+    6 heads 20.1 / 22.3 and 12 heads 25.4 / 22.5. Heads of 128 have one 128-row tile per SM, of which sequences under 512
+    fill half to 60 %: one wave of them is ahead (B1 T320 32 heads 13.7 / 12.3), more are not (B2 17.6 / 21.0, B7 T448 16 heads
+    40 / 47); from 512 on they are (B2 T576 32 heads 39.5 / 35.5, B1 T1088 63 / 35)."""
+    if T % 128 == 0 or not _tc_length(T):
+        return T % 128 == 0
+    if HS == 64:
+        return (T // 64) * B * NH > (2 if T <= 448 else 1) * _sms()
+    return T >= 512 or (T + 127) // 128 * B * NH <= _sms()
+
+
 def attention_fwd(qkv, B, T, NH, NKVH, HS, out=None, lse=None, impl=None):
-    """``qkv``: [B, T, (NH+2*NKVH)*HS] -> ``out`` [B, T, NH*HS], ``lse`` [B, NH, T] fp32."""
+    """``qkv``: [B, T, (NH+2*NKVH)*HS] -> ``out`` [B, T, NH*HS], ``lse`` [B, NH, T] fp32. ``impl`` "warp" / "tc" asks for the
+    warp-level kernels / for the tcgen05 kernels wherever they take the length; both leave what either backward needs."""
     out = torch.empty(B, T, NH * HS, dtype=qkv.dtype, device=qkv.device) if out is None else out
     lse = torch.empty(B, NH, T, dtype=torch.float32, device=qkv.device) if lse is None else lse
-    if (impl or IMPL) == "tc" and _tc_length(T):
+    if _tc_length(T) if impl == "tc" else (impl or IMPL) == "tc" and _tc_forward(B, T, NH, HS):
         N.call("llmk_attention_fwd_tc", out, lse, qkv, B, T, NH, NKVH, HS, N.status_word())
     else:
         N.call("llmk_attention_fwd", out, lse, qkv, B, T, NH, NKVH, HS)
@@ -34,7 +60,7 @@ def attention_fwd(qkv, B, T, NH, NKVH, HS, out=None, lse=None, impl=None):
 
 
 def fused_rope_available(T: int) -> bool:
-    """Whether the tcgen05 kernels run for this sequence length, i.e. whether RoPE can live in the QKV GEMM's epilogue
+    """Whether the tcgen05 backward runs for this sequence length, i.e. whether RoPE can live in the QKV GEMM's epilogue
     and its backward in the output tiles of the attention backward kernels."""
     return IMPL == "tc" and _tc_length(T)
 

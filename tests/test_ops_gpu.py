@@ -415,7 +415,7 @@ def test_attention_fwd_bwd(B, T, NH, NKVH, HS):
 
     qkv = rnd(B, T, (NH + 2 * NKVH) * HS)
     out_w, lse_w = attention.attention_fwd(qkv, B, T, NH, NKVH, HS, impl="warp")
-    out, lse = attention.attention_fwd(qkv, B, T, NH, NKVH, HS, impl="tc")   # tcgen05 path when T % 128 == 0
+    out, lse = attention.attention_fwd(qkv, B, T, NH, NKVH, HS, impl="tc")   # the tcgen05 kernels where they take the length
     _native.check_status()
     assert maxerr(out, out_w) < 0.03 and maxerr(lse, lse_w) < 0.02
     qf = qkv.float().requires_grad_(True)
@@ -433,13 +433,14 @@ def test_attention_fwd_bwd(B, T, NH, NKVH, HS):
     assert torch.equal(dqkv, dqkv2)
 
 
-@pytest.mark.parametrize("dkv", ["1", "2"])
+@pytest.mark.parametrize("dkv,impl", [("1", "tc"), ("2", "tc"), ("2", None)])
 @pytest.mark.parametrize("B,T,NH,NKVH,HS", [(2, 320, 4, 2, 64), (3, 448, 2, 2, 64), (2, 320, 4, 1, 128), (2, 576, 2, 2, 128),
                                             (1, 1088, 4, 1, 64), (73, 1088, 5, 5, 64)])
-def test_attention_of_lengths_that_are_not_whole_tiles(B, T, NH, NKVH, HS, dkv, monkeypatch):
+def test_attention_of_lengths_that_are_not_whole_tiles(B, T, NH, NKVH, HS, dkv, impl, monkeypatch):
     """A ragged last tile reads nothing of the next sequence (which is all infinities here) and writes nothing behind its
     own; output, log-sum-exp and gradients against fp64, with both dK / dV kernels (one query head per key head makes the
-    number of sub-tiles odd). The last case has more heads than one group of the tile order."""
+    number of sub-tiles odd), after the tcgen05 forward and after the one that the size of the call picks. The last case has
+    more heads than one group of the tile order."""
     from llm_kittens_b200.ops import attention as attn
 
     monkeypatch.setenv("LLMK_ATTN_BWD_DKV", dkv)
@@ -451,7 +452,7 @@ def test_attention_of_lengths_that_are_not_whole_tiles(B, T, NH, NKVH, HS, dkv, 
         qkv.view(-1)[T * W:2 * T * W] = float("inf")         # sequence 1
     out, dqkv = torch.full((n + 64, NH * HS), 7.0, device="cuda", dtype=BF), torch.full((n + 64, W), 7.0, device="cuda", dtype=BF)
     lse, dvec = torch.full((B * NH * T + 64,), 7.0, device="cuda"), torch.empty(B, NH, T, device="cuda")
-    attn.attention_fwd(qkv[:n].view(B, T, W), B, T, NH, NKVH, HS, out=out[:n], lse=lse)
+    attn.attention_fwd(qkv[:n].view(B, T, W), B, T, NH, NKVH, HS, out=out[:n], lse=lse, impl=impl)
     attn.attention_bwd(dout[:n], qkv[:n], out[:n], lse, B, T, NH, NKVH, HS, dqkv=dqkv[:n], dvec=dvec)
     assert (out[n:] == 7).all() and (dqkv[n:] == 7).all() and (lse[B * NH * T:] == 7).all()
     for b in ([0] + list(range(2, B)) if small else [0, 36, 72]):
@@ -473,8 +474,8 @@ def test_attention_of_lengths_that_are_not_whole_tiles(B, T, NH, NKVH, HS, dkv, 
                                                   (1, 4096, 32, 8, 128, 1.0), (1, 1024, 12, 12, 64, 3.0), (1, 2048, 8, 2, 128, 3.0)])
 def test_attention_long_sequences(B, T, NH, NKVH, HS, scale, dkv, monkeypatch):
     """The sequence lengths of the training configurations: many key tiles per query tile (the K/V ring wraps
-    around), grouped queries long enough for the pipelined dK/dV kernel (chosen by itself for (T/64)*(NH/NKVH) >= 64,
-    forced both ways through LLMK_ATTN_BWD_DKV), and inputs scaled so that logits reach +-30 and the row maximum
+    around), grouped queries, the pipelined and the plain dK/dV kernel (by the launcher's own choice, and each of them
+    through LLMK_ATTN_BWD_DKV), and inputs scaled so that logits reach +-30 and the row maximum
     jumps by more than 2^8 between key tiles (the lazy rescale of the output accumulator fires)."""
     from llm_kittens_b200.ops import _native, attention
 

@@ -5,7 +5,7 @@ import torch
 
 from llm_kittens_b200.models.config import ModelConfig
 from llm_kittens_b200.models.transformer import Transformer
-from llm_kittens_b200.ops import _native, elementwise, gemm
+from llm_kittens_b200.ops import _native, attention, elementwise, gemm
 
 
 class _Lib:
@@ -25,6 +25,7 @@ def calls(monkeypatch):
     monkeypatch.setattr(_native, "status_word", lambda: None)
     monkeypatch.setattr(_native, "scratch_buffer", lambda pool, nbytes, min_bytes, name: torch.empty(16, dtype=torch.uint8))
     monkeypatch.setattr(gemm, "tile_rows", lambda: 256)
+    monkeypatch.setattr(attention, "_sms", lambda: 148)
     return out
 
 
@@ -104,3 +105,17 @@ def test_zeroing_a_tensor_of_another_device_is_left_to_pytorch(calls, monkeypatc
     t = Tensor()
     assert elementwise.zero_(t) is t
     assert (t.zeroed, [name for name, _ in calls]) == ((False, ["llmk_zero"]) if native else (True, []))
+
+
+@pytest.mark.parametrize("B,T,NH,HS,tc", [(1, 64, 12, 64, False), (64, 192, 12, 64, False), (1, 128, 1, 128, True), (1, 320, 12, 64, False),
+                                          (2, 320, 32, 64, True), (7, 448, 6, 64, False), (7, 448, 12, 64, True), (2, 576, 6, 64, False),
+                                          (2, 576, 12, 64, True), (1, 320, 32, 128, True), (2, 320, 32, 128, False),
+                                          (7, 448, 16, 128, False), (2, 576, 32, 128, True)])
+def test_forward_attention_kernel_by_size(calls, monkeypatch, B, T, NH, HS, tc):
+    """Which kernel a forward takes on a GPU of 148 SMs, and that asking for one gets it where it takes the length."""
+    monkeypatch.setattr(attention, "IMPL", "tc")
+    qkv = torch.empty(B, T, 3 * NH * HS, dtype=torch.bfloat16)
+    for impl in (None, "tc", "warp"):
+        attention.attention_fwd(qkv, B, T, NH, NH, HS, impl=impl)
+    name = lambda on: "llmk_attention_fwd_tc" if on else "llmk_attention_fwd"
+    assert [c[0] for c in calls] == [name(tc), name(T % 128 == 0 or T > 256), name(False)]
