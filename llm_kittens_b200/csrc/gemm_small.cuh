@@ -1,14 +1,21 @@
 // The GEMM of few tiles (included by gemm_tcgen05.cu): outputs too small to give every SM a 256 x 256 tile.
 //
 // One CTA per 128 x BN tile (BN = 64 or 128) and slice of K: a cluster of S CTAs shares a tile, CTA r takes the k-blocks
-// [r * kb / S, (r + 1) * kb / S). Not persistent: warp 0 fills a TMA ring, warp 1 issues the MMAs, then all eight warps
-// move the accumulator from TMEM to shared memory as fp32, and after a cluster barrier CTA r sums rows
-// [r * 128 / S, (r + 1) * 128 / S) over the cluster's S copies, in the order of the slices, through distributed shared
-// memory and applies the epilogue: no partials in global memory, no second launch, the same bits from run to run.
+// [r * kb / S, (r + 1) * kb / S). Not persistent: one thread fills a TMA ring, one issues the MMAs, then all eight warps
+// move the accumulator from TMEM to shared memory as fp32, each CTA sends every other one its share of the tile's rows by
+// a bulk copy into that CTA's shared memory, and each sums its rows over the cluster, in the order of the slices, and
+// applies the epilogue: no partials in global memory, no second launch, the same bits from run to run.
 //
 // What bounds it: a CTA pair's 256 x 256 tile costs 0.3 us of tensor-core time per 64-wide k-block however few of its
 // rows exist, 16 us for K = 3072 on one pair of SMs while 70 pairs have nothing to do. Here a k-block is 24 (32) KiB of
-// operands for 128 x 64 (128 x 128) outputs, bound by what one SM draws from the L2, and S SMs share the k-blocks of a tile.
+// operands for 128 x 64 (128 x 128) outputs, bound by what one SM draws from the L2 (0.14 / 0.19 us), and S SMs share the
+// k-blocks of a tile. With few k-blocks it is a chain of latencies, some 4 us of which the loop is a quarter. What was
+// taken out of that chain (us before / after, weights from HBM): the first loads are issued before the block is set up, no
+// division in front of them, bias, addend and status word are fetched beside them; rows travel as bulk copies that an
+// mbarrier counts (loads from the other CTAs' shared memory between two cluster barriers: 1.2 us more, and a barrier that
+// releases global stores 1 us); little code, since every line of it is fetched anew: NT 64 x 768 x 768 with bias and addend
+// 7.2 / 5.1, 64 x 768 x 3072 8.5 / 6.6, 256 x 3072 x 768 with GELU 9.0 / 6.2, NN 256 x 3072 x 768 with GELU' 7.6 / 5.9, TN 3072 x
+// 768 x 256 with bias gradient 9.2 / 7.0, 768 x 768 x 256 7.3 / 5.2.
 //
 // The bias gradient (mode TN) comes from the tensor core as well: in the CTAs of the first tile column one more MMA of
 // 16 columns multiplies the A stage by a tile of ones, and the column sums arrive in TMEM behind the accumulator, as exact
@@ -18,27 +25,30 @@ namespace small {
 constexpr int THREADS = 256;
 constexpr int MAX_STAGES = 8;
 constexpr int ONES_BYTES = 2048;                 // 16 rows x 64 bf16 ones (EPI_DBIAS)
-constexpr int MAX_SMEM = 200 * 1024;
+constexpr int MAX_SMEM = 227 * 1024;
 template <int BN> struct SGeo {
     static constexpr int STAGE_BYTES = A_STAGE_BYTES + BN * BK * 2;   // 24 / 32 KiB
     static constexpr int LD = BN + 4;            // fp32 row of the accumulator in shared memory; column BN holds the bias sum
     static constexpr int ACC_BYTES = BM * LD * 4;
     static constexpr int STAGES = BN == 64 ? 8 : 6;
+    static constexpr int STAGES_APART = BN == 64 ? 7 : 4;             // with a place of their own for the other CTAs' rows
+    static_assert(STAGES_APART * STAGE_BYTES + ACC_BYTES + ONES_BYTES + 1280 <= MAX_SMEM && STAGES <= MAX_STAGES, "shared memory");
+    static_assert(STAGES * STAGE_BYTES >= 2 * ACC_BYTES, "both over the ring");
     static_assert(ACC_BYTES % 1024 == 0, "the tile of ones behind the accumulator is 1024-byte aligned");
 };
 // A CTA asks for at least its share of shared memory (228 KiB per 512 TMEM columns), so that however many of these CTAs,
 // of whatever instantiation and stream, an SM takes, their columns never add up to more than it has: no CTA waits in
 // tcgen05.alloc for one that waits at a cluster barrier for it.
-static inline int smem_bytes(int stage_bytes, int acc_bytes, int stages, int tmem_cols) {
-    const int ring = stages * stage_bytes;
-    const int need = (ring > acc_bytes ? ring : acc_bytes) + ONES_BYTES + 1024 /*alignment slack*/ + 256 /*barriers*/;
+static inline int smem_bytes(int used, int tmem_cols) {
+    const int need = used + ONES_BYTES + 1024 /*alignment slack*/ + 256 /*barriers*/;
     return need > tmem_cols * 460 ? need : tmem_cols * 460;
 }
 __host__ __device__ constexpr int tmem_cols(int bn, bool db) { return bn + (db ? 16 : 0) <= 64 ? 64 : (bn + (db ? 16 : 0) <= 128 ? 128 : 256); }
 
 struct SParams {
     int M, N, K;               // N counts columns of the accumulator space (EPI_SWIGLU: up and gate, 2 H)
-    int tiles_n, kb_total, S, stages;
+    int kb_total, log_s, stages;   // 1 << log_s CTAs share a tile
+    int over, red_off, ones_off;   // where in shared memory the other CTAs' rows (over: on the ring) and the tile of ones are
     const bf16* bias;
     const bf16* aux;
     bf16* C;
@@ -53,19 +63,21 @@ struct SParams {
     int* status;
 };
 
-__device__ __forceinline__ float4 ld_cluster_f4(uint32_t local, uint32_t cta) {
-    float4 v;
+// `bytes` of this CTA's shared memory to a place in the shared memory of CTA `cta` of the cluster, counted by the barrier there.
+__device__ __forceinline__ void send_bulk(uint32_t local_dst, uint32_t local_src, uint32_t bytes, uint32_t local_bar, uint32_t cta) {
     asm volatile(
-        "{\n\t.reg .b32 remAddr32;\n\t"
-        "mapa.shared::cluster.u32 remAddr32, %4, %5;\n\t"
-        "ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [remAddr32];\n\t}"
-        : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
-        : "r"(local), "r"(cta)
+        "{\n\t.reg .b32 dst, bar;\n\t"
+        "mapa.shared::cluster.u32 dst, %0, %4;\n\t"
+        "mapa.shared::cluster.u32 bar, %3, %4;\n\t"
+        "cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [dst], [%1], %2, [bar];\n\t}" ::"r"(local_dst),
+        "r"(local_src), "r"(bytes), "r"(local_bar), "r"(cta)
         : "memory");
-    return v;
 }
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 
-template <int MODE, int EPI, int BN>
+// CL: a cluster of 2, 4 or 8 CTAs per tile (else one CTA).
+template <int MODE, int EPI, int BN, bool CL>
 __global__ void __launch_bounds__(THREADS, 1)
 gemm_small_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                   const __grid_constant__ CUtensorMap tmB2, const SParams p) {
@@ -76,35 +88,66 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
 
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    uint8_t* ones = smem + max(p.stages * G::STAGE_BYTES, G::ACC_BYTES);
+    // The accumulator goes to shared memory over the ring (every load has landed and every MMA has read it once it is
+    // complete); the rows of other CTAs arrive behind the ring, so that those may send while this CTA still multiplies, or
+    // where a deep ring leaves no room for that, over the ring too, once no CTA uses its ring any more.
+    float* acc_s = reinterpret_cast<float*>(smem);
+    float* red = reinterpret_cast<float*>(smem + p.red_off);
+    uint8_t* ones = smem + p.ones_off;
     uint64_t* full_bar = reinterpret_cast<uint64_t*>(ones + ONES_BYTES);
     uint64_t* empty_bar = full_bar + MAX_STAGES;
     uint64_t* acc_full = empty_bar + MAX_STAGES;
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_full + 1);
+    uint64_t* red_full = acc_full + 1;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(red_full + 1);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-    int* skip_word = reinterpret_cast<int*>(tmem_slot + 2);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int S = p.S;
-    const int rank = S > 1 ? (int)ptx::cluster_ctarank() : 0;
-    const int tile = blockIdx.x / S;
-    const int m0 = (tile / p.tiles_n) * BM, n0 = (tile % p.tiles_n) * BN;
-    const int kb0 = (int)((long long)p.kb_total * rank / S), kb1 = (int)((long long)p.kb_total * (rank + 1) / S);
+    const int S = CL ? 1 << p.log_s : 1;
+    const int rank = CL ? (int)ptx::cluster_ctarank() : 0;
+    const int m0 = blockIdx.y * BM, n0 = (CL ? blockIdx.x >> p.log_s : blockIdx.x) * BN;
+    const int tile = blockIdx.y * gridDim.x + blockIdx.x;   // (for reports)
+    const int kb0 = CL ? (p.kb_total * rank) >> p.log_s : 0, kb1 = CL ? (p.kb_total * (rank + 1)) >> p.log_s : p.kb_total;
     const bool sums = DB && n0 == 0;
+    // the rows of the tile that exist are dealt out to the CTAs of the cluster, which sum and finish them
+    const int m_rows = min(BM, p.M - m0);
+    const int rows = CL ? (m_rows + S - 1) >> p.log_s : m_rows, r0 = rank * rows, my_rows = max(0, min(rows, m_rows - r0));
 
+    auto load_stage = [&](int kb, int s) {
+        uint8_t* sA = smem + s * G::STAGE_BYTES;
+        uint8_t* sB = sA + A_STAGE_BYTES;
+        ptx::mbar_arrive_expect_tx(&full_bar[s], G::STAGE_BYTES);
+        const int k0 = kb * BK;
+        if (B_MN) {
+#pragma unroll
+            for (int j = 0; j < BN / 64; j++) ptx::tma_load_2d(sB + j * CHUNK_BYTES, &tmB, &full_bar[s], n0 + 64 * j, k0);
+        } else if (SWI) {   // BN / 2 hidden units of up, then the same of gate
+            ptx::tma_load_2d(sB, &tmB, &full_bar[s], k0, n0 / 2);
+            ptx::tma_load_2d(sB + BN * BK, &tmB2, &full_bar[s], k0, n0 / 2);
+        } else {
+            ptx::tma_load_2d(sB, &tmB, &full_bar[s], k0, n0);
+        }
+        if (A_MN) {
+#pragma unroll
+            for (int j = 0; j < BM / 64; j++) ptx::tma_load_2d(sA + j * CHUNK_BYTES, &tmA, &full_bar[s], m0 + 64 * j, k0);
+        } else {
+            ptx::tma_load_2d(sA, &tmA, &full_bar[s], k0, m0);
+        }
+    };
+    const int first = min(p.stages, kb1 - kb0);
     if (threadIdx.x == 0) {
-        // a failure already recorded makes the kernel skip its work (the cluster barriers below are reached all the same)
-        *skip_word = (p.status != nullptr && *reinterpret_cast<volatile int*>(p.status) != 0) ? 1 : 0;
+        // the first loads need the barriers and nothing else: they are on their way while the block sets itself up
         for (int i = 0; i < p.stages; i++) {
             ptx::mbar_init(&full_bar[i], 1);
             ptx::mbar_init(&empty_bar[i], 1);
         }
         ptx::mbar_init(acc_full, 1);
+        if (CL) ptx::mbar_init(red_full, 1);
         *abort_flag = 0;
         ptx::fence_barrier_init();
-        ptx::prefetch_tmap(&tmA);
-        ptx::prefetch_tmap(&tmB);
+        for (int i = 0; i < first; i++) load_stage(kb0 + i, i);
+        if (CL) ptx::mbar_arrive_expect_tx(red_full, (S - 1) * my_rows * G::LD * 4);
     }
+    __syncwarp();
     if (warp == 1) {
         ptx::tmem_alloc(tmem_slot, TMEM_ALLOC);
         ptx::tmem_relinquish();
@@ -114,42 +157,51 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
         reinterpret_cast<uint4*>(ones)[threadIdx.x - 128] = make_uint4(0x3f803f80u, 0x3f803f80u, 0x3f803f80u, 0x3f803f80u);
         ptx::fence_proxy_async_smem();
     }
+    // Everything the epilogue reads from memory is fetched now, beside the operands: fetched in the epilogue, the addend of
+    // a 124M model's 256-token weight gradients cost 3 us a call and a bias that no cache holds 0.8. A failure already
+    // recorded makes the kernel leave its outputs alone.
+    const int failed = p.status != nullptr ? *reinterpret_cast<volatile int*>(p.status) : 0;
+    constexpr int VECS = SWI ? BN / 16 : BN / 8;   // groups of 8 output columns per row
+    constexpr bool AUX_IN = (EPI & (EPI_DGELU | EPI_ADD | EPI_DROW)) != 0, ROPE = (EPI & EPI_ROPE) != 0;
+    constexpr int MAX_IT = (CL ? BM / 2 : BM) * VECS / THREADS;
+    static_assert(THREADS % VECS == 0, "a thread keeps its columns");
+    const int c = (threadIdx.x % VECS) * 8, n = n0 + c;
+    const bool col_in = SWI ? n0 / 2 + c < p.N / 2 : n < p.N;
+    bf16x8 aux_v[AUX_IN ? MAX_IT : 1], bias_v;
+    float4 rope_v[ROPE ? 2 * MAX_IT : 1];
+    float db_old = 0.f;
+    if ((EPI & EPI_BIAS) && col_in) bias_v = ld128(p.bias + n);
+#pragma unroll
+    for (int it = 0; it < MAX_IT; it++) {
+        const int lr = (threadIdx.x + it * THREADS) / VECS, m = m0 + r0 + lr;
+        if (lr < my_rows && col_in) {
+            if (AUX_IN) aux_v[AUX_IN ? it : 0] = ld128(p.aux + (size_t)m * p.N + n);
+            if (ROPE && n < p.rope_cols) {
+                const float4* fr = reinterpret_cast<const float4*>(p.rope + (size_t)(m % p.rope_T) * (p.rope_hs >> 1) + ((n % p.rope_hs) >> 1));
+                rope_v[ROPE ? 2 * it : 0] = __ldg(fr);
+                rope_v[ROPE ? 2 * it + 1 : 0] = __ldg(fr + 1);
+            }
+        }
+    }
+    if (DB && sums && p.dbias_add && (int)threadIdx.x < my_rows) db_old = __bfloat162float(p.dbias[m0 + r0 + threadIdx.x]);
     ptx::tc_fence_before();
     __syncthreads();
     ptx::tc_fence_after();
+    if (CL && !p.over) cluster_arrive();   // waited for before the first copy into another CTA's shared memory
     const uint32_t tmem_base = *tmem_slot;
-    const bool skip = *skip_word != 0;
 
     // Producer and issuer are one thread each: a warp that waits and then branches to one lane per k-block spends more
     // cycles on that than the tensor core on a 128 x 64 x 64 product (0.28 us per k-block that way, 0.14 this way).
-    if (!skip && warp == 0 && ptx::elect_one()) {
-        // ------------------------------------------------------------ TMA producer
+    if (warp == 0 && ptx::elect_one()) {
+        // ------------------------------------------------------------ TMA producer (the rest of the k-blocks)
         int s = 0;
         uint32_t ph = 0;
-        for (int kb = kb0; kb < kb1; kb++) {
-            if (!ptx::mbar_wait(&empty_bar[s], ph ^ 1, abort_flag, p.status, LLMK_ST_TIMEOUT_TMA_EMPTY, tile)) break;
-            uint8_t* sA = smem + s * G::STAGE_BYTES;
-            uint8_t* sB = sA + A_STAGE_BYTES;
-            ptx::mbar_arrive_expect_tx(&full_bar[s], G::STAGE_BYTES);
-            const int k0 = kb * BK;
-            if (A_MN) {
-#pragma unroll
-                for (int j = 0; j < BM / 64; j++) ptx::tma_load_2d(sA + j * CHUNK_BYTES, &tmA, &full_bar[s], m0 + 64 * j, k0);
-            } else {
-                ptx::tma_load_2d(sA, &tmA, &full_bar[s], k0, m0);
-            }
-            if (B_MN) {
-#pragma unroll
-                for (int j = 0; j < BN / 64; j++) ptx::tma_load_2d(sB + j * CHUNK_BYTES, &tmB, &full_bar[s], n0 + 64 * j, k0);
-            } else if (SWI) {   // BN / 2 hidden units of up, then the same of gate
-                ptx::tma_load_2d(sB, &tmB, &full_bar[s], k0, n0 / 2);
-                ptx::tma_load_2d(sB + BN * BK, &tmB2, &full_bar[s], k0, n0 / 2);
-            } else {
-                ptx::tma_load_2d(sB, &tmB, &full_bar[s], k0, n0);
-            }
+        for (int kb = kb0 + first; kb < kb1; kb++) {
+            if (!ptx::mbar_wait(&empty_bar[s], ph, abort_flag, p.status, LLMK_ST_TIMEOUT_TMA_EMPTY, tile)) break;
+            load_stage(kb, s);
             if (++s == p.stages) { s = 0; ph ^= 1; }
         }
-    } else if (!skip && warp == 1 && ptx::elect_one()) {
+    } else if (warp == 1 && ptx::elect_one()) {
         // ------------------------------------------------------------ MMA issuer
         constexpr uint32_t idesc = ptx::make_idesc_bf16(BM, BN, A_MN ? 1 : 0, B_MN ? 1 : 0);
         constexpr uint32_t idesc1 = ptx::make_idesc_bf16(BM, 16, A_MN ? 1 : 0, 0);
@@ -159,10 +211,10 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
         const uint64_t one_desc = ptx::make_smem_desc(ptx::smem_u32(ones), 16, 1024);
         int s = 0;
         uint32_t ph = 0;
-        bool ok = true;
+        bool issued = true;
         for (int kb = kb0; kb < kb1; kb++) {
-            ok = ptx::mbar_wait_spin(&full_bar[s], ph, abort_flag, p.status, LLMK_ST_TIMEOUT_TMA_FULL, tile);
-            if (!ok) break;
+            issued = ptx::mbar_wait_spin(&full_bar[s], ph, abort_flag, p.status, LLMK_ST_TIMEOUT_TMA_FULL, tile);
+            if (!issued) break;
             ptx::tc_fence_after();
             const uint64_t ad = a_desc0 + (uint64_t)(s * (G::STAGE_BYTES >> 4));
             const uint64_t bd = b_desc0 + (uint64_t)(s * (G::STAGE_BYTES >> 4));
@@ -177,43 +229,30 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
             ptx::mma_commit(&empty_bar[s]);
             if (++s == p.stages) { s = 0; ph ^= 1; }
         }
-        if (ok) ptx::mma_commit(acc_full);
+        if (issued) ptx::mma_commit(acc_full);
     }
     __syncwarp();
-    const int rows = BM / S, r0 = rank * rows;
-    constexpr int VECS = SWI ? BN / 16 : BN / 8;   // groups of 8 output columns per row
-    // the addend / GELU input / O of this thread's outputs is on its way from HBM while the products are formed (fetched
-    // in the epilogue, the gradients of a 124M model's 256-token weight GEMMs cost 3 us each)
-    constexpr bool AUX_IN = (EPI & (EPI_DGELU | EPI_ADD | EPI_DROW)) != 0;
-    constexpr int MAX_IT = BM * VECS / THREADS;
-    bf16x8 aux_v[AUX_IN ? MAX_IT : 1];
-    if (AUX_IN && !skip) {
-#pragma unroll
-        for (int it = 0; it < MAX_IT; it++) {
-            const int i = threadIdx.x + it * THREADS, r = r0 + i / VECS, c = (i % VECS) * 8;
-            if (i < rows * VECS && m0 + r < p.M && n0 + c < p.N) aux_v[AUX_IN ? it : 0] = ld128(p.aux + (size_t)(m0 + r) * p.N + n0 + c);
-        }
+    // ---------------------------------------------------------------- accumulator -> shared memory
+    bool ok = ptx::mbar_wait(acc_full, 0, abort_flag, p.status, LLMK_ST_TIMEOUT_ACC_FULL, tile);
+    __syncwarp();
+    if (CL) {   // every CTA of the cluster has set up its barriers, and where rows arrive over the ring is done with that
+        if (p.over) cluster_arrive();
+        cluster_wait();
     }
-    // ---------------------------------------------------------------- accumulator -> shared memory (over the ring: every
-    // load has landed and every MMA has read it once the accumulator is complete)
-    bool ok = !skip;
-    if (ok) ok = ptx::mbar_wait(acc_full, 0, abort_flag, p.status, LLMK_ST_TIMEOUT_ACC_FULL, tile);
-    float* acc_s = reinterpret_cast<float*>(smem);
-    if (ok) {
-        __syncwarp();
+    const int lane_group = warp & 3, half = warp >> 2;
+    if (ok && lane_group * 32 < m_rows) {
         ptx::tc_fence_after();
-        const int lane_group = warp & 3, half = warp >> 2;
         float* row = acc_s + (lane_group * 32 + lane) * G::LD;
         const uint32_t t_row = tmem_base + ((uint32_t)(lane_group * 32) << 16);
 #pragma unroll
-        for (int c = half * (BN / 2); c < (half + 1) * (BN / 2); c += 32) {
+        for (int col = half * (BN / 2); col < (half + 1) * (BN / 2); col += 32) {
             uint32_t v[32];
-            ptx::tmem_ld_32x32b_x32(t_row + c, v);
+            ptx::tmem_ld_32x32b_x32(t_row + col, v);
             ptx::tmem_ld_wait();
 #pragma unroll
             for (int q = 0; q < 8; q++)
-                *reinterpret_cast<float4*>(row + c + 4 * q) = make_float4(__uint_as_float(v[4 * q]), __uint_as_float(v[4 * q + 1]),
-                                                                          __uint_as_float(v[4 * q + 2]), __uint_as_float(v[4 * q + 3]));
+                *reinterpret_cast<float4*>(row + col + 4 * q) = make_float4(__uint_as_float(v[4 * q]), __uint_as_float(v[4 * q + 1]),
+                                                                            __uint_as_float(v[4 * q + 2]), __uint_as_float(v[4 * q + 3]));
         }
         if (DB && sums && half == 0) {
             uint32_t v[32];
@@ -221,52 +260,63 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
             ptx::tmem_ld_wait();
             row[BN] = __uint_as_float(v[0]);
         }
-        ptx::tc_fence_before();
+        if (CL) ptx::fence_proxy_async_smem();
     }
-    if (!ok && !skip) {
+    if (!ok) {
         // a wait ran out: copies may still be on their way into this CTA's shared memory
         for (int i = 0; i < 1000; i++) __nanosleep(1000);
     }
+    ptx::tc_fence_before();
     __syncthreads();
-    if (S > 1) ptx::cluster_sync_all();
+    if (CL && warp == 0 && lane < S && lane != rank && ok) {
+        // lane d of the first warp sends the rows that CTA d finishes (place: this CTA's number among the others)
+        const int d_rows = max(0, min(rows, m_rows - lane * rows));
+        if (d_rows > 0)
+            send_bulk(ptx::smem_u32(red + (rank - (rank > lane)) * rows * G::LD), ptx::smem_u32(acc_s + lane * rows * G::LD),
+                      d_rows * G::LD * 4, ptx::smem_u32(red_full), lane);
+    }
+    __syncwarp();
     if (warp == 1) {
         ptx::tc_fence_after();
         ptx::tmem_dealloc(tmem_base, TMEM_ALLOC);
     }
-    // ---------------------------------------------------------------- sum over the cluster, epilogue
-    if (ok) {
-        auto load8 = [&](int r, int c, float* x) {
-            const uint32_t addr = ptx::smem_u32(acc_s + r * G::LD + c);
-            if (S == 1) {
-                const float4 a = *reinterpret_cast<const float4*>(acc_s + r * G::LD + c);
-                const float4 b = *reinterpret_cast<const float4*>(acc_s + r * G::LD + c + 4);
-                x[0] = a.x; x[1] = a.y; x[2] = a.z; x[3] = a.w; x[4] = b.x; x[5] = b.y; x[6] = b.z; x[7] = b.w;
-                return;
-            }
-#pragma unroll
-            for (int j = 0; j < 8; j++) x[j] = 0.f;
-#pragma unroll 4
-            for (int s = 0; s < S; s++) {
-                const float4 a = ld_cluster_f4(addr, s), b = ld_cluster_f4(addr + 16, s);
+    if (CL) {
+        if (ok) ok = ptx::mbar_wait(red_full, 0, abort_flag, p.status, LLMK_ST_TIMEOUT_ACC_FULL, tile);
+        __syncwarp();
+        cluster_arrive();   // what was sent to this CTA is here
+    }
+    // ---------------------------------------------------------------- sum over the cluster, in the order of the slices; epilogue
+    if (ok && !failed) {
+        auto slice = [&](int s) { return !CL || s == rank ? acc_s + r0 * G::LD : red + (s - (s > rank)) * rows * G::LD; };
+        auto load8 = [&](int lr, int col, float* x) {
+            const int off = lr * G::LD + col;
+            const float* src = slice(0) + off;
+            float4 a = *reinterpret_cast<const float4*>(src), b = *reinterpret_cast<const float4*>(src + 4);
+            x[0] = a.x; x[1] = a.y; x[2] = a.z; x[3] = a.w; x[4] = b.x; x[5] = b.y; x[6] = b.z; x[7] = b.w;
+            if (!CL) return;
+#pragma unroll 1
+            for (int s = 1; s < S; s++) {
+                src = slice(s) + off;
+                a = *reinterpret_cast<const float4*>(src);
+                b = *reinterpret_cast<const float4*>(src + 4);
                 x[0] += a.x; x[1] += a.y; x[2] += a.z; x[3] += a.w;
                 x[4] += b.x; x[5] += b.y; x[6] += b.z; x[7] += b.w;
             }
         };
 #pragma unroll
         for (int it = 0; it < MAX_IT; it++) {
-            const int i = threadIdx.x + it * THREADS;
-            if (i >= rows * VECS) break;
-            const int r = r0 + i / VECS, c = (i % VECS) * 8;
-            const int m = m0 + r;
-            const bool in = m < p.M && (SWI ? n0 / 2 + c < p.N / 2 : n0 + c < p.N);
+            const int lr = (threadIdx.x + it * THREADS) / VECS;
+            if (it * (THREADS / VECS) >= my_rows) break;   // (the same for every thread)
+            const int m = m0 + r0 + lr;
+            const bool in = lr < my_rows && col_in;
             // (EPI_DROW exchanges values between the eight lanes of a head: no lane leaves early)
             if (!(EPI & EPI_DROW) && !in) continue;
             float x[8];
-            load8(r, c, x);
+            load8(min(lr, my_rows - 1), c, x);
             if constexpr (SWI) {
                 const size_t off = (size_t)m * (p.N / 2) + n0 / 2 + c;
                 float g[8];
-                load8(r, c + BN / 2, g);
+                load8(lr, c + BN / 2, g);
                 const bf16x8 ub = pack8(x), gb = pack8(g);
                 unpack8(ub, x);
                 unpack8(gb, g);
@@ -277,17 +327,15 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
                 st128(p.C + off, pack8(g));
                 continue;
             }
-            const int n = n0 + c;
             const size_t off = (size_t)m * p.N + n;
             if (EPI & EPI_BIAS) {
                 float b[8];
-                unpack8(ld128(p.bias + n), b);
+                unpack8(bias_v, b);
 #pragma unroll
                 for (int j = 0; j < 8; j++) x[j] += b[j];
             }
-            if ((EPI & EPI_ROPE) && n < p.rope_cols) {
-                const float4* fr = reinterpret_cast<const float4*>(p.rope + (size_t)(m % p.rope_T) * (p.rope_hs >> 1) + ((n % p.rope_hs) >> 1));
-                const float4 f0 = __ldg(fr), f1 = __ldg(fr + 1);
+            if (ROPE && n < p.rope_cols) {
+                const float4 f0 = rope_v[ROPE ? 2 * it : 0], f1 = rope_v[ROPE ? 2 * it + 1 : 0];
                 const float cs[4] = {f0.x, f0.z, f1.x, f1.z}, sn[4] = {f0.y, f0.w, f1.y, f1.w};
 #pragma unroll
                 for (int j = 0; j < 4; j++) {
@@ -335,20 +383,14 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
             }
             st128(p.C + off, out);
         }
-        if (DB && sums && (int)threadIdx.x < rows && m0 + r0 + (int)threadIdx.x < p.M) {
-            const int r = r0 + threadIdx.x;
+        if (DB && sums && (int)threadIdx.x < my_rows) {
             float d = 0.f;
-            if (S == 1) {
-                d = acc_s[r * G::LD + BN];
-            } else {
-                for (int s = 0; s < S; s++) d += ld_cluster_f4(ptx::smem_u32(acc_s + r * G::LD + BN), s).x;
-            }
-            bf16* dst = p.dbias + m0 + r;
-            *dst = __float2bfloat16_rn(p.dbias_add ? __bfloat162float(*dst) + d : d);
+            for (int s = 0; s < S; s++) d += slice(s)[(int)threadIdx.x * G::LD + BN];
+            p.dbias[m0 + r0 + threadIdx.x] = __float2bfloat16_rn(p.dbias_add ? db_old + d : d);
         }
     }
     __syncwarp();
-    if (S > 1) ptx::cluster_sync_all();   // no CTA leaves while another still reads its shared memory
+    if (CL) cluster_wait();   // no CTA leaves before what it sent, and what is sent to it, has arrived
 }
 
 // Clusters of S blocks that the device keeps resident with one block per SM (GPCs are not whole multiples of S, so S times
@@ -357,7 +399,7 @@ static int resident_clusters(int S) {
     static PerDeviceInt known[4];
     int n = 0;
     const cudaError_t e = known[S == 1 ? 0 : (S == 2 ? 1 : (S == 4 ? 2 : 3))].get(&n, [S](int* v) {
-        const cudaError_t a = cudaFuncSetAttribute(gemm_small_kernel<MODE_NT, 0, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize, MAX_SMEM);
+        const cudaError_t a = cudaFuncSetAttribute(gemm_small_kernel<MODE_NT, 0, 64, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, MAX_SMEM);
         if (a != cudaSuccess) return a;
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(S);
@@ -370,7 +412,7 @@ static int resident_clusters(int S) {
         attr[0].val.clusterDim.z = 1;
         cfg.attrs = attr;
         cfg.numAttrs = 1;
-        return cudaOccupancyMaxActiveClusters(v, gemm_small_kernel<MODE_NT, 0, 64>, &cfg);
+        return cudaOccupancyMaxActiveClusters(v, gemm_small_kernel<MODE_NT, 0, 64, true>, &cfg);
     });
     if (e != cudaSuccess) {
         cudaGetLastError();
@@ -379,26 +421,26 @@ static int resident_clusters(int S) {
     return n;
 }
 
-template <int MODE, int EPI, int BN>
-static int launch(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmB2, const SParams& p, int tiles, cudaStream_t stream) {
+template <int MODE, int EPI, int BN, bool CL>
+static int launch(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmB2, const SParams& p, cudaStream_t stream) {
     using G = SGeo<BN>;
     static PerDeviceOnce once_configured;
     if (once_configured.first()) {
-        LLMK_CUDA_TRY(cudaFuncSetAttribute(gemm_small_kernel<MODE, EPI, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, MAX_SMEM));
+        LLMK_CUDA_TRY(cudaFuncSetAttribute(gemm_small_kernel<MODE, EPI, BN, CL>, cudaFuncAttributeMaxDynamicSharedMemorySize, MAX_SMEM));
     }
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(tiles * p.S);
+    cfg.gridDim = dim3(ceil_div(p.N, BN) << p.log_s, ceil_div(p.M, BM));
     cfg.blockDim = dim3(THREADS);
-    cfg.dynamicSmemBytes = smem_bytes(G::STAGE_BYTES, G::ACC_BYTES, p.stages, tmem_cols(BN, (EPI & EPI_DBIAS) != 0));
+    cfg.dynamicSmemBytes = smem_bytes(p.ones_off, tmem_cols(BN, (EPI & EPI_DBIAS) != 0));
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = p.S;
+    attr[0].val.clusterDim.x = 1 << p.log_s;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    LLMK_CUDA_TRY(cudaLaunchKernelEx(&cfg, gemm_small_kernel<MODE, EPI, BN>, tmA, tmB, tmB2, p));
+    cfg.numAttrs = CL ? 1 : 0;
+    LLMK_CUDA_TRY(cudaLaunchKernelEx(&cfg, gemm_small_kernel<MODE, EPI, BN, CL>, tmA, tmB, tmB2, p));
     return LLMK_OK;
 }
 

@@ -1147,14 +1147,15 @@ struct SmallPlan {
 };
 
 // Which kernel a product of few tiles takes: the persistent CTA-pair kernel (256 x 256 tiles) or the kernels of
-// gemm_small.cuh, by estimates in microseconds fitted to 51 shapes with weights read from HBM (64 to 4096 rows, K = 256 to
-// 65536). Per k-block: the pair kernel 0.28, and 0.12 more with every pair busy; a small tile `A` plus `B` times the share
-// of the SMs that have one (the L2 and HBM they share). TN pays for four boxes per k-block and the bias sums. The rest is
-// launch, first load and epilogue, which S > 1 adds an exchange to. The tiles' clusters must fit the chip at once: a second
-// wave of blocks that each fill and drain a pipeline costs more than it splits (1024 x 3072 x 768: 20 us in two waves,
-// pair kernel 14). Measured, pair kernel against the choice, us: NT 64 x 768 x 3072 21.7 / 7.5, 256 x 768 x 3072 22.5 / 9.1,
-// 320 x 2048 x 2048 18.9 / 12.7, 1024 x 768 x 768 11.9 / 6.9; NN 256 x 768 x 50304 226 / 35, 2048 x 1024 x 4096 26.1 / 18.8; TN
-// 768 x 768 x 3136 24.2 / 14.5.
+// gemm_small.cuh, by estimates in microseconds fitted to 520 timings of 150 products with weights read from HBM (64 to 3136
+// rows, K = 256 to 8192, every tile width and cluster size; 4 to 5 % rms). A small tile costs `A` per k-block, what one SM
+// draws from the L2 (24 or 32 KiB at some 75 bytes a cycle; four boxes and the bias sums in mode TN), plus `B` times the
+// share of the SMs that have one; the rest is launch, first load and epilogue, and for clusters the exchange of sums. The
+// tiles' clusters must fit the chip at once: a second wave of blocks that each fill and drain a pipeline costs more than it
+// splits (1024 x 3072 x 768: 15 us in two waves, pair kernel 13.3). Measured, pair kernel against the choice, us: NT 64 x 768
+// x 3072 23.0 / 6.6, 256 x 768 x 3072 23.3 / 8.2, 320 x 2048 x 2048 18.9 / 8.7, 1024 x 768 x 768 12.8 / 5.7, 1024 x 2048 x 8192
+// 48.4 / 29.8, 2048 x 1024 x 4096 28.2 / 16.7; NN 256 x 768 x 50304 226 / 31; TN 768 x 768 x 3136 23.3 / 11.6, 3072 x 768 x 3136
+// 24.5 / 19.4.
 static SmallPlan pick_small(int mode, int M, int N, int K, int num_sms, int pair_clusters) {
     SmallPlan plan = {0, 0};
     const int kb = ceil_div(K, BK);
@@ -1165,15 +1166,16 @@ static SmallPlan pick_small(int mode, int M, int N, int K, int num_sms, int pair
         best += 7.0;
     } else {
         const int units = ceil_div(M, 2 * BM) * ceil_div(N, BN), waves = ceil_div(units, pair_clusters);
-        best = waves * kb * (0.28 + 0.12 * units / ((double)waves * pair_clusters)) + (mode == MODE_NT ? 8.0 : 6.7);
+        best = waves * kb * (0.28 + 0.05 * units / ((double)waves * pair_clusters)) + (mode == MODE_NT ? 9.3 : 7.3);
     }
     best *= 0.95;   // not for a tie
+    const double m_share = (M < BM ? M : BM) / (double)BM;   // rows that a cluster exchanges
     for (int bn = 64; bn <= 128; bn *= 2) {
-        static const double A[3][2] = {{0.13, 0.15}, {0.115, 0.13}, {0.27, 0.34}}, B[3][2] = {{0.14, 0.30}, {0.08, 0.09}, {0.08, 0.04}};
+        static const double A[3][2] = {{0.143, 0.189}, {0.133, 0.171}, {0.234, 0.244}}, B[3][2] = {{0.027, 0.024}, {0.028, 0.034}, {0.002, 0.036}};
+        static const double fixed[3][2] = {{3.8, 4.4}, {3.8, 4.5}, {4.4, 5.7}}, exchange[4][2] = {{0.0, 0.0}, {1.9, 1.8}, {2.2, 2.7}, {2.2, 3.3}};
         const int tiles = ceil_div(M, BM) * ceil_div(N, bn), w = bn == 128;
-        for (int S = 1; S <= 8 && S <= kb && tiles <= small::resident_clusters(S); S *= 2) {
-            const double fixed = (S == 1 ? 4.4 : (S == 2 ? 5.7 : (S == 4 ? 6.2 : 6.6))) + (w ? 1.5 : 0.0);
-            const double cost = fixed + ceil_div(kb, S) * (A[mode][w] + B[mode][w] * tiles * S / num_sms);
+        for (int S = 1, i = 0; S <= 8 && S <= kb && tiles <= small::resident_clusters(S); S *= 2, i++) {
+            const double cost = fixed[mode][w] + exchange[i][w] * m_share + ceil_div(kb, S) * (A[mode][w] + B[mode][w] * tiles * S / num_sms);
             if (cost < best) { best = cost; plan.bn = bn; plan.S = S; }
         }
     }
@@ -1184,12 +1186,20 @@ static int run_small(const SmallPlan& plan, int mode, int epi, const void* A, co
                      const Ready& ready, cudaStream_t stream) {
     small::SParams p = {};
     p.M = q.M; p.N = q.N; p.K = q.K;
-    p.tiles_n = ceil_div(q.N, plan.bn);
     p.kb_total = q.kb_total;
-    p.S = plan.S;
-    const int stages = plan.bn == 64 ? small::SGeo<64>::STAGES : small::SGeo<128>::STAGES;
-    const int kb_max = ceil_div(q.kb_total, plan.S);
+    for (p.log_s = 0; 1 << p.log_s < plan.S;) p.log_s++;
+    // 128-wide tiles of a cluster: six stages over four where the loop is longer than that (320 x 2048 x 8192: 28.2 us with
+    // four, 22.4 with six), at the price of a cluster barrier before rows are sent
+    const bool w = plan.bn == 128;
+    const int kb_max = ceil_div(q.kb_total, plan.S), apart = w ? small::SGeo<128>::STAGES_APART : small::SGeo<64>::STAGES_APART;
+    p.over = plan.S > 1 && w && kb_max > apart;
+    const int stages = plan.S > 1 && !p.over ? apart : (w ? small::SGeo<128>::STAGES : small::SGeo<64>::STAGES);
     p.stages = kb_max < stages ? kb_max : stages;
+    const int acc = w ? small::SGeo<128>::ACC_BYTES : small::SGeo<64>::ACC_BYTES;
+    int ring = p.stages * (w ? small::SGeo<128>::STAGE_BYTES : small::SGeo<64>::STAGE_BYTES);
+    if (ring < (p.over ? 2 : 1) * acc) ring = (p.over ? 2 : 1) * acc;
+    p.red_off = p.over ? acc : ring;
+    p.ones_off = ring + (plan.S > 1 && !p.over ? acc : 0);
     p.bias = q.bias; p.aux = q.aux;
     p.C = static_cast<bf16*>(C); p.C2 = static_cast<bf16*>(C2); p.C3 = static_cast<bf16*>(ready.c3);
     p.dbias = q.dbias;
@@ -1211,11 +1221,12 @@ static int run_small(const SmallPlan& plan, int mode, int epi, const void* A, co
     if (rc) return rc;
     tmB2 = tmB;
     if (swi && (rc = make_tmap_2d(&tmB2, ready.b2, q.K, b_rows, q.K, BK, b_box))) return rc;
-    const int tiles = ceil_div(q.M, BM) * p.tiles_n;
 #define LLMK_SMALL_CASE(MODE_, EPI_)                                                                    \
     if (mode == MODE_ && epi == (EPI_))                                                                 \
-        return plan.bn == 64 ? small::launch<MODE_, EPI_, 64>(tmA, tmB, tmB2, p, tiles, stream)         \
-                             : small::launch<MODE_, EPI_, 128>(tmA, tmB, tmB2, p, tiles, stream);
+        return plan.bn == 64 ? (plan.S > 1 ? small::launch<MODE_, EPI_, 64, true>(tmA, tmB, tmB2, p, stream)    \
+                                           : small::launch<MODE_, EPI_, 64, false>(tmA, tmB, tmB2, p, stream))  \
+                             : (plan.S > 1 ? small::launch<MODE_, EPI_, 128, true>(tmA, tmB, tmB2, p, stream)   \
+                                           : small::launch<MODE_, EPI_, 128, false>(tmA, tmB, tmB2, p, stream));
     LLMK_SMALL_CASE(MODE_NT, 0)
     LLMK_SMALL_CASE(MODE_NT, EPI_BIAS)
     LLMK_SMALL_CASE(MODE_NT, EPI_BIAS | EPI_GELU)

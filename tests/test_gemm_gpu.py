@@ -394,3 +394,31 @@ def test_split_products_get_the_workspace_of_their_split_count(M, N, K, max_ctas
     assert ((out.double() - want).abs() <= 2.0 ** -8 * want.abs() + chain).all()
     assert ((db.double() - a.double().sum(0)).abs() <= 2.0 ** -8 * a.double().sum(0).abs() + 1e-5 * K ** 0.5).all()
     _native.check_status()
+
+
+@pytest.mark.parametrize("M", [1, 5, 60, 130, 200])
+def test_rows_of_few_tiles_dealt_out_unevenly_over_a_cluster(M):
+    """The rows of a tile are summed by the CTAs of its cluster: row counts that are no multiple of the cluster size, fewer
+    rows than CTAs, and the epilogues whose lanes work together (D = rowsum(dO * O), bias gradient) on such rows."""
+    from llm_kittens_b200.ops import gemm, _native
+
+    N, K, T = 768, 3072, 5 if M % 5 == 0 else 1
+    a, w, bias, add = _rand(M, K), _rand(N, K, scale=0.05), _rand(N), _rand(M, N)
+    want = a.double() @ w.double().T
+    tol = lambda x: 2.0 ** -8 * x.abs() + 1e-5 * K ** 0.5   # fp32 sums of K products of order 0.05, one rounding to bf16
+    got = gemm.gemm_nt(a, w, bias=bias, add=add)
+    x = want + bias.double() + add.double()
+    assert ((got.double() - x).abs() <= tol(x)).all()
+    dvec, out = torch.empty(M // T, N // 64, T, device="cuda"), torch.empty(M, N, device="cuda", dtype=torch.bfloat16)
+    assert gemm.gemm_nn(a, w.T.contiguous(), out=out, drow_of=(add, dvec, T)) is not False
+    assert ((out.double() - want).abs() <= tol(want)).all()
+    d = (out.double() * add.double()).view(M // T, T, N // 64, 64).sum(-1).transpose(1, 2)
+    assert ((dvec.double() - d).abs() <= 1e-5 * 64).all()
+    cols = 8 * M
+    b, dout = _rand(3000, 256), _rand(3000, cols)
+    dw, db = _rand(cols, 256), _rand(cols)
+    dw0, db0 = dw.double(), db.double()
+    gemm.gemm_tn(dout, b, out=dw, accumulate=True, dbias=db)
+    for got, x in ((dw, dw0 + dout.double().T @ b.double()), (db, db0 + dout.double().sum(0))):
+        assert ((got.double() - x).abs() <= 2.0 ** -8 * x.abs() + 1e-4 * 3000 ** 0.5).all()
+    _native.check_status()
