@@ -112,6 +112,10 @@ def ledger_start() -> None:
     _LEDGER = []
 
 
+def ledger_running() -> bool:
+    return _LEDGER is not None
+
+
 def ledger_stop() -> dict[str, tuple[int, float]]:
     """Synchronise and return {label: (calls, total milliseconds)}. GEMM calls are labelled by layout, epilogue and
     shape, other entry points by name."""

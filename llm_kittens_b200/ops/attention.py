@@ -47,6 +47,11 @@ def _tc_forward(B: int, T: int, NH: int, HS: int) -> bool:
     return T >= 512 or (T + 127) // 128 * B * NH <= _sms()
 
 
+def forward_is_tc(B: int, T: int, NH: int, HS: int) -> bool:
+    """Whether :func:`attention_fwd` without ``impl`` runs on the tcgen05 kernels."""
+    return IMPL == "tc" and _tc_forward(B, T, NH, HS)
+
+
 def attention_fwd(qkv, B, T, NH, NKVH, HS, out=None, lse=None, impl=None):
     """``qkv``: [B, T, (NH+2*NKVH)*HS] -> ``out`` [B, T, NH*HS], ``lse`` [B, NH, T] fp32. ``impl`` "warp" / "tc" asks for the
     warp-level kernels / for the tcgen05 kernels wherever they take the length; both leave what either backward needs."""

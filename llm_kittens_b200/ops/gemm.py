@@ -29,6 +29,10 @@ def set_max_ctas(n: int) -> None:
     _MAX_CTAS = int(n)
 
 
+def max_ctas() -> int:
+    return _MAX_CTAS
+
+
 def workspace(nbytes: int) -> torch.Tensor:
     return N.scratch_buffer(_WORKSPACE, nbytes, 64 << 20, "split-K partials")
 

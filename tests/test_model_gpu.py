@@ -352,3 +352,56 @@ def test_debug_state_gate_on_the_cuda_path(tmp_path):
     formats.write_model(mp, cfg, ref.params)
     check.write_debug_state(mp, sp, B=4, T=128)
     assert check.check_debug_state(mp, sp, device="cuda") == []
+
+
+@pytest.mark.parametrize("family,recompute,B,T", [("gpt2", 0, 1, 64), ("gpt2", 1, 2, 128), ("gpt2", 2, 3, 64), ("llama3", 0, 1, 64),
+                                                  ("llama3", 1, 1, 320), ("llama3", 2, 2, 128), ("halves", 0, 1, 320)])
+def test_blocks_forward_from_one_native_call_is_the_same_as_block_by_block(family, recompute, B, T, monkeypatch):
+    """Every kept activation bit for bit, and the cases that have to go block by block: a parameter hook, a stacked tensor
+    that is not contiguous, a switch."""
+    from llm_kittens_b200.models.config import ModelConfig
+    from llm_kittens_b200.models.transformer import Transformer
+    from llm_kittens_b200.ops import _native
+
+    llama = family != "gpt2"
+    cfg = ModelConfig(family="llama3" if llama else "gpt2", max_seq_len=512, vocab_size=500, padded_vocab_size=512, num_layers=3, num_heads=4,
+                      num_kv_heads=2 if llama else 4, channels=256, hidden_dim=512)
+    model = Transformer(cfg, device="cuda", recompute=recompute, rope_interleaved=family != "halves")
+    model.init_weights(3)
+    model.params.add_(torch.randn(model.num_parameters, device="cuda").to(torch.bfloat16) * 0.02)
+    x = torch.randint(0, 500, (B, T), dtype=torch.int32, device="cuda")
+    entries = []
+    call = _native.call
+    monkeypatch.setattr(_native, "call", lambda name, *a: (entries.append(name), call(name, *a))[1])
+
+    def run(native):
+        for t in model.acts.values() if model.acts else ():
+            if isinstance(t, torch.Tensor) and t.is_floating_point() and t is not model.acts.get("rope"):
+                t.zero_()
+        entries.clear()
+        before = _native.launch_count()
+        model.forward(x, None)
+        assert ("llmk_forward_layers" in entries) == native
+        kept = {n: t.clone() for n, t in model.acts.items() if isinstance(t, torch.Tensor) and n not in ("dresidual", "d_btc", "d_wide", "d_wide2", "dvec")}
+        return kept, _native.launch_count() - before
+
+    model.allocate(B, T)
+    want, launches = run(True)
+    model.param_hook = lambda layer, phase: None
+    got = [run(False)]
+    model.param_hook = None
+    if not llama:                       # refused by the block-by-block path, as before
+        kept_qkv = model.acts["qkv"]
+        model.acts["qkv"] = torch.empty(*kept_qkv.shape[:-1], 2 * cfg.qkv_width, device="cuda", dtype=torch.bfloat16)[..., :cfg.qkv_width]
+        with pytest.raises(_native.NativeError):
+            model.forward(x, None)
+        model.acts["qkv"] = kept_qkv
+    if llama:
+        monkeypatch.setenv("LLMK_FUSED_SWIGLU", "0")
+        got.append((run(False)[0], launches))
+        monkeypatch.delenv("LLMK_FUSED_SWIGLU")
+    got.append(run(True))
+    for acts, n in got:
+        assert n == launches
+        assert all(torch.equal(acts[k], want[k]) for k in want)
+    _native.check_status()
