@@ -5,19 +5,26 @@
 // which has no sm_100 path; the warp-level implementation in attention.cu remains for short sequences and
 // small calls whose length is not a multiple of 128 (ops/attention.py has the rule).
 //
-// One CTA per (128 query rows, head, batch); 6 warps:
-//   warp 0     TMA producer: Q once, then K/V tiles of 128 rows through a 2-stage ring
+// One CTA per (128 query rows, head, batch); 8 warps:
+//   warp 0     TMA producer: K / V tiles of 128 rows through rings of two, freed apart (K after S, V after P V); prefetches
+//              the tiles after the ring, and the first tiles of the CTA that will take its place, into the L2
 //   warp 1     MMA issuer:   S = Q K^T  (128x128xHS, both operands K-major)  -> TMEM columns [0,128)
-//                            O_j = P V  (128xHSx128, P K-major from smem, V MN-major) -> TMEM [128,128+HS)
-//   warps 2-5  softmax:      one query row per thread (TMEM lane = row, so no cross-thread reductions):
+//                            O += P V   (128xHSx128, P K-major from smem, V MN-major) -> TMEM [128,128+HS)
+//   warps 4-7  softmax:      one query row per thread (TMEM lane = row, so no cross-thread reductions):
 //                            copies its S row into registers and releases the S buffer at once (the next
 //                            S = Q K^T runs during this tile's softmax), writes P = exp2(S*c - m) as bf16
 //                            into 128-byte-swizzled smem for the second MMA. O accumulates in TMEM over
 //                            all tiles; m trails the running maximum and O, l are rescaled (TMEM load,
 //                            multiply, store) only when a row maximum jumps by more than 2^8.
-// TMEM use is 256 columns and shared memory 112 KB for HS = 64, so two CTAs share an SM and one's
-// softmax overlaps the other's MMAs. Every wait is bounded and reports through the status word.
-#include <cstdlib>
+// What bounds it: a chain of latencies per tile (scores ready, TMEM load, maximum, exponentials, P V), 2700 cycles of which the
+// exponentials are half. HS = 64: TMEM use is 256 columns and shared memory 112 KB, so two CTAs share an SM (setmaxnreg gives
+// the softmax threads the registers of the first warpgroup: a whole S row is in registers) and one's softmax overlaps the
+// other's waits, first loads and epilogue. Two query tiles in one CTA instead run in step: both take their exponentials at
+// the same time and wait at the same time (4200 cycles per pair of tiles, 3000 here), and nothing fills a CTA's beginning
+// and end. us, pair of tiles per CTA / this: B64 T1024 12 heads 313 / 240, B16 T1024 16 heads 107 / 79, B8 T2048 12 heads 129 / 94,
+// B1 T1024 12 heads 21.9 / 13.8. HS = 128 (one CTA per SM) with the same code, chunks with branches before: B1 T4096 32/8 heads
+// 242 / 168, B2 T2048 16 heads 81 / 55.
+// Every wait is bounded and reports through the status word.
 
 #include "attention_order.cuh"
 #include "ptx_sm100.cuh"
@@ -29,7 +36,7 @@ int make_tmap_3d(CUtensorMap* m, const void* ptr, uint64_t inner, uint64_t rows,
 namespace attn_tc {
 
 constexpr int BQ = 128, BKV = 128;
-constexpr int THREADS = 192;
+constexpr int THREADS = 256;   // warpgroup 0: producer, MMA issuer, two idle warps; warpgroup 1: softmax
 constexpr int ATOM_BYTES = 128 * 128;  // one 128-row x 64-column (128-byte) swizzle atom column
 
 template <int HS>
@@ -39,7 +46,7 @@ struct Cfg {
     static constexpr int SMEM_MAIN = TILE_BYTES * 5 + P_BYTES;
     static constexpr int SMEM_BYTES = SMEM_MAIN + 128;   // tiles + barriers; the dynamic window itself is 1024-byte aligned
     static constexpr int TMEM_COLS = 256;
-    static constexpr int CTAS_PER_SM = 1;   // 128 S values per thread live in registers: two CTAs per SM would spill
+    static constexpr int CTAS_PER_SM = HS == 64 ? 2 : 1;
 };
 
 
@@ -72,73 +79,66 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
     return d;
 }
 
-// Maximum of one 32-column chunk of this thread's S row; `MASK` drops the columns after `lane`
-// (the chunk that holds the diagonal of a diagonal tile).
-template <bool MASK>
-__device__ __forceinline__ float chunk_max(const uint32_t (&s)[32], int lane, float acc) {
-    float a0 = acc, a1 = -INFINITY;
+// The softmax of a tile is one stretch of code without branches: the groups of eight columns overlap (the sums and stores of
+// one group stand beside the exponentials of the next). With a branch for each 32-column chunk, for the sake of the diagonal
+// tile, each one drained before the next began: 2000 cycles for the exponentials of a tile, of which the transcendental unit
+// needs 1024; now 1400.
+__device__ __forceinline__ float tile_max(const uint32_t (&s)[4][32]) {
+    float a[4];
 #pragma unroll
-    for (int i = 0; i < 32; i += 4) {
-        float x0 = __uint_as_float(s[i]), x1 = __uint_as_float(s[i + 1]);
-        float x2 = __uint_as_float(s[i + 2]), x3 = __uint_as_float(s[i + 3]);
-        if (MASK) {
-            if (i > lane) x0 = -INFINITY;
-            if (i + 1 > lane) x1 = -INFINITY;
-            if (i + 2 > lane) x2 = -INFINITY;
-            if (i + 3 > lane) x3 = -INFINITY;
-        }
-        a0 = max3(a0, x0, x1);
-        a1 = max3(a1, x2, x3);
+    for (int c4 = 0; c4 < 4; c4++) {
+        a[c4] = __uint_as_float(s[c4][0]);
+#pragma unroll
+        for (int i = 1; i < 31; i += 2) a[c4] = max3(a[c4], __uint_as_float(s[c4][i]), __uint_as_float(s[c4][i + 1]));
+        a[c4] = fmaxf(a[c4], __uint_as_float(s[c4][31]));
     }
-    return fmaxf(a0, a1);
+    return fmaxf(max3(a[0], a[1], a[2]), a[3]);
 }
-
-// P = exp2(S*c - m) of one 32-column chunk as bf16 into the swizzled A-operand tile; returns the chunk's sum.
-// MODE 0: plain, 1: mask the columns after `lane`, 2: the whole chunk is masked (zeros).
-template <int MODE, bool ROUND>
-__device__ __forceinline__ float chunk_probs(const uint32_t (&s)[32], uint8_t* atom, int chunk_base, int r, int lane,
-                                             float scale_log2, float neg_m) {
-    // packed fp32 pairs: one FMA-pipe instruction per two columns for the exponent argument and the row sum
-    const ptx::f32x2 c2 = ptx::pack2(scale_log2, scale_log2), m2 = ptx::pack2(neg_m, neg_m);
-    ptx::f32x2 sum2 = ptx::pack2(0.f, 0.f);
+// exp2(S*c - m) of the eight columns of group g, in place
+__device__ __forceinline__ void group_exps(uint32_t (&s)[4][32], int g, ptx::f32x2 c2, ptx::f32x2 m2) {
+    uint32_t* v = &s[g >> 2][(g & 3) * 8];
 #pragma unroll
-    for (int q = 0; q < 4; q++) {
-        float p[8];
+    for (int i = 0; i < 8; i += 2) {
+        float x0, x1;
+        ptx::unpack2(ptx::fma2(ptx::pack2(__uint_as_float(v[i]), __uint_as_float(v[i + 1])), c2, m2), x0, x1);
+        v[i] = __float_as_uint(ex2(x0));
+        v[i + 1] = __float_as_uint(ex2(x1));
+    }
+}
+// Groups [FIRST, 16): exponentials (those before FIRST have been taken already), row sum, and P as bf16 into shared memory.
+template <bool ROUND, int FIRST>
+__device__ __forceinline__ float tile_probs(uint32_t (&s)[4][32], uint8_t* row, int r, ptx::f32x2 c2, ptx::f32x2 m2) {
+    constexpr int LAG = 1;
+    ptx::f32x2 sum[2] = {ptx::pack2(0.f, 0.f), ptx::pack2(0.f, 0.f)};
 #pragma unroll
-        for (int i = 0; i < 8; i += 2) {
-            float e0 = 0.f, e1 = 0.f;
-            if (MODE != 2) {
-                float x0, x1;
-                ptx::unpack2(ptx::fma2(ptx::pack2(__uint_as_float(s[q * 8 + i]), __uint_as_float(s[q * 8 + i + 1])), c2, m2), x0, x1);
-                e0 = ex2(x0);
-                e1 = ex2(x1);
-                if (MODE == 1 && q * 8 + i > lane) e0 = 0.f;
-                if (MODE == 1 && q * 8 + i + 1 > lane) e1 = 0.f;
-            }
-            p[i] = e0;
-            p[i + 1] = e1;
+    for (int g = 0; g < 16 + LAG; g++) {
+        if (g >= FIRST && g < 16) group_exps(s, g, c2, m2);
+        if (g >= LAG) {
+            const int c4 = (g - LAG) >> 2, q = (g - LAG) & 3;
+            float p[8];
+#pragma unroll
+            for (int i = 0; i < 8; i++) p[i] = __uint_as_float(s[c4][q * 8 + i]);
+#pragma unroll
+            for (int i = 0; i < 8; i += 2) sum[(i >> 1) & 1] = ptx::add2(sum[(i >> 1) & 1], ptx::pack2(p[i], p[i + 1]));
+            uint4 w;
+            w.x = ROUND ? pack_round2(p[0], p[1]) : pack_trunc2(p[0], p[1]);
+            w.y = ROUND ? pack_round2(p[2], p[3]) : pack_trunc2(p[2], p[3]);
+            w.z = ROUND ? pack_round2(p[4], p[5]) : pack_trunc2(p[4], p[5]);
+            w.w = ROUND ? pack_round2(p[6], p[7]) : pack_trunc2(p[6], p[7]);
+            *reinterpret_cast<uint4*>(row + (c4 >> 1) * ATOM_BYTES + ((((c4 & 1) * 4 + q) ^ (r & 7)) << 4)) = w;
         }
-        if (MODE != 2) {
-#pragma unroll
-            for (int i = 0; i < 8; i += 2) sum2 = ptx::add2(sum2, ptx::pack2(p[i], p[i + 1]));
-        }
-        uint4 w;
-        w.x = ROUND ? pack_round2(p[0], p[1]) : pack_trunc2(p[0], p[1]);
-        w.y = ROUND ? pack_round2(p[2], p[3]) : pack_trunc2(p[2], p[3]);
-        w.z = ROUND ? pack_round2(p[4], p[5]) : pack_trunc2(p[4], p[5]);
-        w.w = ROUND ? pack_round2(p[6], p[7]) : pack_trunc2(p[6], p[7]);
-        *reinterpret_cast<uint4*>(atom + (((chunk_base + q) ^ (r & 7)) << 4)) = w;
     }
     float s0, s1;
-    ptx::unpack2(sum2, s0, s1);
+    ptx::unpack2(ptx::add2(sum[0], sum[1]), s0, s1);
     return s0 + s1;
 }
 
 template <int HS, bool ROUND>
 __global__ void __launch_bounds__(THREADS, Cfg<HS>::CTAS_PER_SM)
-attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant__ CUtensorMap tmKV, bf16* __restrict__ out,
-                   float* __restrict__ lse, int T, int Tkv, int causal, int NH, int NKVH, float scale_log2, int* status,
-                   const TileOrder order) {
+attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant__ CUtensorMap tmKV,
+                   const __grid_constant__ CUtensorMap tmOut, float* __restrict__ lse, int T, int Tkv, int causal, int NH, int NKVH,
+                   float scale_log2, int* status, const TileOrder order, int ahead) {
+    // ahead: CTAs that the chip holds at once, 0 = nothing is prefetched into the L2 (keys and values of another GPU).
     // tmKV / Tkv / causal: the keys and values may come from ANOTHER packed QKV tensor of the same layout (a peer's
     // chunk of the sequence in context-parallel attention; the map may cover that peer's memory, loads only, no
     // multicast). causal = 1: queries and keys cover the same positions (the usual case, tmKV == tmQKV); causal = 0:
@@ -148,7 +148,6 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_const
     uint8_t* smem = smem_raw;
     // a failure already recorded in the status word (by an earlier CTA or kernel) makes the rest return at once; the word
     // is fetched beside the set-up below, which costs a CTA that lives for 16 us 0.6 us less than in front of it
-    __shared__ int skip;
     const int failed = threadIdx.x == 0 && status != nullptr ? *reinterpret_cast<volatile int*>(status) : 0;
     if (ptx::smem_u32(smem) & 1023u) {  // swizzled tiles need a 1024-byte aligned window: refuse instead of corrupting
         if (threadIdx.x == 0 && status != nullptr) atomicCAS(status, 0, LLMK_ST_BOUNDS);
@@ -160,14 +159,18 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_const
     uint8_t* sP = smem + 5 * C::TILE_BYTES;
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C::SMEM_MAIN);
     uint64_t* q_full = bars;          // [1]
-    uint64_t* kv_full = bars + 1;     // [2]
-    uint64_t* kv_empty = bars + 3;    // [2]
-    uint64_t* s_full = bars + 5;      // [1]
-    uint64_t* p_full = bars + 6;      // [1]
-    uint64_t* o_full = bars + 7;      // [1]
-    uint64_t* s_free = bars + 8;      // [1]
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 9);
+    uint64_t* k_full = bars + 1;      // [2]
+    uint64_t* k_empty = bars + 3;     // [2]
+    uint64_t* v_full = bars + 5;      // [2]
+    uint64_t* v_empty = bars + 7;     // [2]
+    uint64_t* s_full = bars + 9;      // [1]
+    uint64_t* p_full = bars + 10;     // [1]
+    uint64_t* o_full = bars + 11;     // [1]
+    uint64_t* s_free = bars + 12;     // [1]
+    uint64_t* epi = bars + 13;        // [1]
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 14);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+    int* skip = reinterpret_cast<int*>(tmem_slot + 2);   // (no static shared memory: two CTAs fill the SM's)
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     int rank, pair;
@@ -178,35 +181,47 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_const
     const int nkv = causal ? qb + 1 : Tkv / BKV;
     const int q_col = h * HS, k_col = (NH + hk) * HS, v_col = (NH + NKVH + hk) * HS;
 
-    auto load_kv = [&](int j) {   // one thread
-        const int s = j & 1;
-        ptx::mbar_arrive_expect_tx(&kv_full[s], 2 * C::TILE_BYTES);
+    auto load_tile = [&](uint8_t* dst, uint64_t* bar, int col, int j) {   // one thread
+        ptx::mbar_arrive_expect_tx(bar, C::TILE_BYTES);
+#pragma unroll
+        for (int c = 0; c < HS / 64; c++) ptx::tma_load_3d(dst + c * ATOM_BYTES, &tmKV, bar, col + 64 * c, j * BKV, b);
+    };
+    auto prefetch_kv = [&](int j) {
 #pragma unroll
         for (int c = 0; c < HS / 64; c++) {
-            ptx::tma_load_3d(sK + s * C::TILE_BYTES + c * ATOM_BYTES, &tmKV, &kv_full[s], k_col + 64 * c, j * BKV, b);
-            ptx::tma_load_3d(sV + s * C::TILE_BYTES + c * ATOM_BYTES, &tmKV, &kv_full[s], v_col + 64 * c, j * BKV, b);
+            ptx::tma_prefetch_3d(&tmKV, k_col + 64 * c, j * BKV, b);
+            ptx::tma_prefetch_3d(&tmKV, v_col + 64 * c, j * BKV, b);
         }
     };
+    auto load_k = [&](int j) { load_tile(sK + (j & 1) * C::TILE_BYTES, &k_full[j & 1], k_col, j); };
+    auto load_v = [&](int j) { load_tile(sV + (j & 1) * C::TILE_BYTES, &v_full[j & 1], v_col, j); };
     if (threadIdx.x == 0) {
         ptx::mbar_init(q_full, 1);
         for (int i = 0; i < 2; i++) {
-            ptx::mbar_init(&kv_full[i], 1);
-            ptx::mbar_init(&kv_empty[i], 1);
+            ptx::mbar_init(&k_full[i], 1);
+            ptx::mbar_init(&k_empty[i], 1);
+            ptx::mbar_init(&v_full[i], 1);
+            ptx::mbar_init(&v_empty[i], 1);
         }
         ptx::mbar_init(s_full, 1);
         ptx::mbar_init(p_full, 4);
         ptx::mbar_init(o_full, 1);
         ptx::mbar_init(s_free, 4);
+        ptx::mbar_init(epi, 4);
         *abort_flag = 0;
         ptx::fence_barrier_init();
         ptx::fence_proxy_async_smem();
-        skip = failed;
+        *skip = failed;
         if (!failed) {   // the first tiles are on their way while TMEM is allocated
             ptx::mbar_arrive_expect_tx(q_full, C::TILE_BYTES);
 #pragma unroll
             for (int c = 0; c < HS / 64; c++) ptx::tma_load_3d(sQ + c * ATOM_BYTES, &tmQKV, q_full, q_col + 64 * c, qb * BQ, b);
-            for (int j = 0; j < 2 && j < nkv; j++) load_kv(j);
+            for (int j = 0; j < 2 && j < nkv; j++) {
+                load_k(j);
+                load_v(j);
+            }
         }
+        ptx::prefetch_tmap(&tmOut);
     }
     if (warp == 1) {
         ptx::tmem_alloc(tmem_slot, C::TMEM_COLS);
@@ -216,72 +231,94 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_const
     __syncthreads();
     ptx::tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
-    if (skip) {
+    if (*skip) {
         if (warp == 1) ptx::tmem_dealloc(tmem_base, C::TMEM_COLS);
         return;
     }
     const uint32_t tmem_s = tmem_base, tmem_o = tmem_base + 128;
 
-    if (warp == 0) {
-        // ------------------------------------------------------------ TMA producer (Q and the first two K/V tiles: above)
-        for (int j = 2; j < nkv; j++) {
-            if (!ptx::mbar_wait(&kv_empty[j & 1], ((j >> 1) & 1) ^ 1, abort_flag, status, LLMK_ST_TIMEOUT_TMA_EMPTY, j)) break;
-            if (lane == 0) load_kv(j);
-            __syncwarp();
-        }
-    } else if (warp == 1) {
-        // ------------------------------------------------------------ MMA issuer
-        constexpr uint32_t idesc_s = ptx::make_idesc_bf16(BQ, BKV, 0, 0);
-        constexpr uint32_t idesc_o = ptx::make_idesc_bf16(BQ, HS, 0, 1);
-        bool ok = ptx::mbar_wait(q_full, 0, abort_flag, status, LLMK_ST_TIMEOUT_TMA_FULL, -1);
-        // S(j+1) is issued as soon as the softmax warps have copied S(j) into registers (s_free), i.e. while
-        // they are still working on tile j; P V(j) follows when P(j) is in shared memory. O accumulates in TMEM.
-        auto issue_s = [&](int j) -> bool {
-            const int s = j & 1;
-            if (!ptx::mbar_wait(&kv_full[s], (j >> 1) & 1, abort_flag, status, LLMK_ST_TIMEOUT_TMA_FULL, j)) return false;
-            ptx::tc_fence_after();
-            if (ptx::elect_one()) {
-                const uint32_t q_addr = ptx::smem_u32(sQ), k_addr = ptx::smem_u32(sK + s * C::TILE_BYTES);
+    if (warp < 4) {
+        if (C::CTAS_PER_SM == 2) asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
+        if (warp == 0) {
+            // -------------------------------------------------------- TMA producer (Q and the first two K / V tiles: above)
+            // The tiles after the ring are on their way from HBM into the L2 before there is room for them. For the CTA that
+            // will take this one's place (blocks start in order) the first tiles are: without that it waits 3000 cycles for
+            // its first scores.
+            if (ahead > 0 && lane == 0) {
+                for (int j = 2; j < 4 && j < nkv; j++) prefetch_kv(j);
+                const int next = blockIdx.x + ahead;
+                if (next < (int)gridDim.x) {
+                    int n_rank, n_pair;
+                    tile_of(order, next, n_rank, n_pair);
+                    const int n_h = n_pair % NH, n_b = n_pair / NH, n_hk = n_h / (NH / NKVH);
 #pragma unroll
-                for (int kk = 0; kk < HS / 16; kk++) {
-                    const uint32_t off = (kk / 4) * ATOM_BYTES + (kk % 4) * 32;
-                    ptx::mma_f16_ss(tmem_s, ptx::make_smem_desc(q_addr + off, 16, 1024), ptx::make_smem_desc(k_addr + off, 16, 1024),
-                                    idesc_s, kk > 0 ? 1u : 0u);
+                    for (int c = 0; c < HS / 64; c++) {
+                        ptx::tma_prefetch_3d(&tmQKV, n_h * HS + 64 * c, (order.tiles - 1 - n_rank) * BQ, n_b);
+                        ptx::tma_prefetch_3d(&tmKV, (NH + n_hk) * HS + 64 * c, 0, n_b);
+                        ptx::tma_prefetch_3d(&tmKV, (NH + NKVH + n_hk) * HS + 64 * c, 0, n_b);
+                    }
                 }
-                ptx::mma_commit(s_full);
             }
             __syncwarp();
-            return true;
-        };
-        if (ok) ok = issue_s(0);
-        for (int j = 0; j < nkv && ok; j++) {
-            const int s = j & 1;
-            if (j + 1 < nkv) {
-                ok = ptx::mbar_wait(s_free, j & 1, abort_flag, status, LLMK_ST_TIMEOUT_ACC_EMPTY, 3000 + j);
-                if (!ok) break;
-                ptx::tc_fence_after();
-                ok = issue_s(j + 1);
-                if (!ok) break;
+            for (int j = 2; j < nkv; j++) {
+                const uint32_t ph = ((j >> 1) & 1) ^ 1;
+                if (ahead > 0 && lane == 0 && j + 2 < nkv) prefetch_kv(j + 2);
+                if (!ptx::mbar_wait(&k_empty[j & 1], ph, abort_flag, status, LLMK_ST_TIMEOUT_TMA_EMPTY, j)) break;
+                if (lane == 0) load_k(j);
+                __syncwarp();
+                if (!ptx::mbar_wait(&v_empty[j & 1], ph, abort_flag, status, LLMK_ST_TIMEOUT_TMA_EMPTY, j)) break;
+                if (lane == 0) load_v(j);
+                __syncwarp();
             }
-            // P(j) is in shared memory (and O has been rescaled if the row maxima moved)
-            ok = ptx::mbar_wait(p_full, j & 1, abort_flag, status, LLMK_ST_TIMEOUT_ACC_EMPTY, j);
-            if (!ok) break;
-            ptx::tc_fence_after();
-            if (ptx::elect_one()) {
-                const uint32_t p_addr = ptx::smem_u32(sP), v_addr = ptx::smem_u32(sV + s * C::TILE_BYTES);
+        } else if (warp == 1 && lane == 0) {
+            // -------------------------------------------------------- MMA issuer
+            // S(j+1) is issued as soon as the softmax warps have copied S(j) into registers (s_free), i.e. while they are
+            // still working on tile j; P V(j) follows when P(j) is in shared memory. O accumulates in TMEM. The
+            // descriptors are built once: inside the loop an MMA costs one integer add.
+            constexpr uint32_t idesc_s = ptx::make_idesc_bf16(BQ, BKV, 0, 0);
+            constexpr uint32_t idesc_o = ptx::make_idesc_bf16(BQ, HS, 0, 1);
+            const uint64_t q_desc = ptx::make_smem_desc(ptx::smem_u32(sQ), 16, 1024);
+            const uint64_t k_desc = ptx::make_smem_desc(ptx::smem_u32(sK), 16, 1024);
+            const uint64_t p_desc = ptx::make_smem_desc(ptx::smem_u32(sP), 16, 1024);
+            const uint64_t v_desc = ptx::make_smem_desc(ptx::smem_u32(sV), ATOM_BYTES, 1024);
+            bool ok = ptx::mbar_wait_spin(q_full, 0, abort_flag, status, LLMK_ST_TIMEOUT_TMA_FULL, -1);
+            for (int j = 0; j <= nkv && ok; j++) {
+                if (j < nkv) {
+                    const int s = j & 1;
+                    ok = ptx::mbar_wait_spin(&k_full[s], (j >> 1) & 1, abort_flag, status, LLMK_ST_TIMEOUT_TMA_FULL, j);
+                    if (ok && j > 0) ok = ptx::mbar_wait_spin(s_free, (j - 1) & 1, abort_flag, status, LLMK_ST_TIMEOUT_ACC_EMPTY, 3000 + j);
+                    if (!ok) break;
+                    ptx::tc_fence_after();
+                    const uint64_t kd = k_desc + (uint64_t)((s * C::TILE_BYTES) >> 4);
 #pragma unroll
-                for (int kk = 0; kk < BKV / 16; kk++) {
-                    const uint64_t adesc = ptx::make_smem_desc(p_addr + (kk / 4) * ATOM_BYTES + (kk % 4) * 32, 16, 1024);
-                    const uint64_t bdesc = ptx::make_smem_desc(v_addr + kk * 2048, ATOM_BYTES, 1024);
-                    ptx::mma_f16_ss(tmem_o, adesc, bdesc, idesc_o, (j > 0 || kk > 0) ? 1u : 0u);
+                    for (int kk = 0; kk < HS / 16; kk++) {
+                        const uint64_t off = (uint64_t)(((kk / 4) * ATOM_BYTES + (kk % 4) * 32) >> 4);
+                        ptx::mma_f16_ss(tmem_s, q_desc + off, kd + off, idesc_s, kk > 0 ? 1u : 0u);
+                    }
+                    ptx::mma_commit(s_full);
+                    ptx::mma_commit(&k_empty[s]);
                 }
-                ptx::mma_commit(&kv_empty[s]);
-                ptx::mma_commit(o_full);
+                if (j > 0) {
+                    const int jj = j - 1, s = jj & 1;
+                    ok = ptx::mbar_wait_spin(&v_full[s], (jj >> 1) & 1, abort_flag, status, LLMK_ST_TIMEOUT_TMA_FULL, jj);
+                    // P(jj) is in shared memory (and O has been rescaled if the row maxima moved)
+                    if (ok) ok = ptx::mbar_wait_spin(p_full, jj & 1, abort_flag, status, LLMK_ST_TIMEOUT_ACC_EMPTY, jj);
+                    if (!ok) break;
+                    ptx::tc_fence_after();
+                    const uint64_t vd = v_desc + (uint64_t)((s * C::TILE_BYTES) >> 4);
+#pragma unroll
+                    for (int kk = 0; kk < BKV / 16; kk++)
+                        ptx::mma_f16_ss(tmem_o, p_desc + (uint64_t)(((kk / 4) * ATOM_BYTES + (kk % 4) * 32) >> 4),
+                                        vd + (uint64_t)((kk * 2048) >> 4), idesc_o, (jj > 0 || kk > 0) ? 1u : 0u);
+                    ptx::mma_commit(o_full);
+                    ptx::mma_commit(&v_empty[s]);
+                }
             }
-            __syncwarp();
         }
+        __syncwarp();
     } else {
         // ------------------------------------------------------------ softmax warps (one query row per thread)
+        if (C::CTAS_PER_SM == 2) asm volatile("setmaxnreg.inc.sync.aligned.u32 216;");
         const int lane_group = warp & 3;
         const int r = lane_group * 32 + lane;
         const uint32_t lane_off = (uint32_t)(lane_group * 32) << 16;
@@ -294,86 +331,94 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_const
             ok = ptx::mbar_wait(s_full, j & 1, abort_flag, status, LLMK_ST_TIMEOUT_ACC_FULL, j);
             if (!ok) break;
             ptx::tc_fence_after();
-            const bool diag = causal && (j == nkv - 1);
-            const int nchunks = diag ? lane_group + 1 : 4;   // warp-uniform: later chunks are fully masked
             uint32_t s[4][32];
 #pragma unroll
-            for (int c4 = 0; c4 < 4; c4++)
-                if (c4 < nchunks) ptx::tmem_ld_32x32b_x32(tmem_s + lane_off + c4 * 32, s[c4]);
+            for (int c4 = 0; c4 < 4; c4++) ptx::tmem_ld_32x32b_x32(tmem_s + lane_off + c4 * 32, s[c4]);
             ptx::tmem_ld_wait();
             // S(j) now lives in registers: hand the TMEM buffer back so that S(j+1) can be computed meanwhile
             ptx::tc_fence_before();
             __syncwarp();
             if (lane == 0) ptx::mbar_arrive(s_free);
-            float mx = -INFINITY;
+            if (causal && j == nkv - 1) {
+                // the diagonal tile: -infinity after the row's own column, then the same code as every other tile
 #pragma unroll
-            for (int c4 = 0; c4 < 4; c4++) {
-                if (c4 < nchunks) {
-                    if (diag && c4 == lane_group) mx = chunk_max<true>(s[c4], lane, mx);
-                    else mx = chunk_max<false>(s[c4], lane, mx);
+                for (int c4 = 0; c4 < 4; c4++) {
+                    const int last = (lane_group - c4) * 32 + lane;   // last column of this chunk that the row sees
+                    if (c4 >= lane_group) {
+#pragma unroll
+                        for (int i = 0; i < 32; i++)
+                            if (i > last) s[c4][i] = 0xff800000u;
+                    }
                 }
             }
-            const float m_new = fmaxf(m, mx * scale_log2);
+            const float m_new = fmaxf(m, tile_max(s) * scale_log2);
+            // m trails the true running maximum: it moves, and O and l are rescaled, where a row maximum jumps
+            const bool rescale = j > 0 && __any_sync(0xffffffffu, m_new > m + RESCALE_GAP);
+            float alpha = 1.f;
+            if (j == 0 || rescale) {
+                alpha = ex2(m - m_new);
+                m = m_new;
+            }
+            const float neg_m = (ROUND ? 0.f : TRUNC_BIAS_LOG2) - m;   // P is truncated to bf16: see pack_trunc2
+            const ptx::f32x2 c2 = ptx::pack2(scale_log2, scale_log2), m2 = ptx::pack2(neg_m, neg_m);
+            constexpr int EARLY = 4;   // groups whose exponentials are taken before P V(j-1) has to be complete
+#pragma unroll
+            for (int g = 0; g < EARLY; g++) group_exps(s, g, c2, m2);
             if (j > 0) {
                 // P V(j-1) must be complete before P is overwritten and before O may be rescaled
                 ok = ptx::mbar_wait(o_full, (j - 1) & 1, abort_flag, status, LLMK_ST_TIMEOUT_ACC_FULL, 1000 + j);
                 if (!ok) break;
                 ptx::tc_fence_after();
-                if (__any_sync(0xffffffffu, m_new > m + RESCALE_GAP)) {
-                    const float alpha = ex2(m - m_new);
+                if (rescale) {
                     l *= alpha;
-                    m = m_new;
 #pragma unroll
-                    for (int h4 = 0; h4 < HS / 32; h4++) {
-                        uint32_t v[32];
-                        ptx::tmem_ld_32x32b_x32(tmem_o + lane_off + h4 * 32, v);
+                    for (int h8 = 0; h8 < HS / 8; h8++) {   // (eight columns at a time: S takes most of the registers)
+                        uint32_t v[8];
+                        ptx::tmem_ld_32x32b_x8(tmem_o + lane_off + h8 * 8, v);
                         ptx::tmem_ld_wait();
 #pragma unroll
-                        for (int i = 0; i < 32; i++) v[i] = __float_as_uint(__uint_as_float(v[i]) * alpha);
-                        ptx::tmem_st_32x32b_x32(tmem_o + lane_off + h4 * 32, v);
+                        for (int i = 0; i < 8; i++) v[i] = __float_as_uint(__uint_as_float(v[i]) * alpha);
+                        ptx::tmem_st_32x32b_x8(tmem_o + lane_off + h8 * 8, v);
                     }
                     ptx::tmem_st_wait();
                 }
-            } else {
-                m = m_new;
             }
-            const float neg_m = (ROUND ? 0.f : TRUNC_BIAS_LOG2) - m;   // P is truncated to bf16: see pack_trunc2
-            float rs = 0.f;
-#pragma unroll
-            for (int c4 = 0; c4 < 4; c4++) {
-                uint8_t* atom = sP + (c4 >> 1) * ATOM_BYTES + r * 128;
-                const int cb = (c4 & 1) * 4;
-                if (c4 >= nchunks) chunk_probs<2, ROUND>(s[c4], atom, cb, r, lane, scale_log2, neg_m);
-                else if (diag && c4 == lane_group) rs += chunk_probs<1, ROUND>(s[c4], atom, cb, r, lane, scale_log2, neg_m);
-                else rs += chunk_probs<0, ROUND>(s[c4], atom, cb, r, lane, scale_log2, neg_m);
-            }
-            l += rs;
+            l += tile_probs<ROUND, EARLY>(s, sP + r * 128, r, c2, m2);
             ptx::tc_fence_before();
             ptx::fence_proxy_async_smem();
             __syncwarp();
             if (lane == 0) ptx::mbar_arrive(p_full);
         }
+        if (ok) ok = ptx::mbar_wait(o_full, (nkv - 1) & 1, abort_flag, status, LLMK_ST_TIMEOUT_ACC_FULL, 2000);
         if (ok) {
-            ok = ptx::mbar_wait(o_full, (nkv - 1) & 1, abort_flag, status, LLMK_ST_TIMEOUT_ACC_FULL, 2000);
-            if (ok) {
-                ptx::tc_fence_after();
-                const float inv_l = 1.0f / l;
-                const bool in = qb * BQ + r < T;   // rows past the end of the sequence (a ragged last tile) are not stored
-                bf16* orow = out + (((size_t)b * T + qb * BQ + r) * NH + h) * HS;
+            // O -> bf16 -> the P buffer (128 rows x 128 bytes per 64 columns, swizzled like the tensor map) -> TMA store, which
+            // leaves out the rows past the end of the sequence (a ragged last tile)
+            ptx::tc_fence_after();
+            const float inv_l = 1.0f / l;
 #pragma unroll
-                for (int h4 = 0; h4 < HS / 32; h4++) {
-                    uint32_t v[32];
-                    ptx::tmem_ld_32x32b_x32(tmem_o + lane_off + h4 * 32, v);
-                    ptx::tmem_ld_wait();
+            for (int h4 = 0; h4 < HS / 32; h4++) {
+                uint32_t v[32];
+                ptx::tmem_ld_32x32b_x32(tmem_o + lane_off + h4 * 32, v);
+                ptx::tmem_ld_wait();
 #pragma unroll
-                    for (int q = 0; q < 4; q++) {
-                        float f[8];
+                for (int q = 0; q < 4; q++) {
+                    float f[8];
 #pragma unroll
-                        for (int i = 0; i < 8; i++) f[i] = __uint_as_float(v[q * 8 + i]) * inv_l;
-                        if (in) st128(orow + h4 * 32 + q * 8, pack8(f));
-                    }
+                    for (int i = 0; i < 8; i++) f[i] = __uint_as_float(v[q * 8 + i]) * inv_l;
+                    *reinterpret_cast<bf16x8*>(sP + (h4 >> 1) * ATOM_BYTES + r * 128 + ((((h4 & 1) * 4 + q) ^ (r & 7)) << 4)) = pack8(f);
                 }
-                if (in) lse[((size_t)b * NH + h) * T + qb * BQ + r] = (m + log2f(l)) * 0.6931471805599453f;
+            }
+            if (qb * BQ + r < T) lse[((size_t)b * NH + h) * T + qb * BQ + r] = (m + log2f(l)) * 0.6931471805599453f;
+            ptx::fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) ptx::mbar_arrive(epi);
+            if (lane_group == 0 && lane == 0) {
+                if (ptx::mbar_wait(epi, 0, abort_flag, status, LLMK_ST_TIMEOUT_ACC_FULL, 4000)) {
+#pragma unroll
+                    for (int c = 0; c < HS / 64; c++) ptx::tma_store_3d(&tmOut, sP + c * ATOM_BYTES, q_col + 64 * c, qb * BQ, b);
+                    ptx::tma_store_commit();
+                    ptx::tma_store_wait_read<0>();
+                }
             }
         }
     }
@@ -387,323 +432,24 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_const
 }
 
 template <int HS, bool ROUND>
-static int launch(const CUtensorMap& tm, const CUtensorMap& tm_kv, bf16* out, float* lse, int B, int T, int Tkv, int causal, int NH,
-                  int NKVH, int* status, cudaStream_t stream) {
+static int launch(const CUtensorMap& tm, const CUtensorMap& tm_kv, void* out, float* lse, int B, int T, int Tkv, int causal, int NH,
+                  int NKVH, int* status, bool local, cudaStream_t stream) {
     static PerDeviceOnce once_configured;
     if (once_configured.first()) {
         LLMK_CUDA_TRY(cudaFuncSetAttribute(attn_fwd_tc_kernel<HS, ROUND>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<HS>::SMEM_BYTES));
         LLMK_CUDA_TRY(cudaFuncSetAttribute(attn_fwd_tc_kernel<HS, ROUND>, cudaFuncAttributePreferredSharedMemoryCarveout,
                                            cudaSharedmemCarveoutMaxShared));
     }
+    CUtensorMap tm_out;
+    const int rc = gemm::make_tmap_3d(&tm_out, out, (uint64_t)NH * HS, T, B, 64, 128);
+    if (rc) return rc;
     const float scale_log2 = 1.4426950408889634f / sqrtf((float)HS);
     const TileOrder order = make_tile_order(ceil_div(T, BQ), NH * B, 4l * Tkv * HS * NKVH / NH);
-    attn_fwd_tc_kernel<HS, ROUND><<<order.tiles * order.heads, THREADS, Cfg<HS>::SMEM_BYTES, stream>>>(tm, tm_kv, out, lse, T, Tkv,
-        causal, NH, NKVH, scale_log2, status, order);
+    attn_fwd_tc_kernel<HS, ROUND><<<order.tiles * order.heads, THREADS, Cfg<HS>::SMEM_BYTES, stream>>>(tm, tm_kv, tm_out, lse, T, Tkv,
+        causal, NH, NKVH, scale_log2, status, order, local ? Cfg<HS>::CTAS_PER_SM * sm_count_current_device() : 0);
     LLMK_LAUNCH_CHECK();
     return LLMK_OK;
 }
-
-
-// =====================================================================================================
-// HS = 64: two 128-row query tiles per CTA (one CTA per SM), each with its own softmax warpgroup,
-// S / O accumulators and P buffer, sharing the K / V tiles of a 3-stage ring. While one warpgroup runs
-// its softmax the tensor core works for the other one, and K / V are read once for 256 query rows.
-//   warp 0      TMA producer (Q tiles once, K/V ring)
-//   warp 1      MMA issuer: per K/V tile j   S_0(j), S_1(j), then P_0 V(j-1), P_1 V(j-1)
-//   warps 4-7   softmax of query rows [0,128) of the block; warps 8-11 of rows [128,256)
-// The first warpgroup gives most of its registers back (setmaxnreg) so that the softmax threads can hold
-// a whole 128-column S row in registers without spilling.
-// TMEM (all 512 columns): S_0 [0,128)  S_1 [128,256)  O_0 [256,320)  O_1 [320,384).
-// O leaves through shared memory (the warpgroup's P buffer) and one TMA store per 128x64 tile.
-namespace pair {
-constexpr int HS = 64;
-constexpr int STAGES = 3;
-constexpr int THREADS = 384;   // warpgroup 0: producer, MMA issuer, two idle warps; warpgroups 1 and 2: softmax
-constexpr int TILE_BYTES = BQ * HS * 2;
-constexpr int P_BYTES = BQ * BKV * 2;
-constexpr int SMEM_MAIN = 2 * TILE_BYTES + 2 * STAGES * TILE_BYTES + 2 * P_BYTES;
-constexpr int SMEM_BYTES = SMEM_MAIN + 256;
-
-template <bool ROUND>
-__global__ void __launch_bounds__(THREADS, 1)
-attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant__ CUtensorMap tmOut, float* __restrict__ lse,
-                     int T, int NH, int NKVH, float scale_log2, int* status, const TileOrder order) {
-    extern __shared__ __align__(1024) uint8_t smem_raw[];
-    uint8_t* smem = smem_raw;
-    // a failure already recorded in the status word (by an earlier CTA or kernel) makes the rest return at once; the word
-    // is fetched beside the set-up below, which costs a CTA that lives for 16 us 0.6 us less than in front of it
-    __shared__ int skip;
-    const int failed = threadIdx.x == 0 && status != nullptr ? *reinterpret_cast<volatile int*>(status) : 0;
-    if (ptx::smem_u32(smem) & 1023u) {
-        if (threadIdx.x == 0 && status != nullptr) atomicCAS(status, 0, LLMK_ST_BOUNDS);
-        return;
-    }
-    uint8_t* sQ = smem;                                  // [2]
-    uint8_t* sK = smem + 2 * TILE_BYTES;                 // [STAGES]
-    uint8_t* sV = sK + STAGES * TILE_BYTES;              // [STAGES]
-    uint8_t* sP = sV + STAGES * TILE_BYTES;              // [2]
-    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + SMEM_MAIN);
-    uint64_t* q_full = bars;                 // [1]
-    uint64_t* kv_full = bars + 1;            // [STAGES]
-    uint64_t* kv_empty = kv_full + STAGES;   // [STAGES]
-    uint64_t* s_full = kv_empty + STAGES;    // [2]
-    uint64_t* s_free = s_full + 2;           // [2]
-    uint64_t* p_full = s_free + 2;           // [2]
-    uint64_t* o_full = p_full + 2;           // [2]
-    uint64_t* epi = o_full + 2;              // [2]
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(epi + 2);
-    volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    int rank, pair;
-    tile_of(order, blockIdx.x, rank, pair);
-    const int qb2 = order.tiles - 1 - rank;  // late (long) query blocks first
-    const int h = pair % NH, b = pair / NH;
-    const int hk = h / (NH / NKVH);
-    const int q_col = h * HS, k_col = (NH + hk) * HS, v_col = (NH + NKVH + hk) * HS;
-    // tiles per half: the diagonal tile of half i is tile 2*qb2+i; a half past the end of the sequence is idle
-    const int n0 = 2 * qb2 + 1;
-    const int n1 = ((2 * qb2 + 1) * BQ < T) ? 2 * qb2 + 2 : 0;
-    const int nmax = n1 > n0 ? n1 : n0;
-
-    auto load_kv = [&](int j) {   // one thread
-        const int s = j % STAGES;
-        ptx::mbar_arrive_expect_tx(&kv_full[s], 2 * TILE_BYTES);
-        ptx::tma_load_3d(sK + s * TILE_BYTES, &tmQKV, &kv_full[s], k_col, j * BKV, b);
-        ptx::tma_load_3d(sV + s * TILE_BYTES, &tmQKV, &kv_full[s], v_col, j * BKV, b);
-    };
-    if (threadIdx.x == 0) {
-        ptx::mbar_init(q_full, 1);
-        for (int i = 0; i < STAGES; i++) {
-            ptx::mbar_init(&kv_full[i], 1);
-            ptx::mbar_init(&kv_empty[i], 2);   // one arrival per issuer warp
-        }
-        for (int i = 0; i < 2; i++) {
-            ptx::mbar_init(&s_full[i], 1);
-            ptx::mbar_init(&s_free[i], 4);
-            ptx::mbar_init(&p_full[i], 4);
-            ptx::mbar_init(&o_full[i], 1);
-            ptx::mbar_init(&epi[i], 4);
-        }
-        *abort_flag = 0;
-        ptx::fence_barrier_init();
-        ptx::fence_proxy_async_smem();
-        skip = failed;
-        if (!failed) {   // the first tiles are on their way while TMEM is allocated
-            ptx::mbar_arrive_expect_tx(q_full, (n1 ? 2 : 1) * TILE_BYTES);
-            ptx::tma_load_3d(sQ, &tmQKV, q_full, q_col, qb2 * 2 * BQ, b);
-            if (n1) ptx::tma_load_3d(sQ + TILE_BYTES, &tmQKV, q_full, q_col, qb2 * 2 * BQ + BQ, b);
-            for (int j = 0; j < STAGES && j < nmax; j++) load_kv(j);
-        }
-        ptx::prefetch_tmap(&tmOut);
-    }
-    if (warp == 1) {
-        ptx::tmem_alloc(tmem_slot, 512);
-        ptx::tmem_relinquish();
-    }
-    ptx::tc_fence_before();
-    __syncthreads();
-    ptx::tc_fence_after();
-    const uint32_t tmem_base = *tmem_slot;
-    if (skip) {
-        if (warp == 1) ptx::tmem_dealloc(tmem_base, 512);
-        return;
-    }
-
-    if (warp < 4) {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
-    if (warp == 0) {
-        // ------------------------------------------------------------ TMA producer (Q and the first K/V tiles: above)
-        for (int j = STAGES; j < nmax; j++) {
-            if (!ptx::mbar_wait(&kv_empty[j % STAGES], ((j / STAGES) & 1) ^ 1, abort_flag, status, LLMK_ST_TIMEOUT_TMA_EMPTY, j)) break;
-            if (lane == 0) load_kv(j);
-            __syncwarp();
-        }
-    } else if (warp == 1 || warp == 2) {
-        // ------------------------------------------------------------ MMA issuers: warp 1 for half 0, warp 2 for half 1
-        // Per K/V tile j: S_i(j) once K(j) has landed and the warpgroup has copied S_i(j-1) out of TMEM (early in
-        // its tile), then P_i V(j-1) once P_i(j-1) is in shared memory. The descriptors are built once: inside
-        // the loop an MMA costs one integer add, which matters because these warps share their schedulers with
-        // the softmax warps.
-        const int i = warp - 1;
-        const int ni = i ? n1 : n0;
-        if (lane == 0) {
-            constexpr uint32_t idesc_s = ptx::make_idesc_bf16(BQ, BKV, 0, 0);
-            constexpr uint32_t idesc_o = ptx::make_idesc_bf16(BQ, HS, 0, 1);
-            const uint32_t tmem_s = tmem_base + i * 128, tmem_o = tmem_base + 256 + i * HS;
-            const uint64_t q_desc = ptx::make_smem_desc(ptx::smem_u32(sQ + i * TILE_BYTES), 16, 1024);
-            const uint64_t k_desc = ptx::make_smem_desc(ptx::smem_u32(sK), 16, 1024);
-            const uint64_t p_desc = ptx::make_smem_desc(ptx::smem_u32(sP + i * P_BYTES), 16, 1024);
-            const uint64_t v_desc = ptx::make_smem_desc(ptx::smem_u32(sV), ATOM_BYTES, 1024);
-            bool ok = ptx::mbar_wait_spin(q_full, 0, abort_flag, status, LLMK_ST_TIMEOUT_TMA_FULL, -1);
-            if (ni == 0) {
-                // idle half (sequence ends inside this block): still release the K/V stages for the other issuer
-                for (int j = 0; j < nmax && ok; j++) {
-                    ok = ptx::mbar_wait_spin(&kv_full[j % STAGES], (j / STAGES) & 1, abort_flag, status, LLMK_ST_TIMEOUT_TMA_FULL, j);
-                    if (ok) ptx::mbar_arrive(&kv_empty[j % STAGES]);
-                }
-            }
-            for (int j = 0; j <= ni && ok && ni > 0; j++) {
-                if (j < ni) {
-                    const int s = j % STAGES;
-                    ok = ptx::mbar_wait_spin(&kv_full[s], (j / STAGES) & 1, abort_flag, status, LLMK_ST_TIMEOUT_TMA_FULL, j);
-                    if (ok && j > 0) ok = ptx::mbar_wait_spin(&s_free[i], (j - 1) & 1, abort_flag, status, LLMK_ST_TIMEOUT_ACC_EMPTY, 3000 + j);
-                    if (!ok) break;
-                    ptx::tc_fence_after();
-                    const uint64_t kd = k_desc + (uint64_t)((s * TILE_BYTES) >> 4);
-#pragma unroll
-                    for (int kk = 0; kk < HS / 16; kk++)
-                        ptx::mma_f16_ss(tmem_s, q_desc + (uint64_t)(kk * 2), kd + (uint64_t)(kk * 2), idesc_s, kk > 0 ? 1u : 0u);
-                    ptx::mma_commit(&s_full[i]);
-                }
-                if (j > 0) {
-                    const int jj = j - 1, s = jj % STAGES;
-                    ok = ptx::mbar_wait_spin(&p_full[i], jj & 1, abort_flag, status, LLMK_ST_TIMEOUT_ACC_EMPTY, jj);
-                    if (!ok) break;
-                    ptx::tc_fence_after();
-                    const uint64_t vd = v_desc + (uint64_t)((s * TILE_BYTES) >> 4);
-#pragma unroll
-                    for (int kk = 0; kk < BKV / 16; kk++)
-                        ptx::mma_f16_ss(tmem_o, p_desc + (uint64_t)(((kk / 4) * ATOM_BYTES + (kk % 4) * 32) >> 4),
-                                        vd + (uint64_t)((kk * 2048) >> 4), idesc_o, (jj > 0 || kk > 0) ? 1u : 0u);
-                    ptx::mma_commit(&o_full[i]);
-                    ptx::mma_commit(&kv_empty[s]);
-                }
-            }
-        }
-        __syncwarp();
-    }
-    } else {
-        // ------------------------------------------------------------ softmax warpgroups
-        asm volatile("setmaxnreg.inc.sync.aligned.u32 232;");
-        const int half = (warp - 4) >> 2;
-        const int nkv = half ? n1 : n0;
-        const int lane_group = warp & 3;
-        const int r = lane_group * 32 + lane;
-        const uint32_t lane_off = (uint32_t)(lane_group * 32) << 16;
-        const uint32_t tmem_s = tmem_base + half * 128, tmem_o = tmem_base + 256 + half * HS;
-        uint8_t* sPh = sP + half * P_BYTES;
-        constexpr float RESCALE_GAP = 8.f;
-        float m = -INFINITY, l = 0.f;
-        bool ok = nkv > 0;
-        for (int j = 0; j < nkv && ok; j++) {
-            ok = ptx::mbar_wait(&s_full[half], j & 1, abort_flag, status, LLMK_ST_TIMEOUT_ACC_FULL, j);
-            if (!ok) break;
-            ptx::tc_fence_after();
-            const bool diag = (j == nkv - 1);
-            const int nchunks = diag ? lane_group + 1 : 4;
-            uint32_t s[4][32];
-#pragma unroll
-            for (int c4 = 0; c4 < 4; c4++)
-                if (c4 < nchunks) ptx::tmem_ld_32x32b_x32(tmem_s + lane_off + c4 * 32, s[c4]);
-            ptx::tmem_ld_wait();
-            ptx::tc_fence_before();
-            __syncwarp();
-            if (lane == 0) ptx::mbar_arrive(&s_free[half]);
-            float mx = -INFINITY;
-#pragma unroll
-            for (int c4 = 0; c4 < 4; c4++) {
-                if (c4 < nchunks) {
-                    if (diag && c4 == lane_group) mx = chunk_max<true>(s[c4], lane, mx);
-                    else mx = chunk_max<false>(s[c4], lane, mx);
-                }
-            }
-            const float m_new = fmaxf(m, mx * scale_log2);
-            if (j > 0) {
-                ok = ptx::mbar_wait(&o_full[half], (j - 1) & 1, abort_flag, status, LLMK_ST_TIMEOUT_ACC_FULL, 1000 + j);
-                if (!ok) break;
-                ptx::tc_fence_after();
-                if (__any_sync(0xffffffffu, m_new > m + RESCALE_GAP)) {
-                    const float alpha = ex2(m - m_new);
-                    l *= alpha;
-                    m = m_new;
-#pragma unroll
-                    for (int h4 = 0; h4 < HS / 32; h4++) {
-                        uint32_t v[32];
-                        ptx::tmem_ld_32x32b_x32(tmem_o + lane_off + h4 * 32, v);
-                        ptx::tmem_ld_wait();
-#pragma unroll
-                        for (int i = 0; i < 32; i++) v[i] = __float_as_uint(__uint_as_float(v[i]) * alpha);
-                        ptx::tmem_st_32x32b_x32(tmem_o + lane_off + h4 * 32, v);
-                    }
-                    ptx::tmem_st_wait();
-                }
-            } else {
-                m = m_new;
-            }
-            const float neg_m = (ROUND ? 0.f : TRUNC_BIAS_LOG2) - m;   // P is truncated to bf16: see pack_trunc2
-            float rs = 0.f;
-#pragma unroll
-            for (int c4 = 0; c4 < 4; c4++) {
-                uint8_t* atom = sPh + (c4 >> 1) * ATOM_BYTES + r * 128;
-                const int cb = (c4 & 1) * 4;
-                if (c4 >= nchunks) chunk_probs<2, ROUND>(s[c4], atom, cb, r, lane, scale_log2, neg_m);
-                else if (diag && c4 == lane_group) rs += chunk_probs<1, ROUND>(s[c4], atom, cb, r, lane, scale_log2, neg_m);
-                else rs += chunk_probs<0, ROUND>(s[c4], atom, cb, r, lane, scale_log2, neg_m);
-            }
-            l += rs;
-            ptx::tc_fence_before();
-            ptx::fence_proxy_async_smem();
-            __syncwarp();
-            if (lane == 0) ptx::mbar_arrive(&p_full[half]);
-        }
-
-        if (ok) ok = ptx::mbar_wait(&o_full[half], (nkv - 1) & 1, abort_flag, status, LLMK_ST_TIMEOUT_ACC_FULL, 2000);
-        if (ok) {
-            // O -> bf16 -> this warpgroup's P buffer (128 rows x 128 B, swizzled like the tensor map) -> one TMA store
-            ptx::tc_fence_after();
-            const float inv_l = 1.0f / l;
-            const int q_row0 = (2 * qb2 + half) * BQ;
-#pragma unroll
-            for (int h4 = 0; h4 < HS / 32; h4++) {
-                uint32_t v[32];
-                ptx::tmem_ld_32x32b_x32(tmem_o + lane_off + h4 * 32, v);
-                ptx::tmem_ld_wait();
-#pragma unroll
-                for (int q = 0; q < 4; q++) {
-                    float f[8];
-#pragma unroll
-                    for (int i = 0; i < 8; i++) f[i] = __uint_as_float(v[q * 8 + i]) * inv_l;
-                    *reinterpret_cast<bf16x8*>(sPh + r * 128 + (((h4 * 4 + q) ^ (r & 7)) << 4)) = pack8(f);
-                }
-            }
-            if (q_row0 + r < T) lse[((size_t)b * NH + h) * T + q_row0 + r] = (m + log2f(l)) * 0.6931471805599453f;
-            ptx::fence_proxy_async_smem();
-            __syncwarp();
-            if (lane == 0) ptx::mbar_arrive(&epi[half]);
-            if (lane_group == 0 && lane == 0) {
-                if (ptx::mbar_wait(&epi[half], 0, abort_flag, status, LLMK_ST_TIMEOUT_ACC_FULL, 4000)) {
-                    ptx::tma_store_3d(&tmOut, sPh, q_col, q_row0, b);
-                    ptx::tma_store_commit();
-                    ptx::tma_store_wait_read<0>();
-                }
-            }
-        }
-    }
-
-    ptx::tc_fence_before();
-    __syncthreads();
-    if (warp == 1) {
-        ptx::tc_fence_after();
-        ptx::tmem_dealloc(tmem_base, 512);
-    }
-}
-
-template <bool ROUND>
-static int launch(const CUtensorMap& tm, const CUtensorMap& tm_out, float* lse, int B, int T, int NH, int NKVH, int* status,
-                  cudaStream_t stream) {
-    static PerDeviceOnce once_configured;
-    if (once_configured.first()) {
-        LLMK_CUDA_TRY(cudaFuncSetAttribute(attn_fwd_pair_kernel<ROUND>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
-    }
-    const float scale_log2 = 1.4426950408889634f / sqrtf((float)HS);
-    const TileOrder order = make_tile_order(ceil_div(T, 2 * BQ), NH * B, 4l * T * HS * NKVH / NH);
-    attn_fwd_pair_kernel<ROUND><<<order.tiles * order.heads, THREADS, SMEM_BYTES, stream>>>(tm, tm_out, lse, T, NH, NKVH, scale_log2,
-        status, order);
-    LLMK_LAUNCH_CHECK();
-    return LLMK_OK;
-}
-}  // namespace pair
 
 }  // namespace attn_tc
 }  // namespace llmk
@@ -716,25 +462,17 @@ using namespace llmk;
 LLMK_API int llmk_attention_fwd_tc(void* out, void* lse, const void* qkv, int B, int T, int NH, int NKVH, int HS, int* status,
                                    void* stream_) {
     cudaStream_t stream = (cudaStream_t)stream_;
-    static const bool single_tile = getenv("LLMK_ATTN_SINGLE_TILE") != nullptr;   // HS=64: one 128-row tile per CTA instead of two
     if (T % 64 || NH % NKVH || (HS != 64 && HS != 128)) return LLMK_ERR_SHAPE;
     const bool ragged = T % 128 != 0;
     const long width = (long)(NH + 2 * NKVH) * HS;
     CUtensorMap tm;
     const int rc = gemm::make_tmap_3d(&tm, qkv, (uint64_t)width, T, B, 64, 128);
     if (rc) return rc;
-    if (HS == 64 && !single_tile) {
-        CUtensorMap tm_out;
-        const int rc2 = gemm::make_tmap_3d(&tm_out, out, (uint64_t)NH * HS, T, B, 64, 128);
-        if (rc2) return rc2;
-        return ragged ? attn_tc::pair::launch<true>(tm, tm_out, (float*)lse, B, T, NH, NKVH, status, stream)
-                      : attn_tc::pair::launch<false>(tm, tm_out, (float*)lse, B, T, NH, NKVH, status, stream);
-    }
     if (HS == 64)
-        return ragged ? attn_tc::launch<64, true>(tm, tm, (bf16*)out, (float*)lse, B, T, T, 1, NH, NKVH, status, stream)
-                      : attn_tc::launch<64, false>(tm, tm, (bf16*)out, (float*)lse, B, T, T, 1, NH, NKVH, status, stream);
-    return ragged ? attn_tc::launch<128, true>(tm, tm, (bf16*)out, (float*)lse, B, T, T, 1, NH, NKVH, status, stream)
-                  : attn_tc::launch<128, false>(tm, tm, (bf16*)out, (float*)lse, B, T, T, 1, NH, NKVH, status, stream);
+        return ragged ? attn_tc::launch<64, true>(tm, tm, out, (float*)lse, B, T, T, 1, NH, NKVH, status, true, stream)
+                      : attn_tc::launch<64, false>(tm, tm, out, (float*)lse, B, T, T, 1, NH, NKVH, status, true, stream);
+    return ragged ? attn_tc::launch<128, true>(tm, tm, out, (float*)lse, B, T, T, 1, NH, NKVH, status, true, stream)
+                  : attn_tc::launch<128, false>(tm, tm, out, (float*)lse, B, T, T, 1, NH, NKVH, status, true, stream);
 }
 
 // One step of context-parallel (ring) attention, forward: the queries of `qkv` [B, T, W] (this rank's chunk of the
@@ -753,8 +491,8 @@ LLMK_API int llmk_attention_fwd_ring_step(void* out, void* lse, const void* qkv,
     if (rc) return rc;
     rc = gemm::make_tmap_3d(&tm_kv, kv_qkv, (uint64_t)width, Tkv, B, 64, 128);
     if (rc) return rc;
-    if (HS == 64) return attn_tc::launch<64, false>(tm, tm_kv, (bf16*)out, (float*)lse, B, T, Tkv, causal ? 1 : 0, NH, NKVH, status, stream);
-    return attn_tc::launch<128, false>(tm, tm_kv, (bf16*)out, (float*)lse, B, T, Tkv, causal ? 1 : 0, NH, NKVH, status, stream);
+    if (HS == 64) return attn_tc::launch<64, false>(tm, tm_kv, out, (float*)lse, B, T, Tkv, causal ? 1 : 0, NH, NKVH, status, false, stream);
+    return attn_tc::launch<128, false>(tm, tm_kv, out, (float*)lse, B, T, Tkv, causal ? 1 : 0, NH, NKVH, status, false, stream);
 }
 
 namespace llmk {
