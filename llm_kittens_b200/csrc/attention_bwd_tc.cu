@@ -38,20 +38,22 @@ __device__ __forceinline__ float ex2(float x) {
     return y;
 }
 
-// Two columns of the backward softmax with packed fp32 pairs: e = exp2(s * c + nl) (zero where masked) and
-// ds = e * (dp + nd). `nl` / `nd` hold the NEGATED log-sum-exp (exp2 domain) and D, so that the pair forms of
-// FMA / ADD / MUL (which take no operand negation) give the same roundings as the scalar s*c - L and dp - D.
-__device__ __forceinline__ void prob_pair(uint32_t s0, uint32_t s1, uint32_t dp0, uint32_t dp1, ptx::f32x2 c2, ptx::f32x2 nl,
-                                          ptx::f32x2 nd, bool mask0, bool mask1, float* p, float* ds) {
+// e = exp2(s * c + nl) of two columns in place; `nl` holds the NEGATED log-sum-exp (exp2 domain), because the pair forms of
+// FMA / ADD / MUL take no operand negation (D is kept negated for the same reason).
+__device__ __forceinline__ void exp_pair(uint32_t& s0, uint32_t& s1, ptx::f32x2 c2, ptx::f32x2 nl) {
     float x0, x1;
     ptx::unpack2(ptx::fma2(ptx::pack2(__uint_as_float(s0), __uint_as_float(s1)), c2, nl), x0, x1);
-    float e0 = ex2(x0), e1 = ex2(x1);
-    if (mask0) e0 = 0.f;
-    if (mask1) e1 = 0.f;
-    p[0] = e0;
-    p[1] = e1;
+    s0 = __float_as_uint(ex2(x0));
+    s1 = __float_as_uint(ex2(x1));
+}
+// Two columns of the backward softmax: e = exp2(s * c + nl) (zero where masked) and ds = e * (dp + nd).
+__device__ __forceinline__ void prob_pair(uint32_t s0, uint32_t s1, uint32_t dp0, uint32_t dp1, ptx::f32x2 c2, ptx::f32x2 nl,
+                                          ptx::f32x2 nd, bool mask0, bool mask1, float* p, float* ds) {
+    exp_pair(s0, s1, c2, nl);
+    p[0] = mask0 ? 0.f : __uint_as_float(s0);
+    p[1] = mask1 ? 0.f : __uint_as_float(s1);
     const ptx::f32x2 t = ptx::add2(ptx::pack2(__uint_as_float(dp0), __uint_as_float(dp1)), nd);
-    ptx::unpack2(ptx::mul2(ptx::pack2(e0, e1), t), ds[0], ds[1]);
+    ptx::unpack2(ptx::mul2(ptx::pack2(p[0], p[1]), t), ds[0], ds[1]);
 }
 
 // [ROWS x cols] K-major A/B operand at `base`, stored as atoms of 64 columns (ROWS * 128 bytes each):
@@ -107,26 +109,27 @@ __device__ __forceinline__ void store_chunk(uint8_t* tile, int r, int chunk, con
     *reinterpret_cast<bf16x8*>(atom + (((chunk & 7) ^ (r & 7)) << 4)) = v;
 }
 
+// Sub-tiles of the dK / dV kernel are 64 queries long (128 threads' S^T and dP^T rows stay in registers, and the scores of the
+// next one are computed meanwhile); those of the dQ kernel 64 keys for HS = 64 and 128 for HS = 128. HS = 64 has two CTAs per SM.
 template <int HS>
 struct Inner {
-    // HS = 64: 64-query sub-tiles and two CTAs per SM (one CTA's softmax overlaps the other's MMAs); 128-query sub-tiles
-    // with one CTA per SM issue a quarter fewer MMAs but measured 1.06 ms against 0.88 ms at B64 T1024 NH12
-    static constexpr int BN = HS == 64 ? 64 : 128;
+    static constexpr int DQ_BN = HS == 64 ? 64 : 128;
     static constexpr int CTAS = HS == 64 ? 2 : 1;
 };
 
 // ====================================================================================== dK, dV
 template <int HS>
 struct DkvCfg {
-    static constexpr int BN = Inner<HS>::BN;
-    static constexpr int RING = HS == 64 ? 2 : 1;
+    static constexpr int BN = 64;
+    static constexpr int RING = 3;
     static constexpr int TILE = BM * HS * 2;   // K or V
     static constexpr int RT = BN * HS * 2;     // Q or dO sub-tile
     static constexpr int OFF_K = 0, OFF_V = TILE, OFF_RING = 2 * TILE;   // ring: [RING][Q, dO]
     static constexpr int OFF_PT = OFF_RING + RING * 2 * RT, OFF_DST = OFF_PT + BM * BN * 2;
-    static constexpr int OFF_LD = OFF_DST + BM * BN * 2;                  // float [2][2][128]
-    static constexpr int OFF_BAR = OFF_LD + 2 * 2 * 128 * 4;
+    static constexpr int OFF_LD = OFF_DST + BM * BN * 2;                  // float L[2][64], D[64]
+    static constexpr int OFF_BAR = OFF_LD + 3 * BN * 4;
     static constexpr int SMEM_BYTES = OFF_BAR + 128;
+    static_assert(Inner<HS>::CTAS * (SMEM_BYTES + 1024) <= 228 * 1024, "the CTAs of an SM share its shared memory");
     static constexpr int TMEM = (2 * BN + 2 * HS) <= 256 ? 256 : 512;
 };
 
@@ -143,7 +146,6 @@ attn_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_c
     constexpr int RING = C::RING, BN = C::BN;
     extern __shared__ __align__(1024) uint8_t smem[];
     // a failure already recorded makes the CTA return; the word is fetched beside the set-up
-    __shared__ int skip;
     const int failed = threadIdx.x == 0 && status != nullptr ? *reinterpret_cast<volatile int*>(status) : 0;
     if (ptx::smem_u32(smem) & 1023u) {
         if (threadIdx.x == 0 && status != nullptr) atomicCAS(status, 0, LLMK_ST_BOUNDS);
@@ -156,16 +158,19 @@ attn_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_c
     uint8_t* sdSt = smem + C::OFF_DST;
     float* sLD = reinterpret_cast<float*>(smem + C::OFF_LD);
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C::OFF_BAR);
-    uint64_t* kv_full = bars;         // [1]
-    uint64_t* ring_full = bars + 1;   // [2]
-    uint64_t* ring_empty = bars + 3;  // [2]
-    uint64_t* s_full = bars + 5;
-    uint64_t* p_full = bars + 6;
-    uint64_t* acc_done = bars + 7;
-    uint64_t* ld_full = bars + 8;     // [2] LSE / D vectors of a ring slot are in shared memory
-    uint64_t* epi = bars + 10;        // dK / dV staged in shared memory
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 11);
+    uint64_t* kv_full = bars;            // [1]
+    uint64_t* ring_full = bars + 1;      // [3]
+    uint64_t* ring_empty = bars + 4;     // [3]
+    uint64_t* s_full = bars + 7;
+    uint64_t* s_free = bars + 8;         // S^T and dP^T have been read into registers
+    uint64_t* p_full = bars + 9;
+    uint64_t* acc_done = bars + 10;
+    uint64_t* l_full = bars + 11;        // [2] log-sum-exps of a sub-tile are in shared memory
+    uint64_t* d_full = bars + 13;        // its D
+    uint64_t* epi = bars + 14;           // dK / dV staged in shared memory
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 15);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+    int* skip = reinterpret_cast<int*>(smem + C::OFF_LD);   // (no static shared memory; read before the first L is written)
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     int kt, pair;   // early (long) key tiles first
@@ -187,11 +192,14 @@ attn_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_c
     };
     if (threadIdx.x == 0) {
         ptx::mbar_init(kv_full, 1);
-        for (int i = 0; i < 2; i++) {
+        for (int i = 0; i < RING; i++) {
             ptx::mbar_init(&ring_full[i], 1);
             ptx::mbar_init(&ring_empty[i], 1);
-            ptx::mbar_init(&ld_full[i], 1);
         }
+        ptx::mbar_init(&l_full[0], 1);
+        ptx::mbar_init(&l_full[1], 1);
+        ptx::mbar_init(d_full, 1);
+        ptx::mbar_init(s_free, 8);
         ptx::mbar_init(s_full, 1);
         ptx::mbar_init(p_full, 8);
         ptx::mbar_init(acc_done, 1);
@@ -199,7 +207,7 @@ attn_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_c
         *abort_flag = 0;
         ptx::fence_barrier_init();
         ptx::fence_proxy_async_smem();
-        skip = failed;
+        *skip = failed;
         if (!failed) {   // the first tiles are on their way while TMEM is allocated
             ptx::mbar_arrive_expect_tx(kv_full, 2 * C::TILE);
             load_tile<HS, BM>(sK, &tmQKV, kv_full, k_col, kv0, b);
@@ -215,88 +223,100 @@ attn_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_c
     __syncthreads();
     ptx::tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
-    if (skip) {
+    const bool skipped = *skip != 0;
+    __syncthreads();
+    if (skipped) {
         if (warp == 1) ptx::tmem_dealloc(tmem_base, C::TMEM);
         return;
     }
     const uint32_t t_st = tmem_base, t_dpt = tmem_base + BN, t_dv = tmem_base + 2 * BN, t_dk = tmem_base + 2 * BN + HS;
 
     if (warp == 0) {
-        for (int it = 0; it < total; it++) {
-            const int s = it % RING;
-            if (!ptx::mbar_wait(&ring_empty[s], ((it / RING) & 1) ^ 1, abort_flag, status, LLMK_ST_TIMEOUT_TMA_EMPTY, it)) break;
-            const int hq = hk * hr + it / nq, q0 = q_first + (it % nq) * BN;
-            if (lane == 0 && it >= RING) load_q(it);   // (K, V and the first sub-tiles: above)
-            {   // log-sum-exp (in the exp2 domain) and D of the BN queries of this sub-tile
-                float* sL = sLD + s * 256;
-                const size_t off = ((size_t)b * NH + hq) * T + q0;
+        // ------------------------------------------------------------ Q / dO ring, log-sum-exp (exp2 domain) and D, both negated
+        // The vectors are fetched one sub-tile ahead. There is room for two sub-tiles' L and one's D (the softmax needs it
+        // after the exponentials): as soon as sub-tile it-1 is done with, D(it) and L(it+1) take their places.
+        float* sL = sLD;
+        float* sD = sLD + 2 * BN;
+        float L[2], D[2];
+        auto fetch = [&](int it) {
+            const size_t off = ((size_t)b * NH + hk * hr + it / nq) * T + q_first + (it % nq) * BN;
 #pragma unroll
-                for (int i = 0; i < BN / 32; i++) {
-                    // (queries past the end of the sequence, which a 128-row sub-tile can have: probability zero)
-                    const bool in = BN == 64 || q0 + lane + 32 * i < T;
-                    sL[lane + 32 * i] = in ? -lse[off + lane + 32 * i] * LOG2E : -INFINITY;   // negated: the consumers add
-                    sL[128 + lane + 32 * i] = in ? -dvec[off + lane + 32 * i] : 0.f;
-                }
+            for (int i = 0; i < 2; i++) {
+                L[i] = -lse[off + lane + 32 * i] * LOG2E;
+                D[i] = -dvec[off + lane + 32 * i];
+            }
+        };
+        fetch(0);
+#pragma unroll
+        for (int i = 0; i < 2; i++) sL[lane + 32 * i] = L[i];
+        __syncwarp();
+        if (lane == 0) ptx::mbar_arrive(&l_full[0]);
+        for (int it = 0; it < total; it++) {
+            float d[2] = {D[0], D[1]};
+            if (it + 1 < total) fetch(it + 1);
+            if (it > 0 && !ptx::mbar_wait(p_full, (it - 1) & 1, abort_flag, status, LLMK_ST_TIMEOUT_ACC_EMPTY, 5000 + it)) break;
+#pragma unroll
+            for (int i = 0; i < 2; i++) {
+                sD[lane + 32 * i] = d[i];
+                if (it + 1 < total) sL[((it + 1) & 1) * BN + lane + 32 * i] = L[i];
             }
             __syncwarp();
-            if (lane == 0) ptx::mbar_arrive(&ld_full[s]);
+            if (lane == 0) {
+                ptx::mbar_arrive(d_full);
+                if (it + 1 < total) ptx::mbar_arrive(&l_full[(it + 1) & 1]);
+            }
+            const int next = it + RING - 1;   // its slot is free once the products of sub-tile it-1 are in
+            if (it > 0 && next < total) {
+                if (!ptx::mbar_wait(&ring_empty[next % RING], ((next / RING) & 1) ^ 1, abort_flag, status, LLMK_ST_TIMEOUT_TMA_EMPTY, it)) break;
+                if (lane == 0) load_q(next);
+            }
             __syncwarp();
         }
     } else if (warp == 1) {
         constexpr uint32_t idesc_s = ptx::make_idesc_bf16(BM, BN, 0, 0);
         constexpr uint32_t idesc_acc = ptx::make_idesc_bf16(BM, HS, 0, 1);
-        bool ok = ptx::mbar_wait_spin(kv_full, 0, abort_flag, status, LLMK_ST_TIMEOUT_TMA_FULL, -1);
-        // descriptors are built once; only lane 0 runs the issue loop (it shares its scheduler with softmax warps,
-        // so every instruction saved here shortens the critical path)
-        const uint64_t k_desc = kmajor_desc<BM>(ptx::smem_u32(sK), 0), v_desc = kmajor_desc<BM>(ptx::smem_u32(sV), 0);
-        const uint64_t pt_desc = kmajor_desc<BM>(ptx::smem_u32(sPt), 0), dst_desc = kmajor_desc<BM>(ptx::smem_u32(sdSt), 0);
-        const uint32_t ring_addr = ptx::smem_u32(sRing);
-        auto issue_s = [&](int it) -> bool {
-            const int s = it % RING;
-            if (!ptx::mbar_wait_spin(&ring_full[s], (it / RING) & 1, abort_flag, status, LLMK_ST_TIMEOUT_TMA_FULL, it)) return false;
-            ptx::tc_fence_after();
-            if (ptx::elect_one()) {
-                const uint64_t q_desc = kmajor_desc<BN>(ring_addr + s * 2 * C::RT, 0), do_desc = kmajor_desc<BN>(ring_addr + s * 2 * C::RT + C::RT, 0);
+        // One thread; descriptors are built once (the thread shares its scheduler with softmax warps, so every instruction
+        // saved here shortens the critical path). The scores of sub-tile it are issued as soon as the softmax warps have
+        // those of it-1 in registers, i.e. beside their exponentials; the products of it-1 follow when P^T and dS^T are there.
+        if (lane == 0) {
+            bool ok = ptx::mbar_wait_spin(kv_full, 0, abort_flag, status, LLMK_ST_TIMEOUT_TMA_FULL, -1);
+            const uint64_t k_desc = kmajor_desc<BM>(ptx::smem_u32(sK), 0), v_desc = kmajor_desc<BM>(ptx::smem_u32(sV), 0);
+            const uint64_t pt_desc = kmajor_desc<BM>(ptx::smem_u32(sPt), 0), dst_desc = kmajor_desc<BM>(ptx::smem_u32(sdSt), 0);
+            const uint64_t q0_desc = kmajor_desc<BN>(ptx::smem_u32(sRing), 0), qmn0_desc = mnmajor_desc<BN>(ptx::smem_u32(sRing), 0);
+            for (int it = 0; it <= total && ok; it++) {
+                if (it < total) {
+                    const int s = it % RING;
+                    ok = ptx::mbar_wait_spin(&ring_full[s], (it / RING) & 1, abort_flag, status, LLMK_ST_TIMEOUT_TMA_FULL, it);
+                    if (ok && it > 0) ok = ptx::mbar_wait_spin(s_free, (it - 1) & 1, abort_flag, status, LLMK_ST_TIMEOUT_ACC_EMPTY, 3000 + it);
+                    if (!ok) break;
+                    ptx::tc_fence_after();
+                    const uint64_t q_desc = q0_desc + (uint64_t)((s * 2 * C::RT) >> 4), do_desc = q_desc + (uint64_t)(C::RT >> 4);
 #pragma unroll
-                for (int kk = 0; kk < HS / 16; kk++)
-                    ptx::mma_f16_ss(t_st, kmajor_step<BM>(k_desc, kk), kmajor_step<BN>(q_desc, kk), idesc_s, kk > 0 ? 1u : 0u);
+                    for (int kk = 0; kk < HS / 16; kk++)
+                        ptx::mma_f16_ss(t_st, kmajor_step<BM>(k_desc, kk), kmajor_step<BN>(q_desc, kk), idesc_s, kk > 0 ? 1u : 0u);
 #pragma unroll
-                for (int kk = 0; kk < HS / 16; kk++)
-                    ptx::mma_f16_ss(t_dpt, kmajor_step<BM>(v_desc, kk), kmajor_step<BN>(do_desc, kk), idesc_s, kk > 0 ? 1u : 0u);
-                ptx::mma_commit(s_full);
-            }
-            __syncwarp();
-            return true;
-        };
-        auto issue_acc = [&](int it) {
-            const int s = it % RING;
-            if (ptx::elect_one()) {
-                const uint64_t q_mn = mnmajor_desc<BN>(ring_addr + s * 2 * C::RT, 0), do_mn = mnmajor_desc<BN>(ring_addr + s * 2 * C::RT + C::RT, 0);
+                    for (int kk = 0; kk < HS / 16; kk++)
+                        ptx::mma_f16_ss(t_dpt, kmajor_step<BM>(v_desc, kk), kmajor_step<BN>(do_desc, kk), idesc_s, kk > 0 ? 1u : 0u);
+                    ptx::mma_commit(s_full);
+                }
+                if (it > 0) {
+                    const int j = it - 1, s = j % RING;
+                    ok = ptx::mbar_wait_spin(p_full, j & 1, abort_flag, status, LLMK_ST_TIMEOUT_ACC_EMPTY, j);
+                    if (!ok) break;
+                    ptx::tc_fence_after();
+                    const uint64_t q_mn = qmn0_desc + (uint64_t)((s * 2 * C::RT) >> 4), do_mn = q_mn + (uint64_t)(C::RT >> 4);
 #pragma unroll
-                for (int kk = 0; kk < BN / 16; kk++)
-                    ptx::mma_f16_ss(t_dv, kmajor_step<BM>(pt_desc, kk), mnmajor_step(do_mn, kk), idesc_acc, (it > 0 || kk > 0) ? 1u : 0u);
+                    for (int kk = 0; kk < BN / 16; kk++)
+                        ptx::mma_f16_ss(t_dv, kmajor_step<BM>(pt_desc, kk), mnmajor_step(do_mn, kk), idesc_acc, (j > 0 || kk > 0) ? 1u : 0u);
 #pragma unroll
-                for (int kk = 0; kk < BN / 16; kk++)
-                    ptx::mma_f16_ss(t_dk, kmajor_step<BM>(dst_desc, kk), mnmajor_step(q_mn, kk), idesc_acc, (it > 0 || kk > 0) ? 1u : 0u);
-                ptx::mma_commit(&ring_empty[s]);
-                ptx::mma_commit(acc_done);
-            }
-            __syncwarp();
-        };
-        if (ok) ok = issue_s(0);
-        for (int it = 0; it < total && ok; it++) {
-            ok = ptx::mbar_wait_spin(p_full, it & 1, abort_flag, status, LLMK_ST_TIMEOUT_ACC_EMPTY, it);
-            if (!ok) break;
-            ptx::tc_fence_after();
-            if (RING == 2) {
-                if (it + 1 < total) ok = issue_s(it + 1);   // next scores first, so the softmax can overlap the accumulation
-                if (!ok) break;
-                issue_acc(it);
-            } else {
-                issue_acc(it);
-                if (it + 1 < total) ok = issue_s(it + 1);
+                    for (int kk = 0; kk < BN / 16; kk++)
+                        ptx::mma_f16_ss(t_dk, kmajor_step<BM>(dst_desc, kk), mnmajor_step(q_mn, kk), idesc_acc, (j > 0 || kk > 0) ? 1u : 0u);
+                    ptx::mma_commit(&ring_empty[s]);
+                    ptx::mma_commit(acc_done);
+                }
             }
         }
+        __syncwarp();
     } else {
         const int lane_group = warp & 3;
         const int sub = (warp - 2) >> 2;                     // 0 / 1: which half of the columns this warp handles
@@ -305,64 +325,60 @@ attn_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_c
         const ptx::f32x2 c2 = ptx::pack2(scale_log2, scale_log2);
         bool ok = true;
         for (int it = 0; it < total && ok; it++) {
-            const int dq0 = (it % nq) * BN;                  // first query of the sub-tile relative to the first key
-            const int slot = it % RING;
-            const float* sL = sLD + slot * 256;
-            const float* sD = sL + 128;
-            ok = ptx::mbar_wait(&ld_full[slot], (it / RING) & 1, abort_flag, status, LLMK_ST_TIMEOUT_TMA_FULL, 3000 + it);
+            const int dq0 = (it % nq) * BN + sub * 32;       // first query of this warp's half relative to the first key
+            const float* sL = sLD + (it & 1) * BN + sub * 32;
+            const float* sD = sLD + 2 * BN + sub * 32;
+            ok = ptx::mbar_wait(&l_full[it & 1], (it >> 1) & 1, abort_flag, status, LLMK_ST_TIMEOUT_TMA_FULL, 3000 + it);
             if (!ok) break;
             ok = ptx::mbar_wait(s_full, it & 1, abort_flag, status, LLMK_ST_TIMEOUT_ACC_FULL, it);
             if (!ok) break;
             ptx::tc_fence_after();
-            const bool diag = causal && dq0 < BM;            // some (key, query) pairs of this sub-tile are masked
-            // the two TMEM loads of chunk c4+1 are issued before chunk c4 is processed (two register sets)
-            uint32_t vsA[32], vdA[32], vsB[32], vdB[32];
-            // P^T / dS^T of a chunk stay in registers until the accumulation MMAs of the previous sub-tile have read the
-            // buffers they go to: those MMAs run beside the exponentials instead of in front of them
-            bool free_seen = it == 0;
-            auto process = [&](int c4, const uint32_t (&vs)[32], const uint32_t (&vd)[32]) {
-                bf16x8 pk[4], dk[4];
+            uint32_t vs[32], vd[32];
+            ptx::tmem_ld_32x32b_x32(t_st + lane_off + sub * 32, vs);
+            ptx::tmem_ld_32x32b_x32(t_dpt + lane_off + sub * 32, vd);
+            ptx::tmem_ld_wait();
+            ptx::tc_fence_before();
+            __syncwarp();
+            if (lane == 0) ptx::mbar_arrive(s_free);
+            if (causal && dq0 < lane_group * 32 + 32) {      // some (key, query) pairs of this warp are masked: P = 0
 #pragma unroll
-                for (int q = 0; q < 4; q++) {
-                    float p[8], ds[8], L[8], D[8];
-                    *reinterpret_cast<float4*>(L) = *reinterpret_cast<const float4*>(sL + c4 * 32 + q * 8);
-                    *reinterpret_cast<float4*>(L + 4) = *reinterpret_cast<const float4*>(sL + c4 * 32 + q * 8 + 4);
-                    *reinterpret_cast<float4*>(D) = *reinterpret_cast<const float4*>(sD + c4 * 32 + q * 8);
-                    *reinterpret_cast<float4*>(D + 4) = *reinterpret_cast<const float4*>(sD + c4 * 32 + q * 8 + 4);
-#pragma unroll
-                    for (int i = 0; i < 8; i += 2) {
-                        const int c = c4 * 32 + q * 8 + i;   // query column of the sub-tile
-                        prob_pair(vs[q * 8 + i], vs[q * 8 + i + 1], vd[q * 8 + i], vd[q * 8 + i + 1], c2, ptx::pack2(L[i], L[i + 1]),
-                                  ptx::pack2(D[i], D[i + 1]), diag && r > c + dq0, diag && r > c + 1 + dq0, p + i, ds + i);
-                    }
-                    pk[q] = pack8(p);
-                    dk[q] = pack8(ds);
-                }
-                if (!free_seen) ok = ok && ptx::mbar_wait(acc_done, (it - 1) & 1, abort_flag, status, LLMK_ST_TIMEOUT_ACC_FULL, 1000 + it);
-                free_seen = true;
-#pragma unroll
-                for (int q = 0; q < 4; q++) {
-                    store_chunk(sPt, r, c4 * 4 + q, pk[q]);
-                    store_chunk(sdSt, r, c4 * 4 + q, dk[q]);
-                }
-            };
-            // this warp's share of the sub-tile's columns: chunks [sub * NCH, (sub + 1) * NCH)
-            constexpr int NCH = BN / 64;
-            const int c_first = sub * NCH;
-            ptx::tmem_ld_32x32b_x32(t_st + lane_off + c_first * 32, vsA);
-            ptx::tmem_ld_32x32b_x32(t_dpt + lane_off + c_first * 32, vdA);
-#pragma unroll
-            for (int i4 = 0; i4 < NCH; i4++) {
-                const int c4 = c_first + i4;
-                ptx::tmem_ld_wait();
-                if (i4 + 1 < NCH) {
-                    ptx::tmem_ld_32x32b_x32(t_st + lane_off + (c4 + 1) * 32, (i4 & 1) ? vsA : vsB);
-                    ptx::tmem_ld_32x32b_x32(t_dpt + lane_off + (c4 + 1) * 32, (i4 & 1) ? vdA : vdB);
-                }
-                if (i4 & 1) process(c4, vsB, vdB);
-                else process(c4, vsA, vdA);
+                for (int i = 0; i < 32; i++)
+                    if (r > i + dq0) vs[i] = 0xff800000u;
             }
+            // P^T in place of S^T
+#pragma unroll
+            for (int i = 0; i < 32; i += 4) {
+                const float4 L = *reinterpret_cast<const float4*>(sL + i);
+                exp_pair(vs[i], vs[i + 1], c2, ptx::pack2(L.x, L.y));
+                exp_pair(vs[i + 2], vs[i + 3], c2, ptx::pack2(L.z, L.w));
+            }
+            // dS^T = P^T * (dP^T - D)
+            ok = ptx::mbar_wait(d_full, it & 1, abort_flag, status, LLMK_ST_TIMEOUT_TMA_FULL, 6000 + it);
             if (!ok) break;
+            bf16x8 pk[4], dk[4];
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                float p[8], ds[8], D[8];
+                *reinterpret_cast<float4*>(D) = *reinterpret_cast<const float4*>(sD + q * 8);
+                *reinterpret_cast<float4*>(D + 4) = *reinterpret_cast<const float4*>(sD + q * 8 + 4);
+#pragma unroll
+                for (int i = 0; i < 8; i += 2) {
+                    p[i] = __uint_as_float(vs[q * 8 + i]);
+                    p[i + 1] = __uint_as_float(vs[q * 8 + i + 1]);
+                    const ptx::f32x2 t = ptx::add2(ptx::pack2(__uint_as_float(vd[q * 8 + i]), __uint_as_float(vd[q * 8 + i + 1])), ptx::pack2(D[i], D[i + 1]));
+                    ptx::unpack2(ptx::mul2(ptx::pack2(p[i], p[i + 1]), t), ds[i], ds[i + 1]);
+                }
+                pk[q] = pack8(p);
+                dk[q] = pack8(ds);
+            }
+            // (P^T and dS^T stay in registers until the products of the previous sub-tile have read the buffers they go to)
+            if (it > 0) ok = ptx::mbar_wait(acc_done, (it - 1) & 1, abort_flag, status, LLMK_ST_TIMEOUT_ACC_FULL, 1000 + it);
+            if (!ok) break;
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                store_chunk(sPt, r, sub * 4 + q, pk[q]);
+                store_chunk(sdSt, r, sub * 4 + q, dk[q]);
+            }
             ptx::tc_fence_before();
             ptx::fence_proxy_async_smem();
             __syncwarp();
@@ -372,8 +388,9 @@ attn_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_c
         if (ok) {
             ptx::tc_fence_after();
             // dK (scaled) and dV -> bf16 -> the P^T / dS^T buffers as [128 x 64] staging tiles per 64 columns -> TMA stores
-            uint8_t* stage_dk = sPt;    // HS/64 tiles of 16 KB each fit: BM*BN*2 >= BM*HS*2 for both head sizes
-            uint8_t* stage_dv = sdSt;
+            // (HS = 128: dK takes both buffers, dV the ring, whose last reader was the last accumulation)
+            uint8_t* stage_dk = sPt;
+            uint8_t* stage_dv = HS == 64 ? sdSt : sRing;
 #pragma unroll
             for (int h4 = sub; h4 < HS / 32; h4 += 2) {
                 uint32_t v[32];
@@ -692,13 +709,15 @@ attn_bwd_dkv2_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_con
 // ====================================================================================== dQ
 template <int HS>
 struct DqCfg {
-    static constexpr int BN = Inner<HS>::BN;
+    static constexpr int BN = Inner<HS>::DQ_BN;
+    static constexpr int RING = HS == 64 ? 4 : 2;
     static constexpr int TILE = BM * HS * 2;   // Q or dO
     static constexpr int RT = BN * HS * 2;     // K or V sub-tile
-    static constexpr int OFF_Q = 0, OFF_DO = TILE, OFF_RING = 2 * TILE;   // ring: [2][K, V]
-    static constexpr int OFF_DS = OFF_RING + 4 * RT;
+    static constexpr int OFF_Q = 0, OFF_DO = TILE, OFF_RING = 2 * TILE;   // ring: [RING][K, V]
+    static constexpr int OFF_DS = OFF_RING + RING * 2 * RT;
     static constexpr int OFF_BAR = OFF_DS + BM * BN * 2;
     static constexpr int SMEM_BYTES = OFF_BAR + 128;
+    static_assert(Inner<HS>::CTAS * (SMEM_BYTES + 1024) <= 228 * 1024, "the CTAs of an SM share its shared memory");
     static constexpr int TMEM = (2 * BN + HS) <= 256 ? 256 : 512;
 };
 
@@ -710,10 +729,9 @@ attn_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_co
                       int* status, const float2* __restrict__ rope, int Tkv, int causal, const TileOrder order) {
     // Tkv / causal: as in the dK/dV kernel; here tmQKVin (the key / value sub-tiles) may cover another chunk
     using C = DqCfg<HS>;
-    constexpr int BN = C::BN;
+    constexpr int BN = C::BN, RING = C::RING;
     extern __shared__ __align__(1024) uint8_t smem[];
     // a failure already recorded makes the CTA return; the word is fetched beside the set-up
-    __shared__ int skip;
     const int failed = threadIdx.x == 0 && status != nullptr ? *reinterpret_cast<volatile int*>(status) : 0;
     if (ptx::smem_u32(smem) & 1023u) {
         if (threadIdx.x == 0 && status != nullptr) atomicCAS(status, 0, LLMK_ST_BOUNDS);
@@ -725,14 +743,16 @@ attn_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_co
     uint8_t* sdS = smem + C::OFF_DS;
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C::OFF_BAR);
     uint64_t* q_full = bars;
-    uint64_t* ring_full = bars + 1;   // [2]
-    uint64_t* ring_empty = bars + 3;  // [2]
-    uint64_t* s_full = bars + 5;
-    uint64_t* p_full = bars + 6;
-    uint64_t* acc_done = bars + 7;
-    uint64_t* epi = bars + 8;
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 9);
+    uint64_t* ring_full = bars + 1;    // [4]
+    uint64_t* ring_empty = bars + 5;   // [4]
+    uint64_t* s_full = bars + 9;
+    uint64_t* s_free = bars + 10;      // S and dP have been read into registers
+    uint64_t* p_full = bars + 11;
+    uint64_t* acc_done = bars + 12;
+    uint64_t* epi = bars + 13;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 14);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+    int* skip = reinterpret_cast<int*>(tmem_slot + 2);   // (no static shared memory)
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     int rank, pair;
@@ -746,30 +766,31 @@ attn_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_co
     const float scale_log2 = scale * LOG2E;
 
     auto load_kv = [&](int j) {   // one thread
-        const int s = j & 1;
+        const int s = j % RING;
         ptx::mbar_arrive_expect_tx(&ring_full[s], 2 * C::RT);
         load_tile<HS, BN>(sRing + s * 2 * C::RT, &tmQKVin, &ring_full[s], k_col, j * BN, b);
         load_tile<HS, BN>(sRing + s * 2 * C::RT + C::RT, &tmQKVin, &ring_full[s], v_col, j * BN, b);
     };
     if (threadIdx.x == 0) {
         ptx::mbar_init(q_full, 1);
-        for (int i = 0; i < 2; i++) {
+        for (int i = 0; i < RING; i++) {
             ptx::mbar_init(&ring_full[i], 1);
             ptx::mbar_init(&ring_empty[i], 1);
         }
         ptx::mbar_init(s_full, 1);
+        ptx::mbar_init(s_free, 8);
         ptx::mbar_init(p_full, 8);
         ptx::mbar_init(acc_done, 1);
         ptx::mbar_init(epi, 8);
         *abort_flag = 0;
         ptx::fence_barrier_init();
         ptx::fence_proxy_async_smem();
-        skip = failed;
+        *skip = failed;
         if (!failed) {
             ptx::mbar_arrive_expect_tx(q_full, 2 * C::TILE);
             load_tile<HS, BM>(sQ, &tmQKV, q_full, q_col, q0, b);
             load_tile<HS, BM>(sdO, &tmDO, q_full, q_col, q0, b);
-            for (int j = 0; j < 2 && j < nkv; j++) load_kv(j);
+            for (int j = 0; j < RING && j < nkv; j++) load_kv(j);
         }
     }
     if (warp == 1) {
@@ -780,62 +801,57 @@ attn_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_co
     __syncthreads();
     ptx::tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
-    if (skip) {
+    if (*skip) {
         if (warp == 1) ptx::tmem_dealloc(tmem_base, C::TMEM);
         return;
     }
     const uint32_t t_s = tmem_base, t_dp = tmem_base + BN, t_dq = tmem_base + 2 * BN;
 
     if (warp == 0) {
-        for (int j = 2; j < nkv; j++) {   // (Q, dO and the first two sub-tiles: above)
-            if (!ptx::mbar_wait(&ring_empty[j & 1], ((j >> 1) & 1) ^ 1, abort_flag, status, LLMK_ST_TIMEOUT_TMA_EMPTY, j)) break;
+        for (int j = RING; j < nkv; j++) {   // (Q, dO and the first sub-tiles: above)
+            if (!ptx::mbar_wait(&ring_empty[j % RING], ((j / RING) & 1) ^ 1, abort_flag, status, LLMK_ST_TIMEOUT_TMA_EMPTY, j)) break;
             if (lane == 0) load_kv(j);
             __syncwarp();
         }
     } else if (warp == 1) {
         constexpr uint32_t idesc_s = ptx::make_idesc_bf16(BM, BN, 0, 0);
         constexpr uint32_t idesc_acc = ptx::make_idesc_bf16(BM, HS, 0, 1);
-        bool ok = ptx::mbar_wait_spin(q_full, 0, abort_flag, status, LLMK_ST_TIMEOUT_TMA_FULL, -1);
-        const uint64_t q_desc = kmajor_desc<BM>(ptx::smem_u32(sQ), 0), do_desc = kmajor_desc<BM>(ptx::smem_u32(sdO), 0);
-        const uint64_t ds_desc = kmajor_desc<BM>(ptx::smem_u32(sdS), 0);
-        const uint32_t ring_addr = ptx::smem_u32(sRing);
-        auto issue_s = [&](int j) -> bool {
-            const int s = j & 1;
-            if (!ptx::mbar_wait_spin(&ring_full[s], (j >> 1) & 1, abort_flag, status, LLMK_ST_TIMEOUT_TMA_FULL, j)) return false;
-            ptx::tc_fence_after();
-            if (ptx::elect_one()) {
-                const uint64_t k_desc = kmajor_desc<BN>(ring_addr + s * 2 * C::RT, 0), v_desc = kmajor_desc<BN>(ring_addr + s * 2 * C::RT + C::RT, 0);
+        if (lane == 0) {   // as in the dK / dV kernel
+            bool ok = ptx::mbar_wait_spin(q_full, 0, abort_flag, status, LLMK_ST_TIMEOUT_TMA_FULL, -1);
+            const uint64_t q_desc = kmajor_desc<BM>(ptx::smem_u32(sQ), 0), do_desc = kmajor_desc<BM>(ptx::smem_u32(sdO), 0);
+            const uint64_t ds_desc = kmajor_desc<BM>(ptx::smem_u32(sdS), 0);
+            const uint64_t k0_desc = kmajor_desc<BN>(ptx::smem_u32(sRing), 0), kmn0_desc = mnmajor_desc<BN>(ptx::smem_u32(sRing), 0);
+            for (int j = 0; j <= nkv && ok; j++) {
+                if (j < nkv) {
+                    const int s = j % RING;
+                    ok = ptx::mbar_wait_spin(&ring_full[s], (j / RING) & 1, abort_flag, status, LLMK_ST_TIMEOUT_TMA_FULL, j);
+                    if (ok && j > 0) ok = ptx::mbar_wait_spin(s_free, (j - 1) & 1, abort_flag, status, LLMK_ST_TIMEOUT_ACC_EMPTY, 3000 + j);
+                    if (!ok) break;
+                    ptx::tc_fence_after();
+                    const uint64_t k_desc = k0_desc + (uint64_t)((s * 2 * C::RT) >> 4), v_desc = k_desc + (uint64_t)(C::RT >> 4);
 #pragma unroll
-                for (int kk = 0; kk < HS / 16; kk++)
-                    ptx::mma_f16_ss(t_s, kmajor_step<BM>(q_desc, kk), kmajor_step<BN>(k_desc, kk), idesc_s, kk > 0 ? 1u : 0u);
+                    for (int kk = 0; kk < HS / 16; kk++)
+                        ptx::mma_f16_ss(t_s, kmajor_step<BM>(q_desc, kk), kmajor_step<BN>(k_desc, kk), idesc_s, kk > 0 ? 1u : 0u);
 #pragma unroll
-                for (int kk = 0; kk < HS / 16; kk++)
-                    ptx::mma_f16_ss(t_dp, kmajor_step<BM>(do_desc, kk), kmajor_step<BN>(v_desc, kk), idesc_s, kk > 0 ? 1u : 0u);
-                ptx::mma_commit(s_full);
-            }
-            __syncwarp();
-            return true;
-        };
-        if (ok) ok = issue_s(0);
-        for (int j = 0; j < nkv && ok; j++) {
-            const int s = j & 1;
-            ok = ptx::mbar_wait_spin(p_full, j & 1, abort_flag, status, LLMK_ST_TIMEOUT_ACC_EMPTY, j);
-            if (!ok) break;
-            ptx::tc_fence_after();
-            if (j + 1 < nkv) {
-                ok = issue_s(j + 1);
-                if (!ok) break;
-            }
-            if (ptx::elect_one()) {
-                const uint64_t k_mn = mnmajor_desc<BN>(ring_addr + s * 2 * C::RT, 0);
+                    for (int kk = 0; kk < HS / 16; kk++)
+                        ptx::mma_f16_ss(t_dp, kmajor_step<BM>(do_desc, kk), kmajor_step<BN>(v_desc, kk), idesc_s, kk > 0 ? 1u : 0u);
+                    ptx::mma_commit(s_full);
+                }
+                if (j > 0) {
+                    const int jj = j - 1, s = jj % RING;
+                    ok = ptx::mbar_wait_spin(p_full, jj & 1, abort_flag, status, LLMK_ST_TIMEOUT_ACC_EMPTY, jj);
+                    if (!ok) break;
+                    ptx::tc_fence_after();
+                    const uint64_t k_mn = kmn0_desc + (uint64_t)((s * 2 * C::RT) >> 4);
 #pragma unroll
-                for (int kk = 0; kk < BN / 16; kk++)
-                    ptx::mma_f16_ss(t_dq, kmajor_step<BM>(ds_desc, kk), mnmajor_step(k_mn, kk), idesc_acc, (j > 0 || kk > 0) ? 1u : 0u);
-                ptx::mma_commit(&ring_empty[s]);
-                ptx::mma_commit(acc_done);
+                    for (int kk = 0; kk < BN / 16; kk++)
+                        ptx::mma_f16_ss(t_dq, kmajor_step<BM>(ds_desc, kk), mnmajor_step(k_mn, kk), idesc_acc, (jj > 0 || kk > 0) ? 1u : 0u);
+                    ptx::mma_commit(&ring_empty[s]);
+                    ptx::mma_commit(acc_done);
+                }
             }
-            __syncwarp();
         }
+        __syncwarp();
     } else {
         const int lane_group = warp & 3;
         const int sub = (warp - 2) >> 2;                     // 0 / 1: which half of the columns this warp handles
@@ -850,45 +866,49 @@ attn_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_co
             ok = ptx::mbar_wait(s_full, j & 1, abort_flag, status, LLMK_ST_TIMEOUT_ACC_FULL, j);
             if (!ok) break;
             ptx::tc_fence_after();
-            const int dk0 = j * BN - q0;            // first key of the sub-tile relative to the first query
-            const bool diag = causal && dk0 + BN > 0;   // reaches past the first query: some pairs are masked
-            uint32_t vsA[32], vdA[32], vsB[32], vdB[32];
-            bool free_seen = j == 0;   // dS stays in registers until the previous accumulation has read its buffer
-            auto process = [&](int c4, const uint32_t (&vs)[32], const uint32_t (&vd)[32]) {
-                bf16x8 dk[4];
-#pragma unroll
-                for (int q = 0; q < 4; q++) {
-                    float ds[8], p[8];
-#pragma unroll
-                    for (int i = 0; i < 8; i += 2) {
-                        const int c = c4 * 32 + q * 8 + i;   // key column of the sub-tile
-                        prob_pair(vs[q * 8 + i], vs[q * 8 + i + 1], vd[q * 8 + i], vd[q * 8 + i + 1], c2, nl2, nd2,
-                                  diag && c + dk0 > r, diag && c + 1 + dk0 > r, p + i, ds + i);
-                    }
-                    dk[q] = pack8(ds);
-                }
-                if (!free_seen) ok = ok && ptx::mbar_wait(acc_done, (j - 1) & 1, abort_flag, status, LLMK_ST_TIMEOUT_ACC_FULL, 1000 + j);
-                free_seen = true;
-#pragma unroll
-                for (int q = 0; q < 4; q++) store_chunk(sdS, r, c4 * 4 + q, dk[q]);
-            };
-            // this warp's share of the sub-tile's columns: chunks [sub * NCH, (sub + 1) * NCH)
+            // this warp's share of the sub-tile's columns
             constexpr int NCH = BN / 64;
-            const int c_first = sub * NCH;
-            ptx::tmem_ld_32x32b_x32(t_s + lane_off + c_first * 32, vsA);
-            ptx::tmem_ld_32x32b_x32(t_dp + lane_off + c_first * 32, vdA);
+            uint32_t vs[NCH][32], vd[NCH][32];
 #pragma unroll
             for (int i4 = 0; i4 < NCH; i4++) {
-                const int c4 = c_first + i4;
-                ptx::tmem_ld_wait();
-                if (i4 + 1 < NCH) {
-                    ptx::tmem_ld_32x32b_x32(t_s + lane_off + (c4 + 1) * 32, (i4 & 1) ? vsA : vsB);
-                    ptx::tmem_ld_32x32b_x32(t_dp + lane_off + (c4 + 1) * 32, (i4 & 1) ? vdA : vdB);
-                }
-                if (i4 & 1) process(c4, vsB, vdB);
-                else process(c4, vsA, vdA);
+                ptx::tmem_ld_32x32b_x32(t_s + lane_off + (sub * NCH + i4) * 32, vs[i4]);
+                ptx::tmem_ld_32x32b_x32(t_dp + lane_off + (sub * NCH + i4) * 32, vd[i4]);
             }
+            ptx::tmem_ld_wait();
+            ptx::tc_fence_before();
+            __syncwarp();
+            if (lane == 0) ptx::mbar_arrive(s_free);
+            const int dk0 = j * BN + sub * NCH * 32 - q0;   // first key of this warp's columns relative to the first query
+            if (causal && dk0 + NCH * 32 > lane_group * 32) {   // some of them lie after some of its queries: P = 0
+#pragma unroll
+                for (int i4 = 0; i4 < NCH; i4++)
+#pragma unroll
+                    for (int i = 0; i < 32; i++)
+                        if (i4 * 32 + i + dk0 > r) vs[i4][i] = 0xff800000u;
+            }
+            bf16x8 dk[NCH][4];
+#pragma unroll
+            for (int i4 = 0; i4 < NCH; i4++) {
+#pragma unroll
+                for (int i = 0; i < 32; i += 2) exp_pair(vs[i4][i], vs[i4][i + 1], c2, nl2);
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    float ds[8];
+#pragma unroll
+                    for (int i = q * 8; i < q * 8 + 8; i += 2) {
+                        const ptx::f32x2 t = ptx::add2(ptx::pack2(__uint_as_float(vd[i4][i]), __uint_as_float(vd[i4][i + 1])), nd2);
+                        ptx::unpack2(ptx::mul2(ptx::pack2(__uint_as_float(vs[i4][i]), __uint_as_float(vs[i4][i + 1])), t), ds[i - q * 8], ds[i + 1 - q * 8]);
+                    }
+                    dk[i4][q] = pack8(ds);
+                }
+            }
+            // (dS stays in registers until the previous accumulation has read its buffer)
+            if (j > 0) ok = ptx::mbar_wait(acc_done, (j - 1) & 1, abort_flag, status, LLMK_ST_TIMEOUT_ACC_FULL, 1000 + j);
             if (!ok) break;
+#pragma unroll
+            for (int i4 = 0; i4 < NCH; i4++)
+#pragma unroll
+                for (int q = 0; q < 4; q++) store_chunk(sdS, r, (sub * NCH + i4) * 4 + q, dk[i4][q]);
             ptx::tc_fence_before();
             ptx::fence_proxy_async_smem();
             __syncwarp();
@@ -939,7 +959,7 @@ template <int HS>
 static int launch(const void* qkv, const void* dout, bf16* dqkv, const float* lse, const float* dvec, int B, int T, int NH, int NKVH,
                   int* status, const float2* rope, cudaStream_t stream, const void* kv_qkv = nullptr, bf16* dkv_out = nullptr,
                   int Tkv = 0, int causal = 1) {
-    constexpr int BN = Inner<HS>::BN;
+    constexpr int BN = Inner<HS>::DQ_BN, BN_KV = DkvCfg<HS>::BN;
     const bool ring = kv_qkv != nullptr;
     if (!ring) { kv_qkv = qkv; dkv_out = dqkv; Tkv = T; causal = 1; }
     static PerDeviceOnce once_configured;
@@ -956,9 +976,9 @@ static int launch(const void* qkv, const void* dout, bf16* dqkv, const float* ls
     CUtensorMap tq, tq_in, tdo, tdo_in, tdqkv, tkv, tkv_in, tdkv;
     int rc;
     if ((rc = gemm::make_tmap_3d(&tq, qkv, width, T, B, 64, BM))) return rc;
-    if ((rc = gemm::make_tmap_3d(&tq_in, qkv, width, T, B, 64, BN))) return rc;
+    if ((rc = gemm::make_tmap_3d(&tq_in, qkv, width, T, B, 64, BN_KV))) return rc;
     if ((rc = gemm::make_tmap_3d(&tdo, dout, cw, T, B, 64, BM))) return rc;
-    if ((rc = gemm::make_tmap_3d(&tdo_in, dout, cw, T, B, 64, BN))) return rc;
+    if ((rc = gemm::make_tmap_3d(&tdo_in, dout, cw, T, B, 64, BN_KV))) return rc;
     if ((rc = gemm::make_tmap_3d(&tdqkv, dqkv, width, T, B, 64, BM))) return rc;
     if ((rc = gemm::make_tmap_3d(&tkv, kv_qkv, width, Tkv, B, 64, BM))) return rc;
     if ((rc = gemm::make_tmap_3d(&tkv_in, kv_qkv, width, Tkv, B, 64, BN))) return rc;
