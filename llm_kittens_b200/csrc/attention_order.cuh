@@ -33,4 +33,12 @@ __host__ __device__ inline void tile_of(const TileOrder& o, int idx, int& rank, 
     pair = first + r - rank * in_group;
 }
 
+// The k-th tile of block `block` of a grid of fewer blocks than tiles, or `n` behind the last one: back and forth over the
+// blocks. Tiles get shorter along the order, so with every block taking the same place in each turn the first one would
+// have the longest of every turn (32 heads of 32 tiles on 148 blocks: 168 us one tile per block, 184 that way, 163 so).
+__host__ __device__ inline int tile_of_turn(int n, int block, int blocks, int k) {
+    const int idx = k * blocks + ((k & 1) ? blocks - 1 - block : block);
+    return idx < n ? idx : n;
+}
+
 }  // namespace llmk

@@ -5,9 +5,10 @@
 // which has no sm_100 path; the warp-level implementation in attention.cu remains for short sequences and
 // small calls whose length is not a multiple of 128 (ops/attention.py has the rule).
 //
-// One CTA per (128 query rows, head, batch); 8 warps:
-//   warp 0     TMA producer: K / V tiles of 128 rows through rings of two, freed apart (K after S, V after P V); prefetches
-//              the tiles after the ring, and the first tiles of the CTA that will take its place, into the L2
+// Persistent CTAs that take (128 query rows, head, batch) tiles in turns; 8 warps:
+//   warp 0     TMA producer: K / V tiles of 128 rows through rings of two, freed apart (K after S, V after P V); decodes the
+//              tiles (a dozen divisions, 1000 cycles in the path of whoever waits for them) and prefetches the key tiles
+//              after the ring, and the first ones of the next query tile, into the L2
 //   warp 1     MMA issuer:   S = Q K^T  (128x128xHS, both operands K-major)  -> TMEM columns [0,128)
 //                            O += P V   (128xHSx128, P K-major from smem, V MN-major) -> TMEM [128,128+HS)
 //   warps 4-7  softmax:      one query row per thread (TMEM lane = row, so no cross-thread reductions):
@@ -21,9 +22,11 @@
 // the softmax threads the registers of the first warpgroup: a whole S row is in registers) and one's softmax overlaps the
 // other's waits, first loads and epilogue. Two query tiles in one CTA instead run in step: both take their exponentials at
 // the same time and wait at the same time (4200 cycles per pair of tiles, 3000 here), and nothing fills a CTA's beginning
-// and end. us, pair of tiles per CTA / this: B64 T1024 12 heads 313 / 240, B16 T1024 16 heads 107 / 79, B8 T2048 12 heads 129 / 94,
-// B1 T1024 12 heads 21.9 / 13.8. HS = 128 (one CTA per SM) with the same code, chunks with branches before: B1 T4096 32/8 heads
-// 242 / 168, B2 T2048 16 heads 81 / 55.
+// and end. A CTA for each tile spends 8000 cycles on its launch, set-up, first loads and epilogue (at T = 1024 a tile's loop
+// is 12,000); persistent ones load the next tile's Q and compute its first scores beside the epilogue, which leaves 2500.
+// us, pair of tiles per CTA / one CTA per tile / this: B64 T1024 12 heads 313 / 240 / 217, B16 T1024 16 heads 107 / 79 / 75, B16
+// T512 16 heads 40.8 / 30.7 / 28.2, B32 T256 12 heads 25.6 / 19.4 / 15.6, B8 T2048 12 heads 129 / 94 / 95, B1 T1024 12 heads 21.9 / 13.8 /
+// 14.3. HS = 128 (one CTA per SM; before: chunks with branches): B1 T4096 32/8 heads 242 / 168 / 165, B2 T2048 16 heads 81 / 55 / 51.
 // Every wait is bounded and reports through the status word.
 
 #include "attention_order.cuh"
@@ -44,7 +47,8 @@ struct Cfg {
     static constexpr int TILE_BYTES = BQ * HS * 2;         // Q, K or V tile
     static constexpr int P_BYTES = BQ * BKV * 2;
     static constexpr int SMEM_MAIN = TILE_BYTES * 5 + P_BYTES;
-    static constexpr int SMEM_BYTES = SMEM_MAIN + 128;   // tiles + barriers; the dynamic window itself is 1024-byte aligned
+    static constexpr int SMEM_BYTES = SMEM_MAIN + 192;   // tiles + barriers; the dynamic window itself is 1024-byte aligned
+    static_assert((HS == 64 ? 2 : 1) * (SMEM_BYTES + 1024) <= 228 * 1024, "the CTAs of an SM share its shared memory");
     static constexpr int TMEM_COLS = 256;
     static constexpr int CTAS_PER_SM = HS == 64 ? 2 : 1;
 };
@@ -137,8 +141,8 @@ template <int HS, bool ROUND>
 __global__ void __launch_bounds__(THREADS, Cfg<HS>::CTAS_PER_SM)
 attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant__ CUtensorMap tmKV,
                    const __grid_constant__ CUtensorMap tmOut, float* __restrict__ lse, int T, int Tkv, int causal, int NH, int NKVH,
-                   float scale_log2, int* status, const TileOrder order, int ahead) {
-    // ahead: CTAs that the chip holds at once, 0 = nothing is prefetched into the L2 (keys and values of another GPU).
+                   float scale_log2, int* status, const TileOrder order, int local) {
+    // local = 0: nothing is prefetched into the L2 (keys and values of another GPU).
     // tmKV / Tkv / causal: the keys and values may come from ANOTHER packed QKV tensor of the same layout (a peer's
     // chunk of the sequence in context-parallel attention; the map may cover that peer's memory, loads only, no
     // multicast). causal = 1: queries and keys cover the same positions (the usual case, tmKV == tmQKV); causal = 0:
@@ -167,36 +171,44 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_const
     uint64_t* p_full = bars + 10;     // [1]
     uint64_t* o_full = bars + 11;     // [1]
     uint64_t* s_free = bars + 12;     // [1]
-    uint64_t* epi = bars + 13;        // [1]
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 14);
+    uint64_t* q_empty = bars + 13;    // [1] the last S of a query tile is computed
+    uint64_t* o_free = bars + 14;     // [1] O of a query tile has been read
+    uint64_t* info_full = bars + 15;  // [2] the tile that a turn takes has been decoded
+    int4* info = reinterpret_cast<int4*>(bars + 18);   // [2] (key tiles, query tile, head, batch entry), 0 key tiles = no more
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 22);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
     int* skip = reinterpret_cast<int*>(tmem_slot + 2);   // (no static shared memory: two CTAs fill the SM's)
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    int rank, pair;
-    tile_of(order, blockIdx.x, rank, pair);
-    const int qb = order.tiles - 1 - rank;  // late (long) query blocks first
-    const int h = pair % NH, b = pair / NH;
-    const int hk = h / (NH / NKVH);
-    const int nkv = causal ? qb + 1 : Tkv / BKV;
-    const int q_col = h * HS, k_col = (NH + hk) * HS, v_col = (NH + NKVH + hk) * HS;
-
-    auto load_tile = [&](uint8_t* dst, uint64_t* bar, int col, int j) {   // one thread
+    const int n_tiles = order.tiles * order.heads;
+    auto turn = [&](int k) { return tile_of_turn(n_tiles, blockIdx.x, gridDim.x, k); };   // this CTA's tiles
+    struct Tile { int qb, h, b, nkv, q_col, k_col, v_col; };
+    auto tile_at = [&](int idx) {
+        Tile t;
+        int rank, pair;
+        tile_of(order, idx, rank, pair);
+        t.qb = order.tiles - 1 - rank;  // late (long) query blocks first
+        t.h = pair % NH;
+        t.b = pair / NH;
+        const int hk = t.h / (NH / NKVH);
+        t.nkv = causal ? t.qb + 1 : Tkv / BKV;
+        t.q_col = t.h * HS;
+        t.k_col = (NH + hk) * HS;
+        t.v_col = (NH + NKVH + hk) * HS;
+        return t;
+    };
+    // one thread; c counts the key tiles of this CTA
+    auto load_tile = [&](uint8_t* dst, uint64_t* bar, const CUtensorMap* tm, int col, int row, int b) {
         ptx::mbar_arrive_expect_tx(bar, C::TILE_BYTES);
 #pragma unroll
-        for (int c = 0; c < HS / 64; c++) ptx::tma_load_3d(dst + c * ATOM_BYTES, &tmKV, bar, col + 64 * c, j * BKV, b);
+        for (int k = 0; k < HS / 64; k++) ptx::tma_load_3d(dst + k * ATOM_BYTES, tm, bar, col + 64 * k, row, b);
     };
-    auto prefetch_kv = [&](int j) {
-#pragma unroll
-        for (int c = 0; c < HS / 64; c++) {
-            ptx::tma_prefetch_3d(&tmKV, k_col + 64 * c, j * BKV, b);
-            ptx::tma_prefetch_3d(&tmKV, v_col + 64 * c, j * BKV, b);
-        }
-    };
-    auto load_k = [&](int j) { load_tile(sK + (j & 1) * C::TILE_BYTES, &k_full[j & 1], k_col, j); };
-    auto load_v = [&](int j) { load_tile(sV + (j & 1) * C::TILE_BYTES, &v_full[j & 1], v_col, j); };
+    auto load_q = [&](const Tile& t) { load_tile(sQ, q_full, &tmQKV, t.q_col, t.qb * BQ, t.b); };
+    auto load_k = [&](const Tile& t, int j, int c) { load_tile(sK + (c & 1) * C::TILE_BYTES, &k_full[c & 1], &tmKV, t.k_col, j * BKV, t.b); };
+    auto load_v = [&](const Tile& t, int j, int c) { load_tile(sV + (c & 1) * C::TILE_BYTES, &v_full[c & 1], &tmKV, t.v_col, j * BKV, t.b); };
     if (threadIdx.x == 0) {
         ptx::mbar_init(q_full, 1);
+        ptx::mbar_init(q_empty, 1);
         for (int i = 0; i < 2; i++) {
             ptx::mbar_init(&k_full[i], 1);
             ptx::mbar_init(&k_empty[i], 1);
@@ -206,19 +218,22 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_const
         ptx::mbar_init(s_full, 1);
         ptx::mbar_init(p_full, 4);
         ptx::mbar_init(o_full, 1);
+        ptx::mbar_init(o_free, 4);
         ptx::mbar_init(s_free, 4);
-        ptx::mbar_init(epi, 4);
+        ptx::mbar_init(&info_full[0], 1);
+        ptx::mbar_init(&info_full[1], 1);
         *abort_flag = 0;
         ptx::fence_barrier_init();
         ptx::fence_proxy_async_smem();
         *skip = failed;
         if (!failed) {   // the first tiles are on their way while TMEM is allocated
-            ptx::mbar_arrive_expect_tx(q_full, C::TILE_BYTES);
-#pragma unroll
-            for (int c = 0; c < HS / 64; c++) ptx::tma_load_3d(sQ + c * ATOM_BYTES, &tmQKV, q_full, q_col + 64 * c, qb * BQ, b);
-            for (int j = 0; j < 2 && j < nkv; j++) {
-                load_k(j);
-                load_v(j);
+            const Tile t = tile_at(blockIdx.x);
+            info[0] = make_int4(t.nkv, t.qb, t.h, t.b);
+            ptx::mbar_arrive(&info_full[0]);
+            load_q(t);
+            for (int j = 0; j < 2 && j < t.nkv; j++) {
+                load_k(t, j, j);
+                load_v(t, j, j);
             }
         }
         ptx::prefetch_tmap(&tmOut);
@@ -240,79 +255,122 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_const
     if (warp < 4) {
         if (C::CTAS_PER_SM == 2) asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
         if (warp == 0) {
-            // -------------------------------------------------------- TMA producer (Q and the first two K / V tiles: above)
-            // The tiles after the ring are on their way from HBM into the L2 before there is room for them. For the CTA that
-            // will take this one's place (blocks start in order) the first tiles are: without that it waits 3000 cycles for
-            // its first scores.
-            if (ahead > 0 && lane == 0) {
-                for (int j = 2; j < 4 && j < nkv; j++) prefetch_kv(j);
-                const int next = blockIdx.x + ahead;
-                if (next < (int)gridDim.x) {
-                    int n_rank, n_pair;
-                    tile_of(order, next, n_rank, n_pair);
-                    const int n_h = n_pair % NH, n_b = n_pair / NH, n_hk = n_h / (NH / NKVH);
+            // -------------------------------------------------------- TMA producer (the first loads of the first tile: above)
+            // The key tiles behind the ring are on their way from HBM into the L2 before there is room for them, and so are
+            // the first ones of the next query tile: without that it waits 3000 cycles for its first scores.
+            bool ok = true;
+            int c = 0, n = 0;
+            for (int idx = turn(0); idx < n_tiles && ok; idx = turn(++n)) {
+                const Tile t = tile_at(idx);
+                auto prefetch_kv = [&](int j) {
 #pragma unroll
-                    for (int c = 0; c < HS / 64; c++) {
-                        ptx::tma_prefetch_3d(&tmQKV, n_h * HS + 64 * c, (order.tiles - 1 - n_rank) * BQ, n_b);
-                        ptx::tma_prefetch_3d(&tmKV, (NH + n_hk) * HS + 64 * c, 0, n_b);
-                        ptx::tma_prefetch_3d(&tmKV, (NH + NKVH + n_hk) * HS + 64 * c, 0, n_b);
+                    for (int k = 0; k < HS / 64; k++) {
+                        ptx::tma_prefetch_3d(&tmKV, t.k_col + 64 * k, j * BKV, t.b);
+                        ptx::tma_prefetch_3d(&tmKV, t.v_col + 64 * k, j * BKV, t.b);
+                    }
+                };
+                if (local && lane == 0) {
+                    for (int j = 2; j < 4 && j < t.nkv; j++) prefetch_kv(j);
+                    if (turn(n + 1) < n_tiles) {
+                        const Tile u = tile_at(turn(n + 1));
+#pragma unroll
+                        for (int k = 0; k < HS / 64; k++) {
+                            ptx::tma_prefetch_3d(&tmQKV, u.q_col + 64 * k, u.qb * BQ, u.b);
+                            ptx::tma_prefetch_3d(&tmKV, u.k_col + 64 * k, 0, u.b);
+                            ptx::tma_prefetch_3d(&tmKV, u.v_col + 64 * k, 0, u.b);
+                        }
                     }
                 }
+                __syncwarp();
+                for (int j = 0; j < t.nkv && ok; j++, c++) {
+                    if (n == 0 && j < 2) continue;
+                    const uint32_t ph = ((c >> 1) & 1) ^ 1;
+                    ok = ptx::mbar_wait(&k_empty[c & 1], ph, abort_flag, status, LLMK_ST_TIMEOUT_TMA_EMPTY, j);
+                    if (!ok) break;
+                    if (lane == 0) load_k(t, j, c);
+                    __syncwarp();
+                    if (j == 0) {
+                        ok = ptx::mbar_wait(q_empty, (n - 1) & 1, abort_flag, status, LLMK_ST_TIMEOUT_TMA_EMPTY, j);
+                        if (!ok) break;
+                        // (every reader of the slot's last content has waited for it: the scores of tile n-1 needed all of
+                        // them to be past tile n-2)
+                        if (lane == 0) {
+                            info[n & 1] = make_int4(t.nkv, t.qb, t.h, t.b);
+                            ptx::mbar_arrive(&info_full[n & 1]);
+                            load_q(t);
+                        }
+                        __syncwarp();
+                    }
+                    ok = ptx::mbar_wait(&v_empty[c & 1], ph, abort_flag, status, LLMK_ST_TIMEOUT_TMA_EMPTY, j);
+                    if (!ok) break;
+                    if (lane == 0) {
+                        load_v(t, j, c);
+                        if (local && j + 2 < t.nkv) prefetch_kv(j + 2);
+                    }
+                    __syncwarp();
+                }
             }
-            __syncwarp();
-            for (int j = 2; j < nkv; j++) {
-                const uint32_t ph = ((j >> 1) & 1) ^ 1;
-                if (ahead > 0 && lane == 0 && j + 2 < nkv) prefetch_kv(j + 2);
-                if (!ptx::mbar_wait(&k_empty[j & 1], ph, abort_flag, status, LLMK_ST_TIMEOUT_TMA_EMPTY, j)) break;
-                if (lane == 0) load_k(j);
-                __syncwarp();
-                if (!ptx::mbar_wait(&v_empty[j & 1], ph, abort_flag, status, LLMK_ST_TIMEOUT_TMA_EMPTY, j)) break;
-                if (lane == 0) load_v(j);
-                __syncwarp();
+            if (ok) ok = ptx::mbar_wait(q_empty, (n - 1) & 1, abort_flag, status, LLMK_ST_TIMEOUT_TMA_EMPTY, -3);
+            if (ok && lane == 0) {
+                info[n & 1] = make_int4(0, 0, 0, 0);
+                ptx::mbar_arrive(&info_full[n & 1]);
             }
         } else if (warp == 1 && lane == 0) {
             // -------------------------------------------------------- MMA issuer
-            // S(j+1) is issued as soon as the softmax warps have copied S(j) into registers (s_free), i.e. while they are
-            // still working on tile j; P V(j) follows when P(j) is in shared memory. O accumulates in TMEM. The
-            // descriptors are built once: inside the loop an MMA costs one integer add.
+            // S(c+1) is issued as soon as the softmax warps have copied S(c) into registers (s_free), i.e. while they are
+            // still working on tile c; P V(c) follows when P(c) is in shared memory. O accumulates in TMEM. The first S of
+            // the next query tile is computed beside the end of this one. The descriptors are built once: inside the loop
+            // an MMA costs one integer add.
             constexpr uint32_t idesc_s = ptx::make_idesc_bf16(BQ, BKV, 0, 0);
             constexpr uint32_t idesc_o = ptx::make_idesc_bf16(BQ, HS, 0, 1);
             const uint64_t q_desc = ptx::make_smem_desc(ptx::smem_u32(sQ), 16, 1024);
             const uint64_t k_desc = ptx::make_smem_desc(ptx::smem_u32(sK), 16, 1024);
             const uint64_t p_desc = ptx::make_smem_desc(ptx::smem_u32(sP), 16, 1024);
             const uint64_t v_desc = ptx::make_smem_desc(ptx::smem_u32(sV), ATOM_BYTES, 1024);
-            bool ok = ptx::mbar_wait_spin(q_full, 0, abort_flag, status, LLMK_ST_TIMEOUT_TMA_FULL, -1);
-            for (int j = 0; j <= nkv && ok; j++) {
-                if (j < nkv) {
-                    const int s = j & 1;
-                    ok = ptx::mbar_wait_spin(&k_full[s], (j >> 1) & 1, abort_flag, status, LLMK_ST_TIMEOUT_TMA_FULL, j);
-                    if (ok && j > 0) ok = ptx::mbar_wait_spin(s_free, (j - 1) & 1, abort_flag, status, LLMK_ST_TIMEOUT_ACC_EMPTY, 3000 + j);
-                    if (!ok) break;
-                    ptx::tc_fence_after();
-                    const uint64_t kd = k_desc + (uint64_t)((s * C::TILE_BYTES) >> 4);
+            bool ok = true;
+            int c = 0;
+            for (int n = 0; ok; n++) {
+                ok = ptx::mbar_wait_spin(&info_full[n & 1], (n >> 1) & 1, abort_flag, status, LLMK_ST_TIMEOUT_TMA_FULL, -2);
+                if (!ok) break;
+                const int nkv = info[n & 1].x;
+                if (nkv == 0) break;
+                ok = ptx::mbar_wait_spin(q_full, n & 1, abort_flag, status, LLMK_ST_TIMEOUT_TMA_FULL, -1);
+                for (int j = 0; j <= nkv && ok; j++, c++) {
+                    if (j < nkv) {
+                        const int s = c & 1;
+                        ok = ptx::mbar_wait_spin(&k_full[s], (c >> 1) & 1, abort_flag, status, LLMK_ST_TIMEOUT_TMA_FULL, j);
+                        if (ok && c > 0) ok = ptx::mbar_wait_spin(s_free, (c - 1) & 1, abort_flag, status, LLMK_ST_TIMEOUT_ACC_EMPTY, 3000 + j);
+                        if (!ok) break;
+                        ptx::tc_fence_after();
+                        const uint64_t kd = k_desc + (uint64_t)((s * C::TILE_BYTES) >> 4);
 #pragma unroll
-                    for (int kk = 0; kk < HS / 16; kk++) {
-                        const uint64_t off = (uint64_t)(((kk / 4) * ATOM_BYTES + (kk % 4) * 32) >> 4);
-                        ptx::mma_f16_ss(tmem_s, q_desc + off, kd + off, idesc_s, kk > 0 ? 1u : 0u);
+                        for (int kk = 0; kk < HS / 16; kk++) {
+                            const uint64_t off = (uint64_t)(((kk / 4) * ATOM_BYTES + (kk % 4) * 32) >> 4);
+                            ptx::mma_f16_ss(tmem_s, q_desc + off, kd + off, idesc_s, kk > 0 ? 1u : 0u);
+                        }
+                        ptx::mma_commit(s_full);
+                        ptx::mma_commit(&k_empty[s]);
+                        if (j == nkv - 1) ptx::mma_commit(q_empty);
                     }
-                    ptx::mma_commit(s_full);
-                    ptx::mma_commit(&k_empty[s]);
-                }
-                if (j > 0) {
-                    const int jj = j - 1, s = jj & 1;
-                    ok = ptx::mbar_wait_spin(&v_full[s], (jj >> 1) & 1, abort_flag, status, LLMK_ST_TIMEOUT_TMA_FULL, jj);
-                    // P(jj) is in shared memory (and O has been rescaled if the row maxima moved)
-                    if (ok) ok = ptx::mbar_wait_spin(p_full, jj & 1, abort_flag, status, LLMK_ST_TIMEOUT_ACC_EMPTY, jj);
-                    if (!ok) break;
-                    ptx::tc_fence_after();
-                    const uint64_t vd = v_desc + (uint64_t)((s * C::TILE_BYTES) >> 4);
+                    if (j > 0) {
+                        const int cc = c - 1, s = cc & 1;
+                        ok = ptx::mbar_wait_spin(&v_full[s], (cc >> 1) & 1, abort_flag, status, LLMK_ST_TIMEOUT_TMA_FULL, j);
+                        // P(cc) is in shared memory (and O has been rescaled if the row maxima moved, or read if this is the
+                        // first product of a query tile)
+                        if (ok) ok = ptx::mbar_wait_spin(p_full, cc & 1, abort_flag, status, LLMK_ST_TIMEOUT_ACC_EMPTY, j);
+                        if (ok && j == 1 && n > 0) ok = ptx::mbar_wait_spin(o_free, (n - 1) & 1, abort_flag, status, LLMK_ST_TIMEOUT_ACC_EMPTY, 7000);
+                        if (!ok) break;
+                        ptx::tc_fence_after();
+                        const uint64_t vd = v_desc + (uint64_t)((s * C::TILE_BYTES) >> 4);
 #pragma unroll
-                    for (int kk = 0; kk < BKV / 16; kk++)
-                        ptx::mma_f16_ss(tmem_o, p_desc + (uint64_t)(((kk / 4) * ATOM_BYTES + (kk % 4) * 32) >> 4),
-                                        vd + (uint64_t)((kk * 2048) >> 4), idesc_o, (jj > 0 || kk > 0) ? 1u : 0u);
-                    ptx::mma_commit(o_full);
-                    ptx::mma_commit(&v_empty[s]);
+                        for (int kk = 0; kk < BKV / 16; kk++)
+                            ptx::mma_f16_ss(tmem_o, p_desc + (uint64_t)(((kk / 4) * ATOM_BYTES + (kk % 4) * 32) >> 4),
+                                            vd + (uint64_t)((kk * 2048) >> 4), idesc_o, (j > 1 || kk > 0) ? 1u : 0u);
+                        ptx::mma_commit(o_full);
+                        ptx::mma_commit(&v_empty[s]);
+                    }
                 }
+                c--;   // (the loop's last turn has no scores)
             }
         }
         __syncwarp();
@@ -325,10 +383,15 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_const
         // m is the reference maximum of the exponentials (log2 units); it trails the true running maximum by at
         // most RESCALE_GAP, so P stays below 2^RESCALE_GAP and O / l are rescaled only when a row maximum jumps.
         constexpr float RESCALE_GAP = 8.f;
-        float m = -INFINITY, l = 0.f;
         bool ok = true;
-        for (int j = 0; j < nkv && ok; j++) {
-            ok = ptx::mbar_wait(s_full, j & 1, abort_flag, status, LLMK_ST_TIMEOUT_ACC_FULL, j);
+        int c = 0;
+        for (int n = 0; ok; n++) {
+        ok = ptx::mbar_wait(&info_full[n & 1], (n >> 1) & 1, abort_flag, status, LLMK_ST_TIMEOUT_TMA_FULL, -2);
+        const int nkv = info[n & 1].x;
+        if (!ok || nkv == 0) break;
+        float m = -INFINITY, l = 0.f;
+        for (int j = 0; j < nkv && ok; j++, c++) {
+            ok = ptx::mbar_wait(s_full, c & 1, abort_flag, status, LLMK_ST_TIMEOUT_ACC_FULL, j);
             if (!ok) break;
             ptx::tc_fence_after();
             uint32_t s[4][32];
@@ -343,11 +406,13 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_const
                 // the diagonal tile: -infinity after the row's own column, then the same code as every other tile
 #pragma unroll
                 for (int c4 = 0; c4 < 4; c4++) {
-                    const int last = (lane_group - c4) * 32 + lane;   // last column of this chunk that the row sees
-                    if (c4 >= lane_group) {
+                    if (c4 == lane_group) {
 #pragma unroll
                         for (int i = 0; i < 32; i++)
-                            if (i > last) s[c4][i] = 0xff800000u;
+                            if (i > lane) s[c4][i] = 0xff800000u;
+                    } else if (c4 > lane_group) {
+#pragma unroll
+                        for (int i = 0; i < 32; i++) s[c4][i] = 0xff800000u;
                     }
                 }
             }
@@ -364,9 +429,12 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_const
             constexpr int EARLY = 4;   // groups whose exponentials are taken before P V(j-1) has to be complete
 #pragma unroll
             for (int g = 0; g < EARLY; g++) group_exps(s, g, c2, m2);
-            if (j > 0) {
+            if (j == 0) {
+                if (lane == 0) ptx::tma_store_wait_read<0>();   // the previous query tile's O has left these rows of the P buffer
+                __syncwarp();
+            } else {
                 // P V(j-1) must be complete before P is overwritten and before O may be rescaled
-                ok = ptx::mbar_wait(o_full, (j - 1) & 1, abort_flag, status, LLMK_ST_TIMEOUT_ACC_FULL, 1000 + j);
+                ok = ptx::mbar_wait(o_full, (c - 1) & 1, abort_flag, status, LLMK_ST_TIMEOUT_ACC_FULL, 1000 + j);
                 if (!ok) break;
                 ptx::tc_fence_after();
                 if (rescale) {
@@ -389,38 +457,43 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_const
             __syncwarp();
             if (lane == 0) ptx::mbar_arrive(p_full);
         }
-        if (ok) ok = ptx::mbar_wait(o_full, (nkv - 1) & 1, abort_flag, status, LLMK_ST_TIMEOUT_ACC_FULL, 2000);
-        if (ok) {
-            // O -> bf16 -> the P buffer (128 rows x 128 bytes per 64 columns, swizzled like the tensor map) -> TMA store, which
-            // leaves out the rows past the end of the sequence (a ragged last tile)
-            ptx::tc_fence_after();
-            const float inv_l = 1.0f / l;
+        if (ok) ok = ptx::mbar_wait(o_full, (c - 1) & 1, abort_flag, status, LLMK_ST_TIMEOUT_ACC_FULL, 2000);
+        if (!ok) break;
+        // O -> bf16 -> this warp's rows of the P buffer (128 bytes per 64 columns, swizzled like the tensor map) -> TMA store,
+        // which leaves out the rows past the end of the sequence (a ragged last tile)
+        ptx::tc_fence_after();
+        const float inv_l = 1.0f / l;
+        bf16x8 o[HS / 8];
 #pragma unroll
-            for (int h4 = 0; h4 < HS / 32; h4++) {
-                uint32_t v[32];
-                ptx::tmem_ld_32x32b_x32(tmem_o + lane_off + h4 * 32, v);
-                ptx::tmem_ld_wait();
+        for (int h4 = 0; h4 < HS / 32; h4++) {
+            uint32_t v[32];
+            ptx::tmem_ld_32x32b_x32(tmem_o + lane_off + h4 * 32, v);
+            ptx::tmem_ld_wait();
 #pragma unroll
-                for (int q = 0; q < 4; q++) {
-                    float f[8];
+            for (int q = 0; q < 4; q++) {
+                float f[8];
 #pragma unroll
-                    for (int i = 0; i < 8; i++) f[i] = __uint_as_float(v[q * 8 + i]) * inv_l;
-                    *reinterpret_cast<bf16x8*>(sP + (h4 >> 1) * ATOM_BYTES + r * 128 + ((((h4 & 1) * 4 + q) ^ (r & 7)) << 4)) = pack8(f);
-                }
-            }
-            if (qb * BQ + r < T) lse[((size_t)b * NH + h) * T + qb * BQ + r] = (m + log2f(l)) * 0.6931471805599453f;
-            ptx::fence_proxy_async_smem();
-            __syncwarp();
-            if (lane == 0) ptx::mbar_arrive(epi);
-            if (lane_group == 0 && lane == 0) {
-                if (ptx::mbar_wait(epi, 0, abort_flag, status, LLMK_ST_TIMEOUT_ACC_FULL, 4000)) {
-#pragma unroll
-                    for (int c = 0; c < HS / 64; c++) ptx::tma_store_3d(&tmOut, sP + c * ATOM_BYTES, q_col + 64 * c, qb * BQ, b);
-                    ptx::tma_store_commit();
-                    ptx::tma_store_wait_read<0>();
-                }
+                for (int i = 0; i < 8; i++) f[i] = __uint_as_float(v[q * 8 + i]) * inv_l;
+                o[h4 * 4 + q] = pack8(f);
             }
         }
+        ptx::tc_fence_before();
+        __syncwarp();
+        if (lane == 0) ptx::mbar_arrive(o_free);
+#pragma unroll
+        for (int q = 0; q < HS / 8; q++) *reinterpret_cast<bf16x8*>(sP + (q >> 3) * ATOM_BYTES + r * 128 + (((q & 7) ^ (r & 7)) << 4)) = o[q];
+        const int4 tile = info[n & 1];
+        if (tile.y * BQ + r < T) lse[((size_t)tile.w * NH + tile.z) * T + tile.y * BQ + r] = (m + log2f(l)) * 0.6931471805599453f;
+        ptx::fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0 && tile.y * BQ + lane_group * 32 < T) {
+#pragma unroll
+            for (int k = 0; k < HS / 64; k++)
+                ptx::tma_store_3d(&tmOut, sP + k * ATOM_BYTES + lane_group * 4096, tile.z * HS + 64 * k, tile.y * BQ + lane_group * 32, tile.w);
+            ptx::tma_store_commit();
+        }
+        }
+        if (lane == 0) ptx::tma_store_wait_read<0>();
     }
 
     ptx::tc_fence_before();
@@ -441,12 +514,15 @@ static int launch(const CUtensorMap& tm, const CUtensorMap& tm_kv, void* out, fl
                                            cudaSharedmemCarveoutMaxShared));
     }
     CUtensorMap tm_out;
-    const int rc = gemm::make_tmap_3d(&tm_out, out, (uint64_t)NH * HS, T, B, 64, 128);
+    const int rc = gemm::make_tmap_3d(&tm_out, out, (uint64_t)NH * HS, T, B, 64, 32);   // (a warp's rows)
     if (rc) return rc;
+    const int sms = sm_count_current_device();
+    if (sms <= 0) return LLMK_ERR_CUDA;
     const float scale_log2 = 1.4426950408889634f / sqrtf((float)HS);
     const TileOrder order = make_tile_order(ceil_div(T, BQ), NH * B, 4l * Tkv * HS * NKVH / NH);
-    attn_fwd_tc_kernel<HS, ROUND><<<order.tiles * order.heads, THREADS, Cfg<HS>::SMEM_BYTES, stream>>>(tm, tm_kv, tm_out, lse, T, Tkv,
-        causal, NH, NKVH, scale_log2, status, order, local ? Cfg<HS>::CTAS_PER_SM * sm_count_current_device() : 0);
+    const int tiles = order.tiles * order.heads, resident = Cfg<HS>::CTAS_PER_SM * sms;
+    attn_fwd_tc_kernel<HS, ROUND><<<tiles < resident ? tiles : resident, THREADS, Cfg<HS>::SMEM_BYTES, stream>>>(tm, tm_kv, tm_out, lse,
+        T, Tkv, causal, NH, NKVH, scale_log2, status, order, local ? 1 : 0);
     LLMK_LAUNCH_CHECK();
     return LLMK_OK;
 }
