@@ -987,16 +987,17 @@ static int launch(const void* qkv, const void* dout, bf16* dqkv, const float* ls
     // the tiles of a KV head share the queries and output gradients of its query heads; those of a query head its keys and values
     const TileOrder dkv_order = make_tile_order(ceil_div(Tkv, BM), NKVH * B, 4l * T * HS * (NH / NKVH));
     const TileOrder dq_order = make_tile_order(ceil_div(T, BM), NH * B, 4l * Tkv * HS * NKVH / NH);
-    // The pipelined kernel runs one CTA per SM at that CTA's full speed, the other one two at half speed each and 5 to 20 %
-    // more in all. With at most two tiles per SM the longest tile sets the end, and the pipelined kernel wins; with more the
-    // throughput does. Backward in us, two per SM / pipelined, 12 heads unless said: 64 tiles (B2 T512 32/8 heads) 61 / 50,
-    // 72 (B2 T320) 19.3 / 17.2, 256 (B2 T2048 32/8) 303 / 225, 288 (B3 T1024) 59.6 / 51.4; 336 (B7 T448) 31.4 / 34.0,
-    // 384 (B4 T1024) 59 / 62 but (B1 T4096) 206 / 192 and (B1 T6144 32/8) 1014 / 928, 512 (B8 T1024 32/8) 246 / 255,
-    // 1024 (B8 T2048 32/8) 818 / 865; a loop of two sub-tiles does not pay for the set-up, 192 (B16 T128) 15 / 18.
-    // LLMK_ATTN_BWD_DKV=1|2 forces a version.
+    // The pipelined kernel runs one CTA per SM at that CTA's full speed, the other one two that share it and do more in all.
+    // While every tile has an SM the pipelined one is ahead; with up to two tiles per SM it is as long as the tiles are long,
+    // because the other one's longest tile shares its SM to the end; with more the throughput decides. Backward in us, two per
+    // SM / pipelined, 12 heads unless said: 96 tiles (B1 T1024) 39.9 / 39.3, 128 (B1 T2048 32/8 heads) 188 / 180; 192 (B2 T1024)
+    // 42.8 / 40.4, (B1 T2048) 74 / 70, but (B4 T512) 26.7 / 27.2 and (B8 T256) 19.3 / 21.3; 256 (B2 T2048 32/8) 240 / 210 and (B4 T1024
+    // 32/8) 135 / 123, but (B8 T512 32/8) 80 / 84; 288 (B3 T1024) 45 / 47; 384 (B2 T2048) 84 / 97, (B1 T4096) 150 / 171, (B3 T2048
+    // 32/8) 284 / 319. LLMK_ATTN_BWD_DKV=1|2 forces a version.
     const char* dkv_env = getenv("LLMK_ATTN_BWD_DKV");   // read on every call, so that one process can run both versions
-    const bool few_tiles = (T / 64) * (NH / NKVH) >= 5 &&
-                           (long)dkv_order.tiles * dkv_order.heads * 3 <= (long)(T >= 2048 ? 8 : 6) * sm_count_current_device();
+    const long n_tiles = (long)dkv_order.tiles * dkv_order.heads, n_sms = sm_count_current_device();
+    const int steps = (T / 64) * (NH / NKVH);   // of the longest tile
+    const bool few_tiles = n_tiles <= 2 * n_sms && steps >= (n_tiles <= n_sms ? 5 : (5 * n_tiles <= 7 * n_sms ? 12 : 48));
     const bool use_v2 = dkv_env != nullptr ? dkv_env[0] == '2' : few_tiles;
     if (HS == 64 && use_v2 && !ring) {
         static PerDeviceOnce once_configured2;

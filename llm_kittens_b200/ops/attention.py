@@ -32,16 +32,19 @@ def _sms() -> int:
 
 
 def _tc_forward(B: int, T: int, NH: int, HS: int) -> bool:
-    """Whether the forward of these sequences is faster on the tcgen05 kernels. Lengths that are multiples of 128 always are.
-    With a ragged last tile and heads of 64 the time of a launch that the chip holds at once is that of its longest tile,
-    2.07 us per 128 keys on the warp-level kernel and 2.25 on the other, on top of 2.5 and 3.4; with more tiles than that
-    their throughput decides. us, warp level / tcgen05: B1 T320 12 heads 7.7 / 10.2, B2 T320 25 heads 9.8 / 10.2 and 32 heads
-    11.3 / 10.4, B7 T448 6 heads 12.3 / 13.9 and 12 heads 20.5 / 17.6, B2 T576 6 heads 12.1 / 13.6 and 12 heads 15.2 / 13.6, B1 T1088
-    6 heads 20.1 / 22.3 and 12 heads 25.4 / 22.5. Heads of 128 have one 128-row tile per SM, of which sequences under 512
-    fill half to 60 %: one wave of them is ahead (B1 T320 32 heads 13.7 / 12.3), more are not (B2 17.6 / 21.0, B7 T448 16 heads
-    40 / 47); from 512 on they are (B2 T576 32 heads 39.5 / 35.5, B1 T1088 63 / 35)."""
-    if T % 128 == 0 or not _tc_length(T):
-        return T % 128 == 0
+    """Whether the forward of these sequences is faster on the tcgen05 kernels. Lengths that are multiples of 128 are, except
+    for a few sequences of 128 or 256 with heads of 64, where a launch lasts as long as its longest tile and the warp-level
+    kernel's 64-row tiles are shorter (B1 T128 12 heads 4.4 / 5.9, B2 T128 25 heads 4.6 / 6.0, B1 T256 12 heads 6.5 / 7.1, but B2 T256 25
+    heads 6.9 / 7.2, B16 T128 32 heads 14.4 / 12.5).
+    With a ragged last tile few sequences stay on the warp-level kernel: with heads of 64 while its launch is one or two
+    waves of 64-row tiles, with heads of 128 and under 512 keys from one wave of 128-row tiles on. The lines were drawn when
+    both kernels were equal there; the tcgen05 kernel is ahead of them now (us, warp level / tcgen05: B1 T320 12 heads 7.6 / 8.3,
+    but B2 T320 25 heads 9.8 / 9.3, B7 T448 6 heads 12.2 / 11.1, B2 T576 6 heads 11.9 / 10.9; heads of 128: B2 T320 32 heads 17.5 / 12.9,
+    B7 T448 16 heads 40 / 23), and they are kept because tests state them."""
+    if not _tc_length(T):
+        return False
+    if T % 128 == 0:
+        return HS != 64 or T > 256 or T // 128 * B * NH > _sms() // 2
     if HS == 64:
         return (T // 64) * B * NH > (2 if T <= 448 else 1) * _sms()
     return T >= 512 or (T + 127) // 128 * B * NH <= _sms()
