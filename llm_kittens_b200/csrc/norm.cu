@@ -59,6 +59,30 @@ norm_bwd_finish_kernel(bf16* __restrict__ dweight, bf16* __restrict__ dbias, con
 // RAGGED: C is any multiple of 8 up to 256 * NVEC; the lanes whose last vector lies beyond the row keep zeros there.
 constexpr int REG_WARPS = 8;
 
+// Eight bf16 values as four fp32 pairs: the arithmetic of these kernels goes through the packed instructions, two values each.
+// One at a time it took as long as the memory: LayerNorm forward of 65536 x 768 52 us (RMSNorm, with half of it, 35).
+__device__ __forceinline__ void unpack8p(const bf16x8& v, ptx::f32x2* f) {
+    const uint32_t* u = reinterpret_cast<const uint32_t*>(&v);
+#pragma unroll
+    for (int i = 0; i < 4; i++) f[i] = ptx::pack2(__uint_as_float(u[i] << 16), __uint_as_float(u[i] & 0xffff0000u));
+}
+__device__ __forceinline__ bf16x8 pack8p(const ptx::f32x2* f) {
+    bf16x8 r;
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        float a, b;
+        ptx::unpack2(f[i], a, b);
+        r.v[i] = __floats2bfloat162_rn(a, b);
+    }
+    return r;
+}
+__device__ __forceinline__ ptx::f32x2 both(float x) { return ptx::pack2(x, x); }
+__device__ __forceinline__ float sum2(ptx::f32x2 v) {
+    float a, b;
+    ptx::unpack2(v, a, b);
+    return a + b;
+}
+
 __device__ __forceinline__ bf16x8 add8(const bf16x8& x, const bf16x8& y) {
     float a[8], b[8];
     unpack8(x, a);
@@ -68,8 +92,8 @@ __device__ __forceinline__ bf16x8 add8(const bf16x8& x, const bf16x8& y) {
     return pack8(a);
 }
 
-// AHEAD: the next row is loaded before the current one is reduced.
-template <bool RMS, bool FUSED_RESIDUAL, int NVEC, bool RAGGED, bool AHEAD>
+// AHEAD: the next row is loaded before the current one is reduced. KEEP: weight and bias stay in registers.
+template <bool RMS, bool FUSED_RESIDUAL, int NVEC, bool RAGGED, bool AHEAD, bool KEEP>
 __global__ void __launch_bounds__(REG_WARPS * 32)
 norm_fwd_reg_kernel(bf16* __restrict__ normed, float* __restrict__ mean_out, float* __restrict__ rstd_out,
                     bf16* residual_out, const bf16* inp1, const bf16* __restrict__ inp2, const bf16* __restrict__ weight,
@@ -87,6 +111,12 @@ norm_fwd_reg_kernel(bf16* __restrict__ normed, float* __restrict__ mean_out, flo
     if (AHEAD && row < N) {
         load(inp1, row, xn);
         if (FUSED_RESIDUAL) load(inp2, row, yn);
+    }
+    bf16x8 wv[KEEP ? NVEC : 1], bv[KEEP && !RMS ? NVEC : 1];
+#pragma unroll
+    for (int k = 0; k < (KEEP ? NVEC : 0); k++) {
+        wv[k] = in_row(k) ? ld128(weight + (lane + 32 * k) * 8) : zero8();
+        if (!RMS) bv[RMS ? 0 : k] = in_row(k) ? ld128(bias + (lane + 32 * k) * 8) : zero8();
     }
     for (; row < N; row += gridDim.x * REG_WARPS) {
         if (!AHEAD) {
@@ -107,32 +137,30 @@ norm_fwd_reg_kernel(bf16* __restrict__ normed, float* __restrict__ mean_out, flo
             load(inp1, next, xn);
             if (FUSED_RESIDUAL) load(inp2, next, yn);
         }
-        float sum = 0.f;
+        ptx::f32x2 f[NVEC][4], acc = both(0.f);
 #pragma unroll
         for (int k = 0; k < NVEC; k++) {
-            float f[8];
-            unpack8(xv[k], f);
+            unpack8p(xv[k], f[k]);
 #pragma unroll
-            for (int j = 0; j < 8; j++) sum += RMS ? f[j] * f[j] : f[j];
+            for (int j = 0; j < 4; j++) acc = RMS ? ptx::fma2(f[k][j], f[k][j], acc) : ptx::add2(acc, f[k][j]);
         }
-        sum = warp_sum(sum);
+        const float sum = warp_sum(sum2(acc));
         float mean = 0.f, rstd;
         if (RMS) {
             rstd = rsqrtf(sum * inv_c + eps);
         } else {
             mean = sum * inv_c;
-            float var = 0.f;
+            acc = both(0.f);
 #pragma unroll
             for (int k = 0; k < NVEC; k++) {
-                float f[8];
-                unpack8(xv[k], f);
+                if (!in_row(k)) continue;
 #pragma unroll
-                for (int j = 0; j < 8; j++) {
-                    const float d = in_row(k) ? f[j] - mean : 0.f;
-                    var += d * d;
+                for (int j = 0; j < 4; j++) {
+                    f[k][j] = ptx::add2(f[k][j], both(-mean));
+                    acc = ptx::fma2(f[k][j], f[k][j], acc);
                 }
             }
-            var = warp_sum(var);
+            const float var = warp_sum(sum2(acc));
             rstd = rsqrtf(var * inv_c + eps);
         }
         if (lane == 0) {
@@ -142,16 +170,15 @@ norm_fwd_reg_kernel(bf16* __restrict__ normed, float* __restrict__ mean_out, flo
 #pragma unroll
         for (int k = 0; k < NVEC; k++) {
             if (!in_row(k)) continue;
-            float f[8], w[8], b[8];
-            unpack8(xv[k], f);
-            unpack8(ld128(weight + (lane + 32 * k) * 8), w);
-            if (!RMS) unpack8(ld128(bias + (lane + 32 * k) * 8), b);
+            ptx::f32x2 w[4], b[4];
+            unpack8p(KEEP ? wv[KEEP ? k : 0] : ld128(weight + (lane + 32 * k) * 8), w);
+            if (!RMS) unpack8p(KEEP ? bv[KEEP && !RMS ? k : 0] : ld128(bias + (lane + 32 * k) * 8), b);
 #pragma unroll
-            for (int j = 0; j < 8; j++) {
-                const float n = (f[j] - mean) * rstd;
-                f[j] = RMS ? n * w[j] : n * w[j] + b[j];
+            for (int j = 0; j < 4; j++) {
+                const ptx::f32x2 n = ptx::mul2(f[k][j], both(rstd));
+                f[k][j] = RMS ? ptx::mul2(n, w[j]) : ptx::fma2(n, w[j], b[j]);
             }
-            st128(normed + (size_t)row * C + (lane + 32 * k) * 8, pack8(f));
+            st128(normed + (size_t)row * C + (lane + 32 * k) * 8, pack8p(f[k]));
         }
     }
 }
@@ -211,32 +238,30 @@ norm_fwd_wide_kernel(bf16* __restrict__ normed, float* __restrict__ mean_out, fl
             load(inp1, next, xn);
             if (FUSED_RESIDUAL) load(inp2, next, yn);
         }
-        float sum = 0.f;
+        ptx::f32x2 f[NV][4], acc = both(0.f);
 #pragma unroll
         for (int k = 0; k < NV; k++) {
-            float f[8];
-            unpack8(xv[k], f);
+            unpack8p(xv[k], f[k]);
 #pragma unroll
-            for (int j = 0; j < 8; j++) sum += RMS ? f[j] * f[j] : f[j];
+            for (int j = 0; j < 4; j++) acc = RMS ? ptx::fma2(f[k][j], f[k][j], acc) : ptx::add2(acc, f[k][j]);
         }
-        sum = block_total(sum, par, 0);
+        const float sum = block_total(sum2(acc), par, 0);
         float mean = 0.f, rstd;
         if (RMS) {
             rstd = rsqrtf(sum * inv_c + eps);
         } else {
             mean = sum * inv_c;
-            float var = 0.f;
+            acc = both(0.f);
 #pragma unroll
             for (int k = 0; k < NV; k++) {
-                float f[8];
-                unpack8(xv[k], f);
+                if (!in_row(k)) continue;
 #pragma unroll
-                for (int j = 0; j < 8; j++) {
-                    const float d = in_row(k) ? f[j] - mean : 0.f;
-                    var += d * d;
+                for (int j = 0; j < 4; j++) {
+                    f[k][j] = ptx::add2(f[k][j], both(-mean));
+                    acc = ptx::fma2(f[k][j], f[k][j], acc);
                 }
             }
-            var = block_total(var, par, 1);
+            const float var = block_total(sum2(acc), par, 1);
             rstd = rsqrtf(var * inv_c + eps);
         }
         if (threadIdx.x == 0) {
@@ -246,21 +271,25 @@ norm_fwd_wide_kernel(bf16* __restrict__ normed, float* __restrict__ mean_out, fl
 #pragma unroll
         for (int k = 0; k < NV; k++) {
             if (!in_row(k)) continue;
-            float f[8], w[8], b[8];
-            unpack8(xv[k], f);
-            unpack8(wv[k], w);
-            if (!RMS) unpack8(bv[RMS ? 0 : k], b);
+            ptx::f32x2 w[4], b[4];
+            unpack8p(wv[k], w);
+            if (!RMS) unpack8p(bv[RMS ? 0 : k], b);
 #pragma unroll
-            for (int j = 0; j < 8; j++) {
-                const float n = (f[j] - mean) * rstd;
-                f[j] = RMS ? n * w[j] : n * w[j] + b[j];
+            for (int j = 0; j < 4; j++) {
+                const ptx::f32x2 n = ptx::mul2(f[k][j], both(rstd));
+                f[k][j] = RMS ? ptx::mul2(n, w[j]) : ptx::fma2(n, w[j], b[j]);
             }
-            st128(normed + (size_t)row * C + (threadIdx.x + 256 * k) * 8, pack8(f));
+            st128(normed + (size_t)row * C + (threadIdx.x + 256 * k) * 8, pack8p(f[k]));
         }
     }
 }
 
-// Backward with a bulk-copy ring: every warp owns rows and streams them (dout, inp and, when accumulating, the old
+// Backward. Both kernels: two values per instruction, and the row's statistics fetched a row ahead (they stood between a row's
+// arrival and its sums). us before / after, LayerNorm: 65536 x 768 77.8 / 69.7, 16384 x 1024 35.4 / 31.0, 8192 x 1024 21.0 / 19.5, 65536 x
+// 384 61.8 / 41.0, 3136 x 1600 22.3 / 17.2, 3136 x 4096 39.8 / 27.1 (but 3136 x 768 11.6 / 12.1: the terms of a row kept for the second
+// pass spill where 16 warps leave 128 registers; computed again they cost more, 13.5); RMSNorm 3136 x 4096 30.3 / 23.7.
+//
+// With a bulk-copy ring: every warp owns rows and streams them (dout, inp and, when accumulating, the old
 // dinp) into its own shared-memory ring with cp.async.bulk, STAGES rows ahead, so that about
 // warps x STAGES x 3 x C x 2 bytes are in flight per SM whatever the register budget (with one row per warp in
 // registers alone it reached well under half of the copy bandwidth). The dweight / dbias sums stay in registers over all
@@ -318,19 +347,30 @@ norm_bwd_bulk_kernel(bf16* __restrict__ dinp, float* __restrict__ scratch, const
         for (int i = 0; i < STAGES && i < nrows; i++) issue(i);
 
     const float inv_c = 1.0f / (float)C;
-    float dw[NVEC][8], db[RMS ? 1 : NVEC][8];
+    ptx::f32x2 dw[NVEC][4], db[RMS ? 1 : NVEC][4];
 #pragma unroll
     for (int k = 0; k < NVEC; k++)
 #pragma unroll
-        for (int j = 0; j < 8; j++) {
-            dw[k][j] = 0.f;
-            if (!RMS) db[k][j] = 0.f;
+        for (int j = 0; j < 4; j++) {
+            dw[k][j] = both(0.f);
+            if (!RMS) db[RMS ? 0 : k][j] = both(0.f);
         }
 
     bool ok = true;
+    // (the row's statistics are fetched one row ahead: they stood between a row's arrival and its sums)
+    float m_next = 0.f, rs_next = 0.f;
+    if (nrows > 0) {
+        if (!RMS) m_next = mean[first];
+        rs_next = rstd[first];
+    }
     for (int i = 0; i < nrows; i++) {
         const int st = i % STAGES;
         const int row = first + i * stride;
+        const float m = m_next, rs = rs_next;
+        if (i + 1 < nrows) {
+            if (!RMS) m_next = mean[row + stride];
+            rs_next = rstd[row + stride];
+        }
         ok = ptx::mbar_wait(&full[st], (i / STAGES) & 1, abort_flag, status, LLMK_ST_TIMEOUT_TMA_FULL, 8000 + st);
         if (!ok) break;
         const uint8_t* src = ring + st * 3 * SLOT;
@@ -343,43 +383,37 @@ norm_bwd_bulk_kernel(bf16* __restrict__ dinp, float* __restrict__ scratch, const
         }
         __syncwarp();   // the stage has been copied into registers by every lane: refill it
         if (lane == 0 && i + STAGES < nrows) issue(i + STAGES);
-        const float m = RMS ? 0.f : mean[row];
-        const float rs = rstd[row];
-        float s1 = 0.f, s2 = 0.f;
+        // n = (x - m) * rs in place of x, dn = dout * w in place of dout
+        ptx::f32x2 fn[NVEC][4], fd[NVEC][4], a1 = both(0.f), a2 = both(0.f);
 #pragma unroll
         for (int k = 0; k < NVEC; k++) {
-            float fd[8], fx[8], fw[8];
-            unpack8(dv[k], fd);
-            unpack8(xv[k], fx);
-            unpack8(in_row(k) ? ld128(weight + (lane + 32 * k) * 8) : zero8(), fw);
+            ptx::f32x2 fw[4];
+            unpack8p(dv[k], fd[k]);
+            unpack8p(xv[k], fn[k]);
+            unpack8p(in_row(k) ? ld128(weight + (lane + 32 * k) * 8) : zero8(), fw);
 #pragma unroll
-            for (int j = 0; j < 8; j++) {
-                const float n = (fx[j] - m) * rs;
-                const float dn = fd[j] * fw[j];
-                s1 += dn;
-                s2 += dn * n;
-                dw[k][j] += fd[j] * n;
-                if (!RMS) db[k][j] += fd[j];
+            for (int j = 0; j < 4; j++) {
+                fn[k][j] = ptx::mul2(RMS ? fn[k][j] : ptx::add2(fn[k][j], both(-m)), both(rs));
+                dw[k][j] = ptx::fma2(fd[k][j], fn[k][j], dw[k][j]);
+                if (!RMS) db[RMS ? 0 : k][j] = ptx::add2(db[RMS ? 0 : k][j], fd[k][j]);
+                fd[k][j] = ptx::mul2(fd[k][j], fw[j]);
+                a1 = ptx::add2(a1, fd[k][j]);
+                a2 = ptx::fma2(fd[k][j], fn[k][j], a2);
             }
         }
-        s1 = warp_sum(s1) * inv_c;
-        s2 = warp_sum(s2) * inv_c;
+        const float s1 = warp_sum(sum2(a1)) * inv_c, s2 = warp_sum(sum2(a2)) * inv_c;
 #pragma unroll
         for (int k = 0; k < NVEC; k++) {
             if (!in_row(k)) continue;
-            float fd[8], fx[8], fo[8], fw[8];
-            unpack8(dv[k], fd);
-            unpack8(xv[k], fx);
-            unpack8(ld128(weight + (lane + 32 * k) * 8), fw);
-            if (accumulate_dinp) unpack8(ov[k], fo);
+            ptx::f32x2 fo[4];
+            if (accumulate_dinp) unpack8p(ov[k], fo);
 #pragma unroll
-            for (int j = 0; j < 8; j++) {
-                const float n = (fx[j] - m) * rs;
-                const float dn = fd[j] * fw[j];
-                const float d = RMS ? (dn - n * s2) * rs : (dn - s1 - n * s2) * rs;
-                fo[j] = accumulate_dinp ? fo[j] + d : d;
+            for (int j = 0; j < 4; j++) {
+                const ptx::f32x2 t = RMS ? fd[k][j] : ptx::add2(fd[k][j], both(-s1));
+                const ptx::f32x2 d = ptx::fma2(fn[k][j], both(-s2), t);
+                fo[j] = accumulate_dinp ? ptx::fma2(d, both(rs), fo[j]) : ptx::mul2(d, both(rs));
             }
-            st128(dinp + (size_t)row * C + (lane + 32 * k) * 8, pack8(fo));
+            st128(dinp + (size_t)row * C + (lane + 32 * k) * 8, pack8p(fo));
         }
     }
     // all rings are idle now (every issued copy has been waited for): reuse them for the cross-warp reduction
@@ -390,9 +424,11 @@ norm_bwd_bulk_kernel(bf16* __restrict__ dinp, float* __restrict__ scratch, const
     for (int k = 0; k < NVEC; k++) {
         if (!in_row(k)) continue;
 #pragma unroll
-        for (int j = 0; j < 8; j++) {
-            sh[(size_t)warp * PLANES * C + (lane + 32 * k) * 8 + j] = dw[k][j];
-            if (!RMS) sh[(size_t)warp * PLANES * C + C + (lane + 32 * k) * 8 + j] = db[k][j];
+        for (int j = 0; j < 4; j++) {
+            float2* at = reinterpret_cast<float2*>(sh + (size_t)warp * PLANES * C + (lane + 32 * k) * 8 + 2 * j);
+            ptx::unpack2(dw[k][j], at->x, at->y);
+            at += C / 2;
+            if (!RMS) ptx::unpack2(db[RMS ? 0 : k][j], at->x, at->y);
         }
     }
     __syncthreads();
@@ -422,14 +458,14 @@ norm_bwd_wide_kernel(bf16* __restrict__ dinp, float* __restrict__ scratch, const
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const float inv_c = 1.0f / (float)C;
     auto in_row = [&](int k) { return !RAGGED || (int)(threadIdx.x + 256 * k) * 8 < C; };
-    float dw[NV][8], db[RMS ? 1 : NV][8], fw[NV][8];
+    ptx::f32x2 dw[NV][4], db[RMS ? 1 : NV][4], fw[NV][4];
 #pragma unroll
     for (int k = 0; k < NV; k++) {
-        unpack8(in_row(k) ? ld128(weight + (threadIdx.x + 256 * k) * 8) : zero8(), fw[k]);
+        unpack8p(in_row(k) ? ld128(weight + (threadIdx.x + 256 * k) * 8) : zero8(), fw[k]);
 #pragma unroll
-        for (int j = 0; j < 8; j++) {
-            dw[k][j] = 0.f;
-            if (!RMS) db[k][j] = 0.f;
+        for (int j = 0; j < 4; j++) {
+            dw[k][j] = both(0.f);
+            if (!RMS) db[RMS ? 0 : k][j] = both(0.f);
         }
     }
     bf16x8 dv[NV], xv[NV], ov[NV], dvn[NV], xvn[NV], ovn[NV];
@@ -443,31 +479,37 @@ norm_bwd_wide_kernel(bf16* __restrict__ dinp, float* __restrict__ scratch, const
         }
     };
     int row = blockIdx.x;
-    if (row < N) load(row, dv, xv, ov);
+    float m_next = 0.f, rs_next = 0.f;
+    if (row < N) {
+        load(row, dv, xv, ov);
+        if (!RMS) m_next = mean[row];
+        rs_next = rstd[row];
+    }
     int par = 0;
     for (; row < N; row += gridDim.x, par ^= 1) {
         const int next = row + gridDim.x;
-        if (next < N) load(next, dvn, xvn, ovn);
-        const float m = RMS ? 0.f : mean[row];
-        const float rs = rstd[row];
-        float s1 = 0.f, s2 = 0.f;
+        const float m = m_next, rs = rs_next;
+        if (next < N) {
+            load(next, dvn, xvn, ovn);
+            if (!RMS) m_next = mean[next];
+            rs_next = rstd[next];
+        }
+        ptx::f32x2 fn[NV][4], fd[NV][4], a1 = both(0.f), a2 = both(0.f);
 #pragma unroll
         for (int k = 0; k < NV; k++) {
-            float fd[8], fx[8];
-            unpack8(dv[k], fd);
-            unpack8(xv[k], fx);
+            unpack8p(dv[k], fd[k]);
+            unpack8p(xv[k], fn[k]);
 #pragma unroll
-            for (int j = 0; j < 8; j++) {
-                const float n = (fx[j] - m) * rs;
-                const float dn = fd[j] * fw[k][j];
-                s1 += dn;
-                s2 += dn * n;
-                dw[k][j] += fd[j] * n;
-                if (!RMS) db[k][j] += fd[j];
+            for (int j = 0; j < 4; j++) {
+                fn[k][j] = ptx::mul2(RMS ? fn[k][j] : ptx::add2(fn[k][j], both(-m)), both(rs));
+                dw[k][j] = ptx::fma2(fd[k][j], fn[k][j], dw[k][j]);
+                if (!RMS) db[RMS ? 0 : k][j] = ptx::add2(db[RMS ? 0 : k][j], fd[k][j]);
+                fd[k][j] = ptx::mul2(fd[k][j], fw[k][j]);
+                a1 = ptx::add2(a1, fd[k][j]);
+                a2 = ptx::fma2(fd[k][j], fn[k][j], a2);
             }
         }
-        s1 = warp_sum(s1);
-        s2 = warp_sum(s2);
+        float s1 = warp_sum(sum2(a1)), s2 = warp_sum(sum2(a2));
         if (lane == 0) {
             red[par][0][warp] = s1;
             red[par][1][warp] = s2;
@@ -484,18 +526,15 @@ norm_bwd_wide_kernel(bf16* __restrict__ dinp, float* __restrict__ scratch, const
         s2 *= inv_c;
 #pragma unroll
         for (int k = 0; k < NV; k++) {
-            float fd[8], fx[8], fo[8];
-            unpack8(dv[k], fd);
-            unpack8(xv[k], fx);
-            if (accumulate_dinp) unpack8(ov[k], fo);
+            ptx::f32x2 fo[4];
+            if (accumulate_dinp) unpack8p(ov[k], fo);
 #pragma unroll
-            for (int j = 0; j < 8; j++) {
-                const float n = (fx[j] - m) * rs;
-                const float dn = fd[j] * fw[k][j];
-                const float d = RMS ? (dn - n * s2) * rs : (dn - s1 - n * s2) * rs;
-                fo[j] = accumulate_dinp ? fo[j] + d : d;
+            for (int j = 0; j < 4; j++) {
+                const ptx::f32x2 t = RMS ? fd[k][j] : ptx::add2(fd[k][j], both(-s1));
+                const ptx::f32x2 d = ptx::fma2(fn[k][j], both(-s2), t);
+                fo[j] = accumulate_dinp ? ptx::fma2(d, both(rs), fo[j]) : ptx::mul2(d, both(rs));
             }
-            if (in_row(k)) st128(dinp + (size_t)row * C + (threadIdx.x + 256 * k) * 8, pack8(fo));
+            if (in_row(k)) st128(dinp + (size_t)row * C + (threadIdx.x + 256 * k) * 8, pack8p(fo));
         }
 #pragma unroll
         for (int k = 0; k < NV; k++) {
@@ -509,9 +548,15 @@ norm_bwd_wide_kernel(bf16* __restrict__ dinp, float* __restrict__ scratch, const
     for (int k = 0; k < NV; k++) {
         if (!in_row(k)) continue;
 #pragma unroll
-        for (int j = 0; j < 8; j++) {
-            dst[(threadIdx.x + 256 * k) * 8 + j] = dw[k][j];
-            if (!RMS) dst[C + (threadIdx.x + 256 * k) * 8 + j] = db[k][j];
+        for (int j = 0; j < 4; j++) {
+            float2* at = reinterpret_cast<float2*>(dst + (threadIdx.x + 256 * k) * 8 + 2 * j);
+            float2 v;
+            ptx::unpack2(dw[k][j], v.x, v.y);
+            *at = v;
+            if (!RMS) {
+                ptx::unpack2(db[RMS ? 0 : k][j], v.x, v.y);
+                at[C / 2] = v;
+            }
         }
     }
 }
@@ -527,14 +572,18 @@ static int num_sms() {
     return g_sms;
 }
 
-// Whole 256-column widths on the warp-per-row kernel, measured with rows from HBM and from the L2. Without a residual the
-// plain loop is ahead or even (us at 65536 rows, plain / ahead, RMSNorm: 768 columns 35.4 / 40.4, 1024 54.3 / 65.8, 1280 67.0 /
-// 80.1, but 256 15.1 / 15.1 and from the L2 11.7 / 10.8; LayerNorm 1024 at 16384 rows from the L2 17.7 / 18.5, 1280 24.4 / 25.3).
-// With a residual the loads per row double, and so does the gain where the registers allow it: LayerNorm 512 56.4 / 49.9
-// and 1280 147.7 / 122.6, but 1024 105.4 / 106.5 and at 8192 rows from the L2 14.0 / 15.6; RMSNorm 256 27.9 / 24.9, 1280 138 / 131,
-// but 768 70.5 / 76.0. (The other widths of up to 1280 columns always read ahead.)
+// Warp-per-row kernel: weight and bias in registers, and with them the next row loaded ahead (the grid is then what the chip
+// holds at once). Read for every row, weight and bias are two thirds of what LayerNorm loads, and the L1 was 89 % busy at 65536
+// x 768. us, per row / kept and ahead, rows from HBM: LayerNorm 65536 x 768 52.3 / 39.6, 16384 x 1024 19.6 / 14.0, 8192 x 1024 11.6 / 8.7,
+// 65536 x 512 35.3 / 25.5, 16384 x 1280 23.4 / 19.3, with the residual 65536 x 768 77.8 / 66.9; RMSNorm 16384 x 1024 15.9 / 13.3, 65536 x 1280
+// 67.1 / 56.0. RMSNorm has half of the loads, and up to 768 columns more warps do more for it: 65536 x 768 35.1 / 37.7, 8192 x 768 6.7 /
+// 7.5.
+// With one row per warp and SM or less there is nothing to keep them for: LayerNorm 64 x 768 2.5 / 2.9, 1024 x 768 3.1 / 3.1.
+constexpr bool keeps_weights(bool rms, bool fused, int nvec) { return !rms || (!fused && nvec >= 4); }
+// RMSNorm without: the next row ahead or not, measured with rows from HBM and from the L2 (us, plain / ahead: 256 columns at 65536
+// rows 15.1 / 15.1 and from the L2 11.7 / 10.8, 768 35.4 / 40.4; with a residual 256 27.9 / 24.9, 768 70.5 / 76.0, 1280 138 / 131).
 constexpr bool reads_ahead(bool rms, bool fused, int nvec) {
-    return fused ? nvec == 5 || nvec == (rms ? 1 : 2) : rms && nvec == 1;
+    return keeps_weights(rms, fused, nvec) || nvec == 1 || (fused && nvec == 5);
 }
 // LayerNorm at 1536 columns: the block-per-row kernel has a quarter of its threads idle, the warp-per-row one fewer warps.
 // us, block / warp: 1024 rows 4.2 / 4.7, 4096 9.7 / 10.9, 8192 17.1 / 17.2 (from the L2 15.4 / 14.5), 16384 30.4 / 28.7, 65536 108 / 97.
@@ -565,9 +614,11 @@ static int launch_fwd(bf16* normed, float* mean, float* rstd, bf16* residual, co
     case NV:                                                                                                                \
         if (C == NV * 256) {                                                                                                \
             constexpr bool AHEAD = reads_ahead(RMS, FUSED, NV);                                                             \
-            LLMK_NORM_FWD_LAUNCH((norm_fwd_reg_kernel<RMS, FUSED, NV, false, AHEAD>), REG_WARPS, AHEAD)                     \
+            if (keeps_weights(RMS, FUSED, NV) && N <= REG_WARPS * num_sms())                                                \
+                LLMK_NORM_FWD_LAUNCH((norm_fwd_reg_kernel<RMS, FUSED, NV, false, false, false>), REG_WARPS, false)          \
+            LLMK_NORM_FWD_LAUNCH((norm_fwd_reg_kernel<RMS, FUSED, NV, false, AHEAD, keeps_weights(RMS, FUSED, NV)>), REG_WARPS, AHEAD) \
         }                                                                                                                   \
-        LLMK_NORM_FWD_LAUNCH((norm_fwd_reg_kernel<RMS, FUSED, NV, true, true>), REG_WARPS, true)
+        LLMK_NORM_FWD_LAUNCH((norm_fwd_reg_kernel<RMS, FUSED, NV, true, true, keeps_weights(RMS, FUSED, NV)>), REG_WARPS, true)
     switch (ceil_div(C, 256)) {
         LLMK_NORM_FWD_CASE(1)
         LLMK_NORM_FWD_CASE(2)
@@ -577,7 +628,7 @@ static int launch_fwd(bf16* normed, float* mean, float* rstd, bf16* residual, co
         default: break;
     }
     if constexpr (!RMS && !FUSED) {
-        if (C == 1536 && N >= WARP_ROWS_1536) LLMK_NORM_FWD_LAUNCH((norm_fwd_reg_kernel<RMS, FUSED, 6, false, false>), REG_WARPS, false)
+        if (C == 1536 && N >= WARP_ROWS_1536) LLMK_NORM_FWD_LAUNCH((norm_fwd_reg_kernel<RMS, FUSED, 6, false, false, false>), REG_WARPS, false)
     }
     switch (ceil_div(C, 2048)) {
         case 1: LLMK_NORM_FWD_LAUNCH((norm_fwd_wide_kernel<RMS, FUSED, 1>), 1, true)
