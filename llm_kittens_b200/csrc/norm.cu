@@ -716,6 +716,9 @@ namespace norm {
 // below, every row has a block of its own anyway. us, block per row / rings, LayerNorm: 128 columns 256 rows 5.3 / 5.3, 512
 // 6.4 / 5.4, 16384 58 / 13; 384 columns 512 rows 6.9 / 7.5, 1024 8.6 / 7.9, 16384 62 / 19; 640 columns 1024 rows 9.9 / 10.8, 2048
 // 13.6 / 11.3; 1272 columns 512 rows 10.2 / 11.1, 1024 12.4 / 11.8, 16384 74 / 50.
+// Rows of whole vectors per lane take the rings from more than two rows per SM on, i.e. when the other kernel's blocks get a second
+// row: 768 columns 64 rows 5.0 / 7.1, 256 6.3 / 7.4, 512 7.7 / 7.2; 1280 columns 64 5.4 / 6.7, 256 7.2 / 7.3, 512 8.5 / 8.3; 1024 columns 256
+// 6.6 / 6.3.
 constexpr int ragged_bulk_rows(int C) { return C <= 256 ? 512 : 1024; }
 
 // The row kernel plus the fixed-order reduction of its partials.
@@ -735,7 +738,7 @@ static int launch_bwd(bf16* dinp, bf16* dweight, bf16* dbias, float* scratch, co
     }
 #define LLMK_NORM_BWD_BULK(NVEC)                                                    \
     case NVEC:                                                                      \
-        if (C == NVEC * 256) LLMK_NORM_BWD(launch_bwd_bulk, NVEC)                   \
+        if (C == NVEC * 256 && N > 2 * num_sms()) LLMK_NORM_BWD(launch_bwd_bulk, NVEC) \
         if (N >= ragged_bulk_rows(C)) LLMK_NORM_BWD(launch_bwd_bulk, NVEC, true) \
         break;
     switch (ceil_div(C, 256)) {
