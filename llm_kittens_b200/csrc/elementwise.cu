@@ -563,30 +563,56 @@ scan_kernel(int* __restrict__ data, int m) {
     }
 }
 
-// vals_in == nullptr: the value of pair i is i (first pass)
-__global__ void __launch_bounds__(32)
+// vals_in == nullptr: the value of pair i is i (first pass). A tile's pairs keep their order: warp w of the block takes the w-th
+// slice of the tile, the warps count their slices side by side, a prefix over the warps gives each its places, and every
+// warp places its slice 32 pairs at a time. (One warp per tile took 0.55 us for each of the tile's 64 steps. The whole sort by
+// 50,257 tokens, us before / after: 256 positions 28 / 14, 3136 74 / 20, 16384 87 / 28, 65536 117 / 57.)
+constexpr int WARPS = 16, SLICE = TILE / WARPS, STEPS = SLICE / 32;
+__global__ void __launch_bounds__(32 * WARPS)
 scatter_kernel(int* __restrict__ keys_out, int* __restrict__ vals_out, const int* __restrict__ keys_in,
                const int* __restrict__ vals_in, const int* __restrict__ offsets, int n, int shift, int ntiles) {
-    __shared__ int running[BINS];
-    const int lane = threadIdx.x;
-    for (int i = lane; i < BINS; i += 32) running[i] = offsets[i * ntiles + blockIdx.x];
+    __shared__ int place[WARPS][BINS];
+    static_assert(32 * WARPS == BINS, "a thread per bin");
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int first = blockIdx.x * TILE + warp * SLICE + lane;
+    int key[STEPS], val[STEPS];
+#pragma unroll
+    for (int k = 0; k < STEPS; k++) {
+        const int i = first + 32 * k;
+        key[k] = i < n ? keys_in[i] : 0;
+        val[k] = i < n && vals_in != nullptr ? vals_in[i] : i;
+    }
+    int run = offsets[threadIdx.x * ntiles + blockIdx.x];   // of this thread's bin
+    for (int i = lane; i < BINS; i += 32) place[warp][i] = 0;
     __syncwarp();
-    const int base = blockIdx.x * TILE;
-    for (int it = 0; it < TILE / 32; it++) {
-        const int i = base + it * 32 + lane;
-        const bool live = i < n;
-        const unsigned active = __ballot_sync(0xffffffffu, live);
+    unsigned same[STEPS];
+#pragma unroll
+    for (int k = 0; k < STEPS; k++) {
+        const bool live = first + 32 * k < n;
+        const int d = (key[k] >> shift) & (BINS - 1);
+        same[k] = __match_any_sync(0xffffffffu, live ? d : -1);
+        if (live && (same[k] & ((1u << lane) - 1u)) == 0) place[warp][d] += __popc(same[k]);   // the lowest lane of each digit group
+        __syncwarp();
+    }
+    __syncthreads();
+#pragma unroll
+    for (int w = 0; w < WARPS; w++) {
+        const int c = place[w][threadIdx.x];
+        place[w][threadIdx.x] = run;
+        run += c;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < STEPS; k++) {
+        const bool live = first + 32 * k < n;
+        const int d = (key[k] >> shift) & (BINS - 1), rank = __popc(same[k] & ((1u << lane) - 1u));
         if (live) {
-            const int key = keys_in[i];
-            const int d = (key >> shift) & (BINS - 1);
-            const unsigned same = __match_any_sync(active, d);
-            const int rank = __popc(same & ((1u << lane) - 1u));
-            const int dst = running[d] + rank;
-            keys_out[dst] = key;
-            vals_out[dst] = vals_in != nullptr ? vals_in[i] : i;
-            __syncwarp(active);
-            if (rank == 0) running[d] += __popc(same);   // the lowest lane of each digit group
+            const int dst = place[warp][d] + rank;
+            keys_out[dst] = key[k];
+            vals_out[dst] = val[k];
         }
+        __syncwarp();
+        if (live && rank == 0) place[warp][d] += __popc(same[k]);
         __syncwarp();
     }
 }
@@ -617,7 +643,7 @@ LLMK_API int llmk_bucket_sort(void* sorted_tok, void* sorted_pos, const void* to
         LLMK_LAUNCH_CHECK();
         bucket::scan_kernel<<<1, 1024, 0, st>>>(hist, bucket::BINS * ntiles);
         LLMK_LAUNCH_CHECK();
-        bucket::scatter_kernel<<<ntiles, 32, 0, st>>>(kout, vout, kin, vin, hist, n, p * bucket::BITS, ntiles);
+        bucket::scatter_kernel<<<ntiles, 32 * bucket::WARPS, 0, st>>>(kout, vout, kin, vin, hist, n, p * bucket::BITS, ntiles);
         LLMK_LAUNCH_CHECK();
         kin = kout;
         vin = vout;
