@@ -975,6 +975,7 @@ int make_tmap_3d(CUtensorMap* m, const void* ptr, uint64_t inner, uint64_t rows,
 }
 
 #include "gemm_small.cuh"
+#include "gemm_few_rows.cuh"
 
 static int query_pair_clusters();
 
@@ -1156,8 +1157,9 @@ struct SmallPlan {
 // x 3072 23.0 / 6.6, 256 x 768 x 3072 23.3 / 8.2, 320 x 2048 x 2048 18.9 / 8.7, 1024 x 768 x 768 12.8 / 5.7, 1024 x 2048 x 8192
 // 48.4 / 29.8, 2048 x 1024 x 4096 28.2 / 16.7; NN 256 x 768 x 50304 226 / 31; TN 768 x 768 x 3136 23.3 / 11.6, 3072 x 768 x 3136
 // 24.5 / 19.4.
-static SmallPlan pick_small(int mode, int M, int N, int K, int num_sms, int pair_clusters) {
+static SmallPlan pick_small(int mode, int M, int N, int K, int num_sms, int pair_clusters, double* estimate) {
     SmallPlan plan = {0, 0};
+    *estimate = 1e30;   // (of the choice, where one was made)
     const int kb = ceil_div(K, BK);
     if (ceil_div(M, BM) * ceil_div(N, 128) > num_sms) return plan;
     double best;
@@ -1179,7 +1181,15 @@ static SmallPlan pick_small(int mode, int M, int N, int K, int num_sms, int pair
             if (cost < best) { best = cost; plan.bn = bn; plan.S = S; }
         }
     }
+    if (plan.bn) *estimate = best;
     return plan;
+}
+
+// Time of a product of a few rows and a wide output on the CTA-pair kernel (mode NT): as in pick_small, but with every pair busy
+// for several waves a k-block takes 0.40 us, not 0.33.
+static double pair_estimate(int M, int N, int K, int pair_clusters) {
+    const int units = ceil_div(M, 2 * BM) * ceil_div(N, BN), waves = ceil_div(units, pair_clusters);
+    return waves * ceil_div(K, BK) * (0.28 + 0.12 * units / ((double)waves * pair_clusters)) + 9.3;
 }
 
 static int run_small(const SmallPlan& plan, int mode, int epi, const void* A, const void* B, void* C, void* C2, const Params& q,
@@ -1327,7 +1337,15 @@ static int gemm_impl(int mode, int epi, const void* A, const void* B, void* C, v
     // few tiles: kernels of their own (not where flags are polled, rows scattered, problems stacked or the grid limited)
     if (p.pair && groups == 1 && max_ctas <= 0 && p.a_ready == nullptr && p.b_ready == nullptr && p.b_ready2 == nullptr &&
         !(epi & EPI_SCATTER)) {
-        const SmallPlan plan = pick_small(mode, M, N, K, g_num_sms, pair_clusters);
+        double small_us;
+        const SmallPlan plan = pick_small(mode, M, N, K, g_num_sms, pair_clusters, &small_us);
+        const bool swi = (epi & EPI_SWIGLU) != 0;
+        if (mode == MODE_NT && (epi == 0 || epi == EPI_SWIGLU) && M <= few::MAX_TOKENS) {
+            const double us = few::estimate(M, swi ? N / 2 : N, K, swi, pair_clusters);
+            if (us < small_us && us < 0.95 * pair_estimate(M, N, K, pair_clusters))
+                return swi ? few::launch<EPI_SWIGLU>(A, B, ready.b2, C, C2, ready.c3, M, N / 2, K, status, pair_clusters, stream)
+                           : few::launch<0>(A, B, nullptr, C, nullptr, nullptr, M, N, K, status, pair_clusters, stream);
+        }
         if (plan.bn) return run_small(plan, mode, epi, A, B, C, C2, p, ready, stream);
     }
     bool split_accumulate = false;

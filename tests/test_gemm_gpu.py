@@ -422,3 +422,37 @@ def test_rows_of_few_tiles_dealt_out_unevenly_over_a_cluster(M):
     for got, x in ((dw, dw0 + dout.double().T @ b.double()), (db, db0 + dout.double().sum(0))):
         assert ((got.double() - x).abs() <= 2.0 ** -8 * x.abs() + 1e-4 * 3000 ** 0.5).all()
     _native.check_status()
+
+
+@pytest.mark.parametrize("M", [1, 33, 64, 200, 320, 400, 512])
+@pytest.mark.parametrize("N,K", [(50312, 1032), (20008, 72)])
+def test_gemm_of_few_rows_and_a_wide_output(M, N, K):
+    """Rows on the N side of the MMA: counts that are no multiple of 32, one and two MMAs per weight tile, a last weight tile that
+    is cut, K not whole k-blocks; nothing is written behind the rows and columns that exist."""
+    from llm_kittens_b200.ops import gemm, _native
+
+    a, w = _rand(M, K), _rand(N, K, scale=0.05)
+    want = a.double() @ w.double().T
+    whole = torch.full((M * N + 4096,), 7.0, device="cuda", dtype=torch.bfloat16)
+    out = whole[:M * N].view(M, N)
+    gemm.gemm_nt(a, w, out=out)
+    # fp32 sums of K products of order 0.05, one rounding to bf16
+    assert ((out.double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-5 * K ** 0.5).all()
+    assert (whole[M * N:] == 7.0).all()
+    assert torch.equal(out, gemm.gemm_nt(a, w))
+    _native.check_status()
+
+
+@pytest.mark.parametrize("M,H,K", [(320, 8192, 512), (257, 8320, 136), (64, 19072, 264), (512, 8192, 512)])
+def test_swiglu_of_few_rows_and_a_wide_output(M, H, K):
+    from llm_kittens_b200.ops import gemm, _native
+
+    a, wu, wg = _rand(M, K), _rand(H, K, scale=0.05), _rand(H, K, scale=0.05)
+    act, up, gate = (torch.empty(M, H, device="cuda", dtype=torch.bfloat16) for _ in range(3))
+    assert gemm.gemm_swiglu(a, wu, wg, act, up, gate)
+    for got, w in ((up, wu), (gate, wg)):
+        want = a.double() @ w.double().T
+        assert ((got.double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-5 * K ** 0.5).all()
+    want = torch.nn.functional.silu(gate.double()) * up.double()
+    assert ((act.double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-5).all()
+    _native.check_status()
