@@ -22,6 +22,7 @@
 //   owner side   recv[e_local][src][cap][C]   rows routed to local expert e_local by rank src
 //   source side  back[e][cap][C]              expert outputs (or input gradients) returned to this rank
 #include "common.cuh"
+#include "ptx_sm100.cuh"
 
 namespace llmk {
 namespace moe {
@@ -88,86 +89,158 @@ __device__ __forceinline__ bool wait_entries_block(const int* flags, int n, int 
 }
 
 // ------------------------------------------------------------------ router
-// One warp per ROUTER_ROWS tokens: logits = x . Wr^T (fp32), softmax over E, top-K (ties -> lower expert index),
-// weights renormalised to sum 1. Two tokens share a router weight's trip from shared memory and its conversion, where there
-// are enough of them to fill the chip with warps: see launch_router.
-template <int ROUTER_ROWS>
-__global__ void __launch_bounds__(256)
+// Logits = x . Wr^T (fp32), softmax over E, top-K (ties -> lower expert index), weights renormalised to sum 1. A warp works
+// on ROWS tokens at a time and goes on to its next ones; a vector of a row is asked for U vectors, or one row, before its turn.
+// Two experts share an FMA instruction, ROWS tokens a weight's trip from shared memory, where the weights lie once per
+// block: WIDE as fp32 pairs of experts, ready for the FMA (element (pair, quarter of a vector, vector) is two channels of two
+// experts, so the lanes of a warp read consecutive 16 bytes), otherwise as they are, for routers too large for that.
+// EP: E rounded up to a power of two. Bound by issue (about 500 instructions per
+// token at 8 experts and 1024 channels, twice the time of reading the rows): us at 16384 x 1024 with 8 experts, a block per 16
+// tokens with its own copy of the router and a shuffle butterfly per sum 31.5, now 17.0; 65536 113 / 50, 16384 x 768 with 4
+// experts 19.4 / 10.6, 64 tokens 7.7 / 4.3, 8192 x 1024 with 16 experts 29.0 / 23.1.
+template <int EP, int ROWS, bool WIDE>
+__global__ void __launch_bounds__(256, 2)
 router_fwd_kernel(float* __restrict__ probs, int* __restrict__ top_idx, float* __restrict__ top_w, const bf16* __restrict__ x,
                   const bf16* __restrict__ wr, int N, int C, int E, int K) {
+    constexpr int U = ROWS == 4 ? 2 : 4;   // vectors of a row in flight per lane
+    constexpr int V = ROWS * EP;           // dot products of a warp
+    constexpr int W = 32 / ROWS;           // lanes per token at the end
+    static_assert(V <= 32, "one lane per dot product");
     extern __shared__ __align__(16) uint8_t smem_raw[];
-    bf16* wr_s = reinterpret_cast<bf16*>(smem_raw);  // [E][C]
-    for (int i = threadIdx.x * 8; i < E * C; i += blockDim.x * 8) st128(wr_s + i, ld128(wr + i));
-    __syncthreads();
+    float4* pairs = reinterpret_cast<float4*>(smem_raw);                     // [ceil(E / 2)][4][C / 8]
+    __nv_bfloat162* words = reinterpret_cast<__nv_bfloat162*>(smem_raw);     // [E][4][C / 8]
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int row0 = (blockIdx.x * (blockDim.x >> 5) + warp) * ROUTER_ROWS;
-    if (row0 >= N) return;
-    float acc[ROUTER_ROWS][MAXE];
+    const int nv = C / 8, groups = (N + ROWS - 1) / ROWS, stride = gridDim.x * (blockDim.x >> 5);
+    int g = blockIdx.x * (blockDim.x >> 5) + warp;
+    bf16x8 in[ROWS][U];
+    auto fetch = [&](int group, int v0, int u) {
+        const int v = v0 + lane + 32 * u;
+        if (group < groups && v < nv) {
 #pragma unroll
-    for (int r = 0; r < ROUTER_ROWS; r++)
+            for (int r = 0; r < ROWS; r++) in[r][u] = ld128_stream(x + (size_t)min(group * ROWS + r, N - 1) * C + v * 8);
+        }
+    };
 #pragma unroll
-        for (int e = 0; e < MAXE; e++) acc[r][e] = 0.f;
-    for (int v = lane; v < C / 8; v += 32) {
-        float xf[ROUTER_ROWS][8];
+    for (int u = 0; u < U; u++) fetch(g, 0, u);
+    if (WIDE) {
+        for (int i = threadIdx.x; i < (E + 1) / 2 * nv; i += blockDim.x) {
+            const int p = i / nv, v = i % nv;
+            float a[8], b[8];
+            unpack8(ld128(wr + (size_t)(2 * p) * C + v * 8), a);
+            unpack8(2 * p + 1 < E ? ld128(wr + (size_t)(2 * p + 1) * C + v * 8) : zero8(), b);
 #pragma unroll
-        for (int r = 0; r < ROUTER_ROWS; r++) unpack8(ld128_stream(x + (size_t)min(row0 + r, N - 1) * C + v * 8), xf[r]);
+            for (int q = 0; q < 4; q++) pairs[(p * 4 + q) * nv + v] = make_float4(a[2 * q], b[2 * q], a[2 * q + 1], b[2 * q + 1]);
+        }
+    } else {
+        for (int i = threadIdx.x; i < E * nv; i += blockDim.x) {
+            const int e = i / nv, v = i % nv;
+            const bf16x8 w = ld128(wr + (size_t)e * C + v * 8);
 #pragma unroll
-        for (int e = 0; e < MAXE; e++) {
-            if (e < E) {
-                float wf[8];
-                unpack8(ld128(wr_s + (size_t)e * C + v * 8), wf);
-#pragma unroll
-                for (int r = 0; r < ROUTER_ROWS; r++)
-#pragma unroll
-                    for (int j = 0; j < 8; j++) acc[r][e] += xf[r][j] * wf[j];
-            }
+            for (int q = 0; q < 4; q++) words[(e * 4 + q) * nv + v] = w.v[q];
         }
     }
+    __syncthreads();
+    for (; g < groups; g += stride) {
+        ptx::f32x2 acc[ROWS][EP / 2];
 #pragma unroll
-    for (int r = 0; r < ROUTER_ROWS; r++)
+        for (int r = 0; r < ROWS; r++)
 #pragma unroll
-        for (int e = 0; e < MAXE; e++)
-            if (e < E) acc[r][e] = warp_sum(acc[r][e]);
-    // Lane e takes expert e. Sums and comparisons go through the experts in order, by shuffles, so the probabilities and
-    // the choices among equal ones are those of a serial loop (which one lane ran over arrays in local memory: 52 us at
-    // 16384 x 1024 with 8 experts, 43 this way, 29 with two rows a warp).
+            for (int p = 0; p < EP / 2; p++) acc[r][p] = ptx::pack2(0.f, 0.f);
+        for (int v0 = 0; v0 < nv; v0 += 32 * U) {
+            const bool last = v0 + 32 * U >= nv;
 #pragma unroll
-    for (int r = 0; r < ROUTER_ROWS; r++) {
-        const int row = row0 + r;
-        if (row >= N) break;
-        float logit = -INFINITY;
+            for (int u = 0; u < U; u++) {
+                const int v = v0 + lane + 32 * u;
+                bf16x8 xv[ROWS];
 #pragma unroll
-        for (int e = 0; e < MAXE; e++)
-            if (e < E && lane == e) logit = acc[r][e];
-        const float mx = warp_max(logit);
-        float p = lane < E ? __expf(logit - mx) : 0.f;
+                for (int r = 0; r < ROWS; r++) xv[r] = in[r][u];
+                fetch(last ? g + stride : g, last ? 0 : v0 + 32 * U, u);
+                if (v >= nv) continue;
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    float2 xf[ROWS];
+#pragma unroll
+                    for (int r = 0; r < ROWS; r++) xf[r] = __bfloat1622float2(xv[r].v[q]);
+#pragma unroll
+                    for (int p = 0; p < EP / 2; p++) {
+                        if (2 * p >= E) continue;
+                        float4 w;
+                        if (WIDE) {
+                            w = pairs[(p * 4 + q) * nv + v];
+                        } else {
+                            const float2 a = __bfloat1622float2(words[(2 * p * 4 + q) * nv + v]);
+                            const float2 b = 2 * p + 1 < E ? __bfloat1622float2(words[((2 * p + 1) * 4 + q) * nv + v]) : make_float2(0.f, 0.f);
+                            w = make_float4(a.x, b.x, a.y, b.y);
+                        }
+#pragma unroll
+                        for (int r = 0; r < ROWS; r++) {
+                            acc[r][p] = ptx::fma2(ptx::pack2(xf[r].x, xf[r].x), ptx::pack2(w.x, w.y), acc[r][p]);
+                            acc[r][p] = ptx::fma2(ptx::pack2(xf[r].y, xf[r].y), ptx::pack2(w.z, w.w), acc[r][p]);
+                        }
+                    }
+                }
+            }
+        }
+        // The lanes' sums: halves of the list are exchanged, so that each step has half the sums of the one before (the same
+        // pairs of lanes as in a butterfly per sum, so the same bits, with 31 shuffles in place of 160 for 32 sums). Lane l
+        // ends up with dot product l >> SHIFT.
+        float val[V];
+#pragma unroll
+        for (int r = 0; r < ROWS; r++)
+#pragma unroll
+            for (int p = 0; p < EP / 2; p++) ptx::unpack2(acc[r][p], val[r * EP + 2 * p], val[r * EP + 2 * p + 1]);
+        constexpr int SHIFT = V == 32 ? 0 : V == 16 ? 1 : V == 8 ? 2 : V == 4 ? 3 : 4;
+#pragma unroll
+        for (int step = 0; step < 5; step++) {
+            const int n = V >> (step + 1), o = 16 >> step;
+            if (n > 0) {
+                const bool upper = lane & o;
+#pragma unroll
+                for (int i = 0; i < n; i++) {
+                    const float other = __shfl_xor_sync(0xffffffffu, upper ? val[i] : val[i + n], o);
+                    val[i] = (upper ? val[i + n] : val[i]) + other;
+                }
+            } else {
+                val[0] += __shfl_xor_sync(0xffffffffu, val[0], o);
+            }
+        }
+        // W lanes per token, lane e of them takes expert e. Sums and comparisons go through the experts in order, by
+        // shuffles, so the probabilities and the choices among equal ones are those of a serial loop.
+        const int r = lane / W, e = lane % W;
+        const int row = g * ROWS + r;
+        float logit = __shfl_sync(0xffffffffu, val[0], (r * EP + min(e, EP - 1)) << SHIFT);
+        if (e >= E) logit = -INFINITY;
+        float mx = logit;
+#pragma unroll
+        for (int o = W / 2; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        float p = e < E ? __expf(logit - mx) : 0.f;
         float sum = 0.f;
-        for (int e = 0; e < E; e++) sum += __shfl_sync(0xffffffffu, p, e);
+        for (int i = 0; i < E; i++) sum += __shfl_sync(0xffffffffu, p, i, W);
         p /= sum;
-        if (lane < E) probs[(size_t)row * E + lane] = p;
+        if (row < N && e < E) probs[(size_t)row * E + e] = p;
         unsigned taken = 0;
         float wsum = 0.f, w = 0.f;   // lane k keeps choice k
         int idx = 0;
         for (int k = 0; k < K; k++) {
             int best = -1;
             float bv = -1.f;
-            for (int e = 0; e < E; e++) {
-                const float pe = __shfl_sync(0xffffffffu, p, e);
-                if (!(taken & (1u << e)) && pe > bv) {
+            for (int i = 0; i < E; i++) {
+                const float pe = __shfl_sync(0xffffffffu, p, i, W);
+                if (!(taken & (1u << i)) && pe > bv) {
                     bv = pe;
-                    best = e;
+                    best = i;
                 }
             }
             taken |= 1u << best;
-            if (lane == k) {
+            if (e == k) {
                 idx = best;
                 w = bv;
             }
             wsum += bv;
         }
-        if (lane < K) {
-            top_idx[(size_t)row * K + lane] = idx;
-            top_w[(size_t)row * K + lane] = w / wsum;
+        if (row < N && e < K) {
+            top_idx[(size_t)row * K + e] = idx;
+            top_w[(size_t)row * K + e] = w / wsum;
         }
     }
 }
@@ -223,53 +296,91 @@ assign_slots_kernel(int* __restrict__ slot, int* __restrict__ counts, const int*
 }
 
 // ------------------------------------------------------------------ dispatch (all-to-all out)
-// One warp per (token, k): row x[token] * scale -> recv buffer of the owner of expert e at slot s.
-// `scale_by_weight`: 0 copies the row (forward), 1 multiplies by the routing weight (backward: dY = w * dout).
-__global__ void __launch_bounds__(256)
-dispatch_kernel(Peers recv, const bf16* __restrict__ x, const int* __restrict__ top_idx, const int* __restrict__ slot,
-                const float* __restrict__ top_w, int N, int K, int C, int cap, int Eloc, int my_rank, int P, int scale_by_weight) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const size_t a = (size_t)blockIdx.x * (blockDim.x >> 5) + warp;
-    if (a >= (size_t)N * K) return;
-    const int s = slot[a];
-    if (s < 0) return;
-    const int e = top_idx[a];
-    const size_t t = a / K;
-    const int owner = e / Eloc, el = e % Eloc;
-    bf16* dst = static_cast<bf16*>(recv.p[owner]) + ((((size_t)el * P + my_rank) * cap) + s) * C;
-    const bf16* src = x + t * C;
-    const float w = scale_by_weight ? top_w[a] : 1.0f;
-    for (int v = lane; v < C / 8; v += 32) {
-        bf16x8 r = ld128(src + v * 8);
-        if (scale_by_weight) {
-            float f[8];
-            unpack8(r, f);
+// The slots of rows t * K + k0 .. k0 + KK - 1 and the experts they belong to (slot -1: dropped, or beyond K).
+template <int KK>
+__device__ __forceinline__ void token_slots(int (&s)[KK], int (&e)[KK], const int* __restrict__ slot, const int* __restrict__ top_idx,
+                                            size_t t, int K, int k0) {
 #pragma unroll
-            for (int j = 0; j < 8; j++) f[j] *= w;
-            r = pack8(f);
-        }
-        st128(dst + v * 8, r);
+    for (int k = 0; k < KK; k++) {
+        const bool in = k0 + k < K;
+        s[k] = in ? slot[t * K + k0 + k] : -1;
+        e[k] = in ? top_idx[t * K + k0 + k] : 0;
     }
 }
-// Zero the unused slots [counts[e], cap) of this rank's block in every expert's receive buffer.
-// `arrive` (optional): the owners' arrival tables. This kernel runs after dispatch_kernel on the same stream, so when
-// its last CTA is done every row of this rank has been stored: that CTA release-stores `epoch` into entry
-// [e_local * P + my_rank] of the owner of every expert, which is entry (first row of the block) / cap of the
-// owner's receive buffer, the index the expert GEMM derives from the rows of a tile.
-__global__ void __launch_bounds__(256)
-zero_pad_kernel(Peers recv, const int* __restrict__ counts, int E, int C, int cap, int Eloc, int my_rank, int P, Peers arrive,
-                int arrive_off, int* done_counter, int epoch) {
-    const int e = blockIdx.y;
+// Zeros in the unused slots [counts[e], cap) of this rank's block in expert e's receive buffer, by `blocks` blocks.
+__device__ __forceinline__ void zero_slots(const Peers& recv, const int* __restrict__ counts, int e, int block, int blocks, int C,
+                                           int cap, int Eloc, int my_rank, int P) {
     const int owner = e / Eloc, el = e % Eloc;
     const int first = counts[e];
     bf16* base = static_cast<bf16*>(recv.p[owner]) + (((size_t)el * P + my_rank) * cap) * C;
     const size_t begin = (size_t)first * C, end = (size_t)cap * C;
-    bf16x8 z;
+    for (size_t i = begin + ((size_t)block * blockDim.x + threadIdx.x) * 8; i < end; i += (size_t)blocks * blockDim.x * 8)
+        st128(base + i, zero8());
+}
+constexpr int ZERO_BLOCKS = 32;   // per expert
+
+// One warp per token at a time: row x[token], read once, to the receive buffers of the owners of its K experts at its slots.
+// A lane's four vectors are all loaded before the first is stored (a load may not pass a store that could alias it).
+// SCALE: 0 copies the row (forward), 1 multiplies by the routing weight (backward: dY = w * dout).
+// The blocks from token_blocks on, if any, zero the unused slots. Bound by the writes: 16384 rows of 1024 to two experts of 8 with a
+// quarter of unused slots 33.8 us with a warp per copy and a launch for the zeros, now 22.7 (117 MB: 18 at the rate of a
+// copy); 16384 x 1280 to four 71.5 / 44.5, 64 x 1024 4.7 / 2.4.
+template <bool SCALE>
+__global__ void __launch_bounds__(256, 4)
+dispatch_kernel(const __grid_constant__ Peers recv, const bf16* __restrict__ x, const int* __restrict__ top_idx, const int* __restrict__ slot,
+                const float* __restrict__ top_w, const int* __restrict__ counts, int N, int K, int C, int cap, int Eloc, int my_rank,
+                int P, int token_blocks) {
+    if ((int)blockIdx.x >= token_blocks) {
+        const int b = blockIdx.x - token_blocks;
+        zero_slots(recv, counts, b / ZERO_BLOCKS, b % ZERO_BLOCKS, ZERO_BLOCKS, C, cap, Eloc, my_rank, P);
+        return;
+    }
+    constexpr int U = 4;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nv = C / 8;
+    const size_t t = (size_t)blockIdx.x * (blockDim.x >> 5) + warp;
+    if (t >= (size_t)N) return;
+    const bf16* src = x + t * C;
+    for (int k0 = 0; k0 < K; k0 += MAXK) {
+        int s[MAXK], e[MAXK];
+        token_slots(s, e, slot, top_idx, t, K, k0);
+        for (int v0 = lane; v0 < nv; v0 += 32 * U) {
+            bf16x8 r[U];
 #pragma unroll
-    for (int i = 0; i < 4; i++) z.v[i] = __floats2bfloat162_rn(0.f, 0.f);
-    for (size_t i = begin + ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * 8; i < end; i += (size_t)gridDim.x * blockDim.x * 8)
-        st128(base + i, z);
-    if (done_counter != nullptr && last_cta_done(done_counter, gridDim.x * gridDim.y)) {
+            for (int u = 0; u < U; u++)
+                if (v0 + 32 * u < nv) r[u] = ld128(src + (v0 + 32 * u) * 8);
+#pragma unroll
+            for (int k = 0; k < MAXK; k++) {
+                if (s[k] < 0) continue;
+                const float w = SCALE ? top_w[t * K + k0 + k] : 1.f;
+                const int owner = e[k] / Eloc, el = e[k] % Eloc;
+                bf16* dst = static_cast<bf16*>(recv.p[owner]) + ((((size_t)el * P + my_rank) * cap) + s[k]) * C;
+#pragma unroll
+                for (int u = 0; u < U; u++) {
+                    if (v0 + 32 * u >= nv) continue;
+                    bf16x8 o = r[u];
+                    if (SCALE) {
+                        float f[8];
+                        unpack8(o, f);
+#pragma unroll
+                        for (int j = 0; j < 8; j++) f[j] *= w;
+                        o = pack8(f);
+                    }
+                    st128(dst + (v0 + 32 * u) * 8, o);
+                }
+            }
+        }
+    }
+}
+// The unused slots by a kernel of their own, grid (ZERO_BLOCKS, E), for the exchange that publishes its arrival
+// (`arrive`: the owners' arrival tables). This kernel runs after dispatch_kernel on the same stream, so when
+// its last CTA is done every row of this rank has been stored: that CTA release-stores `epoch` into entry
+// [e_local * P + my_rank] of the owner of every expert, which is entry (first row of the block) / cap of the
+// owner's receive buffer, the index the expert GEMM derives from the rows of a tile.
+__global__ void __launch_bounds__(256)
+zero_pad_kernel(const __grid_constant__ Peers recv, const int* __restrict__ counts, int E, int C, int cap, int Eloc, int my_rank, int P,
+                const __grid_constant__ Peers arrive, int arrive_off, int* done_counter, int epoch) {
+    zero_slots(recv, counts, blockIdx.y, blockIdx.x, gridDim.x, C, cap, Eloc, my_rank, P);
+    if (last_cta_done(done_counter, gridDim.x * gridDim.y)) {
         for (int ee = 0; ee < E; ee++)
             st_release_sys(static_cast<int*>(arrive.p[ee / Eloc]) + arrive_off + (ee % Eloc) * P + my_rank, epoch);
     }
@@ -384,29 +495,81 @@ return_kernel(Peers back, const bf16* __restrict__ y, int C, int cap, int Eloc, 
 // With `weights == nullptr` the rows are summed unweighted (input-gradient gather in backward).
 // `returned` (optional): this rank's arrival entries of the E experts; every block waits (bounded) until each holds
 // `epoch`, i.e. until every owner has stored the rows of this rank into `back`.
-__global__ void __launch_bounds__(256)
+// One warp per token at a time, U vectors per lane: a token's rows are all in flight before the first is used, and a warp has
+// the slots and weights of its next token before it turns to it. U is what leaves room for 32 warps: 16384 x 1024, two
+// experts, 2 / 4 vectors 23.0 / 24.4 us. Bound by the reads: 32.5 us a vector at a time, now 22.9 (134 MB: 20.5 at the rate of
+// a copy); 16384 x 1280, four experts, 56 / 38, 65536 x 1024 106 / 79, 64 x 1024 4.9 / 3.2.
+template <int KK, int U>
+__global__ void __launch_bounds__(256, 4)
 combine_kernel(bf16* __restrict__ out, const bf16* __restrict__ base, const bf16* __restrict__ back, const int* __restrict__ top_idx,
                const int* __restrict__ slot, const float* __restrict__ weights, int N, int K, int C, int cap,
                const int* __restrict__ returned, int E, int epoch, long long limit_ns, int* status) {
+    if (returned != nullptr && !wait_entries_block(returned, E, epoch, limit_ns, status, 300)) return;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nv = C / 8;
+    const unsigned stride = gridDim.x * (blockDim.x >> 5), n = N;
+    unsigned t = blockIdx.x * (blockDim.x >> 5) + warp;
+    if (t >= n) return;
+    int s[KK], e[KK];
+    float w[KK];
+    auto choices = [&](unsigned token) {
+        token_slots(s, e, slot, top_idx, token, K, 0);
+#pragma unroll
+        for (int k = 0; k < KK; k++) w[k] = weights != nullptr && k < K ? weights[(size_t)token * K + k] : 1.f;
+    };
+    choices(t);
+    for (; t < n; t += stride) {
+        const bf16* row[KK];
+        float wk[KK];
+#pragma unroll
+        for (int k = 0; k < KK; k++) {
+            row[k] = s[k] < 0 ? nullptr : back + ((size_t)e[k] * cap + s[k]) * C;
+            wk[k] = w[k];
+        }
+        if (t + stride < n) choices(t + stride);
+        for (int v0 = lane; v0 < nv; v0 += 32 * U) {
+            bf16x8 b[U], r[KK][U];
+#pragma unroll
+            for (int k = 0; k < KK; k++)
+#pragma unroll
+                for (int u = 0; u < U; u++)
+                    if (row[k] != nullptr && v0 + 32 * u < nv) r[k][u] = ld128(row[k] + (v0 + 32 * u) * 8);
+#pragma unroll
+            for (int u = 0; u < U; u++) b[u] = base != nullptr && v0 + 32 * u < nv ? ld128(base + (size_t)t * C + (v0 + 32 * u) * 8) : zero8();
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                float acc[8];
+                unpack8(b[u], acc);
+#pragma unroll
+                for (int k = 0; k < KK; k++) {
+                    if (row[k] == nullptr) continue;
+                    float f[8];
+                    unpack8(r[k][u], f);
+#pragma unroll
+                    for (int j = 0; j < 8; j++) acc[j] += wk[k] * f[j];
+                }
+                if (v0 + 32 * u < nv) st128(out + (size_t)t * C + (v0 + 32 * u) * 8, pack8(acc));
+            }
+        }
+    }
+}
+// Any number of experts per token (the router chooses MAXK at most).
+__global__ void __launch_bounds__(256)
+combine_many_kernel(bf16* __restrict__ out, const bf16* __restrict__ base, const bf16* __restrict__ back, const int* __restrict__ top_idx,
+                    const int* __restrict__ slot, const float* __restrict__ weights, int N, int K, int C, int cap,
+                    const int* __restrict__ returned, int E, int epoch, long long limit_ns, int* status) {
     if (returned != nullptr && !wait_entries_block(returned, E, epoch, limit_ns, status, 300)) return;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const size_t t = (size_t)blockIdx.x * (blockDim.x >> 5) + warp;
     if (t >= (size_t)N) return;
     for (int v = lane; v < C / 8; v += 32) {
         float acc[8];
-        if (base != nullptr) {
-            unpack8(ld128(base + t * C + v * 8), acc);
-        } else {
-#pragma unroll
-            for (int j = 0; j < 8; j++) acc[j] = 0.f;
-        }
+        unpack8(base != nullptr ? ld128(base + t * C + v * 8) : zero8(), acc);
         for (int k = 0; k < K; k++) {
             const int s = slot[t * K + k];
             if (s < 0) continue;
-            const int e = top_idx[t * K + k];
             const float w = weights ? weights[t * K + k] : 1.0f;
             float f[8];
-            unpack8(ld128(back + (((size_t)e * cap) + s) * C + v * 8), f);
+            unpack8(ld128(back + ((size_t)top_idx[t * K + k] * cap + s) * C + v * 8), f);
 #pragma unroll
             for (int j = 0; j < 8; j++) acc[j] += w * f[j];
         }
@@ -481,28 +644,56 @@ __global__ void publish_kernel(Peers arrive, int arrive_off, int Eloc, int my_ra
     }
 }
 
-// dw[t,k] = dot(dout[t], back[e][slot])  (gradient of the combine with respect to the routing weight)
-__global__ void __launch_bounds__(256)
+// dw[t,k] = dot(dout[t], back[e][slot])  (gradient of the combine with respect to the routing weight). One warp per token:
+// its row of dout is read once for KK experts, whose rows are all in flight. Bound by the reads: 16384 x 1024,
+// two experts, 20.8 us with a warp per expert, now 18.2 (100 MB: 15.4 at the rate of a copy); four experts of 1280 44 / 33.
+template <int KK, int U>
+__global__ void __launch_bounds__(256, 4)
 combine_dweight_kernel(float* __restrict__ dw, const bf16* __restrict__ dout, const bf16* __restrict__ back,
                        const int* __restrict__ top_idx, const int* __restrict__ slot, int N, int K, int C, int cap) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const size_t a = (size_t)blockIdx.x * (blockDim.x >> 5) + warp;
-    if (a >= (size_t)N * K) return;
-    const int s = slot[a];
-    float acc = 0.f;
-    if (s >= 0) {
-        const int e = top_idx[a];
-        const size_t t = a / K;
-        for (int v = lane; v < C / 8; v += 32) {
-            float d[8], f[8];
-            unpack8(ld128(dout + t * C + v * 8), d);
-            unpack8(ld128(back + (((size_t)e * cap) + s) * C + v * 8), f);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nv = C / 8;
+    const size_t t = (size_t)blockIdx.x * (blockDim.x >> 5) + warp;
+    if (t >= (size_t)N) return;
+    for (int k0 = 0; k0 < K; k0 += KK) {
+        int s[KK], e[KK];
+        token_slots(s, e, slot, top_idx, t, K, k0);
+        float acc[KK];
 #pragma unroll
-            for (int j = 0; j < 8; j++) acc += d[j] * f[j];
+        for (int k = 0; k < KK; k++) acc[k] = 0.f;
+        for (int v0 = lane; v0 < nv; v0 += 32 * U) {
+            bf16x8 d[U], r[KK][U];
+#pragma unroll
+            for (int u = 0; u < U; u++)
+                if (v0 + 32 * u < nv) d[u] = ld128(dout + t * C + (v0 + 32 * u) * 8);
+#pragma unroll
+            for (int k = 0; k < KK; k++) {
+                if (s[k] < 0) continue;
+                const bf16* row = back + ((size_t)e[k] * cap + s[k]) * C;
+#pragma unroll
+                for (int u = 0; u < U; u++)
+                    if (v0 + 32 * u < nv) r[k][u] = ld128(row + (v0 + 32 * u) * 8);
+            }
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                if (v0 + 32 * u >= nv) continue;
+                float df[8];
+                unpack8(d[u], df);
+#pragma unroll
+                for (int k = 0; k < KK; k++) {
+                    if (s[k] < 0) continue;
+                    float f[8];
+                    unpack8(r[k][u], f);
+#pragma unroll
+                    for (int j = 0; j < 8; j++) acc[k] += df[j] * f[j];
+                }
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < KK; k++) {
+            acc[k] = warp_sum(acc[k]);
+            if (lane == 0 && k0 + k < K) dw[t * K + k0 + k] = acc[k];
         }
     }
-    acc = warp_sum(acc);
-    if (lane == 0) dw[a] = acc;
 }
 
 // ------------------------------------------------------------------ load-balance statistics + router backward
@@ -590,19 +781,54 @@ using namespace llmk::moe;
 
 namespace llmk {
 namespace moe {
-// Rows per warp. The work per row is the same trip over the router however many rows share it, so with few tokens one row
-// per warp is the shortest chain, and with many the shared trip pays. us at C = 1024, 8 experts, top 2, one / two / four
-// rows: 64 tokens 7.7 / 10.4 / 14.1, 2048 9.7 / 10.9 / 14.8, 4096 14.0 / 12.4 / 14.9, 16384 43 / 29 / 33, 65536 154 / 110 / 118;
-// four are ahead by 10 % at 8192 tokens with 16 experts only. (768 channels and 4 experts: 2048 tokens 6.1 / 7.1 / 10.2, 4096
-// 7.8 / 8.1 / 10.6, 16384 21 / 17 / 22.)
-template <int ROWS>
+template <int EP, int ROWS, bool WIDE>
 static int launch_router(float* probs, int* top_idx, float* top_w, const bf16* x, const bf16* wr, int N, int C, int E, int K,
                          cudaStream_t stream) {
     static PerDeviceOnce once_configured;
     if (once_configured.first()) {
-        LLMK_CUDA_TRY(cudaFuncSetAttribute(router_fwd_kernel<ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+        LLMK_CUDA_TRY(cudaFuncSetAttribute(router_fwd_kernel<EP, ROWS, WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     }
-    router_fwd_kernel<ROWS><<<ceil_div(N, 8 * ROWS), 256, E * C * 2, stream>>>(probs, top_idx, top_w, x, wr, N, C, E, K);
+    const int smem = WIDE ? (E + 1) / 2 * C * 8 : E * C * 2;
+    const int resident = (smem > 112 * 1024 ? 1 : 2) * sm_count_current_device();
+    const int blocks = ceil_div(N, 8 * ROWS);
+    router_fwd_kernel<EP, ROWS, WIDE><<<resident > 0 && blocks > resident ? resident : blocks, 256, smem, stream>>>(
+        probs, top_idx, top_w, x, wr, N, C, E, K);
+    LLMK_LAUNCH_CHECK();
+    return LLMK_OK;
+}
+// The work for a vector of weights is the same however many tokens share it, so with few tokens one per warp is the shortest
+// chain, and with many the shared trip pays: us at C = 1024, 8 experts, one / two / four tokens a warp, 64 tokens 4.3 / 5.3 /
+// 6.2, 2048 6.8 / 6.4 / 7.1, 4096 10.4 / 8.1 / 7.5, 16384 28 / 22 / 17 (four of 16 experts would be more sums than lanes). fp32
+// pairs against the router as it is, two tokens a warp: 16384 21.9 / 26.1, 8192 with 16 experts 23.0 / 37.6.
+template <int EP>
+static int launch_router(float* probs, int* top_idx, float* top_w, const bf16* x, const bf16* wr, int N, int C, int E, int K,
+                         cudaStream_t stream) {
+    if ((long)((E + 1) / 2) * C * 8 > 200 * 1024) return launch_router<EP, 2, false>(probs, top_idx, top_w, x, wr, N, C, E, K, stream);
+    return N <= 2048 ? launch_router<EP, 1, true>(probs, top_idx, top_w, x, wr, N, C, E, K, stream)
+                     : launch_router<EP, EP == 16 ? 2 : 4, true>(probs, top_idx, top_w, x, wr, N, C, E, K, stream);
+}
+
+static int launch_dispatch(const Peers& recv, const void* x, const void* top_idx, const void* slot, const void* top_w,
+                           const void* counts, int N, int K, int C, int E, int cap, int my_rank, int P, int scale_by_weight,
+                           bool zero, cudaStream_t st) {
+    if (N <= 0 || K <= 0) return LLMK_ERR_SHAPE;
+    const int token_blocks = ceil_div(N, 8);
+    const int grid = token_blocks + (zero ? ZERO_BLOCKS * E : 0);
+    auto kernel = scale_by_weight ? dispatch_kernel<true> : dispatch_kernel<false>;
+    kernel<<<grid, 256, 0, st>>>(recv, (const bf16*)x, (const int*)top_idx, (const int*)slot, (const float*)top_w, (const int*)counts,
+                                 N, K, C, cap, E / P, my_rank, P, token_blocks);
+    LLMK_LAUNCH_CHECK();
+    return LLMK_OK;
+}
+
+static int launch_combine(void* out, const void* base, const void* back, const void* top_idx, const void* slot, const void* weights,
+                          int N, int K, int C, int cap, const void* returned, int E, int epoch, long long limit_ns, int* status,
+                          void* stream) {
+    auto kernel = K > MAXK ? combine_many_kernel : K == 1 ? combine_kernel<1, 4> : K == 2 ? combine_kernel<2, 2> : combine_kernel<MAXK, 1>;
+    const int blocks = ceil_div(N, 8), resident = 4 * sm_count_current_device();
+    kernel<<<K <= MAXK && resident > 0 && blocks > resident ? resident : blocks, 256, 0, (cudaStream_t)stream>>>(
+        (bf16*)out, (const bf16*)base, (const bf16*)back, (const int*)top_idx, (const int*)slot, (const float*)weights, N, K, C, cap,
+        (const int*)returned, E, epoch, limit_ns, status);
     LLMK_LAUNCH_CHECK();
     return LLMK_OK;
 }
@@ -612,9 +838,8 @@ static int launch_router(float* probs, int* top_idx, float* top_w, const bf16* x
 LLMK_API int llmk_moe_router_fwd(void* probs, void* top_idx, void* top_w, const void* x, const void* wr, int N, int C, int E, int K,
                                  void* stream) {
     if (E > MAXE || K > MAXK || K > E || C % 8 || (long)E * C * 2 > 200 * 1024) return LLMK_ERR_SHAPE;
-#define LLMK_ROUTER(ROWS) launch_router<ROWS>((float*)probs, (int*)top_idx, (float*)top_w, (const bf16*)x, (const bf16*)wr, N, C, E, K, (cudaStream_t)stream)
-    return N <= 2048 ? LLMK_ROUTER(1) : LLMK_ROUTER(2);
-#undef LLMK_ROUTER
+    auto launch = E <= 2 ? launch_router<2> : E <= 4 ? launch_router<4> : E <= 8 ? launch_router<8> : launch_router<16>;
+    return launch((float*)probs, (int*)top_idx, (float*)top_w, (const bf16*)x, (const bf16*)wr, N, C, E, K, (cudaStream_t)stream);
 }
 LLMK_API int llmk_moe_assign_slots(void* slot, void* counts, const void* top_idx, int N, int K, int E, int cap, void* stream) {
     cudaStream_t st = (cudaStream_t)stream;
@@ -628,15 +853,8 @@ LLMK_API int llmk_moe_dispatch(const long long* recv_ptrs, const void* x, const 
                                const void* counts, int N, int K, int C, int E, int cap, int my_rank, int P, int scale_by_weight,
                                void* stream) {
     if (P > MAXP || E % P || C % 8) return LLMK_ERR_SHAPE;
-    cudaStream_t st = (cudaStream_t)stream;
-    const Peers recv = make_peers(recv_ptrs, P);
-    const int Eloc = E / P;
-    dispatch_kernel<<<ceil_div((long)N * K, 8), 256, 0, st>>>(recv, (const bf16*)x, (const int*)top_idx, (const int*)slot,
-                                                             (const float*)top_w, N, K, C, cap, Eloc, my_rank, P, scale_by_weight);
-    LLMK_LAUNCH_CHECK();
-    zero_pad_kernel<<<dim3(32, E), 256, 0, st>>>(recv, (const int*)counts, E, C, cap, Eloc, my_rank, P, recv, 0, nullptr, 0);
-    LLMK_LAUNCH_CHECK();
-    return LLMK_OK;
+    return launch_dispatch(make_peers(recv_ptrs, P), x, top_idx, slot, top_w, counts, N, K, C, E, cap, my_rank, P, scale_by_weight, true,
+                           (cudaStream_t)stream);
 }
 // Dispatch that publishes its completion: `arrive_ptrs` = the P ranks' arrival tables (int), `arrive_off` the first
 // entry of this exchange in them, `done_counter` one zeroed int of local scratch, `epoch` the number of the exchange.
@@ -647,11 +865,9 @@ LLMK_API int llmk_moe_dispatch_signal(const long long* recv_ptrs, const void* x,
     if (P > MAXP || E % P || C % 8 || arrive_ptrs == nullptr || done_counter == nullptr) return LLMK_ERR_SHAPE;
     cudaStream_t st = (cudaStream_t)stream;
     const Peers recv = make_peers(recv_ptrs, P);
-    const int Eloc = E / P;
-    dispatch_kernel<<<ceil_div((long)N * K, 8), 256, 0, st>>>(recv, (const bf16*)x, (const int*)top_idx, (const int*)slot,
-                                                             (const float*)top_w, N, K, C, cap, Eloc, my_rank, P, scale_by_weight);
-    LLMK_LAUNCH_CHECK();
-    zero_pad_kernel<<<dim3(32, E), 256, 0, st>>>(recv, (const int*)counts, E, C, cap, Eloc, my_rank, P, make_peers(arrive_ptrs, P),
+    const int rc = launch_dispatch(recv, x, top_idx, slot, top_w, counts, N, K, C, E, cap, my_rank, P, scale_by_weight, false, st);
+    if (rc != LLMK_OK) return rc;
+    zero_pad_kernel<<<dim3(ZERO_BLOCKS, E), 256, 0, st>>>(recv, (const int*)counts, E, C, cap, E / P, my_rank, P, make_peers(arrive_ptrs, P),
                                                  arrive_off, (int*)done_counter, epoch);
     LLMK_LAUNCH_CHECK();
     return LLMK_OK;
@@ -718,23 +934,14 @@ LLMK_API int llmk_moe_return_signal(const long long* back_ptrs, const void* y, i
 }
 LLMK_API int llmk_moe_combine(void* out, const void* base, const void* back, const void* top_idx, const void* slot,
                               const void* weights, int N, int K, int C, int cap, void* stream) {
-    combine_kernel<<<ceil_div(N, 8), 256, 0, (cudaStream_t)stream>>>((bf16*)out, (const bf16*)base, (const bf16*)back,
-                                                                    (const int*)top_idx, (const int*)slot, (const float*)weights,
-                                                                    N, K, C, cap, nullptr, 0, 0, 0, nullptr);
-    LLMK_LAUNCH_CHECK();
-    return LLMK_OK;
+    return launch_combine(out, base, back, top_idx, slot, weights, N, K, C, cap, nullptr, 0, 0, 0, nullptr, stream);
 }
 // Combine that first waits (inside the kernel, for at most limit_ns) until `returned[0..E)` all hold `epoch`.
 LLMK_API int llmk_moe_combine_wait(void* out, const void* base, const void* back, const void* top_idx, const void* slot,
                                    const void* weights, int N, int K, int C, int cap, const void* returned, int E, int epoch,
                                    long limit_ns, int* status, void* stream) {
     if (returned == nullptr || E <= 0 || E > MAXE) return LLMK_ERR_SHAPE;
-    combine_kernel<<<ceil_div(N, 8), 256, 0, (cudaStream_t)stream>>>((bf16*)out, (const bf16*)base, (const bf16*)back,
-                                                                    (const int*)top_idx, (const int*)slot, (const float*)weights,
-                                                                    N, K, C, cap, (const int*)returned, E, epoch,
-                                                                    (long long)limit_ns, status);
-    LLMK_LAUNCH_CHECK();
-    return LLMK_OK;
+    return launch_combine(out, base, back, top_idx, slot, weights, N, K, C, cap, returned, E, epoch, (long long)limit_ns, status, stream);
 }
 LLMK_API int llmk_moe_combine_pull(void* out, const void* base, const long long* y_ptrs, void* save, const void* top_idx,
                                    const void* slot, const void* weights, int N, int K, int C, int E, int cap, int my_rank, int P,
@@ -755,9 +962,10 @@ LLMK_API int llmk_moe_publish(const long long* arrive_ptrs, int arrive_off, int 
 }
 LLMK_API int llmk_moe_combine_dweight(void* dw, const void* dout, const void* back, const void* top_idx, const void* slot, int N,
                                       int K, int C, int cap, void* stream) {
-    combine_dweight_kernel<<<ceil_div((long)N * K, 8), 256, 0, (cudaStream_t)stream>>>((float*)dw, (const bf16*)dout,
-                                                                                      (const bf16*)back, (const int*)top_idx,
-                                                                                      (const int*)slot, N, K, C, cap);
+    if (N <= 0 || K <= 0) return LLMK_ERR_SHAPE;
+    auto kernel = K == 1 ? combine_dweight_kernel<1, 4> : K == 2 ? combine_dweight_kernel<2, 2> : combine_dweight_kernel<MAXK, 1>;
+    kernel<<<ceil_div(N, 8), 256, 0, (cudaStream_t)stream>>>((float*)dw, (const bf16*)dout, (const bf16*)back, (const int*)top_idx,
+                                                             (const int*)slot, N, K, C, cap);
     LLMK_LAUNCH_CHECK();
     return LLMK_OK;
 }

@@ -254,6 +254,49 @@ def test_moe_routing_slots_and_density(N, C, E, K):
     assert abs(aux.item() - 0.01 * E * probs.double().mean(0).pow(2).sum().item()) <= 1e-6
 
 
+@pytest.mark.parametrize("N,C,E,K", [(1, 8, 1, 1), (9, 264, 3, 2), (4740, 1032, 5, 3), (9700, 1024, 8, 2), (5000, 2056, 16, 4), (40, 4096, 16, 2),
+                                     (33, 520, 7, 5)])
+def test_moe_rows_moved_and_summed(N, C, E, K):
+    """Dispatch, its weighted form, combine and the routing weights' gradient with dropped assignments, for rows of less and
+    more than a warp's vectors, tokens beyond one per resident warp, more experts per token than the router gives, and (40, 4096,
+    16) a router too large for shared memory as fp32."""
+    from llm_kittens_b200.ops import moe
+
+    x, base, cap = rnd(N, C), rnd(N, C), max(1, N * K // (E + 1))
+    if K <= 4:
+        wr = rnd(E, C, scale=0.02)
+        probs, idx, w = moe.router_fwd(x, wr, K)
+        assert ((probs.double() - (x.double() @ wr.double().T).softmax(-1)).abs() <= 1e-5).all()
+        assert torch.equal(idx.long(), torch.sort(probs, dim=-1, descending=True, stable=True).indices[:, :K])
+    else:
+        w, idx = (v.contiguous() for v in torch.rand(N, E, device="cuda").topk(K, dim=-1))
+        idx = idx.int()
+    slot, counts = moe.assign_slots(idx, E, cap)
+    kept = slot >= 0
+    assert N == 1 or not kept.all()
+    at = (idx.long() * cap + slot.long())
+    for scaled in (False, True):
+        recv = torch.full((E * cap, C), float("nan"), device="cuda", dtype=BF)
+        want = torch.zeros(E * cap, C, device="cuda", dtype=BF)
+        for k in range(K):
+            rows = (x.float() * w[:, k:k + 1]).to(BF) if scaled else x
+            want[at[kept[:, k], k]] = rows[kept[:, k]]
+        moe.dispatch(moe.ptr_table([recv]), x, idx, slot, w, counts, E, cap, scale_by_weight=scaled)
+        assert torch.equal(recv, want)
+    y, out = rnd(E * cap, C), torch.empty(N, C, device="cuda", dtype=BF)
+    rows = y.double()[at.clamp(min=0)] * kept.unsqueeze(-1)              # [N, K, C], zero where dropped
+    for add, weight in ((base, w), (None, None)):
+        moe.combine(out, add, y, idx, slot, weight, cap)
+        terms = rows if weight is None else rows * weight.double().unsqueeze(-1)
+        ref = terms.sum(1) + (0 if add is None else add.double())
+        size = terms.abs().sum(1) + (0 if add is None else add.double().abs())
+        # one rounding to bf16 and one of fp32 per term
+        assert ((out.double() - ref).abs() <= 2.0 ** -8 * ref.abs() + (K + 1) * 2.0 ** -23 * size).all()
+    dw = moe.combine_dweight(base, y, idx, slot, cap)
+    terms = rows * base.double().unsqueeze(1)
+    assert ((dw.double() - terms.sum(-1)).abs() <= (C / 32 + 6) * 2.0 ** -24 * terms.abs().sum(-1)).all()
+
+
 def test_gelu_swiglu_add():
     from llm_kittens_b200.ops import elementwise as ew
 
