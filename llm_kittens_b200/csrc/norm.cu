@@ -17,7 +17,8 @@ namespace norm {
 
 // dweight[c] += sum_b scratch[b][0][c] ; dbias[c] += sum_b scratch[b][1][c]   (fixed order over b)
 // A few dozen blocks of dependent L2 reads: bound by latency, so the chain per thread is what counts. 32 partial-row
-// lanes instead of 8: 12.2 -> 4.8 us for the partials of 4096 x 1600, 5.0 -> 3.4 us for those of 3136 x 768.
+// lanes instead of 8: 12.2 -> 4.8 us for the partials of 4096 x 1600, 5.0 -> 3.4 us for those of 3136 x 768. The old gradients are
+// asked for at the start: 0.2 us of 64 x 768 (a lane's partials all at once, not four at a time, lost 0.3: more code to fetch).
 constexpr int FIN_LANES = 32;
 __global__ void __launch_bounds__(32 * FIN_LANES)
 norm_bwd_finish_kernel(bf16* __restrict__ dweight, bf16* __restrict__ dbias, const float* __restrict__ scratch, int nblocks, int C) {
@@ -25,6 +26,12 @@ norm_bwd_finish_kernel(bf16* __restrict__ dweight, bf16* __restrict__ dbias, con
     // added in fixed order, so the result does not depend on scheduling
     __shared__ float shw[FIN_LANES][33], shb[FIN_LANES][33];
     const int c = blockIdx.x * 32 + threadIdx.x;
+    const bool last = threadIdx.y == 0 && c < C;
+    bf16 old_w, old_b;
+    if (last) {
+        old_w = dweight[c];
+        if (dbias != nullptr) old_b = dbias[c];
+    }
     float sw = 0.f, sb = 0.f;
     if (c < C) {
 #pragma unroll 4
@@ -36,15 +43,15 @@ norm_bwd_finish_kernel(bf16* __restrict__ dweight, bf16* __restrict__ dbias, con
     shw[threadIdx.y][threadIdx.x] = sw;
     shb[threadIdx.y][threadIdx.x] = sb;
     __syncthreads();
-    if (threadIdx.y == 0 && c < C) {
+    if (last) {
         float tw = 0.f, tb = 0.f;
 #pragma unroll
         for (int y = 0; y < FIN_LANES; y++) {
             tw += shw[y][threadIdx.x];
             tb += shb[y][threadIdx.x];
         }
-        dweight[c] = __float2bfloat16_rn(__bfloat162float(dweight[c]) + tw);
-        if (dbias != nullptr) dbias[c] = __float2bfloat16_rn(__bfloat162float(dbias[c]) + tb);
+        dweight[c] = __float2bfloat16_rn(__bfloat162float(old_w) + tw);
+        if (dbias != nullptr) dbias[c] = __float2bfloat16_rn(__bfloat162float(old_b) + tb);
     }
 }
 
@@ -590,6 +597,13 @@ constexpr bool reads_ahead(bool rms, bool fused, int nvec) {
 // (RMSNorm, and both with a residual: the block is ahead at every count.)
 constexpr int WARP_ROWS_1536 = 8192;
 
+// Few rows: a block per row. A launch is then one latency chain (a row's arrival, two sums, the result), and a warp that holds a
+// whole row has more to do between its steps than eight that share it. The line lies where a block gets a second row while
+// others wait for it. us, warp / block, LayerNorm and RMSNorm, rows in the L2 or HBM as after a write: 64 x 768 2.6 / 1.9 and 2.3 / 1.7, 256 x
+// 768 2.7 / 2.1, 440 x 768 2.8 / 2.5, 512 x 768 2.8 / 2.7 and 2.3 / 2.4, 320 x 512 2.4 / 2.1, 64 x 1280 3.4 / 1.9, 512 x 1280 3.9 / 2.8, 64 x
+// 264 2.3 / 1.9; with a residual 256 x 1024 3.3 / 2.0. (256 columns: the same.)
+constexpr int block_rows_per_sm(int C) { return C <= 256 ? 0 : C <= 768 ? 3 : C <= 1280 ? 4 : 0; }
+
 template <bool RMS, bool FUSED>
 static int launch_fwd(bf16* normed, float* mean, float* rstd, bf16* residual, const bf16* inp1, const bf16* inp2,
                       const bf16* weight, const bf16* bias, int N, int C, float eps, cudaStream_t stream) {
@@ -619,6 +633,7 @@ static int launch_fwd(bf16* normed, float* mean, float* rstd, bf16* residual, co
             LLMK_NORM_FWD_LAUNCH((norm_fwd_reg_kernel<RMS, FUSED, NV, false, AHEAD, keeps_weights(RMS, FUSED, NV)>), REG_WARPS, AHEAD) \
         }                                                                                                                   \
         LLMK_NORM_FWD_LAUNCH((norm_fwd_reg_kernel<RMS, FUSED, NV, true, true, keeps_weights(RMS, FUSED, NV)>), REG_WARPS, true)
+    if (N <= block_rows_per_sm(C) * num_sms()) LLMK_NORM_FWD_LAUNCH((norm_fwd_wide_kernel<RMS, FUSED, 1>), 1, true)
     switch (ceil_div(C, 256)) {
         LLMK_NORM_FWD_CASE(1)
         LLMK_NORM_FWD_CASE(2)
@@ -716,9 +731,9 @@ namespace norm {
 // below, every row has a block of its own anyway. us, block per row / rings, LayerNorm: 128 columns 256 rows 5.3 / 5.3, 512
 // 6.4 / 5.4, 16384 58 / 13; 384 columns 512 rows 6.9 / 7.5, 1024 8.6 / 7.9, 16384 62 / 19; 640 columns 1024 rows 9.9 / 10.8, 2048
 // 13.6 / 11.3; 1272 columns 512 rows 10.2 / 11.1, 1024 12.4 / 11.8, 16384 74 / 50.
-// Rows of whole vectors per lane take the rings from more than two rows per SM on, i.e. when the other kernel's blocks get a second
-// row: 768 columns 64 rows 5.0 / 7.1, 256 6.3 / 7.4, 512 7.7 / 7.2; 1280 columns 64 5.4 / 6.7, 256 7.2 / 7.3, 512 8.5 / 8.3; 1024 columns 256
-// 6.6 / 6.3.
+// Rows of whole vectors per lane take the rings from more than two rows per SM on (the other kernel's blocks then get a second row),
+// wider ones from one on: 768 columns 64 rows 4.7 / 7.0, 256 6.3 / 7.1, 296 7.1 / 7.2, 512 7.6 / 7.3; 512 columns 256 rows 5.6 / 6.1; 1024
+// columns 128 rows 5.1 / 6.2, 192 6.6 / 6.2, 256 6.6 / 6.1; 1280 columns 128 rows 5.2 / 6.7, 192 7.0 / 6.7, 296 8.4 / 7.3.
 constexpr int ragged_bulk_rows(int C) { return C <= 256 ? 512 : 1024; }
 
 // The row kernel plus the fixed-order reduction of its partials.
@@ -738,7 +753,7 @@ static int launch_bwd(bf16* dinp, bf16* dweight, bf16* dbias, float* scratch, co
     }
 #define LLMK_NORM_BWD_BULK(NVEC)                                                    \
     case NVEC:                                                                      \
-        if (C == NVEC * 256 && N > 2 * num_sms()) LLMK_NORM_BWD(launch_bwd_bulk, NVEC) \
+        if (C == NVEC * 256 && N > (NVEC <= 3 ? 2 : 1) * num_sms()) LLMK_NORM_BWD(launch_bwd_bulk, NVEC) \
         if (N >= ragged_bulk_rows(C)) LLMK_NORM_BWD(launch_bwd_bulk, NVEC, true) \
         break;
     switch (ceil_div(C, 256)) {

@@ -148,6 +148,15 @@ def test_norm_forward_of_wide_rows(N, C):
     assert torch.equal(a2, r) and ((out.double() - want).abs() <= ulp * want.abs() + 1e-4).all()
 
 
+@pytest.mark.parametrize("rms", [False, True])
+@pytest.mark.parametrize("N,C", [(1, 264), (444, 768), (445, 768), (592, 1280), (593, 1024), (148, 1024), (149, 1280), (296, 504), (297, 512)])
+def test_norms_of_few_rows(N, C, rms):
+    """Row counts on both sides of where a block per row gives way to a warp per row, forward (three rows per SM up to 768
+    columns, four beyond) and backward (two and one), with 148 SMs."""
+    test_norms_of_widths_that_are_not_whole_vectors_per_lane(N, C, rms)
+    test_norm_forward_of_wide_rows(N, C)
+
+
 @pytest.mark.parametrize("N,C", [(20001, 256), (19000, 512), (20001, 768), (19000, 1024), (19000, 1280), (8191, 1536), (8192, 1536),
                                  (20001, 1536)])
 def test_norm_forward_of_more_rows_than_the_grid_has_warps(N, C):
