@@ -99,6 +99,33 @@ __device__ __forceinline__ bf16x8 add8(const bf16x8& x, const bf16x8& y) {
     return pack8(a);
 }
 
+// The lanes' sums of R values (2, 4 or 8): halves of the list are exchanged, so each step has half the values of the one before
+// (the same pairs of lanes as in a butterfly per value, so the same bits). Lane l ends up with the sum of value l / (32 / R) in v[0].
+template <int R>
+__device__ __forceinline__ void rows_sum(float* v, int lane) {
+#pragma unroll
+    for (int step = 0; step < 5; step++) {
+        const int n = R >> (step + 1), o = 16 >> step;
+        if (n > 0) {
+            const bool upper = lane & o;
+#pragma unroll
+            for (int i = 0; i < n; i++) {
+                const float other = __shfl_xor_sync(0xffffffffu, upper ? v[i] : v[i + n], o);
+                v[i] = (upper ? v[i + n] : v[i]) + other;
+            }
+        } else {
+            v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+        }
+    }
+}
+
+// Eight partial sums in order, two loads (LayerNorm forward, two sums a row, 4096 x 1600 9.4 / 8.9
+// us; with RMSNorm's one sum 256 x 2048 went from 2.5 to 2.6, so that adds them one by one).
+__device__ __forceinline__ float sum8(const float* p) {
+    const float4 a = *reinterpret_cast<const float4*>(p), b = *reinterpret_cast<const float4*>(p + 4);
+    return ((((((a.x + a.y) + a.z) + a.w) + b.x) + b.y) + b.z) + b.w;
+}
+
 // AHEAD: the next row is loaded before the current one is reduced. KEEP: weight and bias stay in registers.
 template <bool RMS, bool FUSED_RESIDUAL, int NVEC, bool RAGGED, bool AHEAD, bool KEEP>
 __global__ void __launch_bounds__(REG_WARPS * 32)
@@ -198,7 +225,7 @@ __global__ void __launch_bounds__(256, NV <= 2 ? 4 : (NV <= 4 ? 2 : 1))
 norm_fwd_wide_kernel(bf16* __restrict__ normed, float* __restrict__ mean_out, float* __restrict__ rstd_out,
                      bf16* residual_out, const bf16* inp1, const bf16* __restrict__ inp2, const bf16* __restrict__ weight,
                      const bf16* __restrict__ bias, int N, int C, float eps) {
-    __shared__ float red[2][2][8];   // [parity][sum | squares][warp]
+    __shared__ __align__(16) float red[2][2][8];   // [parity][sum | squares][warp]
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const float inv_c = 1.0f / (float)C;
     auto in_row = [&](int k) { return (int)(threadIdx.x + 256 * k) * 8 < C; };
@@ -212,6 +239,7 @@ norm_fwd_wide_kernel(bf16* __restrict__ normed, float* __restrict__ mean_out, fl
         v = warp_sum(v);
         if (lane == 0) red[par][slot][warp] = v;
         __syncthreads();
+        if (!RMS) return sum8(red[par][slot]);
         float t = 0.f;
 #pragma unroll
         for (int w = 0; w < 8; w++) t += red[par][slot][w];
@@ -293,7 +321,7 @@ norm_fwd_wide_kernel(bf16* __restrict__ normed, float* __restrict__ mean_out, fl
 
 // Backward. Both kernels: two values per instruction, and the row's statistics fetched a row ahead (they stood between a row's
 // arrival and its sums). us before / after, LayerNorm: 65536 x 768 77.8 / 69.7, 16384 x 1024 35.4 / 31.0, 8192 x 1024 21.0 / 19.5, 65536 x
-// 384 61.8 / 41.0, 3136 x 1600 22.3 / 17.2, 3136 x 4096 39.8 / 27.1 (but 3136 x 768 11.6 / 12.1: the terms of a row kept for the second
+// 384 61.8 / 41.0, 3136 x 4096 39.8 / 27.1 (but 3136 x 768 11.6 / 12.1: the terms of a row kept for the second
 // pass spill where 16 warps leave 128 registers; computed again they cost more, 13.5); RMSNorm 3136 x 4096 30.3 / 23.7.
 //
 // With a bulk-copy ring: every warp owns rows and streams them (dout, inp and, when accumulating, the old
@@ -448,106 +476,121 @@ norm_bwd_bulk_kernel(bf16* __restrict__ dinp, float* __restrict__ scratch, const
     }
 }
 
-// Wide rows (C = NV * 2048): one 256-thread block per row, every thread owns NV 8-element column groups, so the
+// Wide rows (C = NV * 2048): one 256-thread block per R rows, every thread owns NV 8-element column groups, so the
 // weight-gradient accumulators stay at NV * 8 registers per plane however wide the row is and no cross-warp
-// reduction of them is needed (each column has one owner per block). The next row is prefetched into registers
-// while the block reduces the current one. scratch layout [gridDim.x][2][C] as for the other kernels.
+// reduction of them is needed (each column has one owner per block). The next rows are prefetched into registers
+// while the block reduces the current ones. scratch layout [gridDim.x][2][C] as for the other kernels.
 // RAGGED: C is any multiple of 8 up to NV * 2048; threads without a column group in the last round keep zeros.
-// (This replaces a kernel that read dout and x twice and kept the column sums in shared memory, eight-way bank
-// conflicts and all: 4096 x 1600 took 49.0 us, now 23.7; the bytes take 8.)
-template <bool RMS, int NV, bool RAGGED>
-__global__ void __launch_bounds__(256, NV <= 2 ? 2 : 1)
+// Bound by the chain from a row's arrival through two sums and a barrier, then by issue, so up to 2048 columns a step takes
+// several rows: their sums share shuffles, barrier and latency, and more bytes are in flight. us, one row a step / now:
+// LayerNorm 4096 x 1600 20.4 / 17.7, 16384 x 1600 58 / 49, 1024 x 1600 11.3 / 9.7, 256 x 1600 7.8 / 6.1, 8192 x 2048 35.9 / 29.8;
+// RMSNorm 4096 x 1600 18.3 / 15.5, 8192 x 2048 33.4 / 27.1 (the bytes of 4096 x 1600 take 8). LayerNorm has the second sum plane to keep and
+// does more per row: four rows in one block per SM 17.7, two in each of two blocks 19.5 (RMSNorm 15.7 / 15.5); below two rows per SM
+// four to a block would leave SMs idle, 256 x 1600 6.7 / 6.3.
+template <bool RMS, int NV, bool RAGGED, int R, int BLOCKS>
+__global__ void __launch_bounds__(256, BLOCKS)
 norm_bwd_wide_kernel(bf16* __restrict__ dinp, float* __restrict__ scratch, const bf16* __restrict__ dout,
                      const bf16* __restrict__ inp, const bf16* __restrict__ weight, const float* __restrict__ mean,
                      const float* __restrict__ rstd, int N, int C_, int accumulate_dinp) {
     const int C = RAGGED ? C_ : NV * 2048;
-    __shared__ float red[2][2][8];   // [parity][s1 | s2][warp]
+    __shared__ __align__(16) float red[2][2 * R][8];   // [parity][s1, s2 of each row][warp]
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const float inv_c = 1.0f / (float)C;
     auto in_row = [&](int k) { return !RAGGED || (int)(threadIdx.x + 256 * k) * 8 < C; };
-    ptx::f32x2 dw[NV][4], db[RMS ? 1 : NV][4], fw[NV][4];
+    ptx::f32x2 dw[NV][4], db[RMS ? 1 : NV][4];
+    bf16x8 wv[NV];
 #pragma unroll
     for (int k = 0; k < NV; k++) {
-        unpack8p(in_row(k) ? ld128(weight + (threadIdx.x + 256 * k) * 8) : zero8(), fw[k]);
+        wv[k] = in_row(k) ? ld128(weight + (threadIdx.x + 256 * k) * 8) : zero8();
 #pragma unroll
         for (int j = 0; j < 4; j++) {
             dw[k][j] = both(0.f);
             if (!RMS) db[RMS ? 0 : k][j] = both(0.f);
         }
     }
-    bf16x8 dv[NV], xv[NV], ov[NV], dvn[NV], xvn[NV], ovn[NV];
-    auto load = [&](int row, bf16x8* d, bf16x8* x, bf16x8* o) {
+    bf16x8 dvn[R][NV], xvn[R][NV], ovn[R][NV];
+    float m_next[R], rs_next[R];
+    // rows beyond the last are the last again with dout of zero, and are not stored
+    auto load = [&](int first) {
 #pragma unroll
-        for (int k = 0; k < NV; k++) {
-            const size_t off = (size_t)row * C + (threadIdx.x + 256 * k) * 8;
-            d[k] = in_row(k) ? ld128_stream(dout + off) : zero8();
-            x[k] = in_row(k) ? ld128_stream(inp + off) : zero8();
-            if (accumulate_dinp) o[k] = in_row(k) ? ld128(dinp + off) : zero8();
+        for (int r = 0; r < R; r++) {
+            const int row = min(first + r, N - 1);
+#pragma unroll
+            for (int k = 0; k < NV; k++) {
+                const size_t off = (size_t)row * C + (threadIdx.x + 256 * k) * 8;
+                dvn[r][k] = in_row(k) && (R == 1 || first + r < N) ? ld128_stream(dout + off) : zero8();
+                xvn[r][k] = in_row(k) ? ld128_stream(inp + off) : zero8();
+                if (accumulate_dinp) ovn[r][k] = in_row(k) ? ld128(dinp + off) : zero8();
+            }
+            m_next[r] = RMS ? 0.f : mean[row];
+            rs_next[r] = rstd[row];
         }
     };
-    int row = blockIdx.x;
-    float m_next = 0.f, rs_next = 0.f;
-    if (row < N) {
-        load(row, dv, xv, ov);
-        if (!RMS) m_next = mean[row];
-        rs_next = rstd[row];
-    }
+    int row = blockIdx.x * R;
+    if (row < N) load(row);
     int par = 0;
-    for (; row < N; row += gridDim.x, par ^= 1) {
-        const int next = row + gridDim.x;
-        const float m = m_next, rs = rs_next;
-        if (next < N) {
-            load(next, dvn, xvn, ovn);
-            if (!RMS) m_next = mean[next];
-            rs_next = rstd[next];
-        }
-        ptx::f32x2 fn[NV][4], fd[NV][4], a1 = both(0.f), a2 = both(0.f);
+    for (; row < N; row += gridDim.x * R, par ^= 1) {
+        const int next = row + gridDim.x * R;
+        ptx::f32x2 fn[R][NV][4], fd[R][NV][4];
+        bf16x8 ov[R][NV];
+        float rs[R], s[2 * R];
 #pragma unroll
-        for (int k = 0; k < NV; k++) {
-            unpack8p(dv[k], fd[k]);
-            unpack8p(xv[k], fn[k]);
+        for (int r = 0; r < R; r++) {
 #pragma unroll
-            for (int j = 0; j < 4; j++) {
-                fn[k][j] = ptx::mul2(RMS ? fn[k][j] : ptx::add2(fn[k][j], both(-m)), both(rs));
-                dw[k][j] = ptx::fma2(fd[k][j], fn[k][j], dw[k][j]);
-                if (!RMS) db[RMS ? 0 : k][j] = ptx::add2(db[RMS ? 0 : k][j], fd[k][j]);
-                fd[k][j] = ptx::mul2(fd[k][j], fw[k][j]);
-                a1 = ptx::add2(a1, fd[k][j]);
-                a2 = ptx::fma2(fd[k][j], fn[k][j], a2);
+            for (int k = 0; k < NV; k++) {
+                unpack8p(dvn[r][k], fd[r][k]);
+                unpack8p(xvn[r][k], fn[r][k]);
+                ov[r][k] = ovn[r][k];
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    fn[r][k][j] = ptx::mul2(RMS ? fn[r][k][j] : ptx::add2(fn[r][k][j], both(-m_next[r])), both(rs_next[r]));
+                }
             }
+            rs[r] = rs_next[r];
         }
-        float s1 = warp_sum(sum2(a1)), s2 = warp_sum(sum2(a2));
-        if (lane == 0) {
-            red[par][0][warp] = s1;
-            red[par][1][warp] = s2;
+        if (next < N) load(next);
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+            ptx::f32x2 a1 = both(0.f), a2 = both(0.f);
+#pragma unroll
+            for (int k = 0; k < NV; k++) {
+                ptx::f32x2 fw[4];
+                unpack8p(wv[k], fw);
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    dw[k][j] = ptx::fma2(fd[r][k][j], fn[r][k][j], dw[k][j]);
+                    if (!RMS) db[RMS ? 0 : k][j] = ptx::add2(db[RMS ? 0 : k][j], fd[r][k][j]);
+                    fd[r][k][j] = ptx::mul2(fd[r][k][j], fw[j]);
+                    a1 = ptx::add2(a1, fd[r][k][j]);
+                    a2 = ptx::fma2(fd[r][k][j], fn[r][k][j], a2);
+                }
+            }
+            s[2 * r] = sum2(a1);
+            s[2 * r + 1] = sum2(a2);
         }
+        rows_sum<2 * R>(s, lane);
+        constexpr int LANES = 32 / (2 * R);
+        if (lane % LANES == 0) red[par][lane / LANES][warp] = s[0];
         __syncthreads();   // the other parity's slots are free again once every warp has passed this point
-        s1 = 0.f;
-        s2 = 0.f;
 #pragma unroll
-        for (int w = 0; w < 8; w++) {
-            s1 += red[par][0][w];
-            s2 += red[par][1][w];
+        for (int i = 0; i < 2 * R; i++) {
+            s[i] = sum8(red[par][i]) * inv_c;
         }
-        s1 *= inv_c;
-        s2 *= inv_c;
 #pragma unroll
-        for (int k = 0; k < NV; k++) {
-            ptx::f32x2 fo[4];
-            if (accumulate_dinp) unpack8p(ov[k], fo);
+        for (int r = 0; r < R; r++) {
+            if (R > 1 && row + r >= N) continue;
 #pragma unroll
-            for (int j = 0; j < 4; j++) {
-                const ptx::f32x2 t = RMS ? fd[k][j] : ptx::add2(fd[k][j], both(-s1));
-                const ptx::f32x2 d = ptx::fma2(fn[k][j], both(-s2), t);
-                fo[j] = accumulate_dinp ? ptx::fma2(d, both(rs), fo[j]) : ptx::mul2(d, both(rs));
+            for (int k = 0; k < NV; k++) {
+                ptx::f32x2 fo[4];
+                if (accumulate_dinp) unpack8p(ov[r][k], fo);
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    const ptx::f32x2 t = RMS ? fd[r][k][j] : ptx::add2(fd[r][k][j], both(-s[2 * r]));
+                    const ptx::f32x2 d = ptx::fma2(fn[r][k][j], both(-s[2 * r + 1]), t);
+                    fo[j] = accumulate_dinp ? ptx::fma2(d, both(rs[r]), fo[j]) : ptx::mul2(d, both(rs[r]));
+                }
+                if (in_row(k)) st128(dinp + (size_t)(row + r) * C + (threadIdx.x + 256 * k) * 8, pack8p(fo));
             }
-            if (in_row(k)) st128(dinp + (size_t)row * C + (threadIdx.x + 256 * k) * 8, pack8p(fo));
-        }
-#pragma unroll
-        for (int k = 0; k < NV; k++) {
-            dv[k] = dvn[k];
-            xv[k] = xvn[k];
-            ov[k] = ovn[k];
         }
     }
     float* dst = scratch + (size_t)blockIdx.x * 2 * C;
@@ -714,9 +757,20 @@ template <bool RMS, int NV, bool RAGGED = false>
 static int launch_bwd_wide(bf16* dinp, bf16* dweight, bf16* dbias, float* scratch, const bf16* dout, const bf16* inp,
                            const bf16* weight, const float* mean, const float* rstd, int N, int C, int accumulate_dinp,
                            cudaStream_t stream) {
-    int grid = num_sms() * (NV <= 2 ? 2 : 1);
-    if (grid > N) grid = N;
-    norm_bwd_wide_kernel<RMS, NV, RAGGED><<<grid, 256, 0, stream>>>(dinp, scratch, dout, inp, weight, mean, rstd, N, C, accumulate_dinp);
+    auto launch = [&](auto kernel, int rows, int blocks_per_sm) {
+        int grid = num_sms() * blocks_per_sm;
+        if (grid > ceil_div(N, rows)) grid = ceil_div(N, rows);
+        kernel<<<grid, 256, 0, stream>>>(dinp, scratch, dout, inp, weight, mean, rstd, N, C, accumulate_dinp);
+        return grid;
+    };
+    int grid;
+    if constexpr (NV == 1) {
+        grid = !RMS && N >= 2 * num_sms() ? launch(norm_bwd_wide_kernel<RMS, NV, RAGGED, 4, 1>, 4, 1)
+                                          : launch(norm_bwd_wide_kernel<RMS, NV, RAGGED, 2, 2>, 2, 2);
+    } else {
+        constexpr int BLOCKS = NV == 2 ? 2 : 1;
+        grid = launch(norm_bwd_wide_kernel<RMS, NV, RAGGED, 1, BLOCKS>, 1, BLOCKS);
+    }
     LLMK_LAUNCH_CHECK();
     norm_bwd_finish_kernel<<<ceil_div(C, 32), dim3(32, FIN_LANES), 0, stream>>>(dweight, dbias, scratch, grid, C);
     LLMK_LAUNCH_CHECK();
@@ -731,9 +785,10 @@ namespace norm {
 // below, every row has a block of its own anyway. us, block per row / rings, LayerNorm: 128 columns 256 rows 5.3 / 5.3, 512
 // 6.4 / 5.4, 16384 58 / 13; 384 columns 512 rows 6.9 / 7.5, 1024 8.6 / 7.9, 16384 62 / 19; 640 columns 1024 rows 9.9 / 10.8, 2048
 // 13.6 / 11.3; 1272 columns 512 rows 10.2 / 11.1, 1024 12.4 / 11.8, 16384 74 / 50.
-// Rows of whole vectors per lane take the rings from more than two rows per SM on (the other kernel's blocks then get a second row),
-// wider ones from one on: 768 columns 64 rows 4.7 / 7.0, 256 6.3 / 7.1, 296 7.1 / 7.2, 512 7.6 / 7.3; 512 columns 256 rows 5.6 / 6.1; 1024
-// columns 128 rows 5.1 / 6.2, 192 6.6 / 6.2, 256 6.6 / 6.1; 1280 columns 128 rows 5.2 / 6.7, 192 7.0 / 6.7, 296 8.4 / 7.3.
+// Rows of whole vectors per lane take the rings when the other kernel's blocks would get a second step, at more than four rows per SM
+// (256 columns: two): block / rings 768 columns 64 rows 4.7 / 7.0, 320 6.0 / 7.2, 592 6.4 / 8.0, 740 7.5 / 8.4; 512 columns 592 rows 5.8 / 6.3,
+// 740 7.0 / 6.8; 1024 columns 192 rows 5.7 / 6.0, 592 6.7 / 7.7, 888 8.0 / 7.9; 1280 columns 592 rows 7.2 / 8.3, 740 8.8 / 8.6; 256 columns
+// 192 rows 4.8 / 4.8, 592 5.6 / 5.3.
 constexpr int ragged_bulk_rows(int C) { return C <= 256 ? 512 : 1024; }
 
 // The row kernel plus the fixed-order reduction of its partials.
@@ -753,7 +808,7 @@ static int launch_bwd(bf16* dinp, bf16* dweight, bf16* dbias, float* scratch, co
     }
 #define LLMK_NORM_BWD_BULK(NVEC)                                                    \
     case NVEC:                                                                      \
-        if (C == NVEC * 256 && N > (NVEC <= 3 ? 2 : 1) * num_sms()) LLMK_NORM_BWD(launch_bwd_bulk, NVEC) \
+        if (C == NVEC * 256 && N > (NVEC == 1 ? 2 : 4) * num_sms()) LLMK_NORM_BWD(launch_bwd_bulk, NVEC) \
         if (N >= ragged_bulk_rows(C)) LLMK_NORM_BWD(launch_bwd_bulk, NVEC, true) \
         break;
     switch (ceil_div(C, 256)) {

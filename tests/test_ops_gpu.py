@@ -149,10 +149,11 @@ def test_norm_forward_of_wide_rows(N, C):
 
 
 @pytest.mark.parametrize("rms", [False, True])
-@pytest.mark.parametrize("N,C", [(1, 264), (444, 768), (445, 768), (592, 1280), (593, 1024), (148, 1024), (149, 1280), (296, 504), (297, 512)])
+@pytest.mark.parametrize("N,C", [(1, 264), (444, 768), (445, 768), (592, 1280), (593, 1024), (591, 1024), (296, 504), (297, 512), (2, 2048),
+                                 (295, 1600), (297, 1600), (1187, 1600), (5, 2048)])
 def test_norms_of_few_rows(N, C, rms):
     """Row counts on both sides of where a block per row gives way to a warp per row, forward (three rows per SM up to 768
-    columns, four beyond) and backward (two and one), with 148 SMs."""
+    columns, four beyond) and backward (four), with 148 SMs, and counts that are no multiple of the rows of a backward step."""
     test_norms_of_widths_that_are_not_whole_vectors_per_lane(N, C, rms)
     test_norm_forward_of_wide_rows(N, C)
 
