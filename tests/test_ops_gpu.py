@@ -448,6 +448,40 @@ def test_fused_classifier(rows, V, Vp):
     assert abs(tot.item() - ref_losses.mean().item()) < 1e-3
 
 
+@pytest.mark.parametrize("rows,V,Vp", [(1, 1, 8), (449, 50257, 50304), (450, 4999, 5000), (5, 56317, 56320), (149, 56325, 56328), (3, 84473, 84480),
+                                       (7, 84481, 84488), (200, 128001, 128256), (3, 140801, 140808), (77, 225279, 225280), (2, 225281, 225288)])
+def test_fused_classifier_over_blocks_and_clusters(rows, V, Vp):
+    """Row widths on both sides of one, three, five and eight blocks per row, several rows per block, columns that are no whole
+    vectors, rows with entries of -infinity, of the type's lowest value, and of a range whose exponentials leave the normal
+    numbers."""
+    from llm_kittens_b200.ops import classifier
+
+    logits = rnd(rows, Vp, scale=3.0)
+    logits[0, : V // 2] = float("-inf")
+    logits[0, V - 1] = 1.0
+    logits[rows // 2, V // 3 : V - 1] = torch.finfo(BF).min
+    logits[rows - 1, ::3] -= 95.0
+    logits[:, V:] = 60.0                                       # not real: neither maximum nor sum may see them
+    tg = torch.randint(0, V, (rows,), device="cuda", dtype=torch.int32)
+    tg[0], tg[rows // 2], tg[rows - 1] = V - 1, 0, V - 1
+    dloss = 0.5
+    lg, lg2 = logits.clone(), logits.clone()
+    got = classifier.fused_classifier(lg, tg, V, dloss)
+    assert torch.equal(classifier.fused_classifier(lg2, tg, V, dloss, write_dlogits=False), got) and torch.equal(lg2, logits)
+    for r in range(rows):                                      # row by row: a double copy of all would not be small
+        x = logits[r, :V].double()
+        p = torch.softmax(x, -1)
+        ref = torch.logsumexp(x, -1) - x[tg[r].long()]
+        # fp32 sums of exponentials of 2 ulp, and a logarithm of 2 ulp
+        assert abs(got[r].double() - ref) <= 1e-5 * (1 + ref.abs()), (r, got[r], ref)
+        want = p.clone()
+        want[tg[r].long()] -= 1
+        want *= dloss
+        # the exponential is rounded to bf16 and the gradient again (one of each where the row spans blocks), each 2^-9
+        assert ((lg[r, :V].double() - want).abs() <= 2.0 ** -8 * (p.abs() * dloss + want.abs()) + 1e-6).all(), r
+    assert (lg[:, V:] == 0).all()
+
+
 def _ref_attention(qkv, B, T, NH, NKVH, HS):
     x = qkv.float().view(B, T, NH + 2 * NKVH, HS)
     q = x[:, :, :NH].transpose(1, 2)
