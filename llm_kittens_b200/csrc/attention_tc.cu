@@ -39,6 +39,7 @@ int make_tmap_3d(CUtensorMap* m, const void* ptr, uint64_t inner, uint64_t rows,
 namespace attn_tc {
 
 constexpr int BQ = 128, BKV = 128;
+constexpr int INFO_SLOTS = 4;  // decoded tiles on their way from the producer to the others
 constexpr int THREADS = 256;   // warpgroup 0: producer, MMA issuer, two idle warps; warpgroup 1: softmax
 constexpr int ATOM_BYTES = 128 * 128;  // one 128-row x 64-column (128-byte) swizzle atom column
 
@@ -47,7 +48,7 @@ struct Cfg {
     static constexpr int TILE_BYTES = BQ * HS * 2;         // Q, K or V tile
     static constexpr int P_BYTES = BQ * BKV * 2;
     static constexpr int SMEM_MAIN = TILE_BYTES * 5 + P_BYTES;
-    static constexpr int SMEM_BYTES = SMEM_MAIN + 192;   // tiles + barriers; the dynamic window itself is 1024-byte aligned
+    static constexpr int SMEM_BYTES = SMEM_MAIN + 256;   // tiles + barriers; the dynamic window itself is 1024-byte aligned
     static_assert((HS == 64 ? 2 : 1) * (SMEM_BYTES + 1024) <= 228 * 1024, "the CTAs of an SM share its shared memory");
     static constexpr int TMEM_COLS = 256;
     static constexpr int CTAS_PER_SM = HS == 64 ? 2 : 1;
@@ -173,9 +174,9 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_const
     uint64_t* s_free = bars + 12;     // [1]
     uint64_t* q_empty = bars + 13;    // [1] the last S of a query tile is computed
     uint64_t* o_free = bars + 14;     // [1] O of a query tile has been read
-    uint64_t* info_full = bars + 15;  // [2] the tile that a turn takes has been decoded
-    int4* info = reinterpret_cast<int4*>(bars + 18);   // [2] (key tiles, query tile, head, batch entry), 0 key tiles = no more
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 22);
+    uint64_t* info_full = bars + 15;  // [INFO_SLOTS] the tile that a turn takes has been decoded
+    int4* info = reinterpret_cast<int4*>(bars + 20);   // [INFO_SLOTS] (key tiles, query tile, head, batch entry), 0 key tiles = no more
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 28);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
     int* skip = reinterpret_cast<int*>(tmem_slot + 2);   // (no static shared memory: two CTAs fill the SM's)
 
@@ -220,8 +221,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_const
         ptx::mbar_init(o_full, 1);
         ptx::mbar_init(o_free, 4);
         ptx::mbar_init(s_free, 4);
-        ptx::mbar_init(&info_full[0], 1);
-        ptx::mbar_init(&info_full[1], 1);
+        for (int i = 0; i < INFO_SLOTS; i++) ptx::mbar_init(&info_full[i], 1);
         *abort_flag = 0;
         ptx::fence_barrier_init();
         ptx::fence_proxy_async_smem();
@@ -292,11 +292,12 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_const
                     if (j == 0) {
                         ok = ptx::mbar_wait(q_empty, (n - 1) & 1, abort_flag, status, LLMK_ST_TIMEOUT_TMA_EMPTY, j);
                         if (!ok) break;
-                        // (every reader of the slot's last content has waited for it: the scores of tile n-1 needed all of
-                        // them to be past tile n-2)
+                        // (every reader of the slot's last content, tile n-4, is done with it: the last scores of tile n-1
+                        // needed all of them to be in the last key tile of n-2, and they read a tile's slot until its end, so
+                        // two slots would not do where tile n-1 has one key tile)
                         if (lane == 0) {
-                            info[n & 1] = make_int4(t.nkv, t.qb, t.h, t.b);
-                            ptx::mbar_arrive(&info_full[n & 1]);
+                            info[n % INFO_SLOTS] = make_int4(t.nkv, t.qb, t.h, t.b);
+                            ptx::mbar_arrive(&info_full[n % INFO_SLOTS]);
                             load_q(t);
                         }
                         __syncwarp();
@@ -312,8 +313,8 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_const
             }
             if (ok) ok = ptx::mbar_wait(q_empty, (n - 1) & 1, abort_flag, status, LLMK_ST_TIMEOUT_TMA_EMPTY, -3);
             if (ok && lane == 0) {
-                info[n & 1] = make_int4(0, 0, 0, 0);
-                ptx::mbar_arrive(&info_full[n & 1]);
+                info[n % INFO_SLOTS] = make_int4(0, 0, 0, 0);
+                ptx::mbar_arrive(&info_full[n % INFO_SLOTS]);
             }
         } else if (warp == 1 && lane == 0) {
             // -------------------------------------------------------- MMA issuer
@@ -330,9 +331,9 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_const
             bool ok = true;
             int c = 0;
             for (int n = 0; ok; n++) {
-                ok = ptx::mbar_wait_spin(&info_full[n & 1], (n >> 1) & 1, abort_flag, status, LLMK_ST_TIMEOUT_TMA_FULL, -2);
+                ok = ptx::mbar_wait_spin(&info_full[n % INFO_SLOTS], (n / INFO_SLOTS) & 1, abort_flag, status, LLMK_ST_TIMEOUT_TMA_FULL, -2);
                 if (!ok) break;
-                const int nkv = info[n & 1].x;
+                const int nkv = info[n % INFO_SLOTS].x;
                 if (nkv == 0) break;
                 ok = ptx::mbar_wait_spin(q_full, n & 1, abort_flag, status, LLMK_ST_TIMEOUT_TMA_FULL, -1);
                 for (int j = 0; j <= nkv && ok; j++, c++) {
@@ -386,8 +387,8 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_const
         bool ok = true;
         int c = 0;
         for (int n = 0; ok; n++) {
-        ok = ptx::mbar_wait(&info_full[n & 1], (n >> 1) & 1, abort_flag, status, LLMK_ST_TIMEOUT_TMA_FULL, -2);
-        const int nkv = info[n & 1].x;
+        ok = ptx::mbar_wait(&info_full[n % INFO_SLOTS], (n / INFO_SLOTS) & 1, abort_flag, status, LLMK_ST_TIMEOUT_TMA_FULL, -2);
+        const int nkv = info[n % INFO_SLOTS].x;
         if (!ok || nkv == 0) break;
         float m = -INFINITY, l = 0.f;
         for (int j = 0; j < nkv && ok; j++, c++) {
@@ -482,7 +483,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_const
         if (lane == 0) ptx::mbar_arrive(o_free);
 #pragma unroll
         for (int q = 0; q < HS / 8; q++) *reinterpret_cast<bf16x8*>(sP + (q >> 3) * ATOM_BYTES + r * 128 + (((q & 7) ^ (r & 7)) << 4)) = o[q];
-        const int4 tile = info[n & 1];
+        const int4 tile = info[n % INFO_SLOTS];
         if (tile.y * BQ + r < T) lse[((size_t)tile.w * NH + tile.z) * T + tile.y * BQ + r] = (m + log2f(l)) * 0.6931471805599453f;
         ptx::fence_proxy_async_smem();
         __syncwarp();

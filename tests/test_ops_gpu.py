@@ -495,6 +495,26 @@ def _ref_attention(qkv, B, T, NH, NKVH, HS):
     return o, torch.logsumexp(s, -1)
 
 
+@pytest.mark.parametrize("B,T,NH,HS", [(200, 128, 12, 64), (40, 256, 20, 64), (64, 192, 12, 64), (60, 128, 8, 128), (37, 320, 12, 64)])
+def test_attention_forward_of_many_short_tiles(B, T, NH, HS):
+    """Several query tiles per resident block, most of them with one or two key tiles: every tile's rows are written, to their
+    own place, each of many times (a block takes its next tile while the last one's rows leave)."""
+    from llm_kittens_b200.ops import attention
+
+    qkv = rnd(B, T, 3 * NH * HS)
+    q, k, v = (t.view(B, T, NH, HS).transpose(1, 2).float() for t in qkv.split(NH * HS, dim=-1))
+    ref = torch.nn.functional.scaled_dot_product_attention(q, k, v, is_causal=True).transpose(1, 2).reshape(B, T, NH * HS)
+    first = None
+    for _ in range(60):
+        out = torch.full((B, T, NH * HS), float("nan"), device="cuda", dtype=BF)
+        lse = torch.full((B, NH, T), float("nan"), device="cuda", dtype=torch.float32)
+        attention.attention_fwd(qkv, B, T, NH, NH, HS, out=out, lse=lse, impl="tc")
+        if first is None:
+            first = out, lse
+            assert (out.float() - ref).abs().max() < 0.03
+        assert torch.equal(out, first[0]) and torch.equal(lse, first[1])
+
+
 @pytest.mark.parametrize("B,T,NH,NKVH,HS", [(2, 128, 4, 4, 64), (1, 256, 12, 12, 64), (2, 192, 8, 2, 64), (1, 128, 4, 2, 128),
                                             (1, 1024, 2, 1, 128)])
 def test_attention_fwd_bwd(B, T, NH, NKVH, HS):
