@@ -886,41 +886,64 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
     }
 }
 
-// fp32 split-K partials -> bf16 output (optionally += existing contents).
-// With `dbias`: the first M / 8 threads also finish the bias gradient from db_partial [db_rows, M] (EPI_DBIAS).
-__global__ void splitk_reduce_kernel(bf16* __restrict__ out, const float* __restrict__ partial, size_t n, int splits,
-                                     int accumulate, bf16* __restrict__ dbias, const float* __restrict__ db_partial, int M,
-                                     int db_rows) {
-    size_t i = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * 8;
+// fp32 split-K partials -> bf16 output (optionally += existing contents). With `dbias`: the first ceil(M / 64) blocks finish the
+// bias gradient from db_partial [db_rows, M] (EPI_DBIAS), a block 64 columns with 32 lanes of rows, added in fixed order.
+// Bound by latency, so the loads of four splits go out together, and no thread walks through all rows of the bias gradient's
+// partials before its own sums as the first ones did (24 of them at 768 x 768): weight and bias gradient of 768 x 768 over 16384
+// tokens 35.1 -> 30.3 us, 2304 x 768 68.6 -> 63.1, 3072 x 768 67.3 -> 66.0; this kernel inside a step of 65536 tokens 9.8 -> 6.9.
+__global__ void __launch_bounds__(256)
+splitk_reduce_kernel(bf16* __restrict__ out, const float* __restrict__ partial, size_t n, int splits, int accumulate,
+                     bf16* __restrict__ dbias, const float* __restrict__ db_partial, int M, int db_rows, int db_blocks) {
+    if ((int)blockIdx.x < db_blocks) {
+        __shared__ float sh[32][65];
+        const int group = threadIdx.x & 7, row = threadIdx.x >> 3;
+        const int col = blockIdx.x * 64 + group * 8, mine = blockIdx.x * 64 + threadIdx.x;
+        const bool finishes = threadIdx.x < 64 && mine < M;
+        float old = 0.f;
+        if (finishes && accumulate) old = __bfloat162float(dbias[mine]);
+        float d[8] = {};
+        if (col < M) {
+            for (int s = row; s < db_rows; s += 32) {
+                const float4* src = reinterpret_cast<const float4*>(db_partial + (size_t)s * M + col);
+                const float4 a = src[0], b = src[1];
+                d[0] += a.x; d[1] += a.y; d[2] += a.z; d[3] += a.w;
+                d[4] += b.x; d[5] += b.y; d[6] += b.z; d[7] += b.w;
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < 8; j++) sh[row][group * 8 + j] = d[j];
+        __syncthreads();
+        if (finishes) {
+            const int rows = db_rows < 32 ? db_rows : 32;
+            for (int r = 0; r < rows; r++) old += sh[r][threadIdx.x];
+            dbias[mine] = __float2bfloat16_rn(old);
+        }
+        return;
+    }
+    const size_t i = ((size_t)(blockIdx.x - db_blocks) * blockDim.x + threadIdx.x) * 8;
     if (i >= n) return;
-    if (dbias != nullptr && i < (size_t)M) {
-        float d[8];
-        if (accumulate) {
-            unpack8(ld128(dbias + i), d);
-        } else {
-#pragma unroll
-            for (int j = 0; j < 8; j++) d[j] = 0.f;
-        }
-        for (int s = 0; s < db_rows; s++) {
-            const float4* src = reinterpret_cast<const float4*>(db_partial + (size_t)s * M + i);
-            const float4 a = src[0], b = src[1];
-            d[0] += a.x; d[1] += a.y; d[2] += a.z; d[3] += a.w;
-            d[4] += b.x; d[5] += b.y; d[6] += b.z; d[7] += b.w;
-        }
-        st128(dbias + i, pack8(d));
-    }
+    constexpr int U = 4;   // splits in flight
+    bf16x8 old = zero8();
+    if (accumulate) old = ld128(out + i);
     float acc[8];
-    if (accumulate) {
-        unpack8(ld128(out + i), acc);
-    } else {
+    for (int s0 = 0; s0 < splits; s0 += U) {
+        float4 a[U], b[U];
 #pragma unroll
-        for (int j = 0; j < 8; j++) acc[j] = 0.f;
-    }
-    for (int s = 0; s < splits; s++) {
-        const float4* src = reinterpret_cast<const float4*>(partial + (size_t)s * n + i);
-        float4 a = __ldcs(src), b = __ldcs(src + 1);
-        acc[0] += a.x; acc[1] += a.y; acc[2] += a.z; acc[3] += a.w;
-        acc[4] += b.x; acc[5] += b.y; acc[6] += b.z; acc[7] += b.w;
+        for (int u = 0; u < U; u++) {
+            if (s0 + u < splits) {
+                const float4* src = reinterpret_cast<const float4*>(partial + (size_t)(s0 + u) * n + i);
+                a[u] = __ldcs(src);
+                b[u] = __ldcs(src + 1);
+            }
+        }
+        if (s0 == 0) unpack8(old, acc);
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            if (s0 + u < splits) {
+                acc[0] += a[u].x; acc[1] += a[u].y; acc[2] += a[u].z; acc[3] += a[u].w;
+                acc[4] += b[u].x; acc[5] += b[u].y; acc[6] += b[u].z; acc[7] += b[u].w;
+            }
+        }
     }
     st128(out + i, pack8(acc));
 }
@@ -1424,8 +1447,9 @@ static int gemm_impl(int mode, int epi, const void* A, const void* B, void* C, v
     if (rc) return rc;
     if (epi & EPI_PARTIAL) {
         const size_t n = (size_t)M * N;
-        splitk_reduce_kernel<<<ceil_div((long)(n / 8), 256), 256, 0, stream>>>(static_cast<bf16*>(C), p.partial, n, p.splits,
-            split_accumulate ? 1 : 0, with_dbias ? p.dbias : nullptr, p.db_partial, M, p.splits * p.tiles_n);
+        const int db_blocks = with_dbias ? ceil_div(M, 64) : 0;
+        splitk_reduce_kernel<<<db_blocks + ceil_div((long)(n / 8), 256), 256, 0, stream>>>(static_cast<bf16*>(C), p.partial, n, p.splits,
+            split_accumulate ? 1 : 0, with_dbias ? p.dbias : nullptr, p.db_partial, M, p.splits * p.tiles_n, db_blocks);
         LLMK_LAUNCH_CHECK();
     }
     return LLMK_OK;

@@ -456,3 +456,26 @@ def test_swiglu_of_few_rows_and_a_wide_output(M, H, K):
     want = torch.nn.functional.silu(gate.double()) * up.double()
     assert ((act.double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-5).all()
     _native.check_status()
+
+
+@pytest.mark.parametrize("M,N,K", [(200, 8192, 8192), (72, 2056, 32768), (768, 768, 16384), (264, 4104, 12288)])
+@pytest.mark.parametrize("accumulate", [False, True])
+def test_weight_and_bias_gradient_from_split_partials(M, N, K, accumulate):
+    """Column counts that are no multiple of the 64 of a finishing block, and more rows of partials than its 32 lanes."""
+    from llm_kittens_b200.ops import gemm
+
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    a, b = (torch.randn(K, w, device="cuda", generator=g).to(torch.bfloat16) for w in (M, N))
+    c0, d0 = torch.randn(M, N, device="cuda", generator=g).to(torch.bfloat16), torch.randn(M, device="cuda", generator=g).to(torch.bfloat16)
+    out, db = c0.clone(), d0.clone()
+    gemm.gemm_tn(a, b, out=out, accumulate=accumulate, dbias=db)
+    ref, dref = a.double().T @ b.double(), a.double().sum(0)
+    if accumulate:
+        ref, dref = ref + c0.double(), dref + d0.double()
+    # fp32 sums of K terms (3e-6 of their root sum of squares K^0.5), one rounding to bf16
+    tol = K ** 0.5 * 1e-4
+    assert ((out.double() - ref).abs() <= 2.0 ** -8 * ref.abs() + tol).all()
+    assert ((db.double() - dref).abs() <= 2.0 ** -8 * dref.abs() + tol).all()
+    again, db2 = c0.clone(), d0.clone()
+    gemm.gemm_tn(a, b, out=again, accumulate=accumulate, dbias=db2)
+    assert torch.equal(again, out) and torch.equal(db2, db)
