@@ -340,17 +340,20 @@ attn_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_c
             ptx::tc_fence_before();
             __syncwarp();
             if (lane == 0) ptx::mbar_arrive(s_free);
-            if (causal && dq0 < lane_group * 32 + 32) {      // some (key, query) pairs of this warp are masked: P = 0
-#pragma unroll
-                for (int i = 0; i < 32; i++)
-                    if (r > i + dq0) vs[i] = 0xff800000u;
-            }
             // P^T in place of S^T
 #pragma unroll
             for (int i = 0; i < 32; i += 4) {
                 const float4 L = *reinterpret_cast<const float4*>(sL + i);
                 exp_pair(vs[i], vs[i + 1], c2, ptx::pack2(L.x, L.y));
                 exp_pair(vs[i + 2], vs[i + 3], c2, ptx::pack2(L.z, L.w));
+            }
+            // Some (key, query) pairs of this warp are masked: P = 0, whatever the query's log-sum-exp is. (A score of -infinity in
+            // front of the exponential would give the keys after a query whose row is NaN a NaN probability, and their dV with
+            // it. The branch behind the exponentials costs 0.5 % of the backward, selects without it 4 %.)
+            if (causal && dq0 < lane_group * 32 + 32) {
+#pragma unroll
+                for (int i = 0; i < 32; i++)
+                    if (r > i + dq0) vs[i] = 0;
             }
             // dS^T = P^T * (dP^T - D)
             ok = ptx::mbar_wait(d_full, it & 1, abort_flag, status, LLMK_ST_TIMEOUT_TMA_FULL, 6000 + it);

@@ -540,6 +540,38 @@ def test_attention_fwd_bwd(B, T, NH, NKVH, HS):
     assert torch.equal(dqkv, dqkv2)
 
 
+@pytest.mark.parametrize("dkv,HS", [("1", 64), ("2", 64), ("1", 128)])
+@pytest.mark.parametrize("T,bad", [(256, 0), (256, 70), (256, 200), (320, 291)])
+def test_attention_backward_with_one_query_that_is_nan(T, bad, HS, dkv, monkeypatch):
+    """One query's scores, output and log-sum-exp are NaN. The keys after it never saw it: their dV is that of the other queries,
+    and so is every other row of dQ."""
+    from llm_kittens_b200.ops import _native, attention as attn
+
+    monkeypatch.setenv("LLMK_ATTN_BWD_DKV", dkv)
+    B, NH, NKVH = 2, 4, 2
+    W, C = (NH + 2 * NKVH) * HS, NH * HS
+    qkv, dout = rnd(B, T, W), rnd(B, T, C)
+    clean = qkv.double()
+    qkv[0, bad, HS:2 * HS] = float("nan")                     # head 1 of sequence 0, which reads key head 0
+    out, lse = attn.attention_fwd(qkv, B, T, NH, NKVH, HS, impl="tc")
+    assert lse[0, 1, bad].isnan() and lse.isnan().sum() == 1
+    dqkv = attn.attention_bwd(dout, qkv, out, lse, B, T, NH, NKVH, HS)
+    _native.check_status()
+    clean[0, bad, HS:2 * HS] = 0                               # (any finite query: it has no part in what is compared)
+    leaf = clean.requires_grad_(True)
+    x = leaf.view(B, T, NH + 2 * NKVH, HS).transpose(1, 2)
+    q, k, v = x[:, :NH], x[:, NH:NH + NKVH].repeat_interleave(NH // NKVH, 1), x[:, NH + NKVH:].repeat_interleave(NH // NKVH, 1)
+    s = (q @ k.transpose(-1, -2) / math.sqrt(HS)).masked_fill(torch.ones(T, T, device="cuda", dtype=torch.bool).triu(1), float("-inf"))
+    ((s.softmax(-1) @ v).transpose(1, 2).reshape(B, T, C) * dout.double()).sum().backward()
+    got, want = dqkv.double(), leaf.grad
+    # as in the comparison of the gradients of ordinary inputs
+    dv = slice((NH + NKVH) * HS, (NH + NKVH + 1) * HS)
+    assert (got[0, bad + 1:, dv] - want[0, bad + 1:, dv]).abs().max() < 0.08
+    others = [t for t in range(T) if t != bad]
+    assert (got[0, others, :C] - want[0, others, :C]).abs().max() < 0.08
+    assert (got[1] - want[1]).abs().max() < 0.08
+
+
 @pytest.mark.parametrize("dkv,impl", [("1", "tc"), ("2", "tc"), ("2", None)])
 @pytest.mark.parametrize("B,T,NH,NKVH,HS", [(2, 320, 4, 2, 64), (3, 448, 2, 2, 64), (2, 320, 4, 1, 128), (2, 576, 2, 2, 128),
                                             (1, 1088, 4, 1, 64), (73, 1088, 5, 5, 64)])
