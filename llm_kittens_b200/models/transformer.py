@@ -358,17 +358,23 @@ class Transformer:
             self._dweight(d_fch, ln2, g["fcw"][l], g["fcb"][l])
 
     # ------------------------------------------------------------------ all blocks from one native call
+    def _blocks_replaced(self) -> bool:
+        """Whether a method that :meth:`_block_forward` is made of has been replaced, in a subclass, in the class itself or on
+        this object, or an op that it calls, in its module (a timing or tracing wrapper, another MLP): the blocks then run one
+        by one, so that the replacement is called."""
+        cls, own = type(self), vars(self)
+        return (any(n in own or getattr(cls, n) is not f for n, f in _BLOCK_METHODS)
+                or any(getattr(module, n) is not f for module, n, f in _BLOCK_OPS))
+
     def _forward_native(self, x: torch.Tensor) -> torch.Tensor | None:
         """The blocks' forward by ``llmk_forward_layers``, the launches of :meth:`_block_forward` without a Python call for
         each (GPT-2 124M, one window of 64 tokens: 0.71 -> 0.56 ms, no longer bound by the host). Returns the last block's output, or None, having done
         nothing, where something is to happen between the launches (hooks, weights that are still being gathered, the step
-        ledger, checkpointing, an MLP of another kind), a switch asks for other kernels, or the tensors are not what
-        :meth:`allocate` and the layout make. Addresses are taken anew in every forward."""
+        ledger, checkpointing, an MLP of another kind, methods or ops that somebody replaced), a switch asks for other kernels, or
+        the tensors are not what :meth:`allocate` and the layout make. Addresses are taken anew in every forward."""
         cfg, a, p, L = self.config, self._acts, self._p, self.config.num_layers
-        cls = type(self)
-        if (not x.is_cuda or x.dtype != BF16 or not x.is_contiguous() or self.param_hook is not None or self.recompute >= 3 or gemm._B_READY or _native.ledger_running()
-                or cls._mlp_forward is not Transformer._mlp_forward or cls._block_forward is not Transformer._block_forward
-                or cls._norm_fwd is not Transformer._norm_fwd):
+        if (not x.is_cuda or x.dtype != BF16 or not x.is_contiguous() or self.param_hook is not None or self.recompute >= 3
+                or gemm._B_READY or _native.ledger_running() or self._blocks_replaced()):
             return None
         B, T, C, H, NH, KV, HS = self.B, self.T, cfg.channels, cfg.hidden_dim, cfg.num_heads, cfg.num_kv_heads, cfg.head_size
         BT, QW = B * T, cfg.qkv_width
@@ -533,3 +539,10 @@ class Transformer:
 
     def logits_view(self) -> torch.Tensor:
         return self.acts["logits"].view(self.B, self.T, -1)
+
+
+# What the native forward stands in for, as defined: the methods and the ops of a block.
+_BLOCK_METHODS = tuple((n, getattr(Transformer, n)) for n in ("_block_forward", "_mlp_forward", "_norm_fwd", "_layers", "_idx"))
+_BLOCK_OPS = tuple((module, n, getattr(module, n)) for module, names in (
+    (gemm, ("gemm_nt", "gemm_qkv_rope", "gemm_swiglu")), (norm_ops, ("layernorm_fwd", "rmsnorm_fwd")),
+    (attn_ops, ("attention_fwd",)), (ew, ("rope_qk_", "swiglu_fwd"))) for n in names)

@@ -405,3 +405,42 @@ def test_blocks_forward_from_one_native_call_is_the_same_as_block_by_block(famil
         assert n == launches
         assert all(torch.equal(acts[k], want[k]) for k in want)
     _native.check_status()
+
+
+@pytest.mark.parametrize("family", ["gpt2", "llama3"])
+@pytest.mark.parametrize("where,name,per_layer", [("object", "_norm_fwd", 2), ("object", "_mlp_forward", 1), ("object", "_block_forward", 1),
+                                                  ("class", "_norm_fwd", 2), ("class", "_mlp_forward", 1), ("gemm", "gemm_nt", None),
+                                                  ("attn_ops", "attention_fwd", 1), ("norm_ops", None, 2)])
+def test_what_replaces_a_part_of_a_block_is_called_in_every_block(family, where, name, per_layer, monkeypatch):
+    """A wrapper set on one model, on the class or in an ops module sees each block's calls, and changes no bit."""
+    from llm_kittens_b200.models import transformer
+    from llm_kittens_b200.models.config import ModelConfig
+
+    llama = family == "llama3"
+    cfg = ModelConfig(family=family, max_seq_len=128, vocab_size=500, padded_vocab_size=512, num_layers=3, num_heads=4,
+                      num_kv_heads=2 if llama else 4, channels=256, hidden_dim=512)
+    model = transformer.Transformer(cfg, device="cuda")
+    model.init_weights(3)
+    x = torch.randint(0, 500, (2, 128), dtype=torch.int32, device="cuda")
+    model.forward(x, None)
+    want = model.logits_view().clone()
+    if where == "norm_ops":
+        name = "rmsnorm_fwd" if llama else "layernorm_fwd"
+    if per_layer is None:                       # the products that are not in an epilogue of another entry point
+        per_layer = 2 if llama else 4
+    owner = {"object": model, "class": transformer.Transformer}.get(where) or getattr(transformer, where)
+    original, seen = getattr(owner, name), []
+
+    def wrapper(*args, **kwargs):
+        seen.append(name)
+        return original(*args, **kwargs)
+
+    monkeypatch.setattr(owner, name, wrapper)
+    model.forward(x, None)
+    # (the last norm and the head go through the same ops)
+    assert len(seen) == per_layer * cfg.num_layers + (name in ("_norm_fwd", "gemm_nt") or where == "norm_ops")
+    assert torch.equal(model.logits_view(), want)
+    monkeypatch.undo()
+    seen.clear()
+    model.forward(x, None)
+    assert seen == [] and torch.equal(model.logits_view(), want)
