@@ -13,6 +13,7 @@
 //             64-row query tile and loops over the K/V tiles at or before it. Both recompute
 //             P = exp2(S*c - LSE) from the saved log-sum-exp; D = rowsum(dO * O) comes from a small
 //             pre-pass.
+#include "block_ops.cuh"
 #include "common.cuh"
 
 namespace llmk {

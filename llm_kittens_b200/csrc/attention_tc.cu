@@ -30,6 +30,7 @@
 // Every wait is bounded and reports through the status word.
 
 #include "attention_order.cuh"
+#include "block_ops.cuh"
 #include "ptx_sm100.cuh"
 
 namespace llmk {

@@ -5,6 +5,7 @@
 // llmc/encoder.cuh:157-234, matmul_backward_bias (llmc/matmul.cuh:1203-1236) and the Llama-local
 // add/gather kernels (train_llama3.cu:189-251). All use 128-bit accesses; everything that sums over
 // tokens does so in a fixed order (no atomics), so gradients are bit-reproducible.
+#include "block_ops.cuh"
 #include "common.cuh"
 
 namespace llmk {

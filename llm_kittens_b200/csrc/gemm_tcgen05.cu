@@ -29,6 +29,7 @@
 // Every wait is bounded (ptx::mbar_wait) and reports through `status`.
 #include <cstdlib>
 
+#include "block_ops.cuh"
 #include "ptx_sm100.cuh"
 
 namespace llmk {

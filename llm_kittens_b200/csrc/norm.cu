@@ -10,6 +10,7 @@
 //     its dweight/dbias contributions into fp32 accumulators in registers (fixed columns per lane, so no atomics); a
 //     block's accumulators are summed in fixed order into one partial per block in a global scratch buffer, and a second
 //     kernel sums the block partials in fixed order into the bf16 gradients (+=). Bit-reproducible run to run.
+#include "block_ops.cuh"
 #include "ptx_sm100.cuh"
 
 namespace llmk {

@@ -405,7 +405,7 @@ class Transformer:
         head = (L, B, T, C, NH, KV, HS, H, int(llama), rope_mode, int(self.rope_interleaved), int(attn_ops.forward_is_tc(B, T, NH, HS)),
                 gemm.max_ctas(), _native.status_word().data_ptr(), a["rope"].data_ptr() if llama else 0, x.data_ptr())
         block = array.array("q", (*head, *words))
-        _native.call("llmk_forward_layers", block.buffer_info()[0], float(cfg.norm_eps))
+        _native.call("llmk_forward_layers", *block.buffer_info(), float(cfg.norm_eps))
         _native.count_replayed(L * (8 if rope_mode == 2 else 7) - 1)
         return a["res3"][L - 1]
 

@@ -54,6 +54,7 @@ def lib() -> ctypes.CDLL:
                     _build.build()
                 handle = ctypes.CDLL(str(path))
                 handle.llmk_last_error.restype = ctypes.c_char_p
+                handle.llmk_forward_layers_refused.restype = ctypes.c_char_p
                 for fn in ("llmk_gemm_workspace_bytes", "llmk_norm_bwd_scratch_bytes", "llmk_dbias_scratch_bytes",
                            "llmk_bucket_sort_scratch_ints", "llmk_encoder_bwd_scratch_floats"):
                     getattr(handle, fn).restype = ctypes.c_long
@@ -185,6 +186,8 @@ def call(name: str, *args: Any) -> None:
     _LAUNCHES += _KERNELS_PER_CALL.get(name, 1)
     if rc != 0:
         detail = lib().llmk_last_error().decode() if rc == -1 else ""
+        if name == "llmk_forward_layers":      # which of its launches
+            name = lib().llmk_forward_layers_refused().decode()
         raise NativeError(f"{name} failed: {ERRORS.get(rc, rc)} {detail}")
 
 

@@ -1,5 +1,7 @@
 """The launch schedule of the models without a GPU: the native library is replaced by a recorder, so that the order of the
 calls, and what each is handed, can be looked at."""
+import array
+
 import pytest
 import torch
 
@@ -119,3 +121,14 @@ def test_forward_attention_kernel_by_size(calls, monkeypatch, B, T, NH, HS, tc):
         attention.attention_fwd(qkv, B, T, NH, NH, HS, impl=impl)
     name = lambda on: "llmk_attention_fwd_tc" if on else "llmk_attention_fwd"
     assert [c[0] for c in calls] == [name(tc), name(T % 128 == 0 or T > 256), name(False)]
+
+
+@pytest.mark.parametrize("llama,short,entry", [(0, 0, "llmk_layernorm_fwd"), (1, 0, "llmk_rmsnorm_fwd"), (0, 1, "llmk_forward_layers")])
+def test_what_the_native_forward_refuses_is_named(monkeypatch, llama, short, entry):
+    """The entry point that refuses a shape is named, as when the blocks run one by one (an odd width, which the norm refuses
+    before it launches anything); an argument block of another length is not read."""
+    words = [1, 1, 64, 13, 1, 1, 13, 52, llama] + [0] * (7 + 2 * 29 - short)
+    block = array.array("q", words)
+    monkeypatch.setattr(_native, "_invoke", lambda name, args: getattr(_native.lib(), name)(*[_native._conv(a) for a in args], None))
+    with pytest.raises(_native.NativeError, match=f"^{entry} failed: unsupported or misaligned shape"):
+        _native.call("llmk_forward_layers", *block.buffer_info(), 1e-5)
