@@ -322,8 +322,7 @@ norm_fwd_wide_kernel(bf16* __restrict__ normed, float* __restrict__ mean_out, fl
 
 // Backward. Both kernels: two values per instruction, and the row's statistics fetched a row ahead (they stood between a row's
 // arrival and its sums). us before / after, LayerNorm: 65536 x 768 77.8 / 69.7, 16384 x 1024 35.4 / 31.0, 8192 x 1024 21.0 / 19.5, 65536 x
-// 384 61.8 / 41.0, 3136 x 4096 39.8 / 27.1 (but 3136 x 768 11.6 / 12.1: the terms of a row kept for the second
-// pass spill where 16 warps leave 128 registers; computed again they cost more, 13.5); RMSNorm 3136 x 4096 30.3 / 23.7.
+// 384 61.8 / 41.0, 3136 x 4096 39.8 / 27.1; RMSNorm 3136 x 4096 30.3 / 23.7.
 //
 // With a bulk-copy ring: every warp owns rows and streams them (dout, inp and, when accumulating, the old
 // dinp) into its own shared-memory ring with cp.async.bulk, STAGES rows ahead, so that about
@@ -331,6 +330,10 @@ norm_fwd_wide_kernel(bf16* __restrict__ normed, float* __restrict__ mean_out, fl
 // registers alone it reached well under half of the copy bandwidth). The dweight / dbias sums stay in registers over all
 // rows of a warp. scratch layout: [gridDim.x][2][C] fp32 (second plane unused for RMSNorm). Every wait is bounded; a
 // failure goes to `status`. RAGGED: C is any multiple of 8 up to 256 * NVEC (a row is then still whole 16-byte pieces).
+// FEW: the next row's statistics are asked for when this one has arrived, not before: with one or two rows per warp the first
+// one otherwise waits for both. us, one value per instruction / statistics before / FEW, LayerNorm: 3136 x 768 11.7 / 12.2 / 11.6, 4096 x 768
+// 12.5 / 13.1 / 12.3, 2048 x 768 without old gradients 8.8 / 9.0 / 8.7; RMSNorm 4096 x 512 8.8 / 9.1 / 8.8; but LayerNorm 8192 x 512 13.6 / 12.6 /
+// 12.7, 65536 x 512 60.6 / 48.3 / 49.8.
 template <int NVEC>
 struct BulkCfg {
     static constexpr int C = NVEC * 256;   // widest row
@@ -343,7 +346,7 @@ struct BulkCfg {
     static constexpr int SMEM = OFF_BAR + WARPS * STAGES * 8;
 };
 
-template <bool RMS, int NVEC, bool RAGGED>
+template <bool RMS, int NVEC, bool RAGGED, bool FEW>
 __global__ void __launch_bounds__(BulkCfg<NVEC>::WARPS * 32, 1)
 norm_bwd_bulk_kernel(bf16* __restrict__ dinp, float* __restrict__ scratch, const bf16* __restrict__ dout,
                      const bf16* __restrict__ inp, const bf16* __restrict__ weight, const float* __restrict__ mean,
@@ -393,20 +396,18 @@ norm_bwd_bulk_kernel(bf16* __restrict__ dinp, float* __restrict__ scratch, const
         }
 
     bool ok = true;
-    // (the row's statistics are fetched one row ahead: they stood between a row's arrival and its sums)
     float m_next = 0.f, rs_next = 0.f;
-    if (nrows > 0) {
-        if (!RMS) m_next = mean[first];
-        rs_next = rstd[first];
-    }
+    auto statistics = [&](int i) {
+        if (i >= nrows) return;
+        if (!RMS) m_next = mean[first + i * stride];
+        rs_next = rstd[first + i * stride];
+    };
+    statistics(0);
     for (int i = 0; i < nrows; i++) {
         const int st = i % STAGES;
         const int row = first + i * stride;
         const float m = m_next, rs = rs_next;
-        if (i + 1 < nrows) {
-            if (!RMS) m_next = mean[row + stride];
-            rs_next = rstd[row + stride];
-        }
+        if (!FEW) statistics(i + 1);
         ok = ptx::mbar_wait(&full[st], (i / STAGES) & 1, abort_flag, status, LLMK_ST_TIMEOUT_TMA_FULL, 8000 + st);
         if (!ok) break;
         const uint8_t* src = ring + st * 3 * SLOT;
@@ -419,6 +420,7 @@ norm_bwd_bulk_kernel(bf16* __restrict__ dinp, float* __restrict__ scratch, const
         }
         __syncwarp();   // the stage has been copied into registers by every lane: refill it
         if (lane == 0 && i + STAGES < nrows) issue(i + STAGES);
+        if (FEW) statistics(i + 1);
         // n = (x - m) * rs in place of x, dn = dout * w in place of dout
         ptx::f32x2 fn[NVEC][4], fd[NVEC][4], a1 = both(0.f), a2 = both(0.f);
 #pragma unroll
@@ -740,14 +742,15 @@ static int launch_bwd_bulk(bf16* dinp, bf16* dweight, bf16* dbias, float* scratc
                            cudaStream_t stream) {
     using B = BulkCfg<NVEC>;
     static_assert(B::OFF_BAR >= B::WARPS * 2 * B::C * 4, "the rings must be able to hold the final reduction buffer");
-    static PerDeviceOnce once_bulk_configured;
-    if (once_bulk_configured.first()) {
-        LLMK_CUDA_TRY(cudaFuncSetAttribute(norm_bwd_bulk_kernel<RMS, NVEC, RAGGED>, cudaFuncAttributeMaxDynamicSharedMemorySize, B::SMEM));
-    }
+    constexpr bool MAY_BE_FEW = NVEC <= 3;   // (wider rows have half as many warps, four or three rows in flight each: no difference)
+    const bool few = MAY_BE_FEW && N <= 2 * B::WARPS * num_sms();
+    auto kernel = few ? norm_bwd_bulk_kernel<RMS, NVEC, RAGGED, MAY_BE_FEW> : norm_bwd_bulk_kernel<RMS, NVEC, RAGGED, false>;
+    static PerDeviceOnce once_configured[2];
+    if (once_configured[few].first()) LLMK_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, B::SMEM));
     int grid = num_sms();
     const int need = ceil_div(N, B::WARPS);
     if (grid > need) grid = need;
-    norm_bwd_bulk_kernel<RMS, NVEC, RAGGED><<<grid, B::WARPS * 32, B::SMEM, stream>>>(dinp, scratch, dout, inp, weight, mean, rstd, N, C,
+    kernel<<<grid, B::WARPS * 32, B::SMEM, stream>>>(dinp, scratch, dout, inp, weight, mean, rstd, N, C,
         accumulate_dinp, current_status_word());
     LLMK_LAUNCH_CHECK();
     norm_bwd_finish_kernel<<<ceil_div(C, 32), dim3(32, FIN_LANES), 0, stream>>>(dweight, dbias, scratch, grid, C);

@@ -132,6 +132,30 @@ def test_norms_of_widths_that_are_not_whole_vectors_per_lane(N, C, rms):
         assert torch.isnan(whole[view.numel():]).all() and not torch.isnan(view).any()
 
 
+@pytest.mark.parametrize("rms", [False, True])
+@pytest.mark.parametrize("C", [256, 520, 768])
+@pytest.mark.parametrize("extra", [0, 1])
+def test_norm_backward_on_both_sides_of_two_rows_per_warp(C, extra, rms):
+    """Every warp of every SM has two rows, and one of them a third."""
+    from llm_kittens_b200.ops import norm
+
+    N = 32 * torch.cuda.get_device_properties(0).multi_processor_count + extra
+    x, dout, dinp0, w = rnd(N, C), rnd(N, C), rnd(N, C), rnd(C, scale=0.5) + 1
+    xd, wd = x.double().requires_grad_(True), w.double().requires_grad_(True)
+    bd = torch.zeros(C, device="cuda", dtype=torch.float64, requires_grad=True)
+    mean = torch.zeros(N, device="cuda") if rms else x.double().mean(-1).float()
+    rstd = torch.rsqrt((x.double() - mean.double()[:, None]).pow(2).mean(-1) + 1e-5).float()
+    y = xd * torch.rsqrt(xd.pow(2).mean(-1, keepdim=True) + 1e-5) * wd if rms else torch.nn.functional.layer_norm(xd, (C,), wd, bd, 1e-5)
+    y.backward(dout.double())
+    dinp, dw, db = dinp0.clone(), torch.zeros_like(w), torch.zeros_like(w)
+    if rms:
+        norm.rmsnorm_bwd(dinp, dw, dout, x, w, rstd, accumulate_dinp=True)
+    else:
+        norm.layernorm_bwd(dinp, dw, db, dout, x, w, mean, rstd, accumulate_dinp=True)
+        assert rounded(db, bd.grad, 1e-3)
+    assert rounded(dinp, xd.grad + dinp0.double(), 1e-3) and rounded(dw, wd.grad, 1e-3)   # as in the test above
+
+
 @pytest.mark.parametrize("N,C", [(3, 1288), (2, 8200), (300, 16384)])
 def test_norm_forward_of_wide_rows(N, C):
     from llm_kittens_b200.ops import norm
