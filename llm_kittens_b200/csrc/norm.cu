@@ -127,9 +127,106 @@ __device__ __forceinline__ float sum8(const float* p) {
     return ((((((a.x + a.y) + a.z) + a.w) + b.x) + b.y) + b.z) + b.w;
 }
 
+// The arithmetic of a thread's NV vectors of a row, in_row(k) telling which of them exist: two values per instruction with their
+// fp32 values kept (PACKED), or one at a time and converted again in every pass.
+template <bool RMS, int NV, bool PACKED>
+struct RowMath {
+    ptx::f32x2 f[PACKED ? NV : 1][4];
+    // the sum of the values (RMS: of their squares)
+    __device__ __forceinline__ float sum(const bf16x8* x) {
+        if constexpr (PACKED) {
+            ptx::f32x2 acc = both(0.f);
+#pragma unroll
+            for (int k = 0; k < NV; k++) {
+                unpack8p(x[k], f[k]);
+#pragma unroll
+                for (int j = 0; j < 4; j++) acc = RMS ? ptx::fma2(f[k][j], f[k][j], acc) : ptx::add2(acc, f[k][j]);
+            }
+            return sum2(acc);
+        } else {
+            float acc = 0.f;
+#pragma unroll
+            for (int k = 0; k < NV; k++) {
+                float v[8];
+                unpack8(x[k], v);
+#pragma unroll
+                for (int j = 0; j < 8; j++) acc += RMS ? v[j] * v[j] : v[j];
+            }
+            return acc;
+        }
+    }
+    // the sum of the squared distances from the mean
+    template <class InRow>
+    __device__ __forceinline__ float squares(const bf16x8* x, float mean, InRow in_row) {
+        if constexpr (PACKED) {
+            ptx::f32x2 acc = both(0.f);
+#pragma unroll
+            for (int k = 0; k < NV; k++) {
+                if (!in_row(k)) continue;
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    f[k][j] = ptx::add2(f[k][j], both(-mean));
+                    acc = ptx::fma2(f[k][j], f[k][j], acc);
+                }
+            }
+            return sum2(acc);
+        } else {
+            float acc = 0.f;
+#pragma unroll
+            for (int k = 0; k < NV; k++) {
+                float v[8];
+                unpack8(x[k], v);
+#pragma unroll
+                for (int j = 0; j < 8; j++) {
+                    const float d = in_row(k) ? v[j] - mean : 0.f;
+                    acc += d * d;
+                }
+            }
+            return acc;
+        }
+    }
+    // the normalised values of vector k
+    __device__ __forceinline__ bf16x8 result(const bf16x8* x, int k, float mean, float rstd, const bf16x8& weight, const bf16x8& bias) {
+        if constexpr (PACKED) {
+            ptx::f32x2 w[4], b[4], y[4];
+            unpack8p(weight, w);
+            if (!RMS) unpack8p(bias, b);
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                const ptx::f32x2 n = ptx::mul2(f[k][j], both(rstd));
+                y[j] = RMS ? ptx::mul2(n, w[j]) : ptx::fma2(n, w[j], b[j]);
+            }
+            return pack8p(y);
+        } else {
+            float v[8], w[8], b[8];
+            unpack8(x[k], v);
+            unpack8(weight, w);
+            if (!RMS) unpack8(bias, b);
+#pragma unroll
+            for (int j = 0; j < 8; j++) {
+                const float n = (v[j] - mean) * rstd;
+                v[j] = RMS ? n * w[j] : n * w[j] + b[j];
+            }
+            return pack8(v);
+        }
+    }
+};
+
+// Which arithmetic, and how many blocks per SM the registers have to leave room for (0: the compiler's choice). Packed is what LayerNorm's
+// throughput needs; a launch that waits for memory or for its own chain is shorter without. us, one value at a time as
+// before there was the other / packed / now: RMSNorm with a residual 65536 x 512 45.9 / 50.9 / 45.8, 8192 x 512 7.9 / 8.6 / 7.7, 600 x 1024 3.7 / 3.9 /
+// 3.7 (widths that are not whole vectors per lane, and 256, are the same or better packed); LayerNorm without kept weights 1024 x 1280
+// 4.0 / 4.1 / 3.8, 2048 x 768 4.2 / 4.4 / 4.1, with a residual 1024 x 1280 5.25 / 5.36 / 5.1. LayerNorm with a residual and kept weights of 264 to 512
+// columns, 98 registers and two blocks: 65536 x 384 38.2 / 41.8 / 36, 65536 x 512 48.4 / 52.0 / 47, 3136 x 264 4.1 / 4.4 / 4.0 with three.
+constexpr bool fwd_packed(bool rms, bool fused, int nvec, bool ragged, bool keep) {
+    return rms ? !fused || nvec == 1 || ragged : keep || !(nvec == 5 || (nvec == 3 && !fused));
+}
+constexpr int fwd_blocks(bool rms, bool fused, int nvec, bool keep, bool packed) {
+    return !packed ? 1 : (!rms && keep && fused && nvec == 2 ? 3 : 0);
+}
 // AHEAD: the next row is loaded before the current one is reduced. KEEP: weight and bias stay in registers.
 template <bool RMS, bool FUSED_RESIDUAL, int NVEC, bool RAGGED, bool AHEAD, bool KEEP>
-__global__ void __launch_bounds__(REG_WARPS * 32)
+__global__ void __launch_bounds__(REG_WARPS * 32, fwd_blocks(RMS, FUSED_RESIDUAL, NVEC, KEEP, fwd_packed(RMS, FUSED_RESIDUAL, NVEC, RAGGED, KEEP)))
 norm_fwd_reg_kernel(bf16* __restrict__ normed, float* __restrict__ mean_out, float* __restrict__ rstd_out,
                     bf16* residual_out, const bf16* inp1, const bf16* __restrict__ inp2, const bf16* __restrict__ weight,
                     const bf16* __restrict__ bias, int N, int C_, float eps) {
@@ -172,30 +269,14 @@ norm_fwd_reg_kernel(bf16* __restrict__ normed, float* __restrict__ mean_out, flo
             load(inp1, next, xn);
             if (FUSED_RESIDUAL) load(inp2, next, yn);
         }
-        ptx::f32x2 f[NVEC][4], acc = both(0.f);
-#pragma unroll
-        for (int k = 0; k < NVEC; k++) {
-            unpack8p(xv[k], f[k]);
-#pragma unroll
-            for (int j = 0; j < 4; j++) acc = RMS ? ptx::fma2(f[k][j], f[k][j], acc) : ptx::add2(acc, f[k][j]);
-        }
-        const float sum = warp_sum(sum2(acc));
+        RowMath<RMS, NVEC, fwd_packed(RMS, FUSED_RESIDUAL, NVEC, RAGGED, KEEP)> math;
+        const float sum = warp_sum(math.sum(xv));
         float mean = 0.f, rstd;
         if (RMS) {
             rstd = rsqrtf(sum * inv_c + eps);
         } else {
             mean = sum * inv_c;
-            acc = both(0.f);
-#pragma unroll
-            for (int k = 0; k < NVEC; k++) {
-                if (!in_row(k)) continue;
-#pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    f[k][j] = ptx::add2(f[k][j], both(-mean));
-                    acc = ptx::fma2(f[k][j], f[k][j], acc);
-                }
-            }
-            const float var = warp_sum(sum2(acc));
+            const float var = warp_sum(math.squares(xv, mean, in_row));
             rstd = rsqrtf(var * inv_c + eps);
         }
         if (lane == 0) {
@@ -205,15 +286,9 @@ norm_fwd_reg_kernel(bf16* __restrict__ normed, float* __restrict__ mean_out, flo
 #pragma unroll
         for (int k = 0; k < NVEC; k++) {
             if (!in_row(k)) continue;
-            ptx::f32x2 w[4], b[4];
-            unpack8p(KEEP ? wv[KEEP ? k : 0] : ld128(weight + (lane + 32 * k) * 8), w);
-            if (!RMS) unpack8p(KEEP ? bv[KEEP && !RMS ? k : 0] : ld128(bias + (lane + 32 * k) * 8), b);
-#pragma unroll
-            for (int j = 0; j < 4; j++) {
-                const ptx::f32x2 n = ptx::mul2(f[k][j], both(rstd));
-                f[k][j] = RMS ? ptx::mul2(n, w[j]) : ptx::fma2(n, w[j], b[j]);
-            }
-            st128(normed + (size_t)row * C + (lane + 32 * k) * 8, pack8p(f[k]));
+            const bf16x8 w = KEEP ? wv[KEEP ? k : 0] : ld128(weight + (lane + 32 * k) * 8);
+            const bf16x8 b = RMS ? w : (KEEP ? bv[KEEP && !RMS ? k : 0] : ld128(bias + (lane + 32 * k) * 8));
+            st128(normed + (size_t)row * C + (lane + 32 * k) * 8, math.result(xv, k, mean, rstd, w, b));
         }
     }
 }
@@ -221,7 +296,7 @@ norm_fwd_reg_kernel(bf16* __restrict__ normed, float* __restrict__ mean_out, flo
 // Wider rows: one block per row, every thread owns NV 16-byte vectors (C is any multiple of 8 up to NV * 2048). With a warp
 // per row these have few warps and one row each: 4096 x 1600 took 14.5 us, 4096 x 2048 11.8, 4096 x 4096 24.5, 320 x 2048
 // 4.1; here 9.6, 8.4, 13.7 and 2.3. At 4096 x 1280 the warp is still ahead, 8.5 against 9.0 us (and for 1536: WARP_ROWS_1536).
-template <bool RMS, bool FUSED_RESIDUAL, int NV>
+template <bool RMS, bool FUSED_RESIDUAL, int NV, bool PACKED>
 __global__ void __launch_bounds__(256, NV <= 2 ? 4 : (NV <= 4 ? 2 : 1))
 norm_fwd_wide_kernel(bf16* __restrict__ normed, float* __restrict__ mean_out, float* __restrict__ rstd_out,
                      bf16* residual_out, const bf16* inp1, const bf16* __restrict__ inp2, const bf16* __restrict__ weight,
@@ -274,30 +349,14 @@ norm_fwd_wide_kernel(bf16* __restrict__ normed, float* __restrict__ mean_out, fl
             load(inp1, next, xn);
             if (FUSED_RESIDUAL) load(inp2, next, yn);
         }
-        ptx::f32x2 f[NV][4], acc = both(0.f);
-#pragma unroll
-        for (int k = 0; k < NV; k++) {
-            unpack8p(xv[k], f[k]);
-#pragma unroll
-            for (int j = 0; j < 4; j++) acc = RMS ? ptx::fma2(f[k][j], f[k][j], acc) : ptx::add2(acc, f[k][j]);
-        }
-        const float sum = block_total(sum2(acc), par, 0);
+        RowMath<RMS, NV, PACKED> math;
+        const float sum = block_total(math.sum(xv), par, 0);
         float mean = 0.f, rstd;
         if (RMS) {
             rstd = rsqrtf(sum * inv_c + eps);
         } else {
             mean = sum * inv_c;
-            acc = both(0.f);
-#pragma unroll
-            for (int k = 0; k < NV; k++) {
-                if (!in_row(k)) continue;
-#pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    f[k][j] = ptx::add2(f[k][j], both(-mean));
-                    acc = ptx::fma2(f[k][j], f[k][j], acc);
-                }
-            }
-            const float var = block_total(sum2(acc), par, 1);
+            const float var = block_total(math.squares(xv, mean, in_row), par, 1);
             rstd = rsqrtf(var * inv_c + eps);
         }
         if (threadIdx.x == 0) {
@@ -307,15 +366,7 @@ norm_fwd_wide_kernel(bf16* __restrict__ normed, float* __restrict__ mean_out, fl
 #pragma unroll
         for (int k = 0; k < NV; k++) {
             if (!in_row(k)) continue;
-            ptx::f32x2 w[4], b[4];
-            unpack8p(wv[k], w);
-            if (!RMS) unpack8p(bv[RMS ? 0 : k], b);
-#pragma unroll
-            for (int j = 0; j < 4; j++) {
-                const ptx::f32x2 n = ptx::mul2(f[k][j], both(rstd));
-                f[k][j] = RMS ? ptx::mul2(n, w[j]) : ptx::fma2(n, w[j], b[j]);
-            }
-            st128(normed + (size_t)row * C + (threadIdx.x + 256 * k) * 8, pack8p(f[k]));
+            st128(normed + (size_t)row * C + (threadIdx.x + 256 * k) * 8, math.result(xv, k, mean, rstd, wv[k], RMS ? wv[k] : bv[RMS ? 0 : k]));
         }
     }
 }
@@ -631,7 +682,8 @@ static int num_sms() {
 // 65536 x 512 35.3 / 25.5, 16384 x 1280 23.4 / 19.3, with the residual 65536 x 768 77.8 / 66.9; RMSNorm 16384 x 1024 15.9 / 13.3, 65536 x 1280
 // 67.1 / 56.0. RMSNorm has half of the loads, and up to 768 columns more warps do more for it: 65536 x 768 35.1 / 37.7, 8192 x 768 6.7 /
 // 7.5.
-// With one row per warp and SM or less there is nothing to keep them for: LayerNorm 64 x 768 2.5 / 2.9, 1024 x 768 3.1 / 3.1.
+// With one row per warp and SM or less there is nothing to keep them for: LayerNorm 64 x 768 2.5 / 2.9, 1024 x 768 3.1 / 3.1 (768
+// columns, two blocks per SM with the weights kept: 2048 rows 4.1 / 4.4).
 constexpr bool keeps_weights(bool rms, bool fused, int nvec) { return !rms || (!fused && nvec >= 4); }
 // RMSNorm without: the next row ahead or not, measured with rows from HBM and from the L2 (us, plain / ahead: 256 columns at 65536
 // rows 15.1 / 15.1 and from the L2 11.7 / 10.8, 768 35.4 / 40.4; with a residual 256 27.9 / 24.9, 768 70.5 / 76.0, 1280 138 / 131).
@@ -642,6 +694,11 @@ constexpr bool reads_ahead(bool rms, bool fused, int nvec) {
 // us, block / warp: 1024 rows 4.2 / 4.7, 4096 9.7 / 10.9, 8192 17.1 / 17.2 (from the L2 15.4 / 14.5), 16384 30.4 / 28.7, 65536 108 / 97.
 // (RMSNorm, and both with a residual: the block is ahead at every count.)
 constexpr int WARP_ROWS_1536 = 8192;
+// Rows of more than 2048 columns, a block per row. Packed arithmetic shortens LayerNorm (8192 x 8192 49.9 -> 47.9 us), and with a
+// residual the chain of few rows (256 x 8192 7.05 / 6.25, 1024 x 5120 12.5 / 12.2, 2048 x 5120 19.7 / 19.8), not what many rows wait for (4096
+// x 5120 36.3 / 36.8, 8192 x 8192 92.9 / 95.4). RMSNorm has too little of it: 8192 x 8192 47.8 / 50.9, 64 x 8192 2.67 / 2.91, 8192 x 5120 35.8 /
+// 36.8, with a residual 8192 x 4096 45.9 / 47.1 (without one 24.1 / 23.8).
+constexpr int PACKED_ROWS_FUSED = 2048;
 
 // Few rows: a block per row. A launch is then one latency chain (a row's arrival, two sums, the result), and a warp that holds a
 // whole row has more to do between its steps than eight that share it. The line lies where a block gets a second row while
@@ -674,12 +731,12 @@ static int launch_fwd(bf16* normed, float* mean, float* rstd, bf16* residual, co
     case NV:                                                                                                                \
         if (C == NV * 256) {                                                                                                \
             constexpr bool AHEAD = reads_ahead(RMS, FUSED, NV);                                                             \
-            if (keeps_weights(RMS, FUSED, NV) && N <= REG_WARPS * num_sms())                                                \
+            if (keeps_weights(RMS, FUSED, NV) && N <= REG_WARPS * num_sms() * (NV == 3 && !FUSED ? 2 : 1))                  \
                 LLMK_NORM_FWD_LAUNCH((norm_fwd_reg_kernel<RMS, FUSED, NV, false, false, false>), REG_WARPS, false)          \
             LLMK_NORM_FWD_LAUNCH((norm_fwd_reg_kernel<RMS, FUSED, NV, false, AHEAD, keeps_weights(RMS, FUSED, NV)>), REG_WARPS, AHEAD) \
         }                                                                                                                   \
         LLMK_NORM_FWD_LAUNCH((norm_fwd_reg_kernel<RMS, FUSED, NV, true, true, keeps_weights(RMS, FUSED, NV)>), REG_WARPS, true)
-    if (N <= block_rows_per_sm(C) * num_sms()) LLMK_NORM_FWD_LAUNCH((norm_fwd_wide_kernel<RMS, FUSED, 1>), 1, true)
+    if (N <= block_rows_per_sm(C) * num_sms()) LLMK_NORM_FWD_LAUNCH((norm_fwd_wide_kernel<RMS, FUSED, 1, true>), 1, true)
     switch (ceil_div(C, 256)) {
         LLMK_NORM_FWD_CASE(1)
         LLMK_NORM_FWD_CASE(2)
@@ -691,13 +748,23 @@ static int launch_fwd(bf16* normed, float* mean, float* rstd, bf16* residual, co
     if constexpr (!RMS && !FUSED) {
         if (C == 1536 && N >= WARP_ROWS_1536) LLMK_NORM_FWD_LAUNCH((norm_fwd_reg_kernel<RMS, FUSED, 6, false, false, false>), REG_WARPS, false)
     }
-    switch (ceil_div(C, 2048)) {
-        case 1: LLMK_NORM_FWD_LAUNCH((norm_fwd_wide_kernel<RMS, FUSED, 1>), 1, true)
-        case 2: LLMK_NORM_FWD_LAUNCH((norm_fwd_wide_kernel<RMS, FUSED, 2>), 1, true)
-        case 3:
-        case 4: LLMK_NORM_FWD_LAUNCH((norm_fwd_wide_kernel<RMS, FUSED, 4>), 1, true)
-        default: LLMK_NORM_FWD_LAUNCH((norm_fwd_wide_kernel<RMS, FUSED, 8>), 1, true)
+    const int nv = ceil_div(C, 2048);
+    if (nv <= 1) LLMK_NORM_FWD_LAUNCH((norm_fwd_wide_kernel<RMS, FUSED, 1, true>), 1, true)
+    if (RMS ? !FUSED && nv == 2 : !FUSED || N <= PACKED_ROWS_FUSED) {
+        if constexpr (!RMS || !FUSED) {
+            if (nv == 2) LLMK_NORM_FWD_LAUNCH((norm_fwd_wide_kernel<RMS, FUSED, 2, true>), 1, true)
+        }
+        if constexpr (!RMS) {
+            if (nv <= 4) LLMK_NORM_FWD_LAUNCH((norm_fwd_wide_kernel<RMS, FUSED, 4, true>), 1, true)
+            LLMK_NORM_FWD_LAUNCH((norm_fwd_wide_kernel<RMS, FUSED, 8, true>), 1, true)
+        }
     }
+    if constexpr (RMS || FUSED) {
+        if (nv == 2) LLMK_NORM_FWD_LAUNCH((norm_fwd_wide_kernel<RMS, FUSED, 2, false>), 1, true)
+        if (nv <= 4) LLMK_NORM_FWD_LAUNCH((norm_fwd_wide_kernel<RMS, FUSED, 4, false>), 1, true)
+        LLMK_NORM_FWD_LAUNCH((norm_fwd_wide_kernel<RMS, FUSED, 8, false>), 1, true)
+    }
+    return LLMK_ERR_SHAPE;   // (not reached)
 #undef LLMK_NORM_FWD_CASE
 #undef LLMK_NORM_FWD_LAUNCH
 }

@@ -172,6 +172,23 @@ def test_norm_forward_of_wide_rows(N, C):
     assert torch.equal(a2, r) and ((out.double() - want).abs() <= ulp * want.abs() + 1e-4).all()
 
 
+@pytest.mark.parametrize("N,C", [(2048, 4104), (2049, 4104), (2049, 2056), (9, 8200), (2049, 8200), (700, 512), (4000, 392), (700, 1024), (1184, 1280),
+                                 (1185, 1280), (2368, 768), (2369, 768)])
+def test_norm_forward_where_the_arithmetic_changes(N, C):
+    """Row counts and widths on both sides of packed arithmetic, of kept weights and of the register limits, with 148 SMs."""
+    from llm_kittens_b200.ops import norm
+
+    test_norm_forward_of_wide_rows(N, C)
+    x, w, b = rnd(N, C), rnd(C, scale=0.5) + 1, rnd(C, scale=0.1)
+    xd = x.double()
+    out, mean, rstd = norm.layernorm_fwd(x, w, b)
+    assert rounded(out, torch.nn.functional.layer_norm(xd, (C,), w.double(), b.double(), 1e-5), 1e-4)
+    assert (mean - xd.mean(-1)).abs().max() < 1e-5 and (rstd * (xd.var(-1, unbiased=False) + 1e-5).sqrt() - 1).abs().max() < 1e-4
+    out, rstd = norm.rmsnorm_fwd(x, w, 1e-5)
+    rs = torch.rsqrt(xd.pow(2).mean(-1, keepdim=True) + 1e-5)
+    assert rounded(out, xd * rs * w.double(), 1e-4) and (rstd / rs.view(-1) - 1).abs().max() < 1e-4
+
+
 @pytest.mark.parametrize("rms", [False, True])
 @pytest.mark.parametrize("N,C", [(1, 264), (444, 768), (445, 768), (592, 1280), (593, 1024), (591, 1024), (296, 504), (297, 512), (2, 2048),
                                  (295, 1600), (297, 1600), (1187, 1600), (5, 2048)])
