@@ -118,12 +118,16 @@ fused_classifier_kernel(bf16* __restrict__ logits, float* __restrict__ losses, c
 // 946 / 629, 64 x 128256 31 / 21, now 14 / 10. What counted, 16384 x 50304: the maximum per warp 428 -> 389 without the gradient; with it, a
 // barrier after the maximum all the same, because the next load is then asked for before the exponentials (628 -> 607); loads
 // that the L2 lets go of first 607 -> 589. Stores that are not marked as streaming take 1030. Llama 3's row over 5 blocks of 512 threads
-// or 3 of 1024: 940 / 945, without the gradient 618 / 661; 65536 columns over 3 blocks 250 / 329.
+// or 3 of 1024: 940 / 945, without the gradient 618 / 661; 65536 columns over 3 blocks 250 / 329, 151936 over 6 or 8 at 3136 rows 450 / 506,
+// without the gradient 302 / 344 (three passes 329). A row takes the smallest block that holds it, so that the chip works on as many
+// rows as it can: of a block of 1024 threads, 8192 x 1000 columns leave 900 without work at every barrier, 120.8 us with the gradient (89.7
+// before rows were kept in registers), eight blocks of 128 19.7; 8192 x 8000 133 (120), four of 256 51; 8192 x 20000 173 (180), two of 512 113.
 constexpr int NVT = 7;              // 16-byte vectors per thread
 constexpr int BULK_CHUNK = 65536;   // bytes per copy: in pieces of 4 KB 16384 rows of 50304 took 485 us to read, of 16 KB 437, 64 KB 428
-// vectors of a row per block: two slots of shared memory for each of the SM's 1024 / TPB blocks
-constexpr int largest_part(int tpb) { return 220 * 1024 / (1024 / tpb) / 2 / 16; }
-static_assert(largest_part(1024) <= NVT * 1024 && largest_part(512) <= NVT * 512, "in registers");
+// vectors of a row per block: two slots of shared memory for each of the SM's 1024 / TPB blocks (each of which takes 1 KB besides)
+constexpr int largest_part(int tpb) { return (tpb > 128 ? 220 : 218) * 1024 / (1024 / tpb) / 2 / 16; }
+static_assert(largest_part(1024) <= NVT * 1024 && largest_part(512) <= NVT * 512 && largest_part(256) <= NVT * 256 && largest_part(128) <= NVT * 128,
+              "in registers");
 
 __device__ __forceinline__ float ex2(float x) {
     float y;
@@ -382,9 +386,13 @@ LLMK_API int llmk_fused_classifier(void* logits, void* losses, const void* targe
     if (Vp / 8 <= CL * largest_part(TPB_))                                                                           \
         return write_dlogits ? launch_smem<true, CL, TPB_>(lg, ls, tg, dloss, rows, V, Vp, accumulate_loss, stream)  \
                              : launch_smem<false, CL, TPB_>(lg, ls, tg, dloss, rows, V, Vp, accumulate_loss, stream);
+    LLMK_CLASSIFIER(1, 128)
+    LLMK_CLASSIFIER(1, 256)
+    LLMK_CLASSIFIER(1, 512)
     LLMK_CLASSIFIER(1, 1024)
     LLMK_CLASSIFIER(3, 512)
     LLMK_CLASSIFIER(5, 512)
+    LLMK_CLASSIFIER(6, 512)
     LLMK_CLASSIFIER(8, 512)
 #undef LLMK_CLASSIFIER
     if (write_dlogits) fused_classifier_kernel<true><<<rows, TPB, 0, stream>>>(lg, ls, tg, dloss, V, Vp, accumulate_loss);

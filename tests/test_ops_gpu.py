@@ -523,6 +523,13 @@ def test_fused_classifier_over_blocks_and_clusters(rows, V, Vp):
     assert (lg[:, V:] == 0).all()
 
 
+@pytest.mark.parametrize("rows,V,Vp", [(1300, 6975, 6976), (700, 6977, 6984), (650, 14079, 14080), (300, 14081, 14088), (300, 28159, 28160),
+                                       (150, 28161, 28168), (30, 168957, 168960), (3, 168961, 168968)])
+def test_fused_classifier_at_the_edges_of_the_block_sizes(rows, V, Vp):
+    """The widest row of a block size and the narrowest of the next, several rows per block where they are narrow."""
+    test_fused_classifier_over_blocks_and_clusters(rows, V, Vp)
+
+
 def _ref_attention(qkv, B, T, NH, NKVH, HS):
     x = qkv.float().view(B, T, NH + 2 * NKVH, HS)
     q = x[:, :, :NH].transpose(1, 2)
