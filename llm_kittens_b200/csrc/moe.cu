@@ -696,6 +696,30 @@ combine_dweight_kernel(float* __restrict__ dw, const bf16* __restrict__ dout, co
     }
 }
 
+// The same with one warp per (token, expert): the shorter chain for few tokens, which leave warps idle either way. Rule: see
+// llmk_moe_combine_dweight.
+__global__ void __launch_bounds__(256)
+combine_dweight_pairs_kernel(float* __restrict__ dw, const bf16* __restrict__ dout, const bf16* __restrict__ back,
+                             const int* __restrict__ top_idx, const int* __restrict__ slot, int N, int K, int C, int cap) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const size_t a = (size_t)blockIdx.x * (blockDim.x >> 5) + warp;
+    if (a >= (size_t)N * K) return;
+    const int s = slot[a];
+    float acc = 0.f;
+    if (s >= 0) {
+        const bf16 *d = dout + a / K * C, *row = back + ((size_t)top_idx[a] * cap + s) * C;
+        for (int v = lane; v < C / 8; v += 32) {
+            float df[8], f[8];
+            unpack8(ld128(d + v * 8), df);
+            unpack8(ld128(row + v * 8), f);
+#pragma unroll
+            for (int j = 0; j < 8; j++) acc += df[j] * f[j];
+        }
+    }
+    acc = warp_sum(acc);
+    if (lane == 0) dw[a] = acc;
+}
+
 // ------------------------------------------------------------------ load-balance statistics + router backward
 // density[e] = mean_t probs[t,e]  (one block, fixed order). The table is read once, in order: a thread's elements all
 // belong to one expert because the number of threads at work is a multiple of E. (A pass per expert with a stride of E took
@@ -963,9 +987,15 @@ LLMK_API int llmk_moe_publish(const long long* arrive_ptrs, int arrive_off, int 
 LLMK_API int llmk_moe_combine_dweight(void* dw, const void* dout, const void* back, const void* top_idx, const void* slot, int N,
                                       int K, int C, int cap, void* stream) {
     if (N <= 0 || K <= 0) return LLMK_ERR_SHAPE;
-    auto kernel = K == 1 ? combine_dweight_kernel<1, 4> : K == 2 ? combine_dweight_kernel<2, 2> : combine_dweight_kernel<MAXK, 1>;
-    kernel<<<ceil_div(N, 8), 256, 0, (cudaStream_t)stream>>>((float*)dw, (const bf16*)dout, (const bf16*)back, (const int*)top_idx,
-                                                             (const int*)slot, N, K, C, cap);
+    // A warp per (token, expert) while that fills the chip no more than once or twice, and for one expert and many tokens where a row is no whole
+    // number of four vectors per lane. us, per pair / per token: two experts, 64 x 4096 4.9 / 6.8, 512 x 1280 4.3 / 4.7, 1024 x 768 3.8 /
+    // 3.9, but 2048 x 1024 5.3 / 5.0; three, 1024 x 1600 6.1 / 8.1, 2048 8.75 / 9.2, 4096 14.6 / 12.1; four, 512 x 1280 4.6 / 6.6, 2048 7.9 / 8.0,
+    // 4096 14.0 / 11.6; one, 65536 x 768 33.5 / 37.2, but 16384 x 768 11.05 / 10.8, 512 x 4096 7.8 / 6.2.
+    const bool pairs = K == 1 ? N > 32768 && C % 1024 != 0 : N <= (K == 2 ? 1024 : 2048);
+    auto kernel = pairs ? combine_dweight_pairs_kernel
+                        : K == 1 ? combine_dweight_kernel<1, 4> : K == 2 ? combine_dweight_kernel<2, 2> : combine_dweight_kernel<MAXK, 1>;
+    kernel<<<ceil_div(pairs ? (long)N * K : N, 8), 256, 0, (cudaStream_t)stream>>>((float*)dw, (const bf16*)dout, (const bf16*)back,
+                                                                                  (const int*)top_idx, (const int*)slot, N, K, C, cap);
     LLMK_LAUNCH_CHECK();
     return LLMK_OK;
 }

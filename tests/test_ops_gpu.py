@@ -348,6 +348,12 @@ def test_moe_rows_moved_and_summed(N, C, E, K):
     assert ((dw.double() - terms.sum(-1)).abs() <= (C / 32 + 6) * 2.0 ** -24 * terms.abs().sum(-1)).all()
 
 
+@pytest.mark.parametrize("N,C,E,K", [(1024, 264, 4, 2), (1025, 264, 4, 2), (2048, 136, 6, 3), (2049, 136, 6, 3), (32768, 264, 3, 1), (32769, 264, 3, 1)])
+def test_moe_rows_where_the_weight_gradient_changes_kernel(N, C, E, K):
+    """Token counts on both sides of a warp per token and expert."""
+    test_moe_rows_moved_and_summed(N, C, E, K)
+
+
 def test_gelu_swiglu_add():
     from llm_kittens_b200.ops import elementwise as ew
 
