@@ -322,22 +322,24 @@ constexpr int ZERO_BLOCKS = 32;   // per expert
 // One warp per token at a time: row x[token], read once, to the receive buffers of the owners of its K experts at its slots.
 // A lane's four vectors are all loaded before the first is stored (a load may not pass a store that could alias it).
 // SCALE: 0 copies the row (forward), 1 multiplies by the routing weight (backward: dY = w * dout).
-// The blocks from token_blocks on, if any, zero the unused slots. Bound by the writes: 16384 rows of 1024 to two experts of 8 with a
+// ZERO_BLOCKS blocks per expert, if any, zero the unused slots: the last ones of a small call, where they would keep tokens waiting, and the
+// first ones of a large call, where so few of them would be left writing at the end (zeros_first; 65536 x 2048 to one expert of 2 125 us last,
+// 94 first, 118 as a launch of their own; 512 x 4096 to two of 8 7.4 last, 10.6 first). Bound by the writes: 16384 rows of 1024 to two experts of 8 with a
 // quarter of unused slots 33.8 us with a warp per copy and a launch for the zeros, now 22.7 (117 MB: 18 at the rate of a
 // copy); 16384 x 1280 to four 71.5 / 44.5, 64 x 1024 4.7 / 2.4.
 template <bool SCALE>
 __global__ void __launch_bounds__(256, 4)
 dispatch_kernel(const __grid_constant__ Peers recv, const bf16* __restrict__ x, const int* __restrict__ top_idx, const int* __restrict__ slot,
                 const float* __restrict__ top_w, const int* __restrict__ counts, int N, int K, int C, int cap, int Eloc, int my_rank,
-                int P, int token_blocks) {
-    if ((int)blockIdx.x >= token_blocks) {
-        const int b = blockIdx.x - token_blocks;
+                int P, int token_blocks, int zeros_first) {
+    const int zero_blocks = gridDim.x - token_blocks, b = (int)blockIdx.x - (zeros_first ? 0 : token_blocks);
+    if (b >= 0 && b < zero_blocks) {
         zero_slots(recv, counts, b / ZERO_BLOCKS, b % ZERO_BLOCKS, ZERO_BLOCKS, C, cap, Eloc, my_rank, P);
         return;
     }
     constexpr int U = 4;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nv = C / 8;
-    const size_t t = (size_t)blockIdx.x * (blockDim.x >> 5) + warp;
+    const size_t t = (size_t)(blockIdx.x - (zeros_first ? zero_blocks : 0)) * (blockDim.x >> 5) + warp;
     if (t >= (size_t)N) return;
     const bf16* src = x + t * C;
     for (int k0 = 0; k0 < K; k0 += MAXK) {
@@ -838,9 +840,11 @@ static int launch_dispatch(const Peers& recv, const void* x, const void* top_idx
     if (N <= 0 || K <= 0) return LLMK_ERR_SHAPE;
     const int token_blocks = ceil_div(N, 8);
     const int grid = token_blocks + (zero ? ZERO_BLOCKS * E : 0);
+    // us, last / first: 16384 x 2048 to one of 2 32.9 / 26.7, x 1024 to two of 8 22.8 / 21.9, of 16 22.0 / 22.5; 8192 x 1024 of 8 12.4 / 12.9
+    const bool zeros_first = N >= 16384 && E <= 8;
     auto kernel = scale_by_weight ? dispatch_kernel<true> : dispatch_kernel<false>;
     kernel<<<grid, 256, 0, st>>>(recv, (const bf16*)x, (const int*)top_idx, (const int*)slot, (const float*)top_w, (const int*)counts,
-                                 N, K, C, cap, E / P, my_rank, P, token_blocks);
+                                 N, K, C, cap, E / P, my_rank, P, token_blocks, zeros_first ? 1 : 0);
     LLMK_LAUNCH_CHECK();
     return LLMK_OK;
 }

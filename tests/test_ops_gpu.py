@@ -354,6 +354,11 @@ def test_moe_rows_where_the_weight_gradient_changes_kernel(N, C, E, K):
     test_moe_rows_moved_and_summed(N, C, E, K)
 
 
+@pytest.mark.parametrize("N,C,E,K", [(16383, 136, 3, 2), (16384, 136, 3, 2), (16385, 136, 2, 1)])
+def test_moe_rows_where_the_unused_slots_are_zeroed_first(N, C, E, K):
+    test_moe_rows_moved_and_summed(N, C, E, K)
+
+
 def test_gelu_swiglu_add():
     from llm_kittens_b200.ops import elementwise as ew
 
