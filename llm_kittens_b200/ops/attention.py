@@ -36,18 +36,15 @@ def _tc_forward(B: int, T: int, NH: int, HS: int) -> bool:
     for a few sequences of 128 or 256 with heads of 64, where a launch lasts as long as its longest tile and the warp-level
     kernel's 64-row tiles are shorter (B1 T128 12 heads 4.4 / 5.9, B2 T128 25 heads 4.6 / 6.0, B1 T256 12 heads 6.5 / 7.1, but B2 T256 25
     heads 6.9 / 7.2, B16 T128 32 heads 14.4 / 12.5).
-    With a ragged last tile few sequences stay on the warp-level kernel: with heads of 64 while its launch is one or two
-    waves of 64-row tiles, with heads of 128 and under 512 keys from one wave of 128-row tiles on. The lines were drawn when
-    both kernels were equal there; the tcgen05 kernel is ahead of them now (us, warp level / tcgen05: B1 T320 12 heads 7.6 / 8.3,
-    but B2 T320 25 heads 9.8 / 9.3, B7 T448 6 heads 12.2 / 11.1, B2 T576 6 heads 11.9 / 10.9; heads of 128: B2 T320 32 heads 17.5 / 12.9,
-    B7 T448 16 heads 40 / 23), and they are kept because tests state them."""
+    With a ragged last tile they are too, except for heads of 64 and the shortest such length, 320, while the warp-level launch
+    is one wave of 64-row tiles (us, warp level / tcgen05, heads in all: 12 7.7 / 8.4, 24 7.8 / 8.8, but 36 9.6 / 9.0, 50 9.9 / 9.4, 400 38 /
+    30; 448 4 heads 9.2 / 9.2, 12 9.8 / 9.7, 36 12.6 / 10.4; 576 12 heads 11.9 / 10.9; 1088 4 heads 20.5 / 15.7; heads of 128: 320 4 heads 11.2 /
+    8.7, 64 17.5 / 12.9, 448 112 heads 40 / 23, 600 167 / 100)."""
     if not _tc_length(T):
         return False
     if T % 128 == 0:
         return HS != 64 or T > 256 or T // 128 * B * NH > _sms() // 2
-    if HS == 64:
-        return (T // 64) * B * NH > (2 if T <= 448 else 1) * _sms()
-    return T >= 512 or (T + 127) // 128 * B * NH <= _sms()
+    return HS != 64 or T > 320 or T // 64 * B * NH > _sms()
 
 
 def forward_is_tc(B: int, T: int, NH: int, HS: int) -> bool:
