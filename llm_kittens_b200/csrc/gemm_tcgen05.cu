@@ -1216,6 +1216,13 @@ static double pair_estimate(int M, int N, int K, int pair_clusters) {
     return waves * ceil_div(K, BK) * (0.28 + 0.12 * units / ((double)waves * pair_clusters)) + 9.3;
 }
 
+// Whether a product (mode NT, plain or SwiGLU, N columns of the accumulator space) is faster on the kernel of few rows.
+static bool takes_few_rows(int M, int N, int K, bool swi, int pair_clusters, double small_us) {
+    if (M > few::MAX_TOKENS) return false;
+    const double us = few::estimate(M, swi ? N / 2 : N, K, swi, pair_clusters);
+    return us < small_us && us < 0.95 * pair_estimate(M, N, K, pair_clusters);
+}
+
 static int run_small(const SmallPlan& plan, int mode, int epi, const void* A, const void* B, void* C, void* C2, const Params& q,
                      const Ready& ready, cudaStream_t stream) {
     small::SParams p = {};
@@ -1364,12 +1371,9 @@ static int gemm_impl(int mode, int epi, const void* A, const void* B, void* C, v
         double small_us;
         const SmallPlan plan = pick_small(mode, M, N, K, g_num_sms, pair_clusters, &small_us);
         const bool swi = (epi & EPI_SWIGLU) != 0;
-        if (mode == MODE_NT && (epi == 0 || epi == EPI_SWIGLU) && M <= few::MAX_TOKENS) {
-            const double us = few::estimate(M, swi ? N / 2 : N, K, swi, pair_clusters);
-            if (us < small_us && us < 0.95 * pair_estimate(M, N, K, pair_clusters))
-                return swi ? few::launch<EPI_SWIGLU>(A, B, ready.b2, C, C2, ready.c3, M, N / 2, K, status, pair_clusters, stream)
-                           : few::launch<0>(A, B, nullptr, C, nullptr, nullptr, M, N, K, status, pair_clusters, stream);
-        }
+        if (mode == MODE_NT && (epi == 0 || epi == EPI_SWIGLU) && takes_few_rows(M, N, K, swi, pair_clusters, small_us))
+            return swi ? few::launch<EPI_SWIGLU>(A, B, ready.b2, C, C2, ready.c3, M, N / 2, K, status, pair_clusters, stream)
+                       : few::launch<0>(A, B, nullptr, C, nullptr, nullptr, M, N, K, status, pair_clusters, stream);
         if (plan.bn) return run_small(plan, mode, epi, A, B, C, C2, p, ready, stream);
     }
     bool split_accumulate = false;
@@ -1580,6 +1584,27 @@ LLMK_API int llmk_gemm_swiglu(const void* A, const void* Wup, const void* Wgate,
     r.b2 = Wgate;
     r.c3 = gate;
     return gemm_impl(MODE_NT, EPI_SWIGLU, A, Wup, act, up, nullptr, nullptr, M, 2 * H, K, 1, nullptr, 0, status, max_ctas, stream_, r);
+}
+
+// The kernel of few rows whatever the rule says, for shapes on either side of its lines: C[M, N] = A B^T, or with B2 (SwiGLU) C =
+// silu(A B2^T) * (A B^T), C2 = A B^T, C3 = A B2^T. And the rule: 1 where llmk_gemm / llmk_gemm_swiglu take it for `N` columns each.
+LLMK_API int llmk_gemm_few_rows(const void* A, const void* B, const void* B2, void* C, void* C2, void* C3, int M, int N, int K, int* status,
+                                void* stream) {
+    if (M <= 0 || M > few::MAX_TOKENS || N <= 0 || K <= 0 || N % 8 || K % 8) return LLMK_ERR_SHAPE;
+    for (const void* p : {A, B, B2, (const void*)C, (const void*)C2, (const void*)C3})
+        if (reinterpret_cast<uintptr_t>(p) & 15) return LLMK_ERR_SHAPE;
+    if (B2 != nullptr && (C2 == nullptr || C3 == nullptr)) return LLMK_ERR_SHAPE;
+    const int pair_clusters = query_pair_clusters();
+    if (pair_clusters <= 0) return LLMK_ERR_SHAPE;
+    return B2 != nullptr ? few::launch<EPI_SWIGLU>(A, B, B2, C, C2, C3, M, N, K, status, pair_clusters, (cudaStream_t)stream)
+                         : few::launch<0>(A, B, nullptr, C, nullptr, nullptr, M, N, K, status, pair_clusters, (cudaStream_t)stream);
+}
+LLMK_API int llmk_gemm_takes_few_rows(int M, int N, int K, int swiglu) {
+    const int pair_clusters = query_pair_clusters(), sms = sm_count_current_device(), width = swiglu ? 2 * N : N;
+    if (pair_clusters <= 0 || sms <= 0) return 0;
+    double small_us;
+    pick_small(MODE_NT, M, width, K, sms, pair_clusters, &small_us);
+    return takes_few_rows(M, width, K, swiglu != 0, pair_clusters, small_us) ? 1 : 0;
 }
 
 // QKV projection with RoPE in the epilogue: C = A B^T where C is a packed [tokens, (NH + 2 NKVH) * HS] tensor; the

@@ -458,6 +458,61 @@ def test_swiglu_of_few_rows_and_a_wide_output(M, H, K):
     _native.check_status()
 
 
+def _guarded(M, N):
+    whole = torch.full((M * N + 4096,), 7.0, device="cuda", dtype=torch.bfloat16)
+    return whole, whole[:M * N].view(M, N)
+
+
+@pytest.mark.parametrize("M", [1, 33, 64, 200, 257, 320, 400, 512])
+@pytest.mark.parametrize("N,K", [(264, 72), (8, 1032), (20008, 136), (40200, 520)])
+@pytest.mark.parametrize("swiglu", [False, True])
+def test_the_kernel_of_few_rows_itself(M, N, K, swiglu):
+    """Asked for by name, whatever the rule picks: one and two MMAs per weight tile and one and two stretches of tokens, counts that are no
+    multiple of 32, a last weight tile that is cut (or nearly empty), K not whole k-blocks, several units per pair of blocks; guards
+    behind every output."""
+    from llm_kittens_b200.ops import _native
+
+    if swiglu and N > 30000:
+        N = 20104                                              # (several units per pair of blocks too, at half the width)
+    a, wu, wg = _rand(M, K), _rand(N, K, scale=0.05), _rand(N, K, scale=0.05)
+    (cw, c), (uw, up), (gw, gate) = (_guarded(M, N) for _ in range(3))
+    args = (wg, c, up, gate) if swiglu else (None, c, None, None)
+    _native.call("llmk_gemm_few_rows", a, wu, *args, M, N, K, _native.status_word())
+    _native.check_status()
+    # fp32 sums of K products of order 0.05, one rounding to bf16
+    within = lambda got, want: ((got.double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-5 * K ** 0.5).all()
+    u = a.double() @ wu.double().T
+    if swiglu:
+        assert within(up, u) and within(gate, a.double() @ wg.double().T)
+        assert within(c, torch.nn.functional.silu(gate.double()) * up.double())
+    else:
+        assert within(c, u)
+    first = c.clone()
+    _native.call("llmk_gemm_few_rows", a, wu, *args, M, N, K, _native.status_word())
+    assert torch.equal(c, first)
+    for whole in (cw, uw, gw):
+        assert (whole[M * N:] == 7.0).all()
+
+
+@pytest.mark.parametrize("M,N,K,swiglu", [(320, 128256, 2048, 0), (448, 128256, 2048, 0), (320, 50304, 1600, 0), (64, 14336, 4096, 1), (320, 8192, 2048, 1),
+                                          (257, 8192, 2048, 1), (320, 14336, 4096, 1)])
+def test_products_that_take_the_kernel_of_few_rows(M, N, K, swiglu):
+    """What the rule picks gives that kernel's bits; one row more than it can hold does not take it."""
+    from llm_kittens_b200.ops import gemm, _native
+
+    assert _native.lib().llmk_gemm_takes_few_rows(M, N, K, swiglu) == 1 and _native.lib().llmk_gemm_takes_few_rows(513, N, K, swiglu) == 0
+    a, wu, wg = _rand(M, K), _rand(N, K, scale=0.05), _rand(N, K, scale=0.05)
+    got, want = ([torch.empty(M, N, device="cuda", dtype=torch.bfloat16) for _ in range(3)] for _ in range(2))
+    if swiglu:
+        assert gemm.gemm_swiglu(a, wu, wg, *got)
+        _native.call("llmk_gemm_few_rows", a, wu, wg, *want, M, N, K, _native.status_word())
+    else:
+        gemm.gemm_nt(a, wu, out=got[0])
+        _native.call("llmk_gemm_few_rows", a, wu, None, want[0], None, None, M, N, K, _native.status_word())
+    assert all(torch.equal(x, y) for x, y in list(zip(got, want))[: 3 if swiglu else 1])
+    _native.check_status()
+
+
 @pytest.mark.parametrize("M,N,K", [(200, 8192, 8192), (72, 2056, 32768), (768, 768, 16384), (264, 4104, 12288)])
 @pytest.mark.parametrize("accumulate", [False, True])
 def test_weight_and_bias_gradient_from_split_partials(M, N, K, accumulate):
