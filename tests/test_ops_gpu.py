@@ -554,12 +554,15 @@ def _ref_attention(qkv, B, T, NH, NKVH, HS):
     return o, torch.logsumexp(s, -1)
 
 
-@pytest.mark.parametrize("B,T,NH,HS", [(200, 128, 12, 64), (40, 256, 20, 64), (64, 192, 12, 64), (60, 128, 8, 128), (37, 320, 12, 64)])
-def test_attention_forward_of_many_short_tiles(B, T, NH, HS):
+@pytest.mark.parametrize("B,T,NH,HS", [(200, 128, 12, 64), (40, 256, 20, 64), (25, 448, 12, 64), (60, 128, 8, 128), (37, 320, 12, 64), (8, 320, 16, 128)])
+def test_attention_forward_of_many_short_tiles(B, T, NH, HS, monkeypatch):
     """Several query tiles per resident block, most of them with one or two key tiles: every tile's rows are written, to their
     own place, each of many times (a block takes its next tile while the last one's rows leave)."""
-    from llm_kittens_b200.ops import attention
+    from llm_kittens_b200.ops import _native, attention
 
+    assert -(-T // 128) * B * NH > 2 * torch.cuda.get_device_properties(0).multi_processor_count
+    entries, call = [], _native.call
+    monkeypatch.setattr(_native, "call", lambda name, *a: (entries.append(name), call(name, *a))[1])
     qkv = rnd(B, T, 3 * NH * HS)
     q, k, v = (t.view(B, T, NH, HS).transpose(1, 2).float() for t in qkv.split(NH * HS, dim=-1))
     ref = torch.nn.functional.scaled_dot_product_attention(q, k, v, is_causal=True).transpose(1, 2).reshape(B, T, NH * HS)
@@ -572,6 +575,7 @@ def test_attention_forward_of_many_short_tiles(B, T, NH, HS):
             first = out, lse
             assert (out.float() - ref).abs().max() < 0.03
         assert torch.equal(out, first[0]) and torch.equal(lse, first[1])
+    assert entries == ["llmk_attention_fwd_tc"] * 60
 
 
 @pytest.mark.parametrize("B,T,NH,NKVH,HS", [(2, 128, 4, 4, 64), (1, 256, 12, 12, 64), (2, 192, 8, 2, 64), (1, 128, 4, 2, 128),
