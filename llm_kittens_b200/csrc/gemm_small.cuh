@@ -293,14 +293,15 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
             const float* src = slice(0) + off;
             float4 a = *reinterpret_cast<const float4*>(src), b = *reinterpret_cast<const float4*>(src + 4);
             x[0] = a.x; x[1] = a.y; x[2] = a.z; x[3] = a.w; x[4] = b.x; x[5] = b.y; x[6] = b.z; x[7] = b.w;
-            if (!CL) return;
+            if constexpr (CL) {
 #pragma unroll 1
-            for (int s = 1; s < S; s++) {
-                src = slice(s) + off;
-                a = *reinterpret_cast<const float4*>(src);
-                b = *reinterpret_cast<const float4*>(src + 4);
-                x[0] += a.x; x[1] += a.y; x[2] += a.z; x[3] += a.w;
-                x[4] += b.x; x[5] += b.y; x[6] += b.z; x[7] += b.w;
+                for (int s = 1; s < S; s++) {
+                    src = slice(s) + off;
+                    a = *reinterpret_cast<const float4*>(src);
+                    b = *reinterpret_cast<const float4*>(src + 4);
+                    x[0] += a.x; x[1] += a.y; x[2] += a.z; x[3] += a.w;
+                    x[4] += b.x; x[5] += b.y; x[6] += b.z; x[7] += b.w;
+                }
             }
         };
 #pragma unroll
