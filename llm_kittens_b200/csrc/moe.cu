@@ -840,8 +840,9 @@ static int launch_dispatch(const Peers& recv, const void* x, const void* top_idx
     if (N <= 0 || K <= 0) return LLMK_ERR_SHAPE;
     const int token_blocks = ceil_div(N, 8);
     const int grid = token_blocks + (zero ? ZERO_BLOCKS * E : 0);
-    // us, last / first: 16384 x 2048 to one of 2 32.9 / 26.7, x 1024 to two of 8 22.8 / 21.9, of 16 22.0 / 22.5; 8192 x 1024 of 8 12.4 / 12.9
-    const bool zeros_first = N >= 16384 && E <= 8;
+    // us, last / first: 65536 x 1024 to two of 8 85 / 78, x 768 to one of 4 49 / 43; 16384 x 1024 to two of 8 22.8 / 21.9, of 16 22.0 / 22.5, but
+    // a whole expert layer of it 2.08 / 2.09 ms; 8192 x 1024 12.4 / 12.9
+    const bool zeros_first = N >= 32768;
     auto kernel = scale_by_weight ? dispatch_kernel<true> : dispatch_kernel<false>;
     kernel<<<grid, 256, 0, st>>>(recv, (const bf16*)x, (const int*)top_idx, (const int*)slot, (const float*)top_w, (const int*)counts,
                                  N, K, C, cap, E / P, my_rank, P, token_blocks, zeros_first ? 1 : 0);

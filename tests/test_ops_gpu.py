@@ -354,7 +354,7 @@ def test_moe_rows_where_the_weight_gradient_changes_kernel(N, C, E, K):
     test_moe_rows_moved_and_summed(N, C, E, K)
 
 
-@pytest.mark.parametrize("N,C,E,K", [(16383, 136, 3, 2), (16384, 136, 3, 2), (16385, 136, 2, 1)])
+@pytest.mark.parametrize("N,C,E,K", [(32767, 136, 3, 2), (32768, 136, 3, 2), (32769, 136, 2, 1)])
 def test_moe_rows_where_the_unused_slots_are_zeroed_first(N, C, E, K):
     test_moe_rows_moved_and_summed(N, C, E, K)
 
