@@ -37,14 +37,14 @@ def _tc_forward(B: int, T: int, NH: int, HS: int) -> bool:
     kernel's 64-row tiles are shorter (B1 T128 12 heads 4.4 / 5.9, B2 T128 25 heads 4.6 / 6.0, B1 T256 12 heads 6.5 / 7.1, but B2 T256 25
     heads 6.9 / 7.2, B16 T128 32 heads 14.4 / 12.5).
     With a ragged last tile they are too, except for heads of 64 and the shortest such length, 320, while the warp-level launch
-    is one wave of 64-row tiles (us, warp level / tcgen05, heads in all: 12 7.7 / 8.4, 24 7.8 / 8.8, but 36 9.6 / 9.0, 50 9.9 / 9.4, 400 38 /
-    30; 448 4 heads 9.2 / 9.2, 12 9.8 / 9.7, 36 12.6 / 10.4; 576 12 heads 11.9 / 10.9; 1088 4 heads 20.5 / 15.7; heads of 128: 320 4 heads 11.2 /
-    8.7, 64 17.5 / 12.9, 448 112 heads 40 / 23, 600 167 / 100)."""
+    is 1.2 waves of 64-row tiles (us, warp level / tcgen05, heads in all: 12 7.7 / 8.4, 24 7.5 / 8.6, 30 8.4 / 9.0, 34 8.9 / 9.0, but 36 9.6 /
+    9.1, 48 9.8 / 9.3, 400 38 / 30; 448 4 heads 9.2 / 9.2, 12 9.8 / 9.7, 36 12.6 / 10.4; 576 12 heads 11.9 / 10.9; 1088 4 heads 20.5 / 15.7; heads of
+    128: 320 4 heads 11.2 / 8.7, 64 17.5 / 12.9, 448 112 heads 40 / 23, 600 167 / 100)."""
     if not _tc_length(T):
         return False
     if T % 128 == 0:
         return HS != 64 or T > 256 or T // 128 * B * NH > _sms() // 2
-    return HS != 64 or T > 320 or T // 64 * B * NH > _sms()
+    return HS != 64 or T > 320 or 5 * (T // 64) * B * NH > 6 * _sms()
 
 
 def forward_is_tc(B: int, T: int, NH: int, HS: int) -> bool:

@@ -112,7 +112,7 @@ def test_zeroing_a_tensor_of_another_device_is_left_to_pytorch(calls, monkeypatc
 @pytest.mark.parametrize("B,T,NH,HS,tc", [(1, 64, 12, 64, False), (64, 192, 12, 64, False), (1, 128, 1, 128, True), (1, 320, 12, 64, False),
                                           (2, 320, 32, 64, True), (7, 448, 6, 64, True), (7, 448, 12, 64, True), (2, 576, 6, 64, True),
                                           (2, 576, 12, 64, True), (1, 320, 32, 128, True), (2, 320, 32, 128, True),
-                                          (7, 448, 16, 128, True), (2, 576, 32, 128, True), (1, 320, 29, 64, False), (1, 320, 30, 64, True),
+                                          (7, 448, 16, 128, True), (2, 576, 32, 128, True), (1, 320, 35, 64, False), (1, 320, 36, 64, True),
                                           (2, 128, 37, 64, False), (3, 128, 25, 64, True), (1, 256, 37, 64, False), (2, 256, 19, 64, True),
                                           (1, 384, 1, 64, True)])
 def test_forward_attention_kernel_by_size(calls, monkeypatch, B, T, NH, HS, tc):
