@@ -2,8 +2,8 @@
 // TMEM), for MHA and GQA, reading the packed QKV activation [B*T, (NH+2*NKVH)*HS] through one TMA
 // tensor map and writing O as [B*T, NH*HS] plus the log-sum-exp. Same job as attention_forward /
 // attention_gqa_forward of the reference (llmc/attention.cuh:261-338, llmc/attention_gqa.cuh:415-481),
-// which has no sm_100 path; the warp-level implementation in attention.cu remains for short sequences and
-// small calls whose length is not a multiple of 128 (ops/attention.py has the rule).
+// which has no sm_100 path; the warp-level implementation in attention.cu remains for lengths of 64 and 192 and, with heads
+// of 64, for a few sequences of 128, 256 or 320 (ops/attention.py has the rule).
 //
 // Persistent CTAs that take (128 query rows, head, batch) tiles in turns; 8 warps:
 //   warp 0     TMA producer: K / V tiles of 128 rows through rings of two, freed apart (K after S, V after P V); decodes the

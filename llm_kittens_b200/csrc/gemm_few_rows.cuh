@@ -1,8 +1,9 @@
 // GEMM NT of few rows with a wide output (included by gemm_tcgen05.cu): C[M, N] = A[M, K] * B[N, K]^T for up to 512 rows of A,
 // plain or with the SwiGLU epilogue. The roles of the operands are exchanged: the rows of B (weights, 256 per CTA pair) are the
-// M side of the MMA and the rows of A (tokens) its N side, in whatever multiple of 32 there are, so that every weight tile
-// is read once and next to no padding is multiplied. On the 256 x 256 tiles of the other kernel 320 tokens are two row tiles,
-// 60 % more products than exist, and every weight is read twice.
+// M side of the MMA and the rows of A (tokens) its N side, in whatever multiple of 32 there are, so that next to no padding is
+// multiplied and a weight tile is loaded once (SwiGLU, whose two accumulators share TMEM: once per stretch of 256 tokens, so twice for 257
+// to 512, the second time from the L2 where the two units run side by side). On the 256 x 256 tiles of the other kernel
+// 320 tokens are two row tiles, 60 % more products than exist, and every weight is loaded twice.
 //
 // What bounds it: per k-block a pair multiplies 256 x nt; each SM reads its 128 weight rows once per 160 tokens or so and its share of
 // the tokens from shared memory beside what TMA writes there, 0.5 us for 320 tokens where the tensor core alone would take
