@@ -444,3 +444,27 @@ def test_what_replaces_a_part_of_a_block_is_called_in_every_block(family, where,
     seen.clear()
     model.forward(x, None)
     assert seen == [] and torch.equal(model.logits_view(), want)
+
+
+def test_native_forward_where_the_products_take_the_kernel_of_few_rows():
+    """Up and gate of a window of 320 tokens at 2048 -> 8192: the same bits as block by block."""
+    from llm_kittens_b200.models.config import ModelConfig
+    from llm_kittens_b200.models.transformer import Transformer
+    from llm_kittens_b200.ops import _native
+
+    cfg = ModelConfig(family="llama3", max_seq_len=512, vocab_size=500, padded_vocab_size=512, num_layers=2, num_heads=32, num_kv_heads=8,
+                      channels=2048, hidden_dim=8192)
+    assert _native.lib().llmk_gemm_takes_few_rows(320, cfg.hidden_dim, cfg.channels, 1) == 1
+    model = Transformer(cfg, device="cuda")
+    model.init_weights(5)
+    x = torch.randint(0, 500, (1, 320), dtype=torch.int32, device="cuda")
+    names = ("qkv", "atty", "res2", "up", "gate", "act", "res3", "logits")
+
+    def run():
+        model.forward(x, None)
+        return [model.acts[n].clone() for n in names]
+
+    native = run()
+    model.param_hook = lambda layer, phase: None
+    assert all(torch.equal(a, b) for a, b in zip(native, run()))
+    _native.check_status()
